@@ -7,12 +7,18 @@
 // The three operand layouts cover a linear layer's forward (K,K), input gradient (K,MN) and
 // weight gradient (MN,MN) without transposing anything in memory.
 //
-// Persistent kernel, one CTA per SM, 192 threads:
-//   warp 0      TMA producer (one elected lane)
-//   warp 1      TMEM allocator + tcgen05.mma issuer (one elected lane)
-//   warps 2..5  epilogue: tcgen05.ld -> registers -> global
-// A 4-deep shared-memory ring feeds 128x256x16 MMAs; two 256-column TMEM accumulators let the
+// Persistent kernel, one pair of CTAs (cta_group::2) per two SMs and 256 x 256 tile, 192 threads each:
+//   warp 0      TMA producer (one elected lane): this CTA's 128 rows of A and 128 of the 256 rows of B
+//   warp 1      TMEM allocator; in the pair's first CTA also the tcgen05.mma issuer (one elected lane) for both
+//   warps 2..5  epilogue of this CTA's 128 rows: tcgen05.ld -> registers -> (shared memory ->) global
+// A 6-deep shared-memory ring feeds 256x256x16 MMAs; two 256-column TMEM accumulators let the
 // epilogue of tile i overlap the main loop of tile i+1.
+//
+// Why pairs: one CTA's 128 x 256 tile fills and reads 192 bytes of shared memory per cycle of tensor time, above the 128
+// that an SM has; a pair shares the B operand, which brings that to 128 and the L2 reads of a tile from 48 to 32 KB per k-block.
+// Measured in short runs, one CTA per tile -> pairs (5120 rows, d 4096, ffn 14336): forward gate_up 938 -> 850 us (1415 TFLOP/s), input
+// gradient of down 520 -> 441 us, weight gradient of gate_up 1177 -> 950 us, at 700 rows 630 -> 311 us (its rows are written whole, see
+// store_piece). Over seconds the board's power limit, not the kernel, sets the rate of the forward products.
 //
 // Epilogues:
 //   EPI_STORE    C = acc (+ bias) (+ C), bf16 or fp32
@@ -37,19 +43,24 @@ namespace {
 
 using namespace rlb;
 
-constexpr int BM = 128;
+constexpr int BM = 256;       // rows of a pair's tile
+constexpr int CTA_M = 128;    // rows of each of its CTAs
 constexpr int BN = 256;
+constexpr int CTA_N = 128;    // rows of B that each CTA loads
 constexpr int BK = 64;
-constexpr int STAGES = 4;
+constexpr int STAGES = 6;
 constexpr int UMMA_K = 16;
-constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KB
-constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KB
+constexpr int A_STAGE_BYTES = CTA_M * BK * 2;  // 16 KB
+constexpr int B_STAGE_BYTES = CTA_N * BK * 2;  // 16 KB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+constexpr int OUT_COLS = 64;                                  // columns that an epilogue warp passes through shared memory at a time
+constexpr int OUT_WARP_BYTES = 32 * OUT_COLS * 4;
 constexpr int SMEM_BARRIER_BYTES = 256;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + SMEM_BARRIER_BYTES + 1024;  // +1024: manual alignment
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * OUT_WARP_BYTES + SMEM_BARRIER_BYTES + 1024;  // +1024: manual alignment
+static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 constexpr int NUM_THREADS = 192;
 constexpr int TMEM_COLS = 512;
-constexpr int GROUP_M = 16;  // rasterisation: 16 m-tiles share each sweep over n
+constexpr int GROUP_M = 8;  // rasterisation: 8 m-tiles share each sweep over n
 
 enum { EPI_STORE = 0, EPI_LOGPROB = 1, EPI_DLOGITS = 2, EPI_LAYER = 3, EPI_LINEAR = 4 };
 
@@ -85,14 +96,98 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
   n_blk = in_group / rows;
 }
 
+// One 32-row x 64-column piece of fp32 values on its way out: lanes put their rows down, then the warp reads whole rows, so that every
+// access to global memory covers full 32-byte sectors (rows written by single lanes made the weight gradient's fp32 read-add-write
+// as long as its main loop). 16-byte chunks are permuted within the row so that both directions are free of bank conflicts.
+__device__ __forceinline__ uint32_t out_chunk(uint32_t base, int r, int q) { return base + r * (OUT_COLS * 4) + ((q ^ (r & 7)) << 4); }
+__device__ __forceinline__ void st_shared_f4(uint32_t addr, float a, float b, float c, float d) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void add_bf16x4(float4& v, uint32_t lo, uint32_t hi) {
+  const float2 a = unpack_bf16x2(lo), b = unpack_bf16x2(hi);
+  v.x += a.x; v.y += a.y; v.z += b.x; v.w += b.y;
+}
+
+// Writes the staged piece: rows row0.., columns col.. of C. Old values (accumulation) and the residual are fetched by the caller's
+// warp in the same layout before the piece is complete.
+__device__ __forceinline__ void store_piece(const EpiParams& ep, uint32_t buf, int row0, int col, int M, int N, int lane) {
+  if (ep.out_fp32) {
+    const int q = lane & 15, c = col + q * 4;
+    const bool in = c < N;                 // N is a multiple of 8
+    float4 old[16];
+    float* dst = reinterpret_cast<float*>(ep.C) + static_cast<long long>(row0 + (lane >> 4)) * ep.ldc + c;
+    if (ep.accumulate) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        old[i] = in && row0 + 2 * i + (lane >> 4) < M ? *reinterpret_cast<const float4*>(dst + 2 * i * ep.ldc) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (ep.bias && in) bias = make_float4(ep.bias[c], ep.bias[c + 1], ep.bias[c + 2], ep.bias[c + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int r = 2 * i + (lane >> 4);
+      float4 v = ld_shared_f4(out_chunk(buf, r, q));
+      if (!in || row0 + r >= M) continue;
+      v.x += bias.x; v.y += bias.y; v.z += bias.z; v.w += bias.w;
+      if (ep.residual) {
+        const uint2 o = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(ep.residual) + static_cast<long long>(row0 + r) * ep.ldr + c);
+        add_bf16x4(v, o.x, o.y);
+      }
+      if (ep.accumulate) { v.x += old[i].x; v.y += old[i].y; v.z += old[i].z; v.w += old[i].w; }
+      *reinterpret_cast<float4*>(dst + 2 * i * ep.ldc) = v;
+    }
+  } else {
+    const int q = (lane & 7) * 2, c = col + q * 4;
+    const bool in = c < N;
+    uint4 res[8], old[8];
+    const __nv_bfloat16* rsd = reinterpret_cast<const __nv_bfloat16*>(ep.residual) + static_cast<long long>(row0 + (lane >> 3)) * ep.ldr + c;
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(ep.C) + static_cast<long long>(row0 + (lane >> 3)) * ep.ldc + c;
+    if (ep.residual) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        res[i] = in && row0 + 4 * i + (lane >> 3) < M ? *reinterpret_cast<const uint4*>(rsd + 4 * i * ep.ldr) : make_uint4(0, 0, 0, 0);
+    }
+    if (ep.accumulate) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        old[i] = in && row0 + 4 * i + (lane >> 3) < M ? *reinterpret_cast<const uint4*>(dst + 4 * i * ep.ldc) : make_uint4(0, 0, 0, 0);
+    }
+    float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = b0;
+    if (ep.bias && in) {
+      b0 = make_float4(ep.bias[c], ep.bias[c + 1], ep.bias[c + 2], ep.bias[c + 3]);
+      b1 = make_float4(ep.bias[c + 4], ep.bias[c + 5], ep.bias[c + 6], ep.bias[c + 7]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = 4 * i + (lane >> 3);
+      float4 u = ld_shared_f4(out_chunk(buf, r, q)), v = ld_shared_f4(out_chunk(buf, r, q + 1));
+      if (!in || row0 + r >= M) continue;
+      u.x += b0.x; u.y += b0.y; u.z += b0.z; u.w += b0.w;
+      v.x += b1.x; v.y += b1.y; v.z += b1.z; v.w += b1.w;
+      if (ep.residual) { add_bf16x4(u, res[i].x, res[i].y); add_bf16x4(v, res[i].z, res[i].w); }
+      if (ep.accumulate) { add_bf16x4(u, old[i].x, old[i].y); add_bf16x4(v, old[i].z, old[i].w); }
+      *reinterpret_cast<uint4*>(dst + 4 * i * ep.ldc) = make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+    }
+  }
+  __syncwarp();      // the buffer may be written again
+}
+
 template <bool A_MN, bool B_MN, int EPI>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  int M, int N, int K, EpiParams ep, int* status) {
   extern __shared__ uint8_t smem_raw[];
   // 128B swizzle needs 1024-byte aligned stage buffers.
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint8_t* out_smem = smem + STAGES * STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(out_smem + 4 * OUT_WARP_BYTES);
   uint64_t* full_bar = bars;                 // [STAGES]
   uint64_t* empty_bar = bars + STAGES;       // [STAGES]
   uint64_t* tfull_bar = bars + 2 * STAGES;   // [2]
@@ -102,6 +197,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();      // in the pair; the first CTA's barriers count the loads of both
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -110,7 +207,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&tfull_bar[a]), 1);
-      mbar_init(smem_u32(&tempty_bar[a]), 4);  // one arrive per epilogue warp
+      mbar_init(smem_u32(&tempty_bar[a]), 8);  // one arrive per epilogue warp of both CTAs
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -121,11 +218,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     prefetch_tmap(&tmap_b);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
-    tmem_relinquish();
+    tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS);
+    tmem_relinquish_pair();
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();      // both CTAs' barriers exist before either signals the other's
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -139,31 +237,32 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
         int m_blk, n_blk;
         tile_coords(tile, num_m, num_n, m_blk, n_blk);
+        const int row0 = m_blk * BM + rank * CTA_M, brow0 = n_blk * BN + rank * CTA_N;
         for (int kb = 0; kb < num_k; ++kb) {
           if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, status, RLB_ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
-          const uint32_t bar = smem_u32(&full_bar[stage]);
+          const uint32_t bar = mapa_shared(smem_u32(&full_bar[stage]), 0);
           const uint32_t a_dst = smem_u32(smem + stage * STAGE_BYTES);
           const uint32_t b_dst = a_dst + A_STAGE_BYTES;
-          mbar_arrive_expect_tx(bar, STAGE_BYTES);
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), 2 * STAGE_BYTES);
           if (!A_MN) {
-            tma_load_2d(a_dst, &tmap_a, bar, kb * BK, m_blk * BM);
+            tma_load_2d_pair(a_dst, &tmap_a, bar, kb * BK, row0);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d(a_dst + j * (BK * 128), &tmap_a, bar, m_blk * BM + j * 64, kb * BK);
+            for (int j = 0; j < CTA_M / 64; ++j)
+              tma_load_2d_pair(a_dst + j * (BK * 128), &tmap_a, bar, row0 + j * 64, kb * BK);
           }
           if (!B_MN) {
-            tma_load_2d(b_dst, &tmap_b, bar, kb * BK, n_blk * BN);
+            tma_load_2d_pair(b_dst, &tmap_b, bar, kb * BK, brow0);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(b_dst + j * (BK * 128), &tmap_b, bar, n_blk * BN + j * 64, kb * BK);
+            for (int j = 0; j < CTA_N / 64; ++j)
+              tma_load_2d_pair(b_dst + j * (BK * 128), &tmap_b, bar, brow0 + j * 64, kb * BK);
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -171,15 +270,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
         }
       }
+      if (!ok) {      // loads in flight land within microseconds: they must not outlive the CTA
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 1000000ull) {}
+      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (lane == 0 && rank == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
       uint32_t stage = 0, phase = 0;
       uint32_t local_tile = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++local_tile) {
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_phase = (local_tile >> 1) & 1;
         if (!mbar_wait(smem_u32(&tempty_bar[acc]), acc_phase ^ 1, abort_flag, status, RLB_ERR_WAIT_TMEM_EMPTY)) {
@@ -206,23 +309,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           constexpr uint32_t b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            umma_f16(tmem_d, a_desc + kk * a_step, b_desc + kk * b_step, idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma_f16_pair(tmem_d, a_desc + kk * a_step, b_desc + kk * b_step, idesc, (kb | kk) != 0 ? 1u : 0u);
           }
-          umma_commit(smem_u32(&empty_bar[stage]));  // stage reusable once these MMAs have read it
+          umma_commit_pair(smem_u32(&empty_bar[stage]));  // stage reusable, in both CTAs, once these MMAs have read it
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) umma_commit(smem_u32(&tfull_bar[acc]));  // accumulator complete
+        if (ok) umma_commit_pair(smem_u32(&tfull_bar[acc]));  // accumulator complete
       }
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int quarter = warp & 3;  // TMEM lanes 32*quarter .. +31 belong to this warp
+    const uint32_t buf = smem_u32(out_smem) + quarter * OUT_WARP_BYTES;
     uint32_t local_tile = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
+    for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++local_tile) {
       int m_blk, n_blk;
       tile_coords(tile, num_m, num_n, m_blk, n_blk);
       const uint32_t acc = local_tile & 1;
@@ -232,75 +336,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         break;
       }
       tc_fence_after();
-      const int row = m_blk * BM + quarter * 32 + lane;
+      const int row0 = m_blk * BM + rank * CTA_M + quarter * 32, row = row0 + lane;
       const bool row_ok = row < M;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
       const int col0 = n_blk * BN;
 
       if (EPI == EPI_STORE) {
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + c * 32, r);
+        for (int c = 0; c < BN / OUT_COLS && col0 + c * OUT_COLS < N; ++c) {
+          uint32_t r[64];
+          tmem_ld_32x32b_x32(taddr + c * OUT_COLS, *reinterpret_cast<uint32_t(*)[32]>(r));
+          tmem_ld_32x32b_x32(taddr + c * OUT_COLS + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
           tmem_ld_wait();
-          const int col = col0 + c * 32;
-          if (!row_ok || col >= N) continue;
-          float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-          if (ep.bias) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (col + i < N) v[i] += ep.bias[col + i];
-          }
-          if (ep.residual) {
-            const __nv_bfloat16* rsd =
-                reinterpret_cast<const __nv_bfloat16*>(ep.residual) + static_cast<long long>(row) * ep.ldr + col;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              if (col + q * 8 < N) {
-                const uint4 old = *reinterpret_cast<const uint4*>(rsd + q * 8);
-                const float2 o0 = unpack_bf16x2(old.x), o1 = unpack_bf16x2(old.y), o2 = unpack_bf16x2(old.z),
-                             o3 = unpack_bf16x2(old.w);
-                v[q * 8 + 0] += o0.x; v[q * 8 + 1] += o0.y; v[q * 8 + 2] += o1.x; v[q * 8 + 3] += o1.y;
-                v[q * 8 + 4] += o2.x; v[q * 8 + 5] += o2.y; v[q * 8 + 6] += o3.x; v[q * 8 + 7] += o3.y;
-              }
-            }
-          }
-          if (ep.out_fp32) {
-            float* dst = reinterpret_cast<float*>(ep.C) + static_cast<long long>(row) * ep.ldc + col;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              if (col + q * 4 < N) {  // N is a multiple of 8
-                float4 o = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
-                if (ep.accumulate) {
-                  const float4 old = *reinterpret_cast<const float4*>(dst + q * 4);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                *reinterpret_cast<float4*>(dst + q * 4) = o;
-              }
-            }
-          } else {
-            __nv_bfloat16* dst =
-                reinterpret_cast<__nv_bfloat16*>(ep.C) + static_cast<long long>(row) * ep.ldc + col;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              if (col + q * 8 < N) {
-                if (ep.accumulate) {
-                  const uint4 old = *reinterpret_cast<const uint4*>(dst + q * 8);
-                  const float2 o0 = unpack_bf16x2(old.x), o1 = unpack_bf16x2(old.y),
-                               o2 = unpack_bf16x2(old.z), o3 = unpack_bf16x2(old.w);
-                  v[q * 8 + 0] += o0.x; v[q * 8 + 1] += o0.y; v[q * 8 + 2] += o1.x; v[q * 8 + 3] += o1.y;
-                  v[q * 8 + 4] += o2.x; v[q * 8 + 5] += o2.y; v[q * 8 + 6] += o3.x; v[q * 8 + 7] += o3.y;
-                }
-                uint4 o;
-                o.x = pack_bf16x2(v[q * 8 + 0], v[q * 8 + 1]);
-                o.y = pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]);
-                o.z = pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]);
-                o.w = pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]);
-                *reinterpret_cast<uint4*>(dst + q * 8) = o;
-              }
-            }
-          }
+          for (int q = 0; q < OUT_COLS / 4; ++q)
+            st_shared_f4(out_chunk(buf, lane, q), __uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+          store_piece(ep, buf, row0, col0 + c * OUT_COLS, M, N, lane);
         }
       } else if (EPI == EPI_LAYER) {
         const float alpha = ep.layer.x ? __bfloat162float(*ep.layer.alpha) : 0.f;
@@ -430,15 +480,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const float g = row_ok ? ep.coef[row] : 0.f;
         const float ge = (row_ok && ep.ent_coef) ? ep.ent_coef[row] : 0.f;
         const float ent = (row_ok && ep.ent_coef) ? ep.entropy[row] : 0.f;
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + c * 32, r);
+        for (int c = 0; c < BN / OUT_COLS && col0 + c * OUT_COLS < N; ++c) {
+          uint32_t r[64];
+          tmem_ld_32x32b_x32(taddr + c * OUT_COLS, *reinterpret_cast<uint32_t(*)[32]>(r));
+          tmem_ld_32x32b_x32(taddr + c * OUT_COLS + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
           tmem_ld_wait();
-          const int col = col0 + c * 32;
-          if (!row_ok || col >= N) continue;
-          float v[32];
+          const int col = col0 + c * OUT_COLS;
+          float v[64];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < OUT_COLS; ++i) {
             const float z = __uint_as_float(r[i]) * ep.inv_temp;
             const float logp = z - lse;
             const float p = __expf(logp);
@@ -447,32 +497,23 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             d -= ge * p * (logp + ent);
             v[i] = d * ep.inv_temp;
           }
-          __nv_bfloat16* dst =
-              reinterpret_cast<__nv_bfloat16*>(ep.C) + static_cast<long long>(row) * ep.ldc + col;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (col + q * 8 < N) {
-              uint4 o;
-              o.x = pack_bf16x2(v[q * 8 + 0], v[q * 8 + 1]);
-              o.y = pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]);
-              o.z = pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]);
-              o.w = pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]);
-              *reinterpret_cast<uint4*>(dst + q * 8) = o;
-            }
-          }
+          for (int q = 0; q < OUT_COLS / 4; ++q) st_shared_f4(out_chunk(buf, lane, q), v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          store_piece(ep, buf, row0, col, M, N, lane);
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
+      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0));
     }
   }
 
   tc_fence_before();
   __syncthreads();
+  cluster_sync();      // nothing of the pair signals or writes the other CTA any more
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
 }
 
@@ -517,9 +558,9 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int 
     cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev);
   }
   const int num_tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  int grid = num_tiles < g_sm_count ? num_tiles : g_sm_count;
-  if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  kern<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, M, N, K, ep, status);
+  int pairs = num_tiles < g_sm_count / 2 ? num_tiles : g_sm_count / 2;
+  if (max_ctas > 0 && pairs > max_ctas / 2) pairs = max_ctas > 1 ? max_ctas / 2 : 1;
+  kern<<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, M, N, K, ep, status);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -536,14 +577,14 @@ int make_operand_maps(const void* A, const void* B, int M, int N, int K, long lo
                       bool a_mn, bool b_mn, CUtensorMap* ta, CUtensorMap* tb) {
   int rc;
   if (!a_mn)
-    rc = rlb_make_tmap_2d(ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, lda * 2, BK, BM,
+    rc = rlb_make_tmap_2d(ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, lda * 2, BK, CTA_M,
                           CU_TENSOR_MAP_SWIZZLE_128B);
   else
     rc = rlb_make_tmap_2d(ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, lda * 2, 64, BK,
                           CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
   if (!b_mn)
-    rc = rlb_make_tmap_2d(tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, ldb * 2, BK, BN,
+    rc = rlb_make_tmap_2d(tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, ldb * 2, BK, CTA_N,
                           CU_TENSOR_MAP_SWIZZLE_128B);
   else
     rc = rlb_make_tmap_2d(tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldb * 2, 64, BK,

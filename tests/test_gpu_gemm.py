@@ -62,6 +62,31 @@ def test_gemm_epilogues(native_lib):
     assert wide_o[:, :24].abs().max().item() == 0
 
 
+@pytest.mark.parametrize("M", [8, 128, 136, 256, 264, 392])        # one CTA's rows of a 256-row tile, both CTAs', a ragged second tile
+@pytest.mark.parametrize("N", [64, 72, 256, 328])                   # pieces of 64 columns, whole and cut; one tile and two
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gemm_tile_edges(native_lib, M, N, dtype):
+    """Accumulation, bias and residual at the edges of a pair's tile. Products of bf16 values are exact in fp32, so the fp32 result is off by
+    the sums alone (K roundings of terms below 4 sigma^2: 1e-5 of the largest value); a bf16 result also by one
+    rounding, at most 2^-8 of it (8 significant bits)."""
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import check_status
+
+    torch.manual_seed(M + N)
+    K = 456                                                         # seven k-blocks and an eighth that is cut: the ring wraps
+    a, b = torch.randn(M, K, device="cuda", dtype=torch.bfloat16), torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    bias, res = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda", dtype=torch.bfloat16)
+    wide = torch.randn(M + 1, N + 8, device="cuda").to(dtype)
+    old = wide.clone()
+    F.gemm(a, b, out=wide[:M, :N], bias=bias, residual=res, accumulate=True)
+    ref = a.double() @ b.double().t() + bias + res + old[:M, :N]
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    bound = (1e-5 if dtype == torch.float32 else 2.0 ** -8 + 1e-5) * ref.abs().max()
+    assert (wide[:M, :N].double() - ref).abs().max() <= bound
+    assert torch.equal(wide[M:], old[M:]) and torch.equal(wide[:, N:], old[:, N:])      # nothing beside the tile is touched
+
+
 def test_linear_autograd(native_lib):
     from rl_b200.ops import functional as F
 
