@@ -1167,7 +1167,7 @@ class GenerationEngine:
         st = self._static_buffers()
         B = self._bucket(n)
         c = self.cfg
-        num_splits = E.choose_splits(B, self.hkv, max(self.max_model_len // 2, 1), self.block_size, self._sm_count) if self.native else 1
+        num_splits = E.choose_splits(B, self.hkv, max(self.max_model_len // 2, 1), self.block_size, self._sm_count, self.hq) if self.native else 1
         if not self.native:
             self._decode_rows = st["state_rows"][:n]
             logits = self._decode_forward(st["ids"][:n].long(), st["positions"][:n], st["slots"][:n], st["block_table"][:n],

@@ -61,18 +61,42 @@ def skinny_static_weights(on: bool) -> int:
     return int(lib().rlb_gemm_skinny_static_weights(1 if on else 0))
 
 
-def choose_splits(B: int, Hkv: int, max_len: int, block_size: int, sm_count: int = 148) -> int:
-    """Enough KV splits to put ~2 CTAs on every SM, never finer than one cache block per split."""
+def group_rows(B: int, Hq: int, Hkv: int, splits: int, sm_count: int = 148) -> int:
+    """Neighbouring sequences that the plain decode kernel serves together (shared pages are read once): up to eight query heads in all, and
+    as many as leave at least 1.6 CTAs per SM. Sixteen heads were no faster: the soft-max of a tile then takes longer than its bytes (48
+    sequences of 4000 tokens, 16 to a prompt, 8 KV heads, 4 query heads each: 57 us in twos, 59 us in fours; 64 of 1200 tokens: 38 and 39 us;
+    without shared pages 129 and 140 us)."""
+    for rows in (4, 2):
+        if rows * (Hq // Hkv) <= 8 and -(-B // rows) * Hkv * splits * 5 >= 8 * sm_count:
+            return rows
+    return 1
+
+
+def choose_splits(B: int, Hkv: int, max_len: int, block_size: int, sm_count: int = 148, Hq: int = 0) -> int:
+    """KV splits of paged decoding, never finer than one cache block per split. Without ``Hq``: ~2 CTAs on every SM. With ``Hq``: for the plain
+    kernel (``rlb_paged_decode_group``), of which three CTAs fit on an SM and whose groups' tiles are cut evenly: one wave of CTAs, of the
+    largest groups that need at most four splits for it (16 sequences of 4000 tokens take 51 us alone with three splits, 53 us in twos with
+    six). Up to eight splits merge inside a cluster; more cost a second kernel and are taken only where eight leave SMs without work."""
     forced = os.environ.get("RLB_DECODE_SPLITS")
     if forced:
         return max(1, int(forced))
-    ctas = max(1, B * Hkv)
+    B = max(1, B)
+    if Hq:
+        for rows in (4, 2, 1):
+            ctas = -(-B // rows) * Hkv
+            want = max(1, 3 * sm_count // ctas)
+            if rows == 1 or (rows * (Hq // Hkv) <= 8 and want <= 4):
+                break
+        if want > 8 and ctas * 8 >= sm_count:
+            want = 8
+        return int(max(1, min(want, max(1, rows * max_len // max(block_size, 128)), 32)))
+    ctas = B * Hkv
     want = max(1, (2 * sm_count + ctas - 1) // ctas)
     return int(max(1, min(want, max(1, max_len // max(block_size, 128)), 32)))
 
 
 def _paged_decode_gather(q, k_cache, v_cache, block_table, seq_lens, Hq, Hkv, D, scale, out, rows_per_chunk: int = 64, window: int = 0, chunk: int = 0):
-    """Decode attention for head dimensions the native kernels do not cover (they are built for 128): the paged keys and
+    """Decode attention for head dimensions the native kernels do not cover (they are built for 64 and 128): the paged keys and
     values of a chunk of sequences are gathered through the block table and attended with batched matmuls. No host
     synchronisation and static shapes, so it can be captured in a CUDA graph like the native path."""
     B, nb = q.shape[0], block_table.shape[1]
@@ -111,7 +135,8 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     block_size = k_cache.shape[2]
     if out is None:
         out = torch.empty((B, Hq * D), dtype=q.dtype, device=q.device)
-    special = offset is not None or gated or keep > 0       # (forms that the tensor-core kernel alone has)
+    plain = offset is None and not chunk and not window
+    special = offset is not None or gated or keep > 0       # (forms that the tensor-core kernels alone have)
     if not use_native(q):
         assert not special
         g = Hq // Hkv
@@ -129,6 +154,17 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
             p = torch.softmax(qb @ k.transpose(1, 2), dim=-1)
             out[b] = (p @ v).reshape(Hq * D).to(out.dtype)
         return out
+    kernel = os.environ.get("RLB_DECODE_KERNEL", "mma")
+    if plain and (kernel == "mma" or special) and D in (64, 128) and Hq // Hkv <= 16 and (block_size in (16, 32, 64) or block_size % 128 == 0) \
+            and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0:
+        if num_splits > 8 and scratch is None:
+            no, nml = decode_scratch_sizes(B, Hq, num_splits, D)
+            scratch = (torch.empty(no, dtype=torch.float32, device=q.device), torch.empty(nml, dtype=torch.float32, device=q.device))
+        po, pml = scratch if num_splits > 8 else (None, None)
+        call("rlb_paged_decode_group", ptr(q), q.stride(0), ptr(k_cache), ptr(v_cache), k_cache.shape[0], ptr(block_table), block_table.stride(0),
+             ptr(seq_lens), B, Hq, Hkv, D, block_size, group_rows(B, Hq, Hkv, num_splits), int(gated), scale, num_splits, ptr(po), ptr(pml), ptr(out),
+             out.stride(0), ptr(_L.status_word(q.device)), stream_ptr())
+        return out
     if special:
         assert D == 128 and Hq // Hkv <= 8 and (block_size in (16, 32, 64) or block_size % 128 == 0), "shape of the tensor-core decode kernel"
     elif D != 128 or window:
@@ -140,7 +176,6 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
             scratch = (torch.empty(no, dtype=torch.float32, device=q.device),
                        torch.empty(nml, dtype=torch.float32, device=q.device))
         po, pml = scratch
-    kernel = os.environ.get("RLB_DECODE_KERNEL", "mma")
     if (kernel == "mma" or special) and D == 128 and Hq // Hkv <= 8 and (block_size in (16, 32, 64) or block_size % 128 == 0):
         # tensor-core flash-decoding kernel (tcgen05: QK^T and PV as MMAs over 128-token tiles)
         call("rlb_paged_decode_mma", ptr(q), q.stride(0), ptr(k_cache), ptr(v_cache), k_cache.shape[0], ptr(block_table),

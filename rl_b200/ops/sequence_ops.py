@@ -100,7 +100,7 @@ def attention(p: torch.Tensor, m, b: TokenBatch, k_cache: torch.Tensor, v_cache:
         if decode_tiles(p, m, bs):
             seen = min(b.max_ctx, m.chunk) // 2 if m.chunk else min(b.max_ctx // 2, m.window + m.keep) if m.window else b.max_ctx // 2
             E.paged_decode(p[: b.n_paged, m.q_off : m.q_off + H * m.dim], k_cache, v_cache, b.block_table, b.seq_lens, H, G, m.dim, scale=m.scale,
-                           num_splits=E.choose_splits(b.n_paged, G, max(seen, 1), bs), out=y[: b.n_paged], chunk=m.chunk, window=m.window, keep=m.keep,
+                           num_splits=E.choose_splits(b.n_paged, G, max(seen, 1), bs, Hq=0 if m.chunk or m.window or m.offset is not None else H), out=y[: b.n_paged], chunk=m.chunk, window=m.window, keep=m.keep,
                            offset=m.offset, gated=m.gate)
         else:
             call("rlb_gqa_rows", ptr(p), _f32(p), b.n_paged, p.stride(0), m.q_off, H, G, m.dim, m.vdim, bs, k_cache.shape[0], ptr(k_cache),

@@ -334,3 +334,44 @@ def test_fused_clipped_pg_matches_pytorch_statement(native_lib, cfg):
     assert (c1.grad - c2.grad).abs().max().item() <= 2e-4 * c2.grad.abs().max().item() + 1e-8
     for k in ("probs_ratio", "kl_penalty", "token_mult_prob_error"):
         assert m1[k] == pytest.approx(m2[k], rel=1e-3, abs=1e-6), k
+
+
+@pytest.mark.parametrize("Hq,Hkv,D", [(32, 8, 128), (32, 8, 64), (14, 2, 64), (32, 4, 128), (16, 1, 64), (3, 3, 128)])
+@pytest.mark.parametrize("bs", [16, 64, 128])
+@pytest.mark.parametrize("rows,splits", [(1, 1), (1, 8), (1, 11), (4, 1), (4, 3), (4, 8)])
+def test_paged_decode_groups(native_lib, Hq, Hkv, D, bs, rows, splits):
+    """Groups of sequences with all, some and none of their pages shared, lengths at the edges of tiles, empty sequences, a cut last group, gates.
+    Against float64 on the same bf16 inputs: the scaled queries and the weights are rounded to bf16 (2^-9 each, relative), a result too."""
+    from rl_b200.ops import engine_ops as E
+    from rl_b200.ops.lib import call, check_status, ptr, stream_ptr
+    from rl_b200.ops import lib as L
+
+    rows = max(1, min(rows, 16 // (Hq // Hkv)))
+    g = torch.Generator().manual_seed(Hq + bs + splits)
+    lens = torch.tensor([300, 300, 301, 384, 1, 128, 127, 129, 513, 0, 520, 512, 0, 0, 0, 0, 257, 640], dtype=torch.int32)
+    B, NB = len(lens), 18 * (640 // bs + 1) + 1
+    bt = torch.randperm(NB - 1, generator=g)[: B * (640 // bs + 1)].view(B, -1).to(torch.int32) + 1
+    bt[1:4, : 256 // bs] = bt[0, : 256 // bs]                          # two tiles shared, the rest own
+    bt[8:12, : 512 // bs] = bt[8, : 512 // bs]                         # an empty sequence among sharers
+    bt[17, : 128 // bs + 1] = bt[16, : 128 // bs + 1]                  # past a tile's end, not to the next one's
+    q = torch.randn(B, (Hq + 2 * Hkv) * D, generator=g).bfloat16().cuda()
+    kc, vc = (torch.randn(NB, Hkv, bs, D, generator=g).bfloat16().cuda() for _ in range(2))
+    gates = torch.randn(B, Hq * D, generator=g).bfloat16().cuda()
+    btc, lc = bt.cuda(), lens.cuda()
+    for gated in (0, 1):
+        out = gates.clone()
+        no, nml = E.decode_scratch_sizes(B, Hq, splits, D)
+        po, pml = torch.empty(no, device="cuda"), torch.empty(nml, device="cuda")
+        call("rlb_paged_decode_group", ptr(q), q.stride(0), ptr(kc), ptr(vc), NB, ptr(btc), btc.stride(0), ptr(lc), B, Hq, Hkv, D, bs, rows, gated,
+             D ** -0.5, splits, ptr(po), ptr(pml), ptr(out), out.stride(0), ptr(L.status_word(q.device)), stream_ptr())
+        torch.cuda.synchronize()
+        assert check_status() == 0
+        for b, n in enumerate(lens.tolist()):
+            if n == 0:
+                assert out[b].abs().max() == 0
+                continue
+            pages = btc[b, : -(-n // bs)].long()
+            k, v = (c[pages].permute(1, 0, 2, 3).reshape(Hkv, -1, D)[:, :n].double() for c in (kc, vc))
+            w = torch.softmax(q[b, : Hq * D].view(Hkv, Hq // Hkv, D).double() * D ** -0.5 @ k.transpose(1, 2), -1)
+            ref = (w @ v).reshape(-1) * (torch.sigmoid(gates[b].double()) if gated else 1.0)
+            assert (out[b].double() - ref).norm() <= 3 * 2.0 ** -9 * 2 * ref.norm() + 1e-6, (b, n)
