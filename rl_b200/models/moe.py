@@ -199,6 +199,12 @@ class MoEMLP(nn.Module):
                     self.routing_sink(self, self.last_routing)
                 return out
         w, idx, _ = self.route(x)
+        if self.gated and self.ep_size == 1 and self.fc1_latent_proj is None:
+            from rl_b200.ops.moe_ops import expert_layer, expert_layer_takes
+
+            if expert_layer_takes(x, self.gate_up_proj, self.down_proj):
+                out = expert_layer(x, idx, w, residual, self.gate_up_proj, self.down_proj)
+                return out if self.shared_experts is None else self.shared_experts(x, out)
         flat_e = idx.reshape(-1)
         order = torch.argsort(flat_e, stable=True)
         tok = order // k

@@ -118,6 +118,108 @@ def grouped_expert_mlp(xs: torch.Tensor, counts: torch.Tensor, gate_up: torch.Te
     return y.index_select(0, lay.dest)
 
 
+# ------------------------------------------------------------------------------------------- whole layer on one rank
+register("rlb_moe_plan", [P, I, I, I, P, P, P, P, P, P, P])
+register("rlb_moe_gather", [P, L, P, P, I, P, I, I, P])
+register("rlb_moe_combine_rows", [P, P, P, P, L, P, L, I, I, P])
+register("rlb_moe_combine_rows_bwd", [P, P, P, P, P, I, P, P, I, I, P])
+LAYER_MAX_EXPERTS = 256
+
+
+class TokenPlan:
+    """Rows of the grouped GEMMs for the copies of ``idx`` [T, k] (int64 experts), made on the device: ``copy_row`` [T * k], ``row_copy``
+    [mpad] (-1: padding), the experts' row ranges and the tile -> expert table."""
+
+    def __init__(self, idx: torch.Tensor, num_experts: int):
+        self.T, self.k = idx.shape
+        n, dev = idx.numel(), idx.device
+        self.num_experts = num_experts
+        self.mpad = -(-(n + num_experts * 127) // 128) * 128          # static upper bound: no host sync
+        blocks, E = -(-n // 1024), num_experts
+        # one allocation: [scratch | copy_row | row_copy | row0 | rows | tile_expert]
+        sizes = [blocks * E, n, self.mpad, E, E, self.mpad // 128]
+        buf = torch.empty(sum(sizes), dtype=torch.int32, device=dev)
+        scratch, self.copy_row, self.row_copy, self.row0, self.rows, self.tile_expert = buf.split(sizes)
+        idx = idx.contiguous()
+        call("rlb_moe_plan", ptr(idx), n, E, self.mpad, ptr(scratch), ptr(self.copy_row), ptr(self.row_copy), ptr(self.row0), ptr(self.rows),
+             ptr(self.tile_expert), stream_ptr())
+
+
+def _grouped_rows(x, w, transposed: bool, plan) -> torch.Tensor:
+    """Rows of ``x`` times their expert's weight (``transposed``: [E, K, N] as stored, for the input gradient)."""
+    E, N, K = w.shape
+    if transposed:
+        N, K = K, N
+    y = torch.empty((plan.mpad, N), dtype=BF16, device=x.device)      # rows of unused tiles stay unwritten and are never read
+    call("rlb_gemm_grouped_rows", ptr(x), x.stride(0), ptr(w), int(transposed), ptr(y), y.stride(0), plan.mpad, N, K, E, ptr(plan.tile_expert), 0,
+         ptr(_L.status_word(x.device)), stream_ptr())
+    return y
+
+
+def _grouped_wgrad(dy, x, w, plan):
+    """Adds the stacked weight gradient into ``w.main_grad``, or returns it."""
+    E, N, K = w.shape
+    main_grad = getattr(w, "main_grad", None)
+    target = main_grad if main_grad is not None else torch.zeros((E, N, K), dtype=torch.float32, device=dy.device)
+    call("rlb_gemm_grouped_reduce", ptr(dy), dy.stride(0), ptr(x), x.stride(0), ptr(target), plan.mpad, N, K, E, ptr(plan.row0), ptr(plan.rows),
+         int(target.dtype == torch.float32), 1, ptr(_L.status_word(dy.device)), stream_ptr())
+    return None if main_grad is not None else target.to(w.dtype)
+
+
+class _ExpertLayer(torch.autograd.Function):
+    """residual + sum of a token's experts' SwiGLU units, weighted (rl_b200/csrc/moe_layer.cu around the grouped GEMMs)."""
+
+    @staticmethod
+    def forward(ctx, x, w, residual, gate_up, down, plan: TokenPlan):
+        d, f, dev = x.shape[1], down.shape[2], x.device
+        xp = torch.empty((plan.mpad, d), dtype=BF16, device=dev)
+        call("rlb_moe_gather", ptr(x), x.stride(0), ptr(plan.row_copy), ptr(plan.tile_expert), plan.k, ptr(xp), plan.mpad, d, stream_ptr())
+        h = _grouped_rows(xp, gate_up, False, plan)
+        a = torch.empty((plan.mpad, f), dtype=BF16, device=dev)
+        call("rlb_swiglu_fwd", ptr(h), ptr(a), plan.mpad, f, stream_ptr())
+        y = _grouped_rows(a, down, False, plan)
+        out = torch.empty((plan.T, d), dtype=BF16, device=dev)
+        call("rlb_moe_combine_rows", ptr(y), ptr(plan.copy_row), ptr(w), ptr(residual), residual.stride(0) if residual is not None else 0, ptr(out), plan.T,
+             plan.k, d, stream_ptr())
+        ctx.save_for_backward(w, gate_up, down, xp, h, a, y)
+        ctx.plan = plan
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        w, gate_up, down, xp, h, a, y = ctx.saved_tensors
+        plan, (d, f), dev = ctx.plan, (xp.shape[1], a.shape[1]), xp.device
+        g = dout.contiguous()
+        dy, dw = torch.empty_like(y), torch.zeros_like(w)
+        call("rlb_moe_combine_rows_bwd", ptr(g), ptr(y), ptr(plan.row_copy), ptr(plan.tile_expert), ptr(w), plan.k, ptr(dy), ptr(dw), plan.mpad, d, stream_ptr())
+        d_down = _grouped_wgrad(dy, a, down, plan) if ctx.needs_input_grad[4] else None
+        dx = d_gate_up = None
+        if ctx.needs_input_grad[0] or ctx.needs_input_grad[3]:
+            da, dh = _grouped_rows(dy, down, True, plan), torch.empty_like(h)
+            call("rlb_swiglu_bwd", ptr(da), ptr(h), ptr(dh), plan.mpad, f, stream_ptr())
+            if ctx.needs_input_grad[3]:
+                d_gate_up = _grouped_wgrad(dh, xp, gate_up, plan)
+            if ctx.needs_input_grad[0]:
+                dxp, dx = _grouped_rows(dh, gate_up, True, plan), torch.empty((plan.T, d), dtype=BF16, device=dev)
+                call("rlb_moe_combine_rows", ptr(dxp), ptr(plan.copy_row), None, None, 0, ptr(dx), plan.T, plan.k, d, stream_ptr())
+        return dx, dw, (dout if ctx.needs_input_grad[2] else None), d_gate_up, d_down, None
+
+
+def expert_layer_takes(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor) -> bool:
+    """Whether :func:`expert_layer` covers these rows and weights (bf16 on the GPU, widths in whole 64-column blocks, no quantizers)."""
+    return (use_native(x) and x.dtype == BF16 and gate_up.dtype == BF16 and x.shape[0] > 0 and x.shape[1] % 64 == 0 and down.shape[2] % 64 == 0
+            and gate_up.shape[0] <= LAYER_MAX_EXPERTS and getattr(gate_up, "_rlb_qat", None) is None and getattr(down, "_rlb_qat", None) is None)
+
+
+def expert_layer(x: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, residual, gate_up: torch.Tensor, down: torch.Tensor) -> torch.Tensor:
+    """(residual +) sum_j w[t, j] MLP_{idx[t, j]}(x[t]) for tokens ``x`` [T, d]; ``idx``, ``w`` [T, k]. The sum over a token's experts is fp32
+    and in their order."""
+    def rows(t):
+        return t if t is None or (t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 and t.dtype == BF16) else t.to(BF16).contiguous()
+
+    return _ExpertLayer.apply(rows(x), w.float().contiguous(), rows(residual), gate_up, down, TokenPlan(idx, gate_up.shape[0]))
+
+
 # ------------------------------------------------------------------------------------------- small-token path (decode)
 register("rlb_moe_route_topk", [P, L, I, I, I, I, P, P, P])
 register("rlb_moe_decode_plan", [P, I, I, I, I, I, P, P, P, P, P, P, P])

@@ -162,3 +162,51 @@ def test_moe_engine_decodes_from_cuda_graphs(native_lib):
     for a, b in zip(outs[True], outs[False]):
         if a[0] == b[0]:
             assert max(abs(x - y) for x, y in zip(a[1], b[1])) < 0.05
+
+
+@pytest.mark.parametrize("T,E,k,skew", [(1, 8, 2, 0), (127, 128, 8, 0), (1300, 128, 8, 1), (700, 3, 1, 0), (2049, 256, 5, 2)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_expert_layer(native_lib, T, E, k, skew, residual):
+    """Plan, outputs and gradients of a whole layer: more than one block of copies, experts without tokens, one expert with most of them. Against
+    float64 on the same bf16 values; every product's operands are bf16, so an output or gradient is off by a few roundings of 2^-9, relative to
+    its norm: 1e-2."""
+    from rl_b200.ops import moe_ops as M
+    from rl_b200.ops.lib import check_status
+
+    g = torch.Generator("cuda").manual_seed(T + E)
+    d, f = 128, 64
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    score = r(T, E) + (torch.arange(E, device="cuda") == 1) * (5.0 if skew == 1 else 0.0) - (torch.arange(E, device="cuda") % 3 == 0) * (9.0 if skew == 2 else 0.0)
+    idx = score.topk(k, -1)[1]
+    plan = M.TokenPlan(idx, E)
+    rows = plan.copy_row.long()
+    counts = torch.bincount(idx.reshape(-1), minlength=E)
+    assert torch.equal(plan.rows.long(), (counts + 127) // 128 * 128) and torch.equal(plan.row_copy[rows].long(), torch.arange(T * k, device="cuda"))
+    assert torch.equal(plan.tile_expert[rows // 128].long(), idx.reshape(-1)) and (plan.row_copy >= 0).sum() == T * k
+    order = torch.argsort(idx.reshape(-1), stable=True)      # rows of an expert hold its copies in order
+    assert bool((rows[order][1:] > rows[order][:-1]).all())
+    x, res = r(T, d).bfloat16().requires_grad_(), r(T, d).bfloat16().requires_grad_()
+    w = torch.softmax(r(T, k), -1).requires_grad_()
+    gu, dn = (0.2 * r(E, 2 * f, d)).bfloat16().requires_grad_(), (0.2 * r(E, d, f)).bfloat16().requires_grad_()
+    dn.main_grad = torch.ones(E, d, f, device="cuda")
+    out = M.expert_layer(x, idx, w, res if residual else None, gu, dn)
+    up = r(T, d).bfloat16()
+    out.backward(up)
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    X, R, W, G, D = (t.detach().double().requires_grad_() for t in (x, res, w, gu, dn))
+    ref, size = R if residual else torch.zeros_like(R), torch.zeros_like(W)
+    for e in range(E):
+        t, j = (idx == e).nonzero(as_tuple=True)
+        if len(t):
+            a, b = (X[t] @ G[e].T).chunk(2, -1)
+            y = (torch.nn.functional.silu(a) * b) @ D[e].T
+            ref, size[t, j] = ref.index_add(0, t, y * W[t, j, None]), y.detach().norm(dim=-1)
+    ref.backward(up.double())
+    near = lambda a, b: (a.double() - b).norm() <= 1e-2 * b.norm() + 1e-12      # noqa: E731
+    assert near(out, ref) and near(x.grad, X.grad) and near(gu.grad, G.grad) and near(dn.main_grad - 1, D.grad)
+    # a weight's gradient is a scalar product whose terms may cancel: its error is relative to the factors' norms
+    assert bool(((w.grad.double() - W.grad).abs() <= 1e-2 * up.double().norm(dim=-1, keepdim=True) * size.detach()).all())
+    if residual:
+        assert torch.equal(res.grad, up)
+    assert gu.grad[counts == 0].abs().sum() == 0 and dn.grad is None
