@@ -375,3 +375,38 @@ def test_paged_decode_groups(native_lib, Hq, Hkv, D, bs, rows, splits):
             w = torch.softmax(q[b, : Hq * D].view(Hkv, Hq // Hkv, D).double() * D ** -0.5 @ k.transpose(1, 2), -1)
             ref = (w @ v).reshape(-1) * (torch.sigmoid(gates[b].double()) if gated else 1.0)
             assert (out[b].double() - ref).norm() <= 3 * 2.0 ** -9 * 2 * ref.norm() + 1e-6, (b, n)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 2048, 4101])            # whole groups of eight, a tail, a tail alone
+@pytest.mark.parametrize("shift", [0, 1])                          # a start that is not 16-byte aligned goes element by element
+@pytest.mark.parametrize("gdtype", [torch.float32, torch.bfloat16])
+def test_adamw_groups_of_eight(native_lib, n, shift, gdtype):
+    """Every form of the split-master update against the element-wise one on an unaligned copy: the same operations, of which the compiler may
+    contract some to fused ones: a few fp32 roundings of 2^-24."""
+    from rl_b200.ops import functional as F
+
+    gen = torch.Generator().manual_seed(n)
+    w, g0, m0, v0 = (torch.randn(n, generator=gen) for _ in range(4))
+    hi0, lo0 = F.split_master(w)
+
+    def run(off):
+        place = lambda t: torch.cat([torch.zeros(off, dtype=t.dtype), t]).cuda()[off:]      # noqa: E731
+        hi, lo, g, m, v = place(hi0), place(lo0), place(g0.to(gdtype)), place(m0), place(v0.abs())
+        F.adamw_step(hi, lo, None, g, m, v, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3, grad_scale=torch.full((1,), 0.5, device="cuda"))
+        return F.join_master(hi, lo), m, v
+
+    for a, b in zip(run(shift), run(3)):
+        assert bool(((a - b).abs() <= 8 * 2.0 ** -24 * (b.abs() + 1)).all())
+
+
+@pytest.mark.parametrize("n", [1, 3, 8, 1000003])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sumsq_sizes(native_lib, n, dtype):
+    """Against float64; fp32 partial sums of at most some hundred terms each: 1e-5 relative."""
+    from rl_b200.ops import functional as F
+
+    x = torch.randn(n + 1, device="cuda").to(dtype)
+    for part in (x[:n], x[1:]):
+        out = torch.zeros(1, device="cuda")
+        F.sumsq_(part, out)
+        assert abs(out.item() - part.double().pow(2).sum().item()) <= 1e-5 * part.double().pow(2).sum().item()
