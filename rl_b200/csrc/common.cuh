@@ -369,6 +369,16 @@ __device__ __forceinline__ void pdl_sync() {
 }
 
 // ---------------------------------------------------------------- numerics
+// Cosine and sine of `rows` positions for all pairs of a head, [rows][half]: every head of a token turns by the same angles.
+__device__ __forceinline__ void rope_table(float2* table, const int* pos, const float* inv_freq, int rows, int half, float sign) {
+  for (int i = threadIdx.x; i < rows * half; i += blockDim.x) {
+    const int r = i / half, j = i - r * half;
+    float s, c;
+    sincosf(static_cast<float>(pos[r]) * inv_freq[j], &s, &c);
+    table[i] = make_float2(c, s * sign);
+  }
+  __syncthreads();
+}
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -376,6 +386,18 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 __device__ __forceinline__ float2 unpack_bf16x2(uint32_t v) {
   __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162*>(&v);
   return __bfloat1622float2(b);
+}
+// Eight pairs (lo[i], hi[i]) of a head turned by table[i].
+__device__ __forceinline__ void rope_turn8(uint4& lo, uint4& hi, const float2* table) {
+  uint32_t* l = reinterpret_cast<uint32_t*>(&lo);
+  uint32_t* h = reinterpret_cast<uint32_t*>(&hi);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float2 a = unpack_bf16x2(l[q]), b = unpack_bf16x2(h[q]);
+    const float4 t = reinterpret_cast<const float4*>(table)[q];      // (cos, sin) of two pairs
+    l[q] = pack_bf16x2(a.x * t.x - b.x * t.y, a.y * t.z - b.y * t.w);
+    h[q] = pack_bf16x2(b.x * t.x + a.x * t.y, b.y * t.z + a.y * t.w);
+  }
 }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

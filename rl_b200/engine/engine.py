@@ -815,8 +815,7 @@ class GenerationEngine:
             else:
                 qkv = E.skinny_linear(hw, at.qkv_proj, bias=at.qkv_bias, ssq_in=ssq, eps=eps)
             if c.qk_norm:
-                qkv = F.head_rmsnorm(qkv, at.q_norm, 0, at.hq, c.head_dim, eps)
-                qkv = F.head_rmsnorm(qkv, at.k_norm, at.q_local, at.hkv, c.head_dim, eps)
+                qkv = F.qk_rmsnorm(qkv, at.q_norm, at.k_norm, at.hq, at.hkv, c.head_dim, eps)
             qkv = E.rope_kv_cache_write(qkv, positions, m.inv_freq, slots, self.k_cache[li], self.v_cache[li], self.hq, self.hkv, c.head_dim)
             a = E.paged_decode(qkv, self.k_cache[li], self.v_cache[li], block_table, seq_lens, self.hq, self.hkv, c.head_dim,
                                num_splits=num_splits, scratch=scratch)
@@ -861,8 +860,7 @@ class GenerationEngine:
             at = layer.self_attn
             qkv = E.skinny_linear(x, at.qkv_proj, bias=at.qkv_bias)
             if c.qk_norm:
-                qkv = F.head_rmsnorm(qkv, at.q_norm, 0, at.hq, c.head_dim, eps)
-                qkv = F.head_rmsnorm(qkv, at.k_norm, at.q_local, at.hkv, c.head_dim, eps)
+                qkv = F.qk_rmsnorm(qkv, at.q_norm, at.k_norm, at.hq, at.hkv, c.head_dim, eps)
             qkv = E.rope_kv_cache_write(qkv, positions, m.inv_freq, slots, self.k_cache[li], self.v_cache[li], self.hq, self.hkv, c.head_dim)
             a = E.paged_decode(qkv, self.k_cache[li], self.v_cache[li], block_table, seq_lens, self.hq, self.hkv, c.head_dim,
                                num_splits=num_splits, scratch=scratch)

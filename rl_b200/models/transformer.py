@@ -176,8 +176,7 @@ class Attention(nn.Module):
             if d is not None:
                 qkv = qkv + d
         if c.qk_norm:
-            qkv = F.head_rmsnorm(qkv, self.q_norm, 0, self.hq, c.head_dim, c.rms_norm_eps)
-            qkv = F.head_rmsnorm(qkv, self.k_norm, self.q_local, self.hkv, c.head_dim, c.rms_norm_eps)
+            qkv = F.qk_rmsnorm(qkv, self.q_norm, self.k_norm, self.hq, self.hkv, c.head_dim, c.rms_norm_eps)
         if not apply_rope:
             return qkv
         return F.rope(qkv, positions, inv_freq, self.hq + self.hkv, c.head_dim)

@@ -376,6 +376,52 @@ def head_rmsnorm(buf: torch.Tensor, w: torch.Tensor, col0: int, heads: int, D: i
     return _HeadRMSNorm.apply(buf, w, col0, heads, D, eps)
 
 
+class _QKNorm(torch.autograd.Function):
+    """Both norms of fused [q | k | v] rows in one pass over them."""
+
+    @staticmethod
+    def forward(ctx, buf, wq, wk, Hq, Hkv, D, eps):
+        T = buf.shape[0]
+        out = torch.empty(buf.shape, dtype=buf.dtype, device=buf.device)
+        rstd = torch.empty((T, Hq + Hkv), dtype=torch.float32, device=buf.device)
+        call("rlb_qk_rmsnorm_fwd", ptr(buf), ptr(wq), ptr(wk), ptr(out), ptr(rstd), T, Hq, Hkv, D, buf.stride(0), out.stride(0), eps, stream_ptr())
+        ctx.save_for_backward(buf, wq, wk, rstd)
+        ctx.meta = (Hq, Hkv, D)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        buf, wq, wk, rstd = ctx.saved_tensors
+        Hq, Hkv, D = ctx.meta
+        T = buf.shape[0]
+        dout = dout if dout.stride(1) == 1 and dout.stride(0) % 2 == 0 else dout.contiguous()
+        dbuf = torch.empty(buf.shape, dtype=buf.dtype, device=buf.device)
+        part = torch.empty((max(1, _L.lib().rlb_qk_rmsnorm_bwd_parts(T)), 2, D), dtype=torch.float32, device=buf.device)
+        dw = torch.zeros((2, D), dtype=torch.float32, device=buf.device)
+        call("rlb_qk_rmsnorm_bwd", ptr(dout), ptr(buf), ptr(wq), ptr(wk), ptr(rstd), ptr(dbuf), ptr(part), ptr(dw), T, Hq, Hkv, D, buf.stride(0),
+             dout.stride(0), dbuf.stride(0), stream_ptr())
+        grads = []
+        for w, g, need in ((wq, dw[0], ctx.needs_input_grad[1]), (wk, dw[1], ctx.needs_input_grad[2])):
+            main_grad = getattr(w, "main_grad", None)
+            if main_grad is not None:
+                main_grad.add_(g.to(main_grad.dtype))
+            grads.append(g.to(w.dtype) if need and main_grad is None else None)
+        return dbuf, grads[0], grads[1], None, None, None, None
+
+
+def qk_rmsnorm(buf: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, Hq: int, Hkv: int, D: int, eps: float) -> torch.Tensor:
+    """RMSNorms of the ``Hq`` query and ``Hkv`` key heads of fused [q | k | v] rows [T, (Hq + 2 Hkv) * D]. Without autograd on the GPU the rows
+    are changed in place and returned."""
+    if not (use_native(buf) and buf.dtype == BF16 and D % 64 == 0 and D <= 256 and buf.stride(1) == 1 and buf.stride(0) % 2 == 0
+            and buf.shape[1] == (Hq + 2 * Hkv) * D):
+        buf = head_rmsnorm(buf, wq, 0, Hq, D, eps)
+        return head_rmsnorm(buf, wk, Hq * D, Hkv, D, eps)
+    if torch.is_grad_enabled() and (buf.requires_grad or wq.requires_grad or wk.requires_grad):
+        return _QKNorm.apply(buf, wq, wk, Hq, Hkv, D, eps)
+    call("rlb_qk_rmsnorm_fwd", ptr(buf), ptr(wq), ptr(wk), ptr(buf), None, buf.shape[0], Hq, Hkv, D, buf.stride(0), buf.stride(0), eps, stream_ptr())
+    return buf
+
+
 # --------------------------------------------------------------------------------------- RoPE
 def _rope_ref(x, positions, inv_freq, heads, D, sign=1.0):
     T = x.shape[0]

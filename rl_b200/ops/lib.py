@@ -40,6 +40,9 @@ _SIGS: dict[str, list[Any]] = {
     "rlb_rmsnorm_bwd_parts": [L],
     "rlb_rmsnorm_bwd": [P, P, P, P, P, P, P, P, I, L, I, L, L, I, P],
     "rlb_rope": [P, P, P, L, I, I, L, I, P],
+    "rlb_qk_rmsnorm_fwd": [P, P, P, P, P, L, I, I, I, L, L, F, P],
+    "rlb_qk_rmsnorm_bwd_parts": [L],
+    "rlb_qk_rmsnorm_bwd": [P, P, P, P, P, P, P, P, L, I, I, I, L, L, L, P],
     "rlb_head_rmsnorm_fwd": [P, P, P, P, L, I, I, L, L, F, P],
     "rlb_head_rmsnorm_bwd": [P, P, P, P, P, P, L, I, I, L, L, L, P],
     "rlb_swiglu_fwd": [P, P, L, I, P],

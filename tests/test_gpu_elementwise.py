@@ -410,3 +410,79 @@ def test_sumsq_sizes(native_lib, n, dtype):
         out = torch.zeros(1, device="cuda")
         F.sumsq_(part, out)
         assert abs(out.item() - part.double().pow(2).sum().item()) <= 1e-5 * part.double().pow(2).sum().item()
+
+
+@pytest.mark.parametrize("D", [16, 64, 96, 128, 256])
+@pytest.mark.parametrize("T,heads", [(1, 3), (5, 12), (2371, 5)])      # one row per block, four rows per block and a cut last block
+@pytest.mark.parametrize("pad", [0, 8, 4])                             # a row stride without 16-byte alignment takes the plain kernel
+def test_rope_rows(native_lib, D, T, heads, pad):
+    """Both directions against the fp32 statement: one rounding of the result (2^-8 of values up to 8) and the fast sines (2e-6 at these angles)."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(D + T)
+    wide = torch.randn(T, (heads + 2) * D + pad, generator=g, device="cuda").bfloat16()
+    x, keep = wide[:, : (heads + 2) * D], wide.clone()
+    pos = torch.randint(0, 900, (T,), generator=g, device="cuda", dtype=torch.int32)
+    inv = 1.0 / 10000.0 ** (torch.arange(0, D, 2, device="cuda").float() / D)
+    F.call("rlb_rope", x.data_ptr(), pos.data_ptr(), inv.data_ptr(), T, heads, D, x.stride(0), 0, F.stream_ptr())
+    ref = F._rope_ref(keep[:, : (heads + 2) * D].float(), pos, inv, heads, D)
+    assert (x.float() - ref).abs().max() <= 2.0 ** -9 * 8 + 1e-3 and torch.equal(x[:, heads * D :], keep[:, heads * D : (heads + 2) * D])
+    F.call("rlb_rope", x.data_ptr(), pos.data_ptr(), inv.data_ptr(), T, heads, D, x.stride(0), 1, F.stream_ptr())
+    assert (x.float() - keep[:, : (heads + 2) * D].float()).abs().max() <= 4 * 2.0 ** -9 * 8 + 2e-3
+    assert torch.equal(wide[:, (heads + 2) * D :], keep[:, (heads + 2) * D :])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T,bs", [(3, 16), (2370, 64)])
+def test_rope_kv_rows(native_lib, D, T, bs):
+    """Rotation and cache scatter with skipped tokens, against the rotation alone (the same arithmetic, bit for bit) and plain copies."""
+    from rl_b200.ops import engine_ops as E
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import check_status
+
+    Hq, Hkv = 6, 2
+    g = torch.Generator("cuda").manual_seed(D + T)
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * D, generator=g, device="cuda").bfloat16()
+    pos = torch.randint(0, 900, (T,), generator=g, device="cuda", dtype=torch.int32)
+    inv = 1.0 / 10000.0 ** (torch.arange(0, D, 2, device="cuda").float() / D)
+    blocks = T // bs + 2
+    slots = torch.randperm(blocks * bs, generator=g, device="cuda")[:T]
+    slots[1::3] = -1
+    kc, vc = torch.zeros(2, blocks, Hkv, bs, D, device="cuda", dtype=torch.bfloat16)
+    want = F.rope(qkv.clone(), pos, inv, Hq + Hkv, D)
+    v = qkv[:, (Hq + Hkv) * D :].clone()
+    got = E.rope_kv_cache_write(qkv, pos, inv, slots, kc, vc, Hq, Hkv, D)
+    torch.cuda.synchronize()
+    assert check_status() == 0 and torch.equal(got, want)
+    live = slots >= 0
+    b, o = slots[live] // bs, slots[live] % bs
+    assert torch.equal(kc[b, :, o].reshape(-1, Hkv * D), want[live, Hq * D : (Hq + Hkv) * D]) and torch.equal(vc[b, :, o].reshape(-1, Hkv * D), v[live])
+    assert (kc != 0).any(-1).sum() == live.sum() * Hkv and (vc != 0).any(-1).sum() == live.sum() * Hkv
+
+
+@pytest.mark.parametrize("D", [64, 128, 192, 256])
+@pytest.mark.parametrize("T,Hq,Hkv", [(1, 2, 1), (77, 8, 2), (700, 5, 5)])
+def test_qk_rmsnorm(native_lib, D, T, Hq, Hkv):
+    """Forward (a new buffer, and in place without autograd) and gradients against float64; bf16 results: one rounding of 2^-8 and, in the
+    gradient of the rows, the cancellation of two terms of the gradient's size."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(D + T)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    x = r(T, (Hq + 2 * Hkv) * D).bfloat16().requires_grad_()
+    wq, wk = (1 + 0.3 * r(2, D)).bfloat16()
+    wq, wk = wq.clone().requires_grad_(), wk.clone().requires_grad_()
+    wk.main_grad = torch.ones(D, device="cuda")
+    up = r(*x.shape).bfloat16()
+    y = F.qk_rmsnorm(x, wq, wk, Hq, Hkv, D, 1e-6)
+    y.backward(up)
+    X, Q, K = (t.detach().double().requires_grad_() for t in (x, wq, wk))
+    h = X.view(T, Hq + 2 * Hkv, D)
+    n = h[:, : Hq + Hkv] * torch.rsqrt(h[:, : Hq + Hkv].pow(2).mean(-1, keepdim=True) + 1e-6)
+    ref = torch.cat([n[:, :Hq] * Q, n[:, Hq:] * K, h[:, Hq + Hkv :]], 1).reshape(T, -1)
+    ref.backward(up.double())
+    near = lambda a, b, t: (a.double() - b).norm() <= t * b.norm()      # noqa: E731
+    assert near(y, ref, 2.0 ** -8) and near(x.grad, X.grad, 2.0 ** -7) and near(wq.grad, Q.grad, 2.0 ** -7) and near(wk.main_grad - 1, K.grad, 1e-3)
+    with torch.no_grad():
+        z = x.detach().clone()
+        assert F.qk_rmsnorm(z, wq, wk, Hq, Hkv, D, 1e-6) is z and torch.equal(z, y)
