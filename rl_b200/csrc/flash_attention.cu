@@ -5,14 +5,17 @@
 // RoPE) through 2-D TMA tensor maps; `cu_seqlens[B+1]` marks sequence boundaries. The same kernels serve training
 // (packed micro-batches) and the prefill of the generation engine.
 //
-// Forward, one CTA per (128-row query tile, query head), two CTAs per SM so that one CTA's softmax overlaps the
-// other's MMAs:
-//   warp 0      TMA producer: Q once, then K/V tiles of 64 keys through a 2-stage ring
-//   warp 1      tcgen05.mma issuer: S = Q K^T (128x64x128) into TMEM, then O += P V (128x128x64)
+// Forward, one CTA per (128-row query tile, query head), two CTAs per SM, the longest tiles first:
+//   warp 0      TMA producer: Q once, then K tiles of 64 keys through a 3-stage ring and V tiles through a 2-stage ring
+//   warp 1      tcgen05.mma issuer: S = Q K^T (128x64x128) into one of two TMEM buffers, one tile ahead of the softmax, then
+//               O += P V (128x128x64) with P read from TMEM
 //   warps 2..5  softmax: one thread per query row reads its 64 scores from TMEM (no shuffles), keeps the running
-//               max / sum in the exp2 domain, writes P in bf16 into 128B-swizzled shared memory as the A operand of
-//               the second MMA, and rescales the O accumulator in TMEM only when the row maximum moved by more than
-//               2^8 (stale maxima are exact because the final normalisation uses the same reference).
+//               max / sum in the exp2 domain, writes P in bf16 over the scores it has read, and rescales the O accumulator in
+//               TMEM only when the row maximum moved by more than 2^8 (stale maxima are exact because the final normalisation
+//               uses the same reference).
+// Bound by the exponentials and the tensor cores alike (512 cycles each per tile and CTA), so both have to run all the time: the next
+// tile's scores are computed under this one's softmax, and two CTAs cover each other's hand-offs. Measured, 32 query and 8 KV heads of 128
+// (before: one score buffer, P through shared memory): 16 x 4096 tokens 3.77 -> 2.24 ms (984 TFLOP/s); 64 x 1280 2.02 -> 1.18 ms.
 // Output: O[T, Hq*128] bf16 and the per-row log-sum-exp lse[Hq, T] (natural log) for the backward pass.
 //
 // Backward is two kernels without atomics: one per (64-key tile, kv head) accumulating dK / dV over all query tiles
@@ -39,16 +42,16 @@ constexpr int BKV = 64;   // keys per pipeline stage
 constexpr int HD = RLB_HD;
 static_assert(HD == 64 || HD == 128, "head dimension: 64 or 128");
 constexpr int ATOMS = HD / 64;            // [rows x 64] swizzle atoms per operand tile along the head dimension
-constexpr int KV_STAGES = 2;
+constexpr int K_STAGES = 3;
+constexpr int V_STAGES = 2;
 constexpr int Q_BYTES = BQ * HD * 2;         // 32 KB at HD 128: two [128 x 64] swizzle atoms
 constexpr int Q_ATOM = BQ * 64 * 2;
 constexpr int KV_ATOM = BKV * 64 * 2;
 constexpr int K_BYTES = BKV * HD * 2;        // 16 KB: two [64 x 64] atoms
 constexpr int V_BYTES = BKV * HD * 2;        // 16 KB: two boxes of 64 head-dim columns
-constexpr int P_BYTES = BQ * BKV * 2;        // 16 KB: one [128 x 64] atom
-constexpr int FWD_SMEM = Q_BYTES + KV_STAGES * (K_BYTES + V_BYTES) + P_BYTES + 256;  // 2 CTAs fit in 227 KB
+constexpr int FWD_SMEM = Q_BYTES + K_STAGES * K_BYTES + V_STAGES * V_BYTES + 256;  // 2 CTAs fit in 227 KB
 constexpr int FWD_THREADS = 192;
-constexpr int TMEM_COLS_FWD = 256;  // S at column 0 (64 columns), O at column 128 (128 columns)
+constexpr int TMEM_COLS_FWD = 256;  // S of even and odd tiles at columns 0 and 64 (P in the first 32 of each), O at column 128
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // in log2 units
 
@@ -65,29 +68,32 @@ __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_
       : "memory");
 }
 
-// Finds the (sequence, tile-in-sequence) of a flat tile index; tiles of `rows` rows never straddle sequences.
-// Returns false when `tile` is past the last tile. One thread calls it; the result is broadcast through smem.
-__device__ bool locate_tile(const int* __restrict__ cu, int num_seqs, int rows, int tile, int& seq, int& start,
-                            int& len, int& tile_in_seq) {
+// Finds the (sequence, tile-in-sequence) of a flat tile index; tiles of `rows` rows never straddle sequences. Called by a whole warp, 32
+// sequences at a time (one thread walking them waited for memory at every one). Returns false when `tile` is past the last tile.
+__device__ __forceinline__ bool locate_tile(const int* __restrict__ cu, int num_seqs, int rows, int tile, int& start, int& len, int& tile_in_seq) {
+  const int lane = threadIdx.x & 31;
   int acc = 0;
-  for (int s = 0; s < num_seqs; ++s) {
+  for (int s0 = 0; s0 < num_seqs; s0 += 32) {
+    const int s = min(s0 + lane, num_seqs - 1);
     const int b = cu[s], e = cu[s + 1];
-    const int n = (e - b + rows - 1) / rows;
-    if (tile < acc + n) {
-      seq = s;
-      start = b;
-      len = e - b;
-      tile_in_seq = tile - acc;
+    const int n = s0 + lane < num_seqs ? (e - b + rows - 1) / rows : 0;
+    int end = n;      // tiles of the sequences up to this lane's
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, tile < acc + end);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      start = __shfl_sync(0xffffffffu, b, src);
+      len = __shfl_sync(0xffffffffu, e - b, src);
+      tile_in_seq = tile - acc - __shfl_sync(0xffffffffu, end - n, src);
       return true;
     }
-    acc += n;
+    acc += __shfl_sync(0xffffffffu, end, 31);
   }
   return false;
-}
-
-// Writes 8 bf16 (one 16-byte chunk) of row `r` at logical chunk `c` (0..7) of a 128B-swizzled [rows x 64] atom.
-__device__ __forceinline__ void st_swizzled_chunk(uint8_t* atom, int r, int c, uint4 v) {
-  *reinterpret_cast<uint4*>(atom + r * 128 + ((c ^ (r & 7)) << 4)) = v;
 }
 
 struct FwdParams {
@@ -113,17 +119,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   }
   uint8_t* q_s = smem;
   uint8_t* k_s = q_s + Q_BYTES;
-  uint8_t* v_s = k_s + KV_STAGES * K_BYTES;
-  uint8_t* p_s = v_s + KV_STAGES * V_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p_s + P_BYTES);
+  uint8_t* v_s = k_s + K_STAGES * K_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + V_STAGES * V_BYTES);
   uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;    // [2]
-  uint64_t* v_full = bars + 3;    // [2]
-  uint64_t* kv_empty = bars + 5;  // [2]
-  uint64_t* s_full = bars + 7;
-  uint64_t* p_full = bars + 8;
-  uint64_t* o_done = bars + 9;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint64_t* k_full = bars + 1;    // [3]
+  uint64_t* k_empty = bars + 4;   // [3]
+  uint64_t* v_full = bars + 7;    // [2]
+  uint64_t* v_empty = bars + 9;   // [2] also: the product with this V tile is in O
+  uint64_t* s_full = bars + 11;   // [2]
+  uint64_t* p_full = bars + 13;   // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* tile_info = reinterpret_cast<int*>(tmem_slot + 2);  // seq_start, seq_len, tile_in_seq, valid
 
@@ -131,25 +136,29 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int head = blockIdx.y;
   const int kv_head = head / (p.Hq / p.Hkv);
 
-  if (threadIdx.x == 0) {
-    int seq = 0, start = 0, len = 0, tis = 0;
-    const bool ok = locate_tile(p.cu_seqlens, p.num_seqs, BQ, blockIdx.x, seq, start, len, tis);
-    tile_info[0] = start;
-    tile_info[1] = len;
-    tile_info[2] = tis;
-    tile_info[3] = ok ? 1 : 0;
-    mbar_init(smem_u32(q_full), 1);
-    for (int s = 0; s < KV_STAGES; ++s) {
-      mbar_init(smem_u32(&k_full[s]), 1);
-      mbar_init(smem_u32(&v_full[s]), 1);
-      mbar_init(smem_u32(&kv_empty[s]), 1);
+  if (warp == 0) {
+    int start = 0, len = 0, tis = 0;
+    const bool ok = locate_tile(p.cu_seqlens, p.num_seqs, BQ, gridDim.x - 1 - blockIdx.x, start, len, tis);      // late tiles of a sequence see the most keys
+    if (lane == 0) {
+      tile_info[0] = start;
+      tile_info[1] = len;
+      tile_info[2] = tis;
+      tile_info[3] = ok ? 1 : 0;
+      mbar_init(smem_u32(q_full), 1);
+      for (int s = 0; s < K_STAGES; ++s) {
+        mbar_init(smem_u32(&k_full[s]), 1);
+        mbar_init(smem_u32(&k_empty[s]), 1);
+      }
+      for (int s = 0; s < 2; ++s) {
+        mbar_init(smem_u32(&v_full[s]), 1);
+        mbar_init(smem_u32(&v_empty[s]), 1);
+        mbar_init(smem_u32(&s_full[s]), 1);
+        mbar_init(smem_u32(&p_full[s]), 4);
+      }
+      *abort_flag = 0;
+      mbar_fence_init();
+      fence_proxy_async();
     }
-    mbar_init(smem_u32(s_full), 1);
-    mbar_init(smem_u32(p_full), 128);
-    mbar_init(smem_u32(o_done), 1);
-    *abort_flag = 0;
-    mbar_fence_init();
-    fence_proxy_async();
   }
   __syncthreads();
   if (!tile_info[3]) return;  // uniform: past the last tile (before any TMEM allocation)
@@ -161,7 +170,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base;
   const uint32_t tmem_o = tmem_base + 128;
 
   const int seq_start = tile_info[0], seq_len = tile_info[1];
@@ -180,53 +188,61 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll
       for (int a = 0; a < ATOMS; ++a)
         tma_load_2d(smem_u32(q_s + a * Q_ATOM), &tmap_q, smem_u32(q_full), q_col + a * 64, seq_start + q0);
-      for (int j = 0; j < n_kv; ++j) {
-        const int st = j % KV_STAGES;
-        const uint32_t ph = (j / KV_STAGES) & 1;
-        if (!mbar_wait(smem_u32(&kv_empty[st]), ph ^ 1, abort_flag, p.status, RLB_ERR_WAIT_EMPTY)) break;
-        const int row = seq_start + j * BKV;
-        mbar_arrive_expect_tx(smem_u32(&k_full[st]), K_BYTES);
+      bool ok = true;
+      for (int j = 0; j < n_kv && ok; ++j) {
+        const int row = seq_start + j * BKV, ks = j % K_STAGES, vs = j % V_STAGES;
+        ok = mbar_wait(smem_u32(&k_empty[ks]), ((j / K_STAGES) & 1) ^ 1, abort_flag, p.status, RLB_ERR_WAIT_EMPTY);
+        if (!ok) break;
+        mbar_arrive_expect_tx(smem_u32(&k_full[ks]), K_BYTES);
 #pragma unroll
         for (int a = 0; a < ATOMS; ++a)
-          tma_load_2d(smem_u32(k_s + st * K_BYTES + a * KV_ATOM), &tmap_kv, smem_u32(&k_full[st]), k_col + a * 64, row);
-        mbar_arrive_expect_tx(smem_u32(&v_full[st]), V_BYTES);
+          tma_load_2d(smem_u32(k_s + ks * K_BYTES + a * KV_ATOM), &tmap_kv, smem_u32(&k_full[ks]), k_col + a * 64, row);
+        ok = mbar_wait(smem_u32(&v_empty[vs]), ((j / V_STAGES) & 1) ^ 1, abort_flag, p.status, RLB_ERR_WAIT_EMPTY);
+        if (!ok) break;
+        mbar_arrive_expect_tx(smem_u32(&v_full[vs]), V_BYTES);
 #pragma unroll
         for (int a = 0; a < ATOMS; ++a)
-          tma_load_2d(smem_u32(v_s + st * V_BYTES + a * KV_ATOM), &tmap_kv, smem_u32(&v_full[st]), v_col + a * 64, row);
+          tma_load_2d(smem_u32(v_s + vs * V_BYTES + a * KV_ATOM), &tmap_kv, smem_u32(&v_full[vs]), v_col + a * 64, row);
+      }
+      if (!ok) {      // loads in flight land within microseconds: they must not outlive the CTA
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 1000000ull) {}
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(BQ, BKV, false, false);
       constexpr uint32_t idesc_o = make_idesc_bf16(BQ, HD, false, true);
-      bool ok = mbar_wait(smem_u32(q_full), 0, abort_flag, p.status, RLB_ERR_WAIT_FULL);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int st = j % KV_STAGES;
-        const uint32_t ph = (j / KV_STAGES) & 1;
-        if (!mbar_wait(smem_u32(&k_full[st]), ph, abort_flag, p.status, RLB_ERR_WAIT_FULL)) break;
+      // S = Q K^T of tile j over the head dimension: steps of 16, swizzle atoms of 64. Its buffer held P of tile j - 2, whose product has
+      // to be complete.
+      auto scores = [&](int j) -> bool {
+        const int ks = j % K_STAGES;
+        if (j > 1 && !mbar_wait(smem_u32(&v_empty[j % V_STAGES]), ((j - 2) / V_STAGES) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) return false;
+        if (!mbar_wait(smem_u32(&k_full[ks]), (j / K_STAGES) & 1, abort_flag, p.status, RLB_ERR_WAIT_FULL)) return false;
         tc_fence_after();
-        // S = Q K^T over the head dimension: 8 steps of 16, two swizzle atoms of 64
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
           const uint32_t qa = smem_u32(q_s) + (kk / 4) * Q_ATOM + (kk % 4) * 32;
-          const uint32_t ka = smem_u32(k_s + st * K_BYTES) + (kk / 4) * KV_ATOM + (kk % 4) * 32;
-          umma_f16(tmem_s, make_smem_desc_sw128(qa, 16, 1024), make_smem_desc_sw128(ka, 16, 1024), idesc_s,
-                   kk != 0 ? 1u : 0u);
+          const uint32_t ka = smem_u32(k_s + ks * K_BYTES) + (kk / 4) * KV_ATOM + (kk % 4) * 32;
+          umma_f16(tmem_base + (j & 1) * 64, make_smem_desc_sw128(qa, 16, 1024), make_smem_desc_sw128(ka, 16, 1024), idesc_s, kk != 0 ? 1u : 0u);
         }
-        umma_commit(smem_u32(s_full));
-        if (!mbar_wait(smem_u32(p_full), j & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) break;
-        if (!mbar_wait(smem_u32(&v_full[st]), ph, abort_flag, p.status, RLB_ERR_WAIT_FULL)) break;
+        umma_commit(smem_u32(&s_full[j & 1]));
+        umma_commit(smem_u32(&k_empty[ks]));
+        return true;
+      };
+      bool ok = mbar_wait(smem_u32(q_full), 0, abort_flag, p.status, RLB_ERR_WAIT_FULL) && (n_kv == 0 || scores(0));
+      for (int j = 0; j < n_kv && ok; ++j) {
+        const int vs = j % V_STAGES;
+        if (j + 1 < n_kv && !scores(j + 1)) break;
+        if (!mbar_wait(smem_u32(&p_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) break;
+        if (!mbar_wait(smem_u32(&v_full[vs]), (j / V_STAGES) & 1, abort_flag, p.status, RLB_ERR_WAIT_FULL)) break;
         tc_fence_after();
-        // O += P V over the 64 keys: 4 steps of 16 key rows
+        // O += P V over the 64 keys: 4 steps of 16 key rows, 8 columns of P each
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint32_t pa = smem_u32(p_s) + kk * 32;
-          const uint32_t va = smem_u32(v_s + st * V_BYTES) + kk * (16 * 128);
-          umma_f16(tmem_o, make_smem_desc_sw128(pa, 16, 1024), make_smem_desc_sw128(va, KV_ATOM, 1024), idesc_o,
-                   (j | kk) != 0 ? 1u : 0u);
-        }
-        umma_commit(smem_u32(&kv_empty[st]));
-        umma_commit(smem_u32(o_done));
+        for (int kk = 0; kk < BKV / 16; ++kk)
+          umma_f16_ts(tmem_o, tmem_base + (j & 1) * 64 + kk * 8, make_smem_desc_sw128(smem_u32(v_s + vs * V_BYTES) + kk * (16 * 128), KV_ATOM, 1024), idesc_o,
+                      (j | kk) != 0 ? 1u : 0u);
+        umma_commit(smem_u32(&v_empty[vs]));
       }
     }
   } else {
@@ -238,31 +254,49 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     float m_ref = -INFINITY;  // reference maximum used for the exponentials (log2 domain)
     float l = 0.f;
     bool ok = true;
+    // scores are compared before scaling; a negative scale turns the comparison round
+    const bool neg = p.scale_log2 < 0.f;
+    const float hidden = neg ? INFINITY : -INFINITY;
     for (int j = 0; j < n_kv; ++j) {
-      if (!mbar_wait(smem_u32(s_full), j & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL)) {
+      const uint32_t tmem_s = tmem_base + (j & 1) * 64 + lane_addr;
+      if (!mbar_wait(smem_u32(&s_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL)) {
         ok = false;
         break;
       }
       tc_fence_after();
       uint32_t s0[32], s1[32];
-      tmem_ld_32x32b_x32(tmem_s + lane_addr, s0);
-      tmem_ld_32x32b_x32(tmem_s + lane_addr + 32, s1);
+      tmem_ld_32x32b_x32(tmem_s, s0);
+      tmem_ld_32x32b_x32(tmem_s + 32, s1);
       tmem_ld_wait();
       const int k0 = j * BKV;
-      const bool diag = k0 + BKV - 1 > q0;  // tile touches the causal boundary of some row
-      float mx = -INFINITY;
+      if (k0 + BKV - 1 > q0) {  // tile touches the causal boundary of some row
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        float a = __uint_as_float(s0[i]) * p.scale_log2;
-        float b = __uint_as_float(s1[i]) * p.scale_log2;
-        if (diag) {
-          if (k0 + i > qi) a = -INFINITY;
-          if (k0 + 32 + i > qi) b = -INFINITY;
+        for (int i = 0; i < 32; ++i) {
+          if (k0 + i > qi) s0[i] = __float_as_uint(hidden);
+          if (k0 + 32 + i > qi) s1[i] = __float_as_uint(hidden);
         }
-        s0[i] = __float_as_uint(a);
-        s1[i] = __float_as_uint(b);
-        mx = fmaxf(mx, fmaxf(a, b));
       }
+      float best[4] = {__uint_as_float(s0[0]), __uint_as_float(s0[1]), __uint_as_float(s1[0]), __uint_as_float(s1[1])};
+      if (!neg) {
+#pragma unroll
+        for (int i = 2; i < 32; i += 2) {
+          best[0] = fmaxf(best[0], __uint_as_float(s0[i]));
+          best[1] = fmaxf(best[1], __uint_as_float(s0[i + 1]));
+          best[2] = fmaxf(best[2], __uint_as_float(s1[i]));
+          best[3] = fmaxf(best[3], __uint_as_float(s1[i + 1]));
+        }
+        best[0] = fmaxf(fmaxf(best[0], best[1]), fmaxf(best[2], best[3]));
+      } else {
+#pragma unroll
+        for (int i = 2; i < 32; i += 2) {
+          best[0] = fminf(best[0], __uint_as_float(s0[i]));
+          best[1] = fminf(best[1], __uint_as_float(s0[i + 1]));
+          best[2] = fminf(best[2], __uint_as_float(s1[i]));
+          best[3] = fminf(best[3], __uint_as_float(s1[i + 1]));
+        }
+        best[0] = fminf(fminf(best[0], best[1]), fminf(best[2], best[3]));
+      }
+      const float mx = best[0] * p.scale_log2;
       // Lazy rescale: move the reference only when the maximum grew by more than the threshold.
       float factor = 1.f;
       bool need = false;
@@ -274,28 +308,29 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           m_ref = m_new;
         }
       }
-      l *= factor;
-      float rowsum = 0.f;
+      const float mr = (m_ref == -INFINITY) ? 0.f : -m_ref;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
       uint32_t pk[32];
-      const float mr = (m_ref == -INFINITY) ? 0.f : m_ref;
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const float e0 = exp2f(__uint_as_float(s0[2 * i]) - mr), e1 = exp2f(__uint_as_float(s0[2 * i + 1]) - mr);
-        const float f0 = exp2f(__uint_as_float(s1[2 * i]) - mr), f1 = exp2f(__uint_as_float(s1[2 * i + 1]) - mr);
-        rowsum += (e0 + e1) + (f0 + f1);
+        const float e0 = exp2f(fmaf(__uint_as_float(s0[2 * i]), p.scale_log2, mr)), e1 = exp2f(fmaf(__uint_as_float(s0[2 * i + 1]), p.scale_log2, mr));
+        const float f0 = exp2f(fmaf(__uint_as_float(s1[2 * i]), p.scale_log2, mr)), f1 = exp2f(fmaf(__uint_as_float(s1[2 * i + 1]), p.scale_log2, mr));
+        sum[0] += e0;
+        sum[1] += e1;
+        sum[2] += f0;
+        sum[3] += f1;
         pk[i] = pack_bf16x2(e0, e1);
         pk[16 + i] = pack_bf16x2(f0, f1);
       }
-      l += rowsum;
-      // P and O may be touched only after the previous P V product has completed.
-      if (j > 0) {
-        if (!mbar_wait(smem_u32(o_done), (j - 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
+      l = l * factor + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+      tmem_st_32x32b_x32(tmem_s, pk);      // over the scores that this thread has read
+      if (__any_sync(0xffffffffu, need)) {
+        // O may be touched only after the previous P V product has completed (the next one waits for p_full)
+        if (!mbar_wait(smem_u32(&v_empty[(j - 1) % V_STAGES]), ((j - 1) / V_STAGES) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
           ok = false;
           break;
         }
         tc_fence_after();
-      }
-      if (__any_sync(0xffffffffu, need)) {
 #pragma unroll
         for (int c = 0; c < HD / 32; ++c) {
           uint32_t o[32];
@@ -305,16 +340,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
           tmem_st_32x32b_x32(tmem_o + lane_addr + c * 32, o);
         }
-        tmem_st_wait();
       }
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        st_swizzled_chunk(p_s, r, c, make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
-      fence_proxy_async();
+      tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(smem_u32(p_full));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&p_full[j & 1]));
     }
-    if (ok && mbar_wait(smem_u32(o_done), (n_kv - 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
+    if (ok && mbar_wait(smem_u32(&v_empty[(n_kv - 1) % V_STAGES]), ((n_kv - 1) / V_STAGES) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
       tc_fence_after();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       const bool row_ok = r < q_rows;
@@ -399,7 +431,7 @@ RLB_API int RLB_NAME(rlb_flash_attn_fwd)(const void* qkv, long long qkv_stride, 
   p.T = T;
   p.Hq = Hq;
   p.Hkv = Hkv;
-  p.scale_log2 = scale * LOG2E;
+  p.scale_log2 = scale == 0.f ? 1e-30f : scale * LOG2E;      // (hidden scores are infinite: they must not meet a factor of zero)
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.out_stride = out_stride;
   p.lse = lse;
