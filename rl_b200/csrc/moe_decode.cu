@@ -5,10 +5,10 @@
 //   route_topk     one warp per token: soft-max over the router logits, top-k (lowest index wins ties), optional
 //                  renormalisation of the k weights.
 //   decode_plan    one CTA: stable counting sort of the token copies whose expert lives on this rank into the
-//                  padded-by-expert row layout of the grouped GEMM (each expert's rows padded to a multiple of 128);
+//                  padded-by-expert row layout of the expert products (each expert's rows padded to whole tiles of `pad` rows);
 //                  writes, per padded row, the token it holds, per copy its row (or -1: expert of another rank), and
 //                  the tile -> expert table.
-//   gather_rows    padded rows <- token rows (zeros in padding rows of live tiles).
+//   gather_rows    padded rows <- token rows (padding rows of live tiles: zeros, or left as they are).
 //   combine        out[t] = residual[t] + sum_j w[t, j] * y[row(t, j)] over this rank's copies, in copy order.
 //   combine_reduce the expert-parallel form: every rank has ALL ranks' tokens (gathered before the router, which every
 //                  rank evaluates identically), computes the contribution of its own experts to every token, writes
@@ -50,6 +50,7 @@ __device__ __forceinline__ unsigned int ld_acquire_sys_u32(const unsigned int* p
 __global__ void __launch_bounds__(256) route_topk_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int T, int E, int k,
                                                          int renorm, float* __restrict__ out_w, int* __restrict__ out_idx) {
   extern __shared__ float smem[];
+  pdl_sync();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * (blockDim.x >> 5) + warp;
   if (t >= T) return;
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(256) route_topk_kernel(const __nv_bfloat16* __
 
 // ------------------------------------------------------------------------------------------------ layout plan
 // idx [n_copies] global expert of every token copy (copy c belongs to token c / k). Experts [e_lo, e_lo + El) are local.
-__global__ void __launch_bounds__(1024) decode_plan_kernel(const int* __restrict__ idx, int n_copies, int k, int e_lo, int El, int mpad,
+__global__ void __launch_bounds__(1024) decode_plan_kernel(const int* __restrict__ idx, int n_copies, int k, int e_lo, int El, int mpad, int pad,
                                                            int* __restrict__ src_tok, int* __restrict__ copy_row,
                                                            int* __restrict__ tile_expert, int* __restrict__ row0_out,
                                                            int* __restrict__ rows_out, int* status) {
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(1024) decode_plan_kernel(const int* __restrict
   __shared__ int s_cnt[PLAN_MAX_EXPERTS];
   __shared__ int s_row0[PLAN_MAX_EXPERTS + 1];
   const int tid = threadIdx.x, nthr = blockDim.x;
+  pdl_sync();
   for (int e = tid; e < El; e += nthr) s_cnt[e] = 0;
   __syncthreads();
   for (int c = tid; c < n_copies; c += nthr) {
@@ -122,10 +124,10 @@ __global__ void __launch_bounds__(1024) decode_plan_kernel(const int* __restrict
     int at = 0;
     for (int e = 0; e < El; ++e) {
       s_row0[e] = at;
-      at += (s_cnt[e] + 127) / 128 * 128;
+      at += (s_cnt[e] + pad - 1) / pad * pad;
     }
     s_row0[El] = at;
-    if (at > mpad && status) atomicCAS(status, 0, RLB_ERR_BOUNDS);   // cannot happen when mpad >= n_copies + El * 127
+    if (at > mpad && status) atomicCAS(status, 0, RLB_ERR_BOUNDS);   // cannot happen when mpad >= n_copies + El * (pad - 1)
   }
   __syncthreads();
   const int total = min(s_row0[El], mpad);
@@ -133,8 +135,8 @@ __global__ void __launch_bounds__(1024) decode_plan_kernel(const int* __restrict
     row0_out[e] = s_row0[e];
     rows_out[e] = s_row0[e + 1] - s_row0[e];
   }
-  for (int tile = tid; tile < mpad / 128; tile += nthr) {
-    const int start = tile * 128;
+  for (int tile = tid; tile < mpad / pad; tile += nthr) {
+    const int start = tile * pad;
     int te = -1;
     if (start < total) {
       int lo = 0, hi = El - 1;   // last expert whose first row is <= start
@@ -167,13 +169,15 @@ __global__ void __launch_bounds__(1024) decode_plan_kernel(const int* __restrict
   }
 }
 
-// One warp per padded row of a live tile: x_pad[row] = x[src_tok[row]] (zeros when the row is padding).
+// One warp per padded row of a live 128-row tile: x_pad[row] = x[src_tok[row]] (zeros when the row is padding); without tile_expert only the
+// rows that hold a token are written.
 __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ x, long long x_stride_vecs, const int* __restrict__ src_tok,
                                                           const int* __restrict__ tile_expert, uint4* __restrict__ out, int mpad, int vecs) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_sync();
   for (int row = blockIdx.x * (blockDim.x >> 5) + warp; row < mpad; row += gridDim.x * (blockDim.x >> 5)) {
-    if (tile_expert[row >> 7] < 0) continue;
     const int t = src_tok[row];
+    if (tile_expert ? tile_expert[row >> 7] < 0 : t < 0) continue;
     uint4* d = out + static_cast<long long>(row) * vecs;
     if (t < 0) {
       for (int v = lane; v < vecs; v += 32) d[v] = make_uint4(0, 0, 0, 0);
@@ -215,6 +219,7 @@ __device__ __forceinline__ uint4 pack8(const float (&a)[8]) {
 __global__ void __launch_bounds__(256) combine_kernel(const uint4* __restrict__ y, const int* __restrict__ copy_row, const float* __restrict__ w,
                                                       const uint4* __restrict__ residual, uint4* __restrict__ out, int T, int k, int vecs) {
   const long long n = static_cast<long long>(T) * vecs;
+  pdl_sync();
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int t = static_cast<int>(i / vecs), v = static_cast<int>(i - static_cast<long long>(t) * vecs);
     float acc[8];
@@ -314,19 +319,18 @@ RLB_API int rlb_moe_route_topk(const void* logits, long long ld, int T, int E, i
   const int warps = 8;
   const size_t smem = static_cast<size_t>(warps) * E * sizeof(float);
   if (smem > 48 * 1024) cudaFuncSetAttribute(route_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  route_topk_kernel<<<(T + warps - 1) / warps, warps * 32, smem, static_cast<cudaStream_t>(stream)>>>(
+  rlb_launch_pdl(route_topk_kernel, dim3((T + warps - 1) / warps), dim3(warps * 32), smem, static_cast<cudaStream_t>(stream), 
       static_cast<const __nv_bfloat16*>(logits), ld, T, E, k, renorm, out_w, out_idx);
   return static_cast<int>(cudaGetLastError());
 }
 
 // mpad: rows of the padded layout, a multiple of 128 and >= n_copies + El * 127 rounded up (worst case: all copies local).
-RLB_API int rlb_moe_decode_plan(const int* idx, int n_copies, int k, int e_lo, int El, int mpad, int* src_tok, int* copy_row,
+RLB_API int rlb_moe_decode_plan(const int* idx, int n_copies, int k, int e_lo, int El, int mpad, int pad, int* src_tok, int* copy_row,
                                 int* tile_expert, int* row0, int* rows, int* status, void* stream) {
-  if (n_copies <= 0 || n_copies > PLAN_MAX_COPIES || El < 1 || El > PLAN_MAX_EXPERTS || k < 1 || (mpad % 128) ||
-      mpad < n_copies + El * 127)
+  if (n_copies <= 0 || n_copies > PLAN_MAX_COPIES || El < 1 || El > PLAN_MAX_EXPERTS || k < 1 || pad < 1 || (mpad % pad) ||
+      mpad < n_copies + El * (pad - 1))
     return -2;
-  decode_plan_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(idx, n_copies, k, e_lo, El, mpad, src_tok, copy_row, tile_expert,
-                                                                         row0, rows, status);
+  rlb_launch_pdl(decode_plan_kernel, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream), idx, n_copies, k, e_lo, El, mpad, pad, src_tok, copy_row, tile_expert, row0, rows, status);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -336,8 +340,8 @@ RLB_API int rlb_moe_gather_rows(const void* x, long long x_stride_bytes, const i
   if ((row_bytes % 16) || (x_stride_bytes % 16) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return -2;
   int grid = (mpad + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
-  gather_rows_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint4*>(x), x_stride_bytes / 16, src_tok,
-                                                                           tile_expert, static_cast<uint4*>(out), mpad, row_bytes / 16);
+  rlb_launch_pdl(gather_rows_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), x_stride_bytes / 16, src_tok, tile_expert,
+                 static_cast<uint4*>(out), mpad, row_bytes / 16);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -349,8 +353,8 @@ RLB_API int rlb_moe_combine(const void* y, const int* copy_row, const float* w, 
   const long long n = static_cast<long long>(T) * (d / 8);
   int grid = static_cast<int>((n + 255) / 256);
   if (grid > 148 * 8) grid = 148 * 8;
-  combine_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint4*>(y), copy_row, w,
-                                                                       static_cast<const uint4*>(residual), static_cast<uint4*>(out), T, k, d / 8);
+  rlb_launch_pdl(combine_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(y), copy_row, w, static_cast<const uint4*>(residual),
+                 static_cast<uint4*>(out), T, k, d / 8);
   return static_cast<int>(cudaGetLastError());
 }
 

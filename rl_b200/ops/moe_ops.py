@@ -222,7 +222,8 @@ def expert_layer(x: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, residual, 
 
 # ------------------------------------------------------------------------------------------- small-token path (decode)
 register("rlb_moe_route_topk", [P, L, I, I, I, I, P, P, P])
-register("rlb_moe_decode_plan", [P, I, I, I, I, I, P, P, P, P, P, P, P])
+register("rlb_moe_decode_plan", [P, I, I, I, I, I, I, P, P, P, P, P, P, P])
+register("rlb_moe_skinny", [P, L, P, P, L, I, I, I, I, I, P, I, P, P])
 register("rlb_moe_gather_rows", [P, L, P, P, P, I, I, P])
 register("rlb_moe_combine", [P, P, P, P, P, I, I, I, P])
 
@@ -268,13 +269,13 @@ class SmallTokenMoE:
         self.wait_limit_s = wait_limit_s
         n_all = self.W * self.maxT
         assert n_all * top_k <= SMALL_MAX_COPIES and hidden % 8 == 0 and self.El <= 256 and top_k <= 16
-        self.max_mpad = self.mpad_for(self.maxT)
+        self.max_mpad = max(self.mpad_for(self.maxT), -(-(n_all * top_k + self.El * 127) // 128) * 128)
         i32 = dict(dtype=torch.int32, device=device)
         self.w = torch.empty((n_all, top_k), dtype=torch.float32, device=device)
         self.idx = torch.empty((n_all, top_k), **i32)
         self.src_tok = torch.empty(self.max_mpad, **i32)
         self.copy_row = torch.empty(n_all * top_k, **i32)
-        self.tile_expert = torch.empty(self.max_mpad // 128, **i32)
+        self.tile_expert = torch.empty(self.max_mpad // 32, **i32)
         self.row0 = torch.empty(self.El, **i32)
         self.rows = torch.empty(self.El, **i32)
         self.xp = torch.empty((self.max_mpad, hidden), dtype=BF16, device=device)
@@ -303,8 +304,15 @@ class SmallTokenMoE:
             self.scratch = torch.zeros(2, dtype=torch.int32, device=device)
             self.x_all = torch.empty((n_all, hidden), dtype=BF16, device=device)
 
+    def tile_rows(self, T: int) -> int:
+        """Rows of a tile. Few tokens per expert: 32 or 64, the columns of the weight-streaming products (twice the mean load, so that nearly every
+        expert's weights are read once); from 32 on the 128-row tiles of the grouped GEMM, which then read more weights than padding."""
+        mean = self.W * T * self.k / self.E
+        return 32 if mean <= 16 else 64 if mean <= 32 else 128
+
     def mpad_for(self, T: int) -> int:
-        return -(-(self.W * T * self.k + self.El * 127) // 128) * 128
+        pad = self.tile_rows(T)
+        return -(-(self.W * T * self.k + self.El * (pad - 1)) // pad) * pad
 
     def fits(self, T: int) -> bool:
         return 0 < T <= self.maxT
@@ -330,16 +338,22 @@ class SmallTokenMoE:
         logits = F.linear(xa, router)
         wts, idx = self.w[:n_all], self.idx[:n_all]
         call("rlb_moe_route_topk", ptr(logits), logits.stride(0), n_all, self.E, k, int(renorm), ptr(wts), ptr(idx), st)
-        mpad = self.mpad_for(T)
-        call("rlb_moe_decode_plan", ptr(idx), n_all * k, k, self.e_lo, self.El, mpad, ptr(self.src_tok), ptr(self.copy_row),
+        mpad, pad = self.mpad_for(T), self.tile_rows(T)
+        call("rlb_moe_decode_plan", ptr(idx), n_all * k, k, self.e_lo, self.El, mpad, pad, ptr(self.src_tok), ptr(self.copy_row),
              ptr(self.tile_expert), ptr(self.row0), ptr(self.rows), status, st)
-        xp, h, y = self.xp[:mpad], self.h[:mpad], self.y[:mpad]
-        call("rlb_moe_gather_rows", ptr(xa), xa.stride(0) * 2, ptr(self.src_tok), ptr(self.tile_expert), ptr(xp), mpad, d * 2, st)
-        call("rlb_gemm_grouped_rows", ptr(xp), xp.stride(0), ptr(gate_up), 0, ptr(h), h.stride(0), mpad, 2 * self.f, d, self.El,
-             ptr(self.tile_expert), 0, status, st)
-        a = F.swiglu(h)
-        call("rlb_gemm_grouped_rows", ptr(a), a.stride(0), ptr(down), 0, ptr(y), y.stride(0), mpad, d, self.f, self.El,
-             ptr(self.tile_expert), 0, status, st)
+        xp, y = self.xp[:mpad], self.y[:mpad]
+        call("rlb_moe_gather_rows", ptr(xa), xa.stride(0) * 2, ptr(self.src_tok), ptr(self.tile_expert) if pad == 128 else None, ptr(xp), mpad, d * 2, st)
+        if pad < 128:
+            a = self.h.view(-1)[: mpad * self.f].view(mpad, self.f)
+            call("rlb_moe_skinny", ptr(xp), xp.stride(0), ptr(gate_up), ptr(a), a.stride(0), mpad, pad, self.f, d, self.El, ptr(self.tile_expert), 1, status, st)
+            call("rlb_moe_skinny", ptr(a), a.stride(0), ptr(down), ptr(y), y.stride(0), mpad, pad, d, self.f, self.El, ptr(self.tile_expert), 0, status, st)
+        else:
+            h = self.h[:mpad]
+            call("rlb_gemm_grouped_rows", ptr(xp), xp.stride(0), ptr(gate_up), 0, ptr(h), h.stride(0), mpad, 2 * self.f, d, self.El,
+                 ptr(self.tile_expert), 0, status, st)
+            a = F.swiglu(h)
+            call("rlb_gemm_grouped_rows", ptr(a), a.stride(0), ptr(down), 0, ptr(y), y.stride(0), mpad, d, self.f, self.El,
+                 ptr(self.tile_expert), 0, status, st)
         out = torch.empty((T, d), dtype=BF16, device=x.device)
         res = ptr(residual.contiguous()) if residual is not None else None
         if W > 1:

@@ -210,3 +210,36 @@ def test_expert_layer(native_lib, T, E, k, skew, residual):
     if residual:
         assert torch.equal(res.grad, up)
     assert gu.grad[counts == 0].abs().sum() == 0 and dn.grad is None
+
+
+@pytest.mark.parametrize("T,E,k,load", [(1, 8, 2, 32), (33, 16, 4, 32), (126, 64, 8, 32), (60, 12, 4, 64), (64, 4, 2, 64), (128, 4, 2, 128)])
+@pytest.mark.parametrize("one", [False, True])
+def test_few_token_layer(native_lib, T, E, k, load, one):
+    """Every tile size, experts without tokens, one expert with all of them (several tiles), widths that cut the last weight tile. Against float64:
+    bf16 products, a unit rounded to bf16, weighted rows rounded to bf16: 1e-2 of the norm."""
+    from rl_b200.ops import moe_ops as M
+    from rl_b200.ops.lib import check_status
+
+    g = torch.Generator("cuda").manual_seed(T + E)
+    d, f = 192, 64
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    x, res, router = r(T, d).bfloat16(), r(T, d).bfloat16(), r(E, d).bfloat16()
+    if one:
+        x[:, 0], router[1] = 40.0, 0
+        router[1, 0] = 1.0
+    gu, dn = (0.2 * r(E, 2 * f, d)).bfloat16(), (0.2 * r(E, d, f)).bfloat16()
+    ws = M.SmallTokenMoE(d, f, E, k, None, T, x.device)
+    assert ws.tile_rows(T) == load
+    for _ in range(2):      # the workspace is used again
+        out, idx = ws.forward(x, res, router, gu, dn, True)
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    W, ref = ws.w[:T].double(), res.double()
+    for e in range(E):
+        t, j = (idx == e).nonzero(as_tuple=True)
+        if len(t):
+            a, b = (x[t].double() @ gu[e].double().T).chunk(2, -1)
+            ref = ref.index_add(0, t, (torch.nn.functional.silu(a) * b) @ dn[e].double().T * W[t, j, None])
+    assert (out.double() - ref).norm() <= 1e-2 * ref.norm()
+    if one:
+        assert bool((idx == 1).any(-1).all())
