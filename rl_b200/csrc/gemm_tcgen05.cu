@@ -33,6 +33,7 @@
 // Replaces the cuBLAS calls behind nn.Linear and the chunked hidden->logprob path of the reference
 // (nemo_rl/distributed/model_utils.py:2137-2316).
 #include "common.cuh"
+#include "out_piece.cuh"
 
 #include <cstdlib>
 
@@ -53,8 +54,6 @@ constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = CTA_M * BK * 2;  // 16 KB
 constexpr int B_STAGE_BYTES = CTA_N * BK * 2;  // 16 KB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-constexpr int OUT_COLS = 64;                                  // columns that an epilogue warp passes through shared memory at a time
-constexpr int OUT_WARP_BYTES = 32 * OUT_COLS * 4;
 constexpr int SMEM_BARRIER_BYTES = 256;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * OUT_WARP_BYTES + SMEM_BARRIER_BYTES + 1024;  // +1024: manual alignment
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
@@ -94,89 +93,6 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
   const int in_group = tile - group * per_group;
   m_blk = first_m + in_group % rows;
   n_blk = in_group / rows;
-}
-
-// One 32-row x 64-column piece of fp32 values on its way out: lanes put their rows down, then the warp reads whole rows, so that every
-// access to global memory covers full 32-byte sectors (rows written by single lanes made the weight gradient's fp32 read-add-write
-// as long as its main loop). 16-byte chunks are permuted within the row so that both directions are free of bank conflicts.
-__device__ __forceinline__ uint32_t out_chunk(uint32_t base, int r, int q) { return base + r * (OUT_COLS * 4) + ((q ^ (r & 7)) << 4); }
-__device__ __forceinline__ void st_shared_f4(uint32_t addr, float a, float b, float c, float d) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ void add_bf16x4(float4& v, uint32_t lo, uint32_t hi) {
-  const float2 a = unpack_bf16x2(lo), b = unpack_bf16x2(hi);
-  v.x += a.x; v.y += a.y; v.z += b.x; v.w += b.y;
-}
-
-// Writes the staged piece: rows row0.., columns col.. of C. Old values (accumulation) and the residual are fetched by the caller's
-// warp in the same layout before the piece is complete.
-__device__ __forceinline__ void store_piece(const EpiParams& ep, uint32_t buf, int row0, int col, int M, int N, int lane) {
-  if (ep.out_fp32) {
-    const int q = lane & 15, c = col + q * 4;
-    const bool in = c < N;                 // N is a multiple of 8
-    float4 old[16];
-    float* dst = reinterpret_cast<float*>(ep.C) + static_cast<long long>(row0 + (lane >> 4)) * ep.ldc + c;
-    if (ep.accumulate) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        old[i] = in && row0 + 2 * i + (lane >> 4) < M ? *reinterpret_cast<const float4*>(dst + 2 * i * ep.ldc) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (ep.bias && in) bias = make_float4(ep.bias[c], ep.bias[c + 1], ep.bias[c + 2], ep.bias[c + 3]);
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int r = 2 * i + (lane >> 4);
-      float4 v = ld_shared_f4(out_chunk(buf, r, q));
-      if (!in || row0 + r >= M) continue;
-      v.x += bias.x; v.y += bias.y; v.z += bias.z; v.w += bias.w;
-      if (ep.residual) {
-        const uint2 o = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(ep.residual) + static_cast<long long>(row0 + r) * ep.ldr + c);
-        add_bf16x4(v, o.x, o.y);
-      }
-      if (ep.accumulate) { v.x += old[i].x; v.y += old[i].y; v.z += old[i].z; v.w += old[i].w; }
-      *reinterpret_cast<float4*>(dst + 2 * i * ep.ldc) = v;
-    }
-  } else {
-    const int q = (lane & 7) * 2, c = col + q * 4;
-    const bool in = c < N;
-    uint4 res[8], old[8];
-    const __nv_bfloat16* rsd = reinterpret_cast<const __nv_bfloat16*>(ep.residual) + static_cast<long long>(row0 + (lane >> 3)) * ep.ldr + c;
-    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(ep.C) + static_cast<long long>(row0 + (lane >> 3)) * ep.ldc + c;
-    if (ep.residual) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        res[i] = in && row0 + 4 * i + (lane >> 3) < M ? *reinterpret_cast<const uint4*>(rsd + 4 * i * ep.ldr) : make_uint4(0, 0, 0, 0);
-    }
-    if (ep.accumulate) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        old[i] = in && row0 + 4 * i + (lane >> 3) < M ? *reinterpret_cast<const uint4*>(dst + 4 * i * ep.ldc) : make_uint4(0, 0, 0, 0);
-    }
-    float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = b0;
-    if (ep.bias && in) {
-      b0 = make_float4(ep.bias[c], ep.bias[c + 1], ep.bias[c + 2], ep.bias[c + 3]);
-      b1 = make_float4(ep.bias[c + 4], ep.bias[c + 5], ep.bias[c + 6], ep.bias[c + 7]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = 4 * i + (lane >> 3);
-      float4 u = ld_shared_f4(out_chunk(buf, r, q)), v = ld_shared_f4(out_chunk(buf, r, q + 1));
-      if (!in || row0 + r >= M) continue;
-      u.x += b0.x; u.y += b0.y; u.z += b0.z; u.w += b0.w;
-      v.x += b1.x; v.y += b1.y; v.z += b1.z; v.w += b1.w;
-      if (ep.residual) { add_bf16x4(u, res[i].x, res[i].y); add_bf16x4(v, res[i].z, res[i].w); }
-      if (ep.accumulate) { add_bf16x4(u, old[i].x, old[i].y); add_bf16x4(v, old[i].z, old[i].w); }
-      *reinterpret_cast<uint4*>(dst + 4 * i * ep.ldc) = make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-    }
-  }
-  __syncwarp();      // the buffer may be written again
 }
 
 template <bool A_MN, bool B_MN, int EPI>
