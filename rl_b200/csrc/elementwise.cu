@@ -77,6 +77,124 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
   }
 }
 
+// The same without a residual for many rows: one warp per row, which stays in registers between the two passes, all its loads in flight and no
+// barrier. NV: pieces of 8 elements per lane. From 8 rows per SM on: with fewer, several warps per row are sooner done. 20480 rows of 4096:
+// 99 us with a CTA per row, now 69 us (4.9 TB/s).
+template <int NV>
+__global__ void __launch_bounds__(256, 2) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                                                           float* __restrict__ rstd_out, long long rows, int d, long long x_stride, long long y_stride, float eps) {
+  pdl_sync();
+  const int lane = threadIdx.x & 31;
+  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const __nv_bfloat16* xr = x + row * x_stride;
+  __nv_bfloat16* yr = y + row * y_stride;
+  BF8 v[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = (lane + 32 * j) * 8;
+    if (i < d) v[j] = *reinterpret_cast<const BF8*>(xr + i);
+    else v[j].w[0] = v[j].w[1] = v[j].w[2] = v[j].w[3] = 0u;
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 f = unpack_bf16x2(v[j].w[k]);
+      t += f.x * f.x + f.y * f.y;
+    }
+    ss += t;
+  }
+  ss = warp_sum(ss);
+  const float rstd = rsqrtf(ss / d + eps);
+  if (rstd_out && lane == 0) rstd_out[row] = rstd;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = (lane + 32 * j) * 8;
+    if (i < d) {
+      float g[8];
+      load8(w + i, g);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = unpack_bf16x2(v[j].w[k]);
+        v[j].w[k] = pack_bf16x2(f.x * rstd * g[2 * k], f.y * rstd * g[2 * k + 1]);
+      }
+      *reinterpret_cast<BF8*>(yr + i) = v[j];
+    }
+  }
+}
+
+// Gradient for d up to 8 columns per thread: a CTA takes four rows at a time, so that a barrier and a trip to memory serve four of them, and keeps
+// them in registers. 4000 rows of 2048: 28 us with one row at a time, now 19 us.
+constexpr int NORM_BWD_ROWS = 4;
+__global__ void __launch_bounds__(512) rmsnorm_bwd4_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                           const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial, int rows, int d,
+                                                           long long x_stride, long long dy_stride, int add_to_dx) {
+  __shared__ float red[2][NORM_BWD_ROWS][16];
+  const int i = threadIdx.x * 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const bool in = i < d;
+  float fw[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (in) load8(w + i, fw);
+  int turn = 0;
+  for (long long row0 = blockIdx.x; row0 < rows; row0 += static_cast<long long>(gridDim.x) * NORM_BWD_ROWS, turn ^= 1) {
+    BF8 vx[NORM_BWD_ROWS], vd[NORM_BWD_ROWS];
+    float rs[NORM_BWD_ROWS];
+#pragma unroll
+    for (int q = 0; q < NORM_BWD_ROWS; ++q) {
+      const long long row = row0 + static_cast<long long>(q) * gridDim.x;
+      const bool ok = in && row < rows;
+      rs[q] = row < rows ? rstd[row] : 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) vx[q].w[k] = vd[q].w[k] = 0u;
+      if (ok) {
+        vx[q] = *reinterpret_cast<const BF8*>(x + row * x_stride + i);
+        vd[q] = *reinterpret_cast<const BF8*>(dy + row * dy_stride + i);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NORM_BWD_ROWS; ++q) {
+      float dot = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 a = unpack_bf16x2(vx[q].w[k]), b = unpack_bf16x2(vd[q].w[k]);
+        dot += b.x * fw[2 * k] * a.x + b.y * fw[2 * k + 1] * a.y;
+        acc[2 * k] += b.x * a.x * rs[q];
+        acc[2 * k + 1] += b.y * a.y * rs[q];
+      }
+      dot = warp_sum(dot);
+      if (lane == 0) red[turn][q][warp] = dot;
+    }
+    __syncthreads();      // (the other half of `red` is written next: everyone has read it by the next barrier but one)
+#pragma unroll
+    for (int q = 0; q < NORM_BWD_ROWS; ++q) {
+      const long long row = row0 + static_cast<long long>(q) * gridDim.x;
+      float dot = 0.f;
+      for (int t = 0; t < warps; ++t) dot += red[turn][q][t];
+      const float c = dot * rs[q] * rs[q] / d;
+      if (in && row < rows) {
+        __nv_bfloat16* dst = dx + row * static_cast<long long>(d) + i;
+        float o[8];
+        if (add_to_dx) load8(dst, o);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 a = unpack_bf16x2(vx[q].w[k]), b = unpack_bf16x2(vd[q].w[k]);
+          const float v0 = rs[q] * (b.x * fw[2 * k] - a.x * c), v1 = rs[q] * (b.y * fw[2 * k + 1] - a.y * c);
+          o[2 * k] = add_to_dx ? o[2 * k] + v0 : v0;
+          o[2 * k + 1] = add_to_dx ? o[2 * k + 1] + v1 : v1;
+        }
+        store8(dst, o);
+      }
+    }
+  }
+  if (in) {
+    float* p = dw_partial + static_cast<long long>(blockIdx.x) * d + i;
+    *reinterpret_cast<float4*>(p) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  }
+}
+
 // dx = rstd * (dy*w - x * rstd^2 * mean(dy*w*x)); dw partial per CTA (rows strided over the grid).
 __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
@@ -807,6 +925,11 @@ RLB_API int rlb_rmsnorm_fwd(const void* x, const void* res, const void* w, void*
                             void* stream) {
   if (rows <= 0) return 0;
   if (d % 8 || x_stride % 8 || y_stride % 8) return -2;
+  if (!res && rows >= 148 * 8 && d <= 5120) {
+    auto kern = d <= 1024 ? rmsnorm_rows_kernel<4> : d <= 2048 ? rmsnorm_rows_kernel<8> : d <= 4096 ? rmsnorm_rows_kernel<16> : rmsnorm_rows_kernel<20>;
+    rlb_launch_pdl(kern, dim3(static_cast<unsigned>((rows + 7) / 8)), dim3(256), 0, S(stream), CBF(x), CBF(w), BF(y), rstd, rows, d, x_stride, y_stride, eps);
+    return static_cast<int>(cudaGetLastError());
+  }
   rlb_launch_pdl(rmsnorm_fwd_kernel, dim3(static_cast<unsigned>(rows)), dim3(rms_threads(d)), 0, S(stream), 
       CBF(x), CBF(res), CBF(w), BF(y), BF(res_out), rstd, d, x_stride, y_stride, eps);
   return static_cast<int>(cudaGetLastError());
@@ -825,8 +948,11 @@ RLB_API int rlb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   const int threads = rms_threads(d);
   if (d > threads * 8 * 8) return -4;
   const int parts = rlb_rmsnorm_bwd_parts(rows);
-  rmsnorm_bwd_kernel<<<parts, threads, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial,
-                                                       static_cast<int>(rows), d, x_stride, dy_stride, add_to_dx);
+  if (d <= threads * 8)
+    rmsnorm_bwd4_kernel<<<parts, threads, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial, static_cast<int>(rows), d, x_stride, dy_stride, add_to_dx);
+  else
+    rmsnorm_bwd_kernel<<<parts, threads, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial,
+                                                         static_cast<int>(rows), d, x_stride, dy_stride, add_to_dx);
   colsum_kernel<<<(d + 255) / 256, 256, 0, S(stream)>>>(dw_partial, parts, d, dw_f32, BF(dw_bf16), dw_accumulate);
   return static_cast<int>(cudaGetLastError());
 }

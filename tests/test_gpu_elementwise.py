@@ -486,3 +486,36 @@ def test_qk_rmsnorm(native_lib, D, T, Hq, Hkv):
     with torch.no_grad():
         z = x.detach().clone()
         assert F.qk_rmsnorm(z, wq, wk, Hq, Hkv, D, 1e-6) is z and torch.equal(z, y)
+
+
+@pytest.mark.parametrize("d", [8, 512, 1032, 2048, 4096, 5120, 5128])      # one register count each, cut rows of pieces, beyond the last
+@pytest.mark.parametrize("rows", [3, 1184, 1187])                           # a CTA per row; a warp per row, a cut last CTA
+def test_rmsnorm_many_rows(native_lib, d, rows):
+    """Values, statistics and both gradients against float64: one bf16 rounding of a result (2^-8), a few in the gradient's two terms."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(d + rows)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    wide = r(rows, d + 8).bfloat16()
+    x, w, up = wide[:, :d].requires_grad_(), (1 + 0.3 * r(d)).bfloat16().requires_grad_(), r(rows, d).bfloat16()
+    y = F.rmsnorm(x, w, 1e-6)
+    y.backward(up)
+    X, W = (t.detach().double().requires_grad_() for t in (x, w))
+    ref = X * torch.rsqrt(X.pow(2).mean(-1, keepdim=True) + 1e-6) * W
+    ref.backward(up.double())
+    near = lambda a, b, t: (a.double() - b).norm() <= t * b.norm()      # noqa: E731
+    assert near(y, ref, 2.0 ** -8) and near(x.grad, X.grad, 2.0 ** -7) and near(w.grad, W.grad, 2.0 ** -7)
+
+
+@pytest.mark.parametrize("M", [1, 31, 33, 300])
+@pytest.mark.parametrize("V", [8, 256, 1800, 2304])                         # fewer parts than warps, one, as many, one more
+def test_logprob_combine(native_lib, M, V):
+    """Log-probability and entropy of the fused head against float64 on the same bf16 operands (fp32 logits of size 8: 1e-5)."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(M + V)
+    h, w = (torch.randn(n, 64, generator=g, device="cuda").bfloat16() for n in (M, V))
+    t = torch.randint(0, V, (M,), generator=g, device="cuda")
+    lp, ent = F.lm_head_logprobs(h, w, t, 1.0, True)
+    z = torch.log_softmax(h.double() @ w.double().T, -1)
+    assert (lp.double() - z.gather(1, t[:, None])[:, 0]).abs().max() < 1e-4 and (ent.double() + (z.exp() * z).sum(-1)).abs().max() < 1e-3

@@ -212,7 +212,7 @@ def test_expert_layer(native_lib, T, E, k, skew, residual):
     assert gu.grad[counts == 0].abs().sum() == 0 and dn.grad is None
 
 
-@pytest.mark.parametrize("T,E,k,load", [(1, 8, 2, 32), (33, 16, 4, 32), (126, 64, 8, 32), (60, 12, 4, 64), (64, 4, 2, 64), (128, 4, 2, 128)])
+@pytest.mark.parametrize("T,E,k,load", [(1, 8, 2, 32), (33, 16, 4, 32), (126, 64, 8, 32), (60, 16, 6, 64), (64, 8, 4, 64), (128, 8, 4, 128)])
 @pytest.mark.parametrize("one", [False, True])
 def test_few_token_layer(native_lib, T, E, k, load, one):
     """Every tile size, experts without tokens, one expert with all of them (several tiles), widths that cut the last weight tile. Against float64:
@@ -225,7 +225,7 @@ def test_few_token_layer(native_lib, T, E, k, load, one):
     r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
     x, res, router = r(T, d).bfloat16(), r(T, d).bfloat16(), r(E, d).bfloat16()
     if one:
-        x[:, 0], router[1] = 40.0, 0
+        x[:, 0], router[:, 0], router[1] = 100.0, 0, 0      # expert 1 scores 100, the others some 14 (sigma)
         router[1, 0] = 1.0
     gu, dn = (0.2 * r(E, 2 * f, d)).bfloat16(), (0.2 * r(E, d, f)).bfloat16()
     ws = M.SmallTokenMoE(d, f, E, k, None, T, x.device)
