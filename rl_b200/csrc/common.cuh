@@ -412,12 +412,10 @@ __device__ __forceinline__ float warp_max(float v) {
 // tanh that keeps its relative accuracy near zero whatever math mode the file is compiled with: the odd Taylor series below 1/4
 // (remainder under 1e-8 relative), 1 - 2 / (1 + exp(2|x|)) above.
 __device__ __forceinline__ float tanh_acc(float x) {
-  const float a = fabsf(x);
-  if (a < 0.25f) {
-    const float q = x * x;
-    return x * (1.f + q * (-1.f / 3.f + q * (2.f / 15.f + q * (-17.f / 315.f + q * (62.f / 2835.f)))));
-  }
-  return copysignf(1.f - 2.f / (1.f + expf(2.f * a)), x);
+  const float a = fabsf(x), q = x * x;
+  const float near = x * (1.f + q * (-1.f / 3.f + q * (2.f / 15.f + q * (-17.f / 315.f + q * (62.f / 2835.f)))));
+  const float far = copysignf(1.f - 2.f / (1.f + expf(2.f * a)), x);      // (both, so that a row of values stays one straight piece of code)
+  return a < 0.25f ? near : far;
 }
 
 // What follows a product in a layer-list model. LIN_GLU, LIN_SILU: columns 2i and 2i + 1 are gate and up of a gated unit (clamped, or silu

@@ -95,6 +95,15 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
   n_blk = in_group / rows;
 }
 
+__device__ __forceinline__ void unpack8(const uint4 r, float (&v)[8]) {
+  const float2 a = unpack_bf16x2(r.x), b = unpack_bf16x2(r.y), c = unpack_bf16x2(r.z), d = unpack_bf16x2(r.w);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
+}
+__device__ __forceinline__ float4 square_relu4(float4 v) {
+  v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f);
+  return make_float4(v.x * v.x, v.y * v.y, v.z * v.z, v.w * v.w);
+}
+
 template <bool A_MN, bool B_MN, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -269,24 +278,86 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           store_piece(ep, buf, row0, col0 + c * OUT_COLS, M, N, lane);
         }
       } else if (EPI == EPI_LAYER) {
-        const float alpha = ep.layer.x ? __bfloat162float(*ep.layer.alpha) : 0.f;
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + c * 32, r);
+        // Through shared memory like store_piece. With one row to a lane the epilogue was longer than the main loop of short contractions and
+        // than the fp32 stream of long ones: 11200 x 11264 x 2048 with the squared ReLU 452 -> 350 us (plain store 358), 11200 x 2048 x
+        // 10240 onto the stream 404 -> 337 (with embeddings and step 453 -> 344), 700 rows of it 130 -> 88. The norm's loop is kept small:
+        // unrolled over the rows, with branches in tanh, the same layout was slower than a row to a lane.
+        const LayerEpilogue& le = ep.layer;
+        const float alpha = le.x ? __bfloat162float(*le.alpha) : 0.f;
+        const int q = (lane & 7) * 2, r0 = lane >> 3;      // eight lanes a row, eight columns each
+        for (int c = 0; c < BN / OUT_COLS && col0 + c * OUT_COLS < N; ++c) {
+          uint32_t t[64];
+          tmem_ld_32x32b_x32(taddr + c * OUT_COLS, *reinterpret_cast<uint32_t(*)[32]>(t));
+          tmem_ld_32x32b_x32(taddr + c * OUT_COLS + 32, *reinterpret_cast<uint32_t(*)[32]>(t + 32));
           tmem_ld_wait();
-          const int col = col0 + c * 32;
-          if (!row_ok || col >= N) continue;
-          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(ep.C) + static_cast<long long>(row) * ep.ldc + col;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (col + q * 8 < N) {
-              const float4 a = layer_epilogue4(ep.layer, make_float4(__uint_as_float(r[q * 8]), __uint_as_float(r[q * 8 + 1]),
-                                                                     __uint_as_float(r[q * 8 + 2]), __uint_as_float(r[q * 8 + 3])), row, col + q * 8, alpha);
-              const float4 b = layer_epilogue4(ep.layer, make_float4(__uint_as_float(r[q * 8 + 4]), __uint_as_float(r[q * 8 + 5]),
-                                                                     __uint_as_float(r[q * 8 + 6]), __uint_as_float(r[q * 8 + 7])), row, col + q * 8 + 4, alpha);
-              *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
+          for (int i = 0; i < OUT_COLS / 4; ++i)
+            st_shared_f4(out_chunk(buf, lane, i), __uint_as_float(t[4 * i]), __uint_as_float(t[4 * i + 1]), __uint_as_float(t[4 * i + 2]), __uint_as_float(t[4 * i + 3]));
+          const int col = col0 + c * OUT_COLS + q * 4;
+          const bool in = col < N;
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(ep.C) + static_cast<long long>(row0 + r0) * ep.ldc + col;
+          __syncwarp();
+          if (!le.x) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int r = 4 * i + r0;
+              float4 u = ld_shared_f4(out_chunk(buf, r, q)), v = ld_shared_f4(out_chunk(buf, r, q + 1));
+              if (!in || row0 + r >= M) continue;
+              if (col >= le.act_from) { u = square_relu4(u); v = square_relu4(v); }      // act_from is a multiple of 8
+              *reinterpret_cast<uint4*>(dst + 4 * i * ep.ldc) = make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+            }
+          } else {
+            // The residual stream of four rows at a time is fetched before any of it is written; its new values go back into the
+            // piece, and the norm follows in a loop that stays small.
+            float step[8] = {}, nw[8] = {}, nb[8] = {};
+            if (in) {
+              if (le.step) unpack8(*reinterpret_cast<const uint4*>(le.step + col), step);
+              unpack8(*reinterpret_cast<const uint4*>(le.nw + col), nw);
+              unpack8(*reinterpret_cast<const uint4*>(le.nb + col), nb);
+            }
+            float* xp = le.x + static_cast<long long>(row0 + r0) * le.ldx + col;
+            const float* e = le.e ? le.e + static_cast<long long>(row0 + r0) * le.ldx + col : nullptr;
+#pragma unroll 1
+            for (int h = 0; h < 8; h += 4) {
+              float4 old[4][2], ev[4][2];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const long long off = 4 * (h + i) * le.ldx;
+                const bool ok_x = in && row0 + 4 * (h + i) + r0 < M, ok_e = ok_x && e;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  old[i][k] = ok_x ? *reinterpret_cast<const float4*>(xp + off + 4 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                  ev[i][k] = ok_e ? *reinterpret_cast<const float4*>(e + off + 4 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int r = 4 * (h + i) + r0;
+                const bool ok_x = in && row0 + r < M;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  float4 u = ld_shared_f4(out_chunk(buf, r, q + k));
+                  u.x = u.x + old[i][k].x + ev[i][k].x + step[4 * k];
+                  u.y = u.y + old[i][k].y + ev[i][k].y + step[4 * k + 1];
+                  u.z = u.z + old[i][k].z + ev[i][k].z + step[4 * k + 2];
+                  u.w = u.w + old[i][k].w + ev[i][k].w + step[4 * k + 3];
+                  st_shared_f4(out_chunk(buf, r, q + k), u.x, u.y, u.z, u.w);      // (read again by this lane alone)
+                  if (ok_x) *reinterpret_cast<float4*>(xp + 4 * (h + i) * le.ldx + 4 * k) = u;
+                }
+              }
+            }
+#pragma unroll 1
+            for (int i = 0; i < 8; ++i) {
+              const int r = 4 * i + r0;
+              const float4 u = ld_shared_f4(out_chunk(buf, r, q)), v = ld_shared_f4(out_chunk(buf, r, q + 1));
+              float t8[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int k = 0; k < 8; ++k) t8[k] = tanh_acc(alpha * t8[k]) * nw[k] + nb[k];
+              if (in && row0 + r < M)
+                *reinterpret_cast<uint4*>(dst + 4 * i * ep.ldc) = make_uint4(pack_bf16x2(t8[0], t8[1]), pack_bf16x2(t8[2], t8[3]), pack_bf16x2(t8[4], t8[5]), pack_bf16x2(t8[6], t8[7]));
             }
           }
+          __syncwarp();      // the buffer may be written again
         }
       } else if (EPI == EPI_LINEAR) {
         const LinearEpi& le = ep.layer.lin;

@@ -226,6 +226,12 @@ def test_products(M, N, K, act, dt):
             assert rel(h, torch.tanh(n.alpha.float() * want) * n.weight.float() + n.bias.float()) < tol
 
 
+@pytest.mark.parametrize("M,N,K,act", [(257, 8, 64, 0), (511, 72, 72, 40), (513, 264, 136, 128), (300, 320, 64, 1000)])
+def test_tiled_product_edges(M, N, K, act):
+    """The tiled kernel's pieces of 32 rows and 64 columns: one row or eight columns over, the relu's border inside a piece, at its edge and outside."""
+    test_products(M, N, K, act, BF)
+
+
 def test_presets_generate_with_captured_steps():
     m = build_model(preset("tiny-gadarax"), device=DEV, dtype=BF, seed=1)
     prompts = [G.tokens({"vocab": 264}, n, n) for n in (5, 70, 129, 1)]
