@@ -1,5 +1,5 @@
 // Mixture-of-experts layer for small token counts (decode steps, short prefills) on sm_100a: the whole routing /
-// layout / combine chain as five small kernels around the two grouped GEMMs, with fixed shapes and no host visit, so a
+// layout / combine chain as five small kernels around the experts' products (moe_skinny.cu, or the grouped GEMM), with fixed shapes and no host visit, so a
 // decode step of an MoE model can be captured in a CUDA graph.
 //
 //   route_topk     one warp per token: soft-max over the router logits, top-k (lowest index wins ties), optional

@@ -5,6 +5,7 @@
 synchronisation: the per-expert segments are re-laid out with zero padding to multiples of 128 rows, so each 128-row tile
 of the grouped GEMM belongs to one expert, and the tile -> expert table is computed on the device from ``counts``.
 Weight gradients use the reduction form of the grouped GEMM and accumulate straight into the stacked gradient buffers.
+``expert_layer`` is the whole layer on one rank, from tokens to tokens, with the rows planned, gathered and combined by kernels of its own.
 On CPU (and for dtypes other than bf16) the per-expert loop of plain linears is used.
 """
 
@@ -251,7 +252,7 @@ def route_topk(logits: torch.Tensor, k: int, renorm: bool, out_w=None, out_idx=N
 class SmallTokenMoE:
     """Buffers and launchers of the few-token MoE layer (rl_b200/csrc/moe_decode.cu): gather the tokens of all expert-
     parallel ranks, route them identically everywhere, run the local experts' grouped MLP over the copies routed to them
-    and reduce the partial sums to the tokens' owners. Nine launches per layer, fixed shapes, no host visit: a decode
+    and reduce the partial sums to the tokens' owners. Seven to nine launches per layer, fixed shapes, no host visit: a decode
     step that contains it can be captured in a CUDA graph. One instance serves all layers of a model.
 
     With ``ep.world > 1`` every rank of the group must call :meth:`forward` with the same number of tokens (the generation
