@@ -464,19 +464,16 @@ struct LayerEpilogue {
   int act_from;
   LinearEpi lin;
 };
-// Four consecutive columns of one row (col a multiple of 4). Gated units: the two outputs are in .x and .y.
-__device__ __forceinline__ float4 layer_epilogue4(const LayerEpilogue& le, float4 v, long long row, int col, float alpha) {
+// Four consecutive columns of one row (col a multiple of 4). Gated units: the two outputs are in .x and .y. `old`, `ev`: these columns of x and e.
+__device__ __forceinline__ float4 layer_epilogue4(const LayerEpilogue& le, float4 v, long long row, int col, float alpha, float4 old, float4 ev) {
   if (le.lin.bias) {
     const uint2 bv = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(le.lin.bias) + col);
     const float2 b0 = unpack_bf16x2(bv.x), b1 = unpack_bf16x2(bv.y);
     v.x += b0.x; v.y += b0.y; v.z += b1.x; v.w += b1.y;
   }
   if (le.x) {
-    float4* xp = reinterpret_cast<float4*>(le.x + row * le.ldx + col);
-    const float4 old = *xp;
     v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
     if (le.e) {
-      const float4 ev = *reinterpret_cast<const float4*>(le.e + row * le.ldx + col);
       v.x += ev.x; v.y += ev.y; v.z += ev.z; v.w += ev.w;
     }
     if (le.step) {
@@ -484,7 +481,7 @@ __device__ __forceinline__ float4 layer_epilogue4(const LayerEpilogue& le, float
       const float2 s0 = unpack_bf16x2(sv.x), s1 = unpack_bf16x2(sv.y);
       v.x += s0.x; v.y += s0.y; v.z += s1.x; v.w += s1.y;
     }
-    *xp = v;
+    *reinterpret_cast<float4*>(le.x + row * le.ldx + col) = v;
     const uint2 wv = *reinterpret_cast<const uint2*>(le.nw + col), bv = *reinterpret_cast<const uint2*>(le.nb + col);
     const float2 w0 = unpack_bf16x2(wv.x), w1 = unpack_bf16x2(wv.y), b0 = unpack_bf16x2(bv.x), b1 = unpack_bf16x2(bv.y);
     v.x = tanh_acc(alpha * v.x) * w0.x + b0.x;
