@@ -13,6 +13,7 @@ import argparse
 import concurrent.futures as cf
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -48,7 +49,10 @@ def sources() -> list[Path]:
 
 def _digest(path: Path, flags: list[str]) -> str:
     h = hashlib.sha256()
-    h.update(path.read_bytes())
+    text = path.read_bytes()
+    h.update(text)
+    for inc in re.findall(rb'#include "(\w+\.cu)"', text):      # one source compiled twice, for another head dimension
+        h.update((path.parent / inc.decode()).read_bytes())
     for hdr in sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")):
         h.update(hdr.read_bytes())
     h.update(" ".join(flags).encode())

@@ -124,3 +124,14 @@ def test_flops_formulas_per_architecture():
     mc = ModelConfig(model_type="llama", vocab_size=32, hidden_size=8, intermediate_size=16, num_hidden_layers=3, num_attention_heads=2,
                      num_key_value_heads=1, head_dim=4)
     assert FL.transformer_flops(mc, 4, 4, backward=False) == pytest.approx(FL.model_flops(llama, 4, backward=False))
+
+
+def test_native_build_sees_included_sources(tmp_path):
+    """A source that another one includes (the head-dimension-64 instantiations) is part of what that one was built from."""
+    from rl_b200.csrc.build import _digest
+
+    (tmp_path / "a.cu").write_text("int a;\n")
+    (tmp_path / "a_d64.cu").write_text('#define RLB_HD 64\n#include "a.cu"\n')
+    before = _digest(tmp_path / "a_d64.cu", [])
+    (tmp_path / "a.cu").write_text("int b;\n")
+    assert _digest(tmp_path / "a_d64.cu", []) != before
