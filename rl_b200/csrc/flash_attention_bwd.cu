@@ -120,7 +120,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   uint64_t* s_full = bars + 15;    // [2]
   uint64_t* p_full = bars + 17;    // [2]
   uint64_t* dq_done = bars + 19;   // [2] the second product of the buffer's tile is complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  uint64_t* all_done = bars + 21;  // every product is
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* info = reinterpret_cast<int*>(tmem_slot + 2);
 
@@ -139,6 +140,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         mbar_init(smem_u32(&p_full[i]), 4);
         mbar_init(smem_u32(&dq_done[i]), 1);
       }
+      mbar_init(smem_u32(all_done), 1);
       *abort_flag = 0;
       mbar_fence_init();
       fence_proxy_async();
@@ -226,6 +228,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           umma_f16_ts(tmem_dq, tmem_base + (j & 1) * 64 + kk * 8, make_smem_desc_sw128(ka + kk * 2048, DQ_KV_ATOM, 1024), idesc_dq, (j | kk) != 0);
         umma_commit(smem_u32(&k_empty[j % DQ_K_STAGES]));
         umma_commit(smem_u32(&dq_done[j & 1]));
+        if (j + 1 == n_kv) umma_commit(smem_u32(all_done));
       }
     }
   } else {
@@ -275,7 +278,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&p_full[group]));
     }
-    if (ok && mbar_wait(smem_u32(&dq_done[(n_kv - 1) & 1]), ((n_kv - 1) >> 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
+    // A barrier of its own: a group may be two phases of the other group's dq_done behind, where a wait for that parity passes at once.
+    if (ok && mbar_wait(smem_u32(all_done), 0, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
       tc_fence_after();
       __nv_bfloat16* dst = p.dqkv + static_cast<long long>(seq_start + qi) * p.dqkv_stride + q_col;
 #pragma unroll
@@ -321,7 +325,8 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_kv128, const __gri
   uint64_t* s_full = bars + 9;      // [2]
   uint64_t* p_full = bars + 11;     // [2]
   uint64_t* acc_done = bars + 13;   // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* all_done = bars + 15;   // every product is complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* info = reinterpret_cast<int*>(tmem_slot + 2);
 
@@ -338,6 +343,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_kv128, const __gri
         mbar_init(smem_u32(&p_full[i]), 4);
         mbar_init(smem_u32(&acc_done[i]), 1);
       }
+      mbar_init(smem_u32(all_done), 1);
       *abort_flag = 0;
       mbar_fence_init();
       fence_proxy_async();
@@ -428,6 +434,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_kv128, const __gri
           umma_f16_ts(tmem_dk, tmem_base + 128 + (it & 1) * 64 + kk * 8, make_smem_desc_sw128(smem_u32(q_s + st * KV_Q_BYTES) + kk * 2048, KV_Q_ATOM, 1024), idesc_acc, (it | kk) != 0);
         umma_commit(smem_u32(&qdo_empty[st]));
         umma_commit(smem_u32(&acc_done[it & 1]));
+        if (it + 1 == n_iter) umma_commit(smem_u32(all_done));
       }
     }
   } else {
@@ -489,7 +496,8 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_kv128, const __gri
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&p_full[group]));
     }
-    if (ok && n_iter > 0 && mbar_wait(smem_u32(&acc_done[(n_iter - 1) & 1]), ((n_iter - 1) >> 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
+    // (a barrier of its own, as for dQ)
+    if (ok && n_iter > 0 && mbar_wait(smem_u32(all_done), 0, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
       tc_fence_after();
       // the first group writes dK, the second dV
       __nv_bfloat16* dst = p.dqkv + static_cast<long long>(seq_start + kj) * p.dqkv_stride + (group == 0 ? k_col : v_col);

@@ -58,3 +58,25 @@ def test_flash_autograd(native_lib, lens, Hq, Hkv, D):
     assert (y.float() - yr).abs().max().item() < 3e-2
     rel = (x.grad.float() - xr.grad).abs().max().item() / (xr.grad.abs().max().item() + 1e-6)
     assert rel < 3e-2, f"relative grad err {rel}"
+
+
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("Hq,Hkv", [(2, 2), (3, 1), (8, 2)])
+@pytest.mark.parametrize("n", [65, 129, 160, 192, 193, 257, 320, 321])
+def test_flash_bwd_few_tiles(native_lib, n, Hq, Hkv, D):
+    """Gradients where a tile has one to six tiles opposite it, both parities, next to a sequence of another length. Bound: that of test_flash_autograd.
+    Nothing is summed by atomics, so repeats are equal bit for bit."""
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import check_status
+
+    lens = [n, 70, n]
+    qkv, cu, D = _case(lens, Hq, Hkv, seed=n, D=D)
+    x = qkv.clone().requires_grad_()
+    y = F.attention_varlen(x, cu, n, Hq, Hkv, D)
+    g = torch.randn_like(y)
+    grads = [torch.autograd.grad(y, x, g, retain_graph=True)[0] for _ in range(100)]
+    torch.cuda.synchronize()
+    assert check_status() == 0 and all(torch.equal(t, grads[0]) for t in grads[1:])
+    xr = qkv.float().requires_grad_()
+    F._attention_ref(xr, cu, Hq, Hkv, D, 1.0 / math.sqrt(D)).backward(g.float())
+    assert (grads[0].float() - xr.grad).abs().max() <= 3e-2 * xr.grad.abs().max()
