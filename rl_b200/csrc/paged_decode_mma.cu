@@ -392,6 +392,9 @@ __global__ void dm_combine_kernel(const float* __restrict__ part_o, const float*
 // all. A CTA is (group of sequences, KV head, split): the group's tiles are listed as the shared ones, then every sequence's own, and the list
 // is cut evenly over the splits, so that a ragged batch spreads as evenly as an even one. The splits of a group form a cluster whose CTAs merge
 // their results through distributed shared memory; more than eight splits (few sequences, long contexts) merge in dm_combine_kernel.
+// A tile of one sequence is multiplied with the weights of all columns, zeros in the others', and zero times an infinite or undefined value is
+// undefined. So the accumulator starts anew with every run of tiles (the shared ones, then each sequence's own), and at the end of a run
+// only its own columns are taken from it: what one sequence holds does not reach its neighbours (1 to 3 % of a group's time).
 // Bound by the cache stream: K and V buffers of three CTAs per SM are in flight; one CTA-wide barrier per tile.
 // Measured, 8 KV heads of 128, 4 query heads each (one CTA per sequence, split and KV head, two per SM, before -> now): 48 sequences of 4000
 // tokens, 16 to a prompt, 169 -> 57 us, every prompt its own 206 -> 129 us (5.9 TB/s); 64 of 256 tokens, 8 to a prompt, 23 -> 18 us; 64 of 2000
@@ -432,8 +435,8 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   return v;
 }
 
-// NC: columns in use, sequences of a group * G, rounded up
-template <int HD, int NC>
+// NC: columns in use, sequences of a group * G, rounded up; RUNS: several sequences in a group, so that runs of tiles have to be kept apart
+template <int HD, int NC, bool RUNS>
 __global__ void __launch_bounds__(DM_THREADS, 3)
 paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, DgParams p) {
   using Cfg = DgCfg<HD>;
@@ -618,10 +621,15 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         return true;
       };
       bool ok = n_tiles > 0 ? issue_qk(0) : true;
+      int run = -2;      // whose tiles the accumulator holds
       for (int i = 0; i < n_tiles && ok; ++i) {
         const uint32_t ph = i & 1;
         if (i + 1 < n_tiles) ok = issue_qk(i + 1);   // overlaps the softmax of tile i
         if (!ok) break;
+        int j = 0;
+        if (RUNS) tile_at(i, j);
+        const bool fresh = j != run;
+        run = j;
         if (!mbar_wait(smem_u32(p_ready), ph, abort_flag, p.status, RLB_ERR_WAIT_FLAG) ||
             !mbar_wait(smem_u32(v_full), ph, abort_flag, p.status, RLB_ERR_WAIT_FULL))
           break;
@@ -631,7 +639,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
           // V^T: M = dims (two 64-dim chunks 16 KB apart), K = tokens: 16 token rows of 128 B per MMA
           const uint64_t a = make_smem_desc_sw128(smem_u32(v_sm) + kk * 2048, DM_CHUNK, 1024);
           const uint64_t b = make_smem_desc_sw128(smem_u32(p_sm) + (kk >> 2) * (DM_N * 128) + (kk & 3) * 32, 16, 1024);
-          umma_f16(tmem_o, a, b, idesc_pv, (i | kk) != 0 ? 1u : 0u);
+          umma_f16(tmem_o, a, b, idesc_pv, !fresh || kk != 0 ? 1u : 0u);
         }
         umma_commit(smem_u32(o_full));
         umma_commit(smem_u32(v_empty));
@@ -644,13 +652,14 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     // O accumulates in TMEM against a reference maximum per column that moves only when a tile's maximum is far above it
     // (the final division and the merge use the same reference, so a stale one is exact)
-    float m_run[NC], l_own[NC];      // l_own: this thread's tokens' share of the soft-max sum
+    float m_run[NC], l_own[NC], o_run[NC];      // l_own: this thread's tokens' share of the soft-max sum; o_run: O of the runs before this one
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       m_run[c] = -INFINITY;
-      l_own[c] = 0.f;
+      l_own[c] = o_run[c] = 0.f;
     }
     uint32_t last = 0;      // columns whose P differs from zero
+    int run = -2;
     bool ok = true;
     for (int i = 0; i < n_tiles; ++i) {
       const uint32_t ph = i & 1;
@@ -708,14 +717,23 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         if (!ok) continue;
         tc_fence_after();
       }
-      if (moved && i > 0) {
+      const bool fresh = RUNS && j != run;      // the product of this tile overwrites O: what the run before left there is taken out first
+      run = j;
+      if (i > 0 && (moved || fresh)) {
         uint32_t orr[DM_N];
         tmem_ld_32x32b_x16(tmem_o + lane_addr, orr);
         tmem_ld_wait();
 #pragma unroll
-        for (int c = 0; c < NC; ++c) orr[c] = __float_as_uint(__uint_as_float(orr[c]) * k[c]);      // (columns behind them hold zeros)
-        tmem_st_32x32b_x16(tmem_o + lane_addr, orr);
-        tmem_st_wait();
+        for (int c = 0; c < NC; ++c) {
+          const float o = __uint_as_float(orr[c]);
+          if (fresh && (last >> c & 1)) o_run[c] += o;
+          if (RUNS) o_run[c] *= k[c];
+          orr[c] = __float_as_uint(o * k[c]);      // (columns behind them hold zeros)
+        }
+        if (!fresh) {
+          tmem_st_32x32b_x16(tmem_o + lane_addr, orr);
+          tmem_st_wait();
+        }
       }
 #pragma unroll
       for (int c = 0; c < NC; ++c)
@@ -727,16 +745,14 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(p_ready));
     }
-    float o_run[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) o_run[c] = 0.f;
     if (n_tiles > 0 && ok && mbar_wait(smem_u32(o_full), (n_tiles - 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL)) {
       tc_fence_after();
       uint32_t orr[DM_N];
       tmem_ld_32x32b_x16(tmem_o + lane_addr, orr);
       tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < NC; ++c) o_run[c] = __uint_as_float(orr[c]);
+      for (int c = 0; c < NC; ++c)
+        if (last >> c & 1) o_run[c] += __uint_as_float(orr[c]);
     }
     // sums over the tile rows; thread r owns head dimension r
     named_bar_sync(1, 128);
@@ -809,9 +825,9 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   }
 }
 
-template <int HD, int NC>
+template <int HD, int NC, bool RUNS>
 int launch_group_nc(const CUtensorMap& tk, const CUtensorMap& tv, const DgParams& p, cudaStream_t s) {
-  auto kern = paged_decode_group_kernel<HD, NC>;
+  auto kern = paged_decode_group_kernel<HD, NC, RUNS>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DgCfg<HD>::SMEM);
@@ -840,10 +856,10 @@ int launch_group_nc(const CUtensorMap& tk, const CUtensorMap& tv, const DgParams
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, tk, tv, p));
 }
 
-template <int HD>
+template <int HD, bool RUNS>
 int launch_group(const CUtensorMap& tk, const CUtensorMap& tv, const DgParams& p, cudaStream_t s) {
   const int columns = p.rows * p.G;
-  return columns <= 4 ? launch_group_nc<HD, 4>(tk, tv, p, s) : columns <= 8 ? launch_group_nc<HD, 8>(tk, tv, p, s) : launch_group_nc<HD, 16>(tk, tv, p, s);
+  return columns <= 4 ? launch_group_nc<HD, 4, RUNS>(tk, tv, p, s) : columns <= 8 ? launch_group_nc<HD, 8, RUNS>(tk, tv, p, s) : launch_group_nc<HD, 16, RUNS>(tk, tv, p, s);
 }
 }  // namespace
 
@@ -949,7 +965,8 @@ RLB_API int rlb_paged_decode_group(const void* q, long long q_stride, const void
   p.status = status;
   p.gated = gated;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  rc = D == 64 ? launch_group<64>(tk, tv, p, s) : launch_group<128>(tk, tv, p, s);
+  if (rows > 1) rc = D == 64 ? launch_group<64, true>(tk, tv, p, s) : launch_group<128, true>(tk, tv, p, s);
+  else rc = D == 64 ? launch_group<64, false>(tk, tv, p, s) : launch_group<128, false>(tk, tv, p, s);
   if (rc) return rc;
   if (num_splits > DG_CLUSTER)
     rlb_launch_pdl(dm_combine_kernel, dim3(B, Hq), dim3(D), 0, s, part_o, part_ml, num_splits, Hq, 0, gated, static_cast<__nv_bfloat16*>(out), out_stride);

@@ -377,6 +377,42 @@ def test_paged_decode_groups(native_lib, Hq, Hkv, D, bs, rows, splits):
             assert (out[b].double() - ref).norm() <= 3 * 2.0 ** -9 * 2 * ref.norm() + 1e-6, (b, n)
 
 
+@pytest.mark.parametrize("Hq,Hkv,D", [(8, 2, 128), (8, 2, 64), (2, 2, 128)])
+@pytest.mark.parametrize("rows,splits", [(2, 1), (4, 1), (4, 3), (2, 11)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_paged_decode_groups_stay_apart(native_lib, Hq, Hkv, D, rows, splits, bad):
+    """Undefined values in one sequence's own pages, and behind another one's end, leave the other sequences of the group as they are, bit for bit."""
+    from rl_b200.ops import engine_ops as E
+    from rl_b200.ops import lib as L
+    from rl_b200.ops.lib import call, check_status, ptr, stream_ptr
+
+    bs, lens = 64, [300, 450, 390, 500, 200, 130, 129, 640]
+    B, pages = len(lens), 10
+    g = torch.Generator().manual_seed(rows + splits)
+    bt = torch.arange(1, B * pages + 1, dtype=torch.int32).view(B, pages)
+    bt[1:4, :2] = bt[0, :2]                                            # the first tile of four sequences is shared
+    q = torch.randn(B, Hq * D, generator=g).bfloat16().cuda()
+    kc, vc = (torch.randn(B * pages + 1, Hkv, bs, D, generator=g).bfloat16().cuda() for _ in range(2))
+    btc, lc = bt.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+    def run(v):
+        out = torch.zeros(B, Hq * D, dtype=torch.bfloat16, device="cuda")
+        no, nml = E.decode_scratch_sizes(B, Hq, splits, D)
+        po, pml = torch.empty(no, device="cuda"), torch.empty(nml, device="cuda")
+        call("rlb_paged_decode_group", ptr(q), q.stride(0), ptr(kc), ptr(v), len(kc), ptr(btc), btc.stride(0), ptr(lc), B, Hq, Hkv, D, bs, rows, 0,
+             D ** -0.5, splits, ptr(po), ptr(pml), ptr(out), out.stride(0), ptr(L.status_word(q.device)), stream_ptr())
+        torch.cuda.synchronize()
+        assert check_status() == 0
+        return out
+
+    clean, spoilt = run(vc), vc.clone()
+    spoilt[bt[1, 3].item()] = bad                                      # tokens 192 to 255 of sequence 1
+    spoilt[bt[6, 2].item(), :, 2:] = bad                               # behind the end of sequence 6
+    got = run(spoilt)
+    others = [b for b in range(B) if b not in (1, 6)]
+    assert torch.equal(got[others], clean[others]) and not got[1].isfinite().all()
+
+
 @pytest.mark.parametrize("n", [1, 7, 8, 9, 2048, 4101])            # whole groups of eight, a tail, a tail alone
 @pytest.mark.parametrize("shift", [0, 1])                          # a start that is not 16-byte aligned goes element by element
 @pytest.mark.parametrize("gdtype", [torch.float32, torch.bfloat16])
