@@ -121,6 +121,13 @@ def _paged_decode_gather(q, k_cache, v_cache, block_table, seq_lens, Hq, Hkv, D,
     return out
 
 
+def _kernel_layout(q, k_cache, v_cache, block_table, seq_lens, out) -> bool:
+    """Whether a decode kernel can read these: what the gather path takes beside them (64-bit tables, caches of another type or order) stays with it."""
+    return (q.stride(1) == 1 and k_cache.dtype == v_cache.dtype == out.dtype == torch.bfloat16 and k_cache.is_contiguous() and v_cache.is_contiguous()
+            and (k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0 and block_table.dtype == seq_lens.dtype == torch.int32 and block_table.stride(1) == 1
+            and seq_lens.is_contiguous() and out.stride(1) == 1)
+
+
 def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
                  seq_lens: torch.Tensor, Hq: int, Hkv: int, D: int, *, scale: Optional[float] = None,
                  num_splits: int = 1, scratch: Optional[tuple[torch.Tensor, torch.Tensor]] = None,
@@ -156,7 +163,7 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
         return out
     kernel = os.environ.get("RLB_DECODE_KERNEL", "mma")
     if plain and (kernel == "mma" or special) and D in (64, 128) and Hq // Hkv <= 16 and (block_size in (16, 32, 64) or block_size % 128 == 0) \
-            and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0:
+            and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and (D == 128 or _kernel_layout(q, k_cache, v_cache, block_table, seq_lens, out)):
         if num_splits > 8 and scratch is None:
             no, nml = decode_scratch_sizes(B, Hq, num_splits, D)
             scratch = (torch.empty(no, dtype=torch.float32, device=q.device), torch.empty(nml, dtype=torch.float32, device=q.device))

@@ -377,6 +377,37 @@ def test_paged_decode_groups(native_lib, Hq, Hkv, D, bs, rows, splits):
             assert (out[b].double() - ref).norm() <= 3 * 2.0 ** -9 * 2 * ref.norm() + 1e-6, (b, n)
 
 
+@pytest.mark.parametrize("form", ["kernel", "int64 table", "int64 lengths", "fp32 caches", "permuted caches", "fp32 output", "strided table"])
+def test_paged_decode_d64_forms(native_lib, form):
+    """Heads of 64 with the tables, caches and outputs that the gather path takes, whatever path serves them, against the statement on the CPU."""
+    from rl_b200.ops import engine_ops as E
+    from rl_b200.ops.lib import check_status
+
+    Hq, Hkv, D, bs, lens = 8, 2, 64, 16, [5, 100, 64, 33]
+    g = torch.Generator().manual_seed(3)
+    q = torch.randn(len(lens), Hq * D, generator=g).bfloat16()
+    kc, vc = (torch.randn(40, Hkv, bs, D, generator=g).bfloat16() for _ in range(2))
+    bt, ln = torch.randperm(40, generator=g)[:28].view(4, 7).to(torch.int32), torch.tensor(lens, dtype=torch.int32)
+    ref = E.paged_decode(q, kc, vc, bt, ln, Hq, Hkv, D).float()
+    q, kc, vc, bt, ln = (t.cuda() for t in (q, kc, vc, bt, ln))
+    out = None
+    if form == "int64 table":
+        bt = bt.long()
+    elif form == "int64 lengths":
+        ln = ln.long()
+    elif form == "fp32 caches":
+        kc, vc = kc.float(), vc.float()
+    elif form == "permuted caches":
+        kc, vc = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (kc, vc))
+    elif form == "fp32 output":
+        out = torch.empty(len(lens), Hq * D, device="cuda")
+    elif form == "strided table":
+        bt = torch.stack([bt, bt.flip(0)], -1)[..., 0]
+    got = E.paged_decode(q, kc, vc, bt, ln, Hq, Hkv, D, out=out)
+    torch.cuda.synchronize()
+    assert check_status() == 0 and (got.cpu().float() - ref).norm() <= 2e-2 * ref.norm()
+
+
 @pytest.mark.parametrize("Hq,Hkv,D", [(8, 2, 128), (8, 2, 64), (2, 2, 128)])
 @pytest.mark.parametrize("rows,splits", [(2, 1), (4, 1), (4, 3), (2, 11)])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
