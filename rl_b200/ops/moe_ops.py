@@ -309,7 +309,9 @@ class SmallTokenMoE:
         """Rows of a tile. Few tokens per expert: 32 or 64, the columns of the weight-streaming products (twice the mean load, so that nearly every
         expert's weights are read once); from 32 on the 128-row tiles of the grouped GEMM, which then read more weights than padding."""
         mean = self.W * T * self.k / self.E
-        return 32 if mean <= 16 else 64 if mean <= 32 else 128
+        if mean > 32 or self.d % 64 or self.f % 64:      # (the weight-streaming products have whole 64-column blocks)
+            return 128
+        return 32 if mean <= 16 else 64
 
     def mpad_for(self, T: int) -> int:
         pad = self.tile_rows(T)

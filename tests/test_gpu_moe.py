@@ -243,3 +243,27 @@ def test_few_token_layer(native_lib, T, E, k, load, one):
     assert (out.double() - ref).norm() <= 1e-2 * ref.norm()
     if one:
         assert bool((idx == 1).any(-1).all())
+
+
+@pytest.mark.parametrize("d,f", [(200, 64), (192, 72), (136, 40)])
+def test_few_token_layer_widths(native_lib, d, f):
+    """Widths that are not whole 64-column blocks take the grouped GEMM, as they did before there was another product. Bounds as above."""
+    from rl_b200.ops import moe_ops as M
+    from rl_b200.ops.lib import check_status
+
+    T, E, k = 5, 8, 2
+    g = torch.Generator("cuda").manual_seed(d)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    x, router = r(T, d).bfloat16(), r(E, d).bfloat16()
+    gu, dn = (0.2 * r(E, 2 * f, d)).bfloat16(), (0.2 * r(E, d, f)).bfloat16()
+    ws = M.SmallTokenMoE(d, f, E, k, None, T, x.device)
+    out, idx = ws.forward(x, None, router, gu, dn, True)
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    ref = torch.zeros(T, d, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        t, j = (idx == e).nonzero(as_tuple=True)
+        if len(t):
+            a, b = (x[t].double() @ gu[e].double().T).chunk(2, -1)
+            ref = ref.index_add(0, t, (torch.nn.functional.silu(a) * b) @ dn[e].double().T * ws.w[:T].double()[t, j, None])
+    assert (out.double() - ref).norm() <= 1e-2 * ref.norm()
