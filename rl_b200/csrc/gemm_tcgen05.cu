@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(256) logprob_combine_kernel(const float* __res
 #pragma unroll 4
     for (int p = warp; p < num_parts; p += 8) {
       const long long i = static_cast<long long>(p) * M + row;
-      const float s = __expf(part_max[i] - mx);
+      const float s = part_max[i] == -INFINITY ? 0.f : __expf(part_max[i] - mx);      // (a part without columns, or all of this warp's)
       sum += part_sum[i] * s;
       zsum += part_zsum[i] * s;
     }
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(256) logprob_combine_kernel(const float* __res
   for (int w = 1; w < 8; ++w) mx = fmaxf(mx, s_max[w][lane]);
   sum = zsum = 0.f;
   for (int w = 0; w < 8; ++w) {
-    const float s = s_max[w][lane] == -INFINITY ? 0.f : __expf(s_max[w][lane] - mx);      // (a warp without parts)
+    const float s = s_max[w][lane] == -INFINITY ? 0.f : __expf(s_max[w][lane] - mx);
     sum += s_sum[w][lane] * s;
     zsum += s_zsum[w][lane] * s;
   }

@@ -130,6 +130,27 @@ def test_lm_head_logprob(native_lib, M, V, K):
     assert _rel_err(w.grad, wr.grad) < 3e-2
 
 
+@pytest.mark.parametrize("parts", [1, 3, 8, 21])
+def test_logprob_combine_empty_parts(native_lib, parts):
+    """Parts without columns (maximum -inf, sums 0), as many as all of a warp's, count for nothing. Against float64: fp32 sums of at most 21 terms
+    and the fast exponentials, 1e-5."""
+    from rl_b200.ops.lib import call, ptr, stream_ptr
+
+    M = 70
+    g = torch.Generator("cuda").manual_seed(parts)
+    mx, sm = torch.randn(parts, M, generator=g, device="cuda"), 1 + 50 * torch.rand(parts, M, generator=g, device="cuda")
+    zs, tl = sm * torch.randn(parts, M, generator=g, device="cuda"), torch.randn(M, generator=g, device="cuda")
+    empty = torch.rand(parts, M, generator=g, device="cuda") < 0.5
+    empty[torch.randint(0, parts, (M,), generator=g, device="cuda"), torch.arange(M, device="cuda")] = False
+    mx[empty], sm[empty], zs[empty] = -float("inf"), 0.0, 0.0
+    lp, ent, lse = torch.empty(3, M, device="cuda")
+    call("rlb_logprob_combine", ptr(mx), ptr(sm), ptr(zs), ptr(tl), M, parts, ptr(lp), ptr(ent), ptr(lse), stream_ptr())
+    w = torch.exp(mx.double())
+    total = (w * sm).sum(0)
+    for got, ref in ((lse, total.log()), (lp, tl - total.log()), (ent, total.log() - (w * zs).sum(0) / total)):
+        assert (got - ref).abs().max() <= 1e-5 * (1 + ref.abs().max())
+
+
 @pytest.mark.parametrize("M", [1, 7, 32, 64, 100, 128, 200, 256])
 @pytest.mark.parametrize("N,K", [(4096, 4096), (6144, 4096), (4096, 14336), (1000, 512), (128256, 1024)])
 def test_skinny_gemm(native_lib, M, N, K):
