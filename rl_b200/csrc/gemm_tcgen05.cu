@@ -12,7 +12,8 @@
 //   warp 1      TMEM allocator; in the pair's first CTA also the tcgen05.mma issuer (one elected lane) for both
 //   warps 2..5  epilogue of this CTA's 128 rows: tcgen05.ld -> registers -> (shared memory ->) global
 // A 6-deep shared-memory ring feeds 256x256x16 MMAs; two 256-column TMEM accumulators let the
-// epilogue of tile i overlap the main loop of tile i+1.
+// epilogue of tile i overlap the main loop of tile i+1. Where tiles of 256 rows would leave the last wave nearly empty (takes_pairs) the same
+// kernel runs with one CTA per 128 x 256 tile and a 4-deep ring.
 //
 // Why pairs: one CTA's 128 x 256 tile fills and reads 192 bytes of shared memory per cycle of tensor time, above the 128
 // that an SM has; a pair shares the B operand, which brings that to 128 and the L2 reads of a tile from 48 to 32 KB per k-block.
@@ -44,22 +45,27 @@ namespace {
 
 using namespace rlb;
 
-constexpr int BM = 256;       // rows of a pair's tile
-constexpr int CTA_M = 128;    // rows of each of its CTAs
+constexpr int CTA_M = 128;    // rows of one CTA
 constexpr int BN = 256;
-constexpr int CTA_N = 128;    // rows of B that each CTA loads
 constexpr int BK = 64;
-constexpr int STAGES = 6;
 constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = CTA_M * BK * 2;  // 16 KB
-constexpr int B_STAGE_BYTES = CTA_N * BK * 2;  // 16 KB
-constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int SMEM_BARRIER_BYTES = 256;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * OUT_WARP_BYTES + SMEM_BARRIER_BYTES + 1024;  // +1024: manual alignment
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 constexpr int NUM_THREADS = 192;
 constexpr int TMEM_COLS = 512;
-constexpr int GROUP_M = 8;  // rasterisation: 8 m-tiles share each sweep over n
+constexpr int GROUP_ROWS = 2048;  // rasterisation: the m-tiles of so many rows share each sweep over n
+
+// A tile of a pair of CTAs, or of one.
+template <bool PAIR>
+struct Tile {
+  static constexpr int CTAS = PAIR ? 2 : 1;
+  static constexpr int BM = CTAS * CTA_M;
+  static constexpr int CTA_N = BN / CTAS;                  // rows of B that each CTA loads
+  static constexpr int STAGES = PAIR ? 6 : 4;
+  static constexpr int STAGE_BYTES = A_STAGE_BYTES + CTA_N * BK * 2;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * OUT_WARP_BYTES + SMEM_BARRIER_BYTES + 1024;  // +1024: manual alignment
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
+};
 
 enum { EPI_STORE = 0, EPI_LOGPROB = 1, EPI_DLOGITS = 2, EPI_LAYER = 3, EPI_LINEAR = 4 };
 
@@ -85,7 +91,9 @@ struct EpiParams {
   LayerEpilogue layer;    // EPI_LAYER
 };
 
+template <int BM>
 __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int& m_blk, int& n_blk) {
+  constexpr int GROUP_M = GROUP_ROWS / BM;
   const int per_group = GROUP_M * num_n;
   const int group = tile / per_group;
   const int first_m = group * GROUP_M;
@@ -104,10 +112,23 @@ __device__ __forceinline__ float4 square_relu4(float4 v) {
   return make_float4(v.x * v.x, v.y * v.y, v.z * v.z, v.w * v.w);
 }
 
-template <bool A_MN, bool B_MN, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+// A load of this CTA's operands, signalling `bar`: with PAIR the first CTA's barrier.
+template <bool PAIR>
+__device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  if constexpr (PAIR) tma_load_2d_pair(dst, map, bar, c0, c1);
+  else tma_load_2d(dst, map, bar, c0, c1);
+}
+template <bool PAIR>
+__device__ __forceinline__ void commit_tile(uint32_t bar) {
+  if constexpr (PAIR) umma_commit_pair(bar);
+  else umma_commit(bar);
+}
+
+template <bool PAIR, bool A_MN, bool B_MN, int EPI>
+__global__ void __cluster_dims__(Tile<PAIR>::CTAS, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  int M, int N, int K, EpiParams ep, int* status) {
+  constexpr int BM = Tile<PAIR>::BM, CTA_N = Tile<PAIR>::CTA_N, STAGES = Tile<PAIR>::STAGES, STAGE_BYTES = Tile<PAIR>::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   // 128B swizzle needs 1024-byte aligned stage buffers.
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -122,8 +143,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();      // in the pair; the first CTA's barriers count the loads of both
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0;      // in the pair; the first CTA's barriers count the loads of both
+  const int first = blockIdx.x / Tile<PAIR>::CTAS, step = gridDim.x / Tile<PAIR>::CTAS;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -132,7 +153,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&tfull_bar[a]), 1);
-      mbar_init(smem_u32(&tempty_bar[a]), 8);  // one arrive per epilogue warp of both CTAs
+      mbar_init(smem_u32(&tempty_bar[a]), 4 * Tile<PAIR>::CTAS);  // one arrive per epilogue warp
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -143,12 +164,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     prefetch_tmap(&tmap_b);
   }
   if (warp == 1) {
-    tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS);
-    tmem_relinquish_pair();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync();      // both CTAs' barriers exist before either signals the other's
+  if (PAIR) cluster_sync();      // both CTAs' barriers exist before either signals the other's
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -162,32 +188,32 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
+      for (int tile = first; tile < num_tiles && ok; tile += step) {
         int m_blk, n_blk;
-        tile_coords(tile, num_m, num_n, m_blk, n_blk);
+        tile_coords<BM>(tile, num_m, num_n, m_blk, n_blk);
         const int row0 = m_blk * BM + rank * CTA_M, brow0 = n_blk * BN + rank * CTA_N;
         for (int kb = 0; kb < num_k; ++kb) {
           if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, status, RLB_ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
-          const uint32_t bar = mapa_shared(smem_u32(&full_bar[stage]), 0);
+          const uint32_t bar = PAIR ? mapa_shared(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
           const uint32_t a_dst = smem_u32(smem + stage * STAGE_BYTES);
           const uint32_t b_dst = a_dst + A_STAGE_BYTES;
-          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), 2 * STAGE_BYTES);
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), Tile<PAIR>::CTAS * STAGE_BYTES);
           if (!A_MN) {
-            tma_load_2d_pair(a_dst, &tmap_a, bar, kb * BK, row0);
+            load_tile<PAIR>(a_dst, &tmap_a, bar, kb * BK, row0);
           } else {
 #pragma unroll
             for (int j = 0; j < CTA_M / 64; ++j)
-              tma_load_2d_pair(a_dst + j * (BK * 128), &tmap_a, bar, row0 + j * 64, kb * BK);
+              load_tile<PAIR>(a_dst + j * (BK * 128), &tmap_a, bar, row0 + j * 64, kb * BK);
           }
           if (!B_MN) {
-            tma_load_2d_pair(b_dst, &tmap_b, bar, kb * BK, brow0);
+            load_tile<PAIR>(b_dst, &tmap_b, bar, kb * BK, brow0);
           } else {
 #pragma unroll
             for (int j = 0; j < CTA_N / 64; ++j)
-              tma_load_2d_pair(b_dst + j * (BK * 128), &tmap_b, bar, brow0 + j * 64, kb * BK);
+              load_tile<PAIR>(b_dst + j * (BK * 128), &tmap_b, bar, brow0 + j * 64, kb * BK);
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -207,7 +233,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       uint32_t stage = 0, phase = 0;
       uint32_t local_tile = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++local_tile) {
+      for (int tile = first; tile < num_tiles && ok; tile += step, ++local_tile) {
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_phase = (local_tile >> 1) & 1;
         if (!mbar_wait(smem_u32(&tempty_bar[acc]), acc_phase ^ 1, abort_flag, status, RLB_ERR_WAIT_TMEM_EMPTY)) {
@@ -234,15 +260,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           constexpr uint32_t b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            umma_f16_pair(tmem_d, a_desc + kk * a_step, b_desc + kk * b_step, idesc, (kb | kk) != 0 ? 1u : 0u);
+            if constexpr (PAIR) umma_f16_pair(tmem_d, a_desc + kk * a_step, b_desc + kk * b_step, idesc, (kb | kk) != 0 ? 1u : 0u);
+            else umma_f16(tmem_d, a_desc + kk * a_step, b_desc + kk * b_step, idesc, (kb | kk) != 0 ? 1u : 0u);
           }
-          umma_commit_pair(smem_u32(&empty_bar[stage]));  // stage reusable, in both CTAs, once these MMAs have read it
+          commit_tile<PAIR>(smem_u32(&empty_bar[stage]));  // stage reusable, in both CTAs, once these MMAs have read it
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) umma_commit_pair(smem_u32(&tfull_bar[acc]));  // accumulator complete
+        if (ok) commit_tile<PAIR>(smem_u32(&tfull_bar[acc]));  // accumulator complete
       }
     }
   } else {
@@ -251,9 +278,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const uint32_t buf = smem_u32(out_smem) + quarter * OUT_WARP_BYTES;
     uint32_t local_tile = 0;
     bool ok = true;
-    for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++local_tile) {
+    for (int tile = first; tile < num_tiles && ok; tile += step, ++local_tile) {
       int m_blk, n_blk;
-      tile_coords(tile, num_m, num_n, m_blk, n_blk);
+      tile_coords<BM>(tile, num_m, num_n, m_blk, n_blk);
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;
       if (!mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase, abort_flag, status, RLB_ERR_WAIT_TMEM_FULL)) {
@@ -491,16 +518,20 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0));
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0));
+        else mbar_arrive(smem_u32(&tempty_bar[acc]));
+      }
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  cluster_sync();      // nothing of the pair signals or writes the other CTA any more
+  if (PAIR) cluster_sync();      // nothing of the pair signals or writes the other CTA any more
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
@@ -542,28 +573,57 @@ __global__ void __launch_bounds__(256) logprob_combine_kernel(const float* __res
   if (entropy) entropy[row] = lse - zsum / sum;  // H = lse - E[z]
 }
 
-int g_sm_count = 0;
+int sm_count() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return n;
+}
+
+// Tiles of this size, and the waves of them on at most `max_ctas` CTAs (0: as many as there are SMs).
+template <bool PAIR>
+int num_tiles(int M, int N) { return ((M + Tile<PAIR>::BM - 1) / Tile<PAIR>::BM) * ((N + BN - 1) / BN); }
+template <bool PAIR>
+int slots(int max_ctas) {
+  const int ctas = max_ctas > 0 && max_ctas < sm_count() ? max_ctas : sm_count();
+  return ctas / Tile<PAIR>::CTAS;
+}
+
+// Pairs unless single CTAs need so many waves fewer that these, each some 10 to 15 % longer, are sooner done. Timed both ways over 250 products
+// (64 to 9000 rows; forward, input and weight gradients, vocabulary): at equal waves pairs took 0.90 of single CTAs' time (0.84 to 1.05), at
+// 1.11 to 1.14 times as many waves 0.98 to 0.99, at 1.17 1.00 to 1.05, at 1.25 to 1.33 1.02 to 1.17, at 1.5 to 2 1.05 to 1.6. So 640 x 14336 x 4096
+// runs in 91 us (pairs 116), 1100 x 4096 x 14336 in 163 (267), 257 rows of a vocabulary of 128256 x 2048 in 228 (257).
+constexpr int TILE_RATIO = 115;      // percent
+bool takes_pairs(int M, int N, int max_ctas) {
+  const int p = slots<true>(max_ctas), c = slots<false>(max_ctas);
+  if (p == 0) return false;
+  const int waves_p = (num_tiles<true>(M, N) + p - 1) / p, waves_c = (num_tiles<false>(M, N) + c - 1) / c;
+  return 100 * waves_p <= TILE_RATIO * waves_c;
+}
+
+template <bool PAIR, bool A_MN, bool B_MN, int EPI>
+int launch_tiles(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, const EpiParams& ep,
+                 int* status, int max_ctas, cudaStream_t stream) {
+  auto kern = gemm_bf16_kernel<PAIR, A_MN, B_MN, EPI>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<PAIR>::SMEM_BYTES);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  const int tiles = num_tiles<PAIR>(M, N), most = slots<PAIR>(max_ctas);
+  kern<<<Tile<PAIR>::CTAS * (tiles < most ? tiles : most), NUM_THREADS, Tile<PAIR>::SMEM_BYTES, stream>>>(ta, tb, M, N, K, ep, status);
+  return static_cast<int>(cudaGetLastError());
+}
 
 template <bool A_MN, bool B_MN, int EPI>
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, const EpiParams& ep,
                 int* status, int max_ctas, cudaStream_t stream) {
-  auto kern = gemm_bf16_kernel<A_MN, B_MN, EPI>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
-  if (g_sm_count == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev);
-  }
-  const int num_tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  int pairs = num_tiles < g_sm_count / 2 ? num_tiles : g_sm_count / 2;
-  if (max_ctas > 0 && pairs > max_ctas / 2) pairs = max_ctas > 1 ? max_ctas / 2 : 1;
-  kern<<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, M, N, K, ep, status);
-  return static_cast<int>(cudaGetLastError());
+  return takes_pairs(M, N, max_ctas) ? launch_tiles<true, A_MN, B_MN, EPI>(ta, tb, M, N, K, ep, status, max_ctas, stream)
+                                     : launch_tiles<false, A_MN, B_MN, EPI>(ta, tb, M, N, K, ep, status, max_ctas, stream);
 }
 
 template <int EPI>
@@ -576,7 +636,8 @@ int dispatch_layout(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorM
 }
 
 int make_operand_maps(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb,
-                      bool a_mn, bool b_mn, CUtensorMap* ta, CUtensorMap* tb) {
+                      bool a_mn, bool b_mn, CUtensorMap* ta, CUtensorMap* tb, int max_ctas = 0) {
+  const int b_rows = takes_pairs(M, N, max_ctas) ? Tile<true>::CTA_N : Tile<false>::CTA_N;
   int rc;
   if (!a_mn)
     rc = rlb_make_tmap_2d(ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, lda * 2, BK, CTA_M,
@@ -586,7 +647,7 @@ int make_operand_maps(const void* A, const void* B, int M, int N, int K, long lo
                           CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
   if (!b_mn)
-    rc = rlb_make_tmap_2d(tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, ldb * 2, BK, CTA_N,
+    rc = rlb_make_tmap_2d(tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, ldb * 2, BK, b_rows,
                           CU_TENSOR_MAP_SWIZZLE_128B);
   else
     rc = rlb_make_tmap_2d(tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldb * 2, 64, BK,
@@ -654,7 +715,7 @@ RLB_API int rlb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15)
     return -3;
   CUtensorMap ta, tb;
-  int rc = make_operand_maps(A, B, M, N, K, lda, ldb, a_mn_major != 0, b_mn_major != 0, &ta, &tb);
+  int rc = make_operand_maps(A, B, M, N, K, lda, ldb, a_mn_major != 0, b_mn_major != 0, &ta, &tb, max_ctas);
   if (rc) return -100 - rc;
   EpiParams ep{};
   ep.C = C;

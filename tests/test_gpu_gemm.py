@@ -87,6 +87,29 @@ def test_gemm_tile_edges(native_lib, M, N, dtype):
     assert torch.equal(wide[M:], old[M:]) and torch.equal(wide[:, N:], old[:, N:])      # nothing beside the tile is touched
 
 
+@pytest.mark.parametrize("M,N,K,ctas", [(8, 72, 456, 1), (136, 328, 456, 1), (304, 584, 136, 1), (304, 584, 136, 3), (120, 20480, 128, 0), (1160, 4096, 72, 0)])
+@pytest.mark.parametrize("layout", ["kk", "k_mn", "mn_mn", "mn_k"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gemm_single_ctas(native_lib, M, N, K, ctas, layout, dtype):
+    """One CTA a tile: asked for by the number of CTAs, or because it takes fewer waves than pairs (the last two sizes). Bounds as in test_gemm_tile_edges."""
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import check_status
+
+    torch.manual_seed(M + N)
+    a_mn, b_mn = layout.startswith("mn"), layout.endswith("mn")
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    bias, res = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda").bfloat16()
+    wide = torch.randn(M + 1, N + 8, device="cuda").to(dtype)
+    old = wide.clone()
+    F.gemm(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, a_mn=a_mn, b_mn=b_mn, out=wide[:M, :N], bias=bias, residual=res,
+           accumulate=True, max_ctas=ctas)
+    ref = a.double() @ b.double().t() + bias + res + old[:M, :N]
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    assert (wide[:M, :N].double() - ref).abs().max() <= (1e-5 if dtype == torch.float32 else 2.0 ** -8 + 1e-5) * ref.abs().max()
+    assert torch.equal(wide[M:], old[M:]) and torch.equal(wide[:, N:], old[:, N:])
+
+
 def test_linear_autograd(native_lib):
     from rl_b200.ops import functional as F
 
