@@ -431,7 +431,8 @@ RLB_API int RLB_NAME(rlb_flash_attn_fwd)(const void* qkv, long long qkv_stride, 
   p.T = T;
   p.Hq = Hq;
   p.Hkv = Hkv;
-  p.scale_log2 = scale == 0.f ? 1e-30f : scale * LOG2E;      // (hidden scores are infinite: they must not meet a factor of zero)
+  // (hidden scores are infinite: they must not meet a factor of zero, nor one that the kernel would flush to zero)
+  p.scale_log2 = fabsf(scale) < 1e-30f ? copysignf(1e-30f, scale) : scale * LOG2E;
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.out_stride = out_stride;
   p.lse = lse;

@@ -80,3 +80,19 @@ def test_flash_bwd_few_tiles(native_lib, n, Hq, Hkv, D):
     xr = qkv.float().requires_grad_()
     F._attention_ref(xr, cu, Hq, Hkv, D, 1.0 / math.sqrt(D)).backward(g.float())
     assert (grads[0].float() - xr.grad).abs().max() <= 3e-2 * xr.grad.abs().max()
+
+
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("scale", [0.0, -0.0, 1e-39, -1e-39, -0.09, 1e-3])
+def test_flash_fwd_scales(native_lib, D, scale):
+    """Scales of zero, too small for a normal number, and negative ones, where the least score has the largest weight. Bounds of test_flash_fwd."""
+    from rl_b200.ops import attention as A
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import check_status
+
+    qkv, cu, D = _case([200, 1, 333], 4, 2, seed=3, D=D)
+    out, lse = A.flash_fwd(qkv, cu, 4, 2, D, scale)
+    torch.cuda.synchronize()
+    assert check_status() == 0 and bool(lse.isfinite().all())
+    ref = F._attention_ref(qkv.float(), cu, 4, 2, D, scale)
+    assert (out.float() - ref).abs().max() < 3e-2
