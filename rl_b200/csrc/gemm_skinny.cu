@@ -28,6 +28,7 @@
 #include "common.cuh"
 
 #include <cooperative_groups.h>
+#include <type_traits>
 
 namespace {
 using namespace rlb;
@@ -251,86 +252,95 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // squares for the next norm is one warp reduction
     const int items = max(m_end - m_begin, 0) * groups;
     const int items_pad = (items + 31) & ~31;
-    for (int it = threadIdx.x; it < items_pad; it += SK_THREADS) {
-      const bool live = it < items;
-      const int m = m_begin + (live ? it / groups : 0);
-      const int n4 = (live ? it % groups : 0) * 4;
-      const int n = n0 + n4;
-      const bool valid = live && n < p.N;  // N is a multiple of 8, so a group of 4 is all in or all out
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc_u = acc, x_old = acc, x_e = acc;
-      uint2 rv = make_uint2(0u, 0u), wv = rv;
-      if (valid) {
-        // All that the item needs from memory and from the other CTAs is requested before any of it is waited for: one latency instead of one
-        // per CTA of the cluster (projections of an 8B layer in a captured chain, 64 sequences 98.7 -> 97.0 us, one 85.5 -> 83.6; of a 1B
-        // layer 46.5 -> 45.1 and 37.9 -> 36.9).
-        const uint32_t off = static_cast<uint32_t>((m * SK_BM + n4) * 4);
-        if (p.residual) rv = *reinterpret_cast<const uint2*>(p.residual + static_cast<long long>(m) * p.ldr + n);
-        if (p.ssq_out) wv = *reinterpret_cast<const uint2*>(p.norm_w + n);
-        if (p.use_layer && p.layer.x) {
-          x_old = *reinterpret_cast<const float4*>(p.layer.x + m * p.layer.ldx + n);
-          if (p.layer.e) x_e = *reinterpret_cast<const float4*>(p.layer.e + m * p.layer.ldx + n);
-        }
-        float4 part[8], part_u[8];      // 8: the largest cluster
+    auto finish = [&](auto alone) {      // alone: a CTA on its own, without the loops over the cluster, whose instructions cost more than they hide
+      for (int it = threadIdx.x; it < items_pad; it += SK_THREADS) {
+        const bool live = it < items;
+        const int m = m_begin + (live ? it / groups : 0);
+        const int n4 = (live ? it % groups : 0) * 4;
+        const int n = n0 + n4;
+        const bool valid = live && n < p.N;  // N is a multiple of 8, so a group of 4 is all in or all out
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc_u = acc, x_old = acc, x_e = acc;
+        uint2 rv = make_uint2(0u, 0u), wv = rv;
+        if (valid) {
+          // All that the item needs from memory and from the other CTAs is requested before any of it is waited for: one latency instead of one
+          // per CTA of the cluster (projections of an 8B layer in a captured chain, 64 sequences 98.7 -> 97.0 us, one 85.5 -> 83.6; of a 1B
+          // layer 46.5 -> 45.1 and 37.9 -> 36.9).
+          const uint32_t off = static_cast<uint32_t>((m * SK_BM + n4) * 4);
+          if (p.residual) rv = *reinterpret_cast<const uint2*>(p.residual + static_cast<long long>(m) * p.ldr + n);
+          if (p.ssq_out) wv = *reinterpret_cast<const uint2*>(p.norm_w + n);
+          if (p.use_layer && p.layer.x) {
+            x_old = *reinterpret_cast<const float4*>(p.layer.x + m * p.layer.ldx + n);
+            if (p.layer.e) x_e = *reinterpret_cast<const float4*>(p.layer.e + m * p.layer.ldx + n);
+          }
+          if constexpr (decltype(alone)::value) {
+            acc = *reinterpret_cast<const float4*>(smem + off);
+            if (p.swiglu) acc_u = *reinterpret_cast<const float4*>(smem + off + 64 * 4);
+          } else {
+            float4 part[8], part_u[8];      // 8: the largest cluster
 #pragma unroll
-        for (uint32_t r = 0; r < 8; ++r) {
-          if (r < split) {
-            part[r] = ld_dsmem_f4(mapa_shared(part_addr + off, r));
-            if (p.swiglu) part_u[r] = ld_dsmem_f4(mapa_shared(part_addr + off + 64 * 4, r));
-          }
-        }
+            for (uint32_t r = 0; r < 8; ++r) {
+              if (r < split) {
+                part[r] = ld_dsmem_f4(mapa_shared(part_addr + off, r));
+                if (p.swiglu) part_u[r] = ld_dsmem_f4(mapa_shared(part_addr + off + 64 * 4, r));
+              }
+            }
 #pragma unroll
-        for (uint32_t r = 0; r < 8; ++r) {
-          if (r < split) {
-            acc.x += part[r].x; acc.y += part[r].y; acc.z += part[r].z; acc.w += part[r].w;
-            if (p.swiglu) { acc_u.x += part_u[r].x; acc_u.y += part_u[r].y; acc_u.z += part_u[r].z; acc_u.w += part_u[r].w; }
+            for (uint32_t r = 0; r < 8; ++r) {
+              if (r < split) {
+                acc.x += part[r].x; acc.y += part[r].y; acc.z += part[r].z; acc.w += part[r].w;
+                if (p.swiglu) { acc_u.x += part_u[r].x; acc_u.y += part_u[r].y; acc_u.z += part_u[r].z; acc_u.w += part_u[r].w; }
+              }
+            }
+          }
+          if (p.ssq_in) {
+            const float rs = s_rstd[m];
+            acc.x *= rs; acc.y *= rs; acc.z *= rs; acc.w *= rs;
+            acc_u.x *= rs; acc_u.y *= rs; acc_u.z *= rs; acc_u.w *= rs;
+          }
+          if (p.swiglu) {
+            acc.x = acc.x / (1.f + __expf(-acc.x)) * acc_u.x;
+            acc.y = acc.y / (1.f + __expf(-acc.y)) * acc_u.y;
+            acc.z = acc.z / (1.f + __expf(-acc.z)) * acc_u.z;
+            acc.w = acc.w / (1.f + __expf(-acc.w)) * acc_u.w;
+          }
+          if (p.bias) {
+            acc.x += p.bias[n]; acc.y += p.bias[n + 1]; acc.z += p.bias[n + 2]; acc.w += p.bias[n + 3];
+          }
+          if (p.residual) {
+            const float2 r0 = unpack_bf16x2(rv.x), r1 = unpack_bf16x2(rv.y);
+            acc.x += r0.x; acc.y += r0.y; acc.z += r1.x; acc.w += r1.y;
+          }
+          if (p.use_layer) acc = layer_epilogue4(p.layer, acc, m, n, layer_alpha, x_old, x_e);
+          if (p.out_fp32) {
+            *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.Y) + static_cast<long long>(m) * p.ldy + n) = acc;
+          } else if (p.use_layer && lin_gated(p.layer.lin.act)) {
+            *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.Y) + static_cast<long long>(m) * p.ldy + n / 2) = pack_bf16x2(acc.x, acc.y);
+          } else {
+            uint2 o;
+            o.x = pack_bf16x2(acc.x, acc.y);
+            o.y = pack_bf16x2(acc.z, acc.w);
+            *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.Y) + static_cast<long long>(m) * p.ldy + n) = o;
+            if (p.ssq_out) {
+              // what the next norm sees is the bf16 value that was just stored
+              const float2 h0 = unpack_bf16x2(o.x), h1 = unpack_bf16x2(o.y);
+              acc = make_float4(h0.x, h0.y, h1.x, h1.y);
+              const float2 w0 = unpack_bf16x2(wv.x), w1 = unpack_bf16x2(wv.y);
+              uint2 o2;
+              o2.x = pack_bf16x2(acc.x * w0.x, acc.y * w0.y);
+              o2.y = pack_bf16x2(acc.z * w1.x, acc.w * w1.y);
+              *reinterpret_cast<uint2*>(p.Y2 + static_cast<long long>(m) * p.ldy2 + n) = o2;
+            }
           }
         }
-        if (p.ssq_in) {
-          const float rs = s_rstd[m];
-          acc.x *= rs; acc.y *= rs; acc.z *= rs; acc.w *= rs;
-          acc_u.x *= rs; acc_u.y *= rs; acc_u.z *= rs; acc_u.w *= rs;
-        }
-        if (p.swiglu) {
-          acc.x = acc.x / (1.f + __expf(-acc.x)) * acc_u.x;
-          acc.y = acc.y / (1.f + __expf(-acc.y)) * acc_u.y;
-          acc.z = acc.z / (1.f + __expf(-acc.z)) * acc_u.z;
-          acc.w = acc.w / (1.f + __expf(-acc.w)) * acc_u.w;
-        }
-        if (p.bias) {
-          acc.x += p.bias[n]; acc.y += p.bias[n + 1]; acc.z += p.bias[n + 2]; acc.w += p.bias[n + 3];
-        }
-        if (p.residual) {
-          const float2 r0 = unpack_bf16x2(rv.x), r1 = unpack_bf16x2(rv.y);
-          acc.x += r0.x; acc.y += r0.y; acc.z += r1.x; acc.w += r1.y;
-        }
-        if (p.use_layer) acc = layer_epilogue4(p.layer, acc, m, n, layer_alpha, x_old, x_e);
-        if (p.out_fp32) {
-          *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.Y) + static_cast<long long>(m) * p.ldy + n) = acc;
-        } else if (p.use_layer && lin_gated(p.layer.lin.act)) {
-          *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.Y) + static_cast<long long>(m) * p.ldy + n / 2) = pack_bf16x2(acc.x, acc.y);
-        } else {
-          uint2 o;
-          o.x = pack_bf16x2(acc.x, acc.y);
-          o.y = pack_bf16x2(acc.z, acc.w);
-          *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.Y) + static_cast<long long>(m) * p.ldy + n) = o;
-          if (p.ssq_out) {
-            // what the next norm sees is the bf16 value that was just stored
-            const float2 h0 = unpack_bf16x2(o.x), h1 = unpack_bf16x2(o.y);
-            acc = make_float4(h0.x, h0.y, h1.x, h1.y);
-            const float2 w0 = unpack_bf16x2(wv.x), w1 = unpack_bf16x2(wv.y);
-            uint2 o2;
-            o2.x = pack_bf16x2(acc.x * w0.x, acc.y * w0.y);
-            o2.y = pack_bf16x2(acc.z * w1.x, acc.w * w1.y);
-            *reinterpret_cast<uint2*>(p.Y2 + static_cast<long long>(m) * p.ldy2 + n) = o2;
-          }
+        if (p.ssq_out) {
+          float sq = valid ? acc.x * acc.x + acc.y * acc.y + acc.z * acc.z + acc.w * acc.w : 0.f;
+          sq = warp_sum(sq);
+          if (live && (threadIdx.x & 31) == 0) p.ssq_out[n_blk * p.ssq_out_stride + m] = sq;
         }
       }
-      if (p.ssq_out) {
-        float sq = valid ? acc.x * acc.x + acc.y * acc.y + acc.z * acc.z + acc.w * acc.w : 0.f;
-        sq = warp_sum(sq);
-        if (live && (threadIdx.x & 31) == 0) p.ssq_out[n_blk * p.ssq_out_stride + m] = sq;
-      }
-    }
+    };
+    if (split == 1) finish(std::true_type{});
+    else finish(std::false_type{});
   }
   cluster.sync();  // peers may still be reading this CTA's partial tile
 }
