@@ -463,6 +463,8 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int seq0 = blockIdx.x * p.rows, kvh = blockIdx.y, split = blockIdx.z;
   const int rows = min(p.rows, p.B - seq0), G = p.G, Hq = p.Hkv * G, bs = p.block_size;
+  auto row_of = [&](int c) { return RUNS ? c / G : 0; };      // column c: which sequence of the group, and which of its heads
+  auto head_of = [&](int c) { return RUNS ? c % G : c; };
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(k_full), 1);
     mbar_init(smem_u32(k_empty), 1);
@@ -510,7 +512,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     const int which = i / (Cfg::QP_BYTES / 16), j = i % (Cfg::QP_BYTES / 16);
     const int c = j / 16, piece = j % 16;
     if (which == 0 && c < rows * G && piece < HD / 8) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(p.q + (seq0 + c / G) * p.q_stride + static_cast<long long>(kvh * G + c % G) * HD + piece * 8);
+      const uint4 raw = *reinterpret_cast<const uint4*>(p.q + (seq0 + row_of(c)) * p.q_stride + static_cast<long long>(kvh * G + head_of(c)) * HD + piece * 8);
       const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
       uint32_t o[4];
 #pragma unroll
@@ -552,6 +554,8 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   // tile i of this CTA: its sequence of the group (-1: all of them) and its first token
   auto tile_at = [&](int i, int& j) {
     i += i_begin;
+    j = 0;
+    if (!RUNS) return i * DM_TOK;
     j = -1;
     if (i < shared) return i * DM_TOK;
     j = 0;
@@ -626,8 +630,8 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         const uint32_t ph = i & 1;
         if (i + 1 < n_tiles) ok = issue_qk(i + 1);   // overlaps the softmax of tile i
         if (!ok) break;
-        int j = 0;
-        if (RUNS) tile_at(i, j);
+        int j;
+        tile_at(i, j);
         const bool fresh = j != run;
         run = j;
         if (!mbar_wait(smem_u32(p_ready), ph, abort_flag, p.status, RLB_ERR_WAIT_FLAG) ||
@@ -658,7 +662,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
       m_run[c] = -INFINITY;
       l_own[c] = o_run[c] = 0.f;
     }
-    uint32_t last = 0;      // columns whose P differs from zero
+    uint32_t last = 0;      // columns that the tile before concerned
     int run = -2;
     bool ok = true;
     for (int i = 0; i < n_tiles; ++i) {
@@ -669,7 +673,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
 #pragma unroll
       for (int k = 1; k < DG_ROWS; ++k) n = j == k ? len[k] : n;
       const bool valid = j < 0 || tok < n;
-      const uint32_t active = j < 0 ? live : ((1u << G) - 1u) << (j * G);
+      const uint32_t active = !RUNS ? 0xffffffffu : j < 0 ? live : ((1u << G) - 1u) << (j * G);      // (columns behind the heads are computed and not used)
       float* red_max = red + ph * 4 * DM_N;
       ok = ok && mbar_wait(smem_u32(s_full), ph, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
       if (!ok) {      // every warp meets every barrier, also after a wait that ran out
@@ -683,34 +687,38 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(s_empty));
+      // Columns go in fours, so that their chains of shuffles and exponentials overlap (with a branch for each column they ran one after the other).
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (!(active >> c & 1)) continue;
-        if (!valid) sr[c] = 0xff800000u;   // -inf
-        float mx = __uint_as_float(sr[c]);
+      for (int c0 = 0; c0 < NC; c0 += 4) {
+        if (RUNS && !(active >> c0 & 15u)) continue;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        if (lane == 0) red_max[quarter * DM_N + c] = mx;
+        for (int c = c0; c < c0 + 4; ++c) {
+          if (!valid || !(active >> c & 1)) sr[c] = 0xff800000u;   // -inf
+          float mx = __uint_as_float(sr[c]);
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+          if (lane == 0) red_max[quarter * DM_N + c] = mx;
+        }
       }
       named_bar_sync(1, 128);   // (this tile's half of `red` is written again two tiles on, behind the next tile's barrier)
       uint32_t moved = 0;       // columns whose O has to be scaled
       float k[NC];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        k[c] = 1.f;
-        if (!(active >> c & 1)) continue;
-        const float mt = fmaxf(fmaxf(red_max[c], red_max[DM_N + c]), fmaxf(red_max[2 * DM_N + c], red_max[3 * DM_N + c]));
-        if (mt > m_run[c] + DG_SLACK || m_run[c] == -INFINITY) {      // the same in all threads
-          if (m_run[c] != -INFINITY) {
-            k[c] = __expf(m_run[c] - mt);
-            l_own[c] *= k[c];
-            moved |= 1u << c;
-          }
-          m_run[c] = mt;
+      for (int c0 = 0; c0 < NC; c0 += 4) {
+#pragma unroll
+        for (int c = c0; c < c0 + 4; ++c) k[c] = 1.f;
+        if (RUNS && !(active >> c0 & 15u)) continue;      // (their scores are not read: P of these columns is written as zeros below)
+#pragma unroll
+        for (int c = c0; c < c0 + 4; ++c) {
+          const float mt = fmaxf(fmaxf(red_max[c], red_max[DM_N + c]), fmaxf(red_max[2 * DM_N + c], red_max[3 * DM_N + c]));
+          const bool move = mt > m_run[c] + DG_SLACK, scaled = move && m_run[c] != -INFINITY;      // the same in all threads
+          if (scaled) moved |= 1u << c;
+          k[c] = scaled ? __expf(m_run[c] - mt) : 1.f;
+          m_run[c] = move ? mt : m_run[c];
+          const float s = __uint_as_float(sr[c]), pr = s == -INFINITY ? 0.f : __expf(s - m_run[c]);
+          l_own[c] = l_own[c] * k[c] + pr;
+          sr[c] = __float_as_uint(pr);
         }
-        const float s = __uint_as_float(sr[c]), pr = s == -INFINITY ? 0.f : __expf(s - m_run[c]);
-        l_own[c] += pr;
-        sr[c] = __float_as_uint(pr);
       }
       if (i > 0) {      // the previous product has read P and written O
         ok = mbar_wait(smem_u32(o_full), ph ^ 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
@@ -736,9 +744,12 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         }
       }
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if ((active | last) >> c & 1)
-          *reinterpret_cast<__nv_bfloat16*>(p_sm + sw128_off(c, r, DM_N * 128)) = __float2bfloat16(active >> c & 1 ? __uint_as_float(sr[c]) : 0.f);
+      for (int c0 = 0; c0 < NC; c0 += 4) {
+        if (RUNS && !((active | last) >> c0 & 15u)) continue;
+#pragma unroll
+        for (int c = c0; c < c0 + 4; ++c)
+          *reinterpret_cast<__nv_bfloat16*>(p_sm + sw128_off(c, r, DM_N * 128)) = __float2bfloat16(active >> c0 & 15u ? __uint_as_float(sr[c]) : 0.f);
+      }
       last = active;
       fence_proxy_async();           // P^T is read by the tensor core (async proxy)
       tc_fence_before();
@@ -760,8 +771,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     float* s_ml = red + 4 * DM_N;         // [16][2] merged by the cluster
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      if (c >= rows * G) break;
-      const float l = warp_sum(l_own[c]);
+      const float l = warp_sum(l_own[c]);      // (all columns: with a way out of the loop the sums came one after the other)
       if (lane == 0) red_sum[quarter * DM_N + c] = l;
     }
     named_bar_sync(1, 128);
@@ -770,7 +780,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     for (int c = 0; c < NC; ++c) {
       if (c >= rows * G) break;
       const float l = (red_sum[c] + red_sum[DM_N + c]) + (red_sum[2 * DM_N + c] + red_sum[3 * DM_N + c]);
-      const int seq = seq0 + c / G, hq = kvh * G + c % G;
+      const int seq = seq0 + row_of(c), hq = kvh * G + head_of(c);
       if (p.in_cluster) {
         if (r < HD) o_sm[c * HD + r] = o_run[c];
         if (r == 0) {
@@ -818,7 +828,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         ll += ls[z] * k;
         acc += os[z] * k;
       }
-      __nv_bfloat16* dst = p.out + (seq0 + c / G) * p.out_stride + static_cast<long long>(kvh * G + c % G) * HD + d;
+      __nv_bfloat16* dst = p.out + (seq0 + row_of(c)) * p.out_stride + static_cast<long long>(kvh * G + head_of(c)) * HD + d;
       *dst = __float2bfloat16(dm_gated(ll > 0.f ? acc / ll : 0.f, dst, p.gated));
     }
     cluster_sync();        // the others may still read this CTA's results
