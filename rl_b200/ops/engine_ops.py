@@ -76,23 +76,32 @@ def choose_splits(B: int, Hkv: int, max_len: int, block_size: int, sm_count: int
     """KV splits of paged decoding, never finer than one cache block per split. Without ``Hq``: ~2 CTAs on every SM. With ``Hq``: for the plain
     kernel (``rlb_paged_decode_group``), of which three CTAs fit on an SM and whose groups' tiles are cut evenly: one wave of CTAs, of the
     largest groups that need at most four splits for it (16 sequences of 4000 tokens take 51 us alone with three splits, 53 us in twos with
-    six). Up to eight splits merge inside a cluster; more cost a second kernel and are taken only where eight leave SMs without work."""
+    six). Up to eight splits merge inside a cluster; more cost a second kernel and are taken only where eight leave SMs without work. Where
+    one split each is as much as fits, or more, up to four (two, beyond two waves) that fill the last wave better, of eight tiles and more (8 KV heads
+    of 128, four query heads each: 64 sequences of 3000 tokens with one split 176 us, with three 136; 128 of 4000 444 and, with four, 352; 256 of 2000
+    372 and, with two, 355, with three 389; but 128 of 500 66 and, with two, 68. One query head each, 256 of 1000: 223 and, with three, 192).
+    Sequences of one whole tile are not split (256 of 200 tokens, one KV head: 9 us, with three splits 14)."""
     forced = os.environ.get("RLB_DECODE_SPLITS")
     if forced:
         return max(1, int(forced))
     B = max(1, B)
+    tiles = max(1, max_len // max(block_size, 128))
     if Hq:
+        slots = 3 * sm_count
         for rows in (4, 2, 1):
             ctas = -(-B // rows) * Hkv
-            want = max(1, 3 * sm_count // ctas)
+            want = max(1, slots // ctas)
             if rows == 1 or (rows * (Hq // Hkv) <= 8 and want <= 4):
                 break
-        if want > 8 and ctas * 8 >= sm_count:
+        if want == 1:
+            most = 4 if ctas <= 2 * slots else 2
+            want = min((n for n in range(1, most + 1) if n == 1 or rows * tiles >= 8 * n), key=lambda n: (-(-ctas * n // slots) / n, n))
+        elif want > 8 and ctas * 8 >= sm_count:
             want = 8
-        return int(max(1, min(want, max(1, rows * max_len // max(block_size, 128)), 32)))
+        return int(max(1, min(want, rows * tiles if tiles > 1 else 1, 32)))
     ctas = B * Hkv
     want = max(1, (2 * sm_count + ctas - 1) // ctas)
-    return int(max(1, min(want, max(1, max_len // max(block_size, 128)), 32)))
+    return int(max(1, min(want, tiles, 32)))
 
 
 def _paged_decode_gather(q, k_cache, v_cache, block_table, seq_lens, Hq, Hkv, D, scale, out, rows_per_chunk: int = 64, window: int = 0, chunk: int = 0):

@@ -286,3 +286,21 @@ def test_rollout_routing_replay_end_to_end():
     train = BatchedDataDict(input_ids=out["output_ids"], input_lengths=tot, token_mask=tm, sample_mask=torch.ones(3), routed_experts=re)
     res = w.train(train.slice(0, 2), NLLLossFn(), gbs=2, mbs=2)
     assert torch.isfinite(res["loss"]).all()
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(32, 8), (32, 4), (8, 8), (4, 1), (64, 8)])
+@pytest.mark.parametrize("block_size", [16, 64, 256])
+def test_decode_splits(Hq, Hkv, block_size):
+    """Splits of the grouped decode kernel: never more than the tiles of a group, no group of more than eight query heads, and where one wave of
+    CTAs is full, more splits only where the last wave is the fuller for it."""
+    from rl_b200.ops.engine_ops import choose_splits, group_rows
+
+    for B in (1, 2, 7, 16, 33, 64, 100, 128, 256, 300):
+        for n in (1, 100, 255, 256, 300, 1000, 4000, 30000):
+            s = choose_splits(B, Hkv, n, block_size, 148, Hq)
+            rows = group_rows(B, Hq, Hkv, s)
+            tiles = max(1, n // max(block_size, 128))
+            assert 1 <= s <= min(32, 4 * tiles) and (s == 1 or tiles > 1) and (rows == 1 or rows * (Hq // Hkv) <= 8)
+            ctas = -(-B // rows) * Hkv
+            if ctas > 444 and s > 1:
+                assert s <= 4 and -(-ctas * s // 444) < s * -(-ctas // 444)
