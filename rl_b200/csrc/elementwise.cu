@@ -78,8 +78,10 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
 }
 
 // The same without a residual for many rows: one warp per row, which stays in registers between the two passes, all its loads in flight and no
-// barrier. NV: pieces of 8 elements per lane. From 8 rows per SM on: with fewer, several warps per row are sooner done. 20480 rows of 4096:
-// 99 us with a CTA per row, now 69 us (4.9 TB/s).
+// barrier. NV: pieces of 8 elements per lane. Wide rows leave two CTAs to an SM, so that a few thousand of them end in a nearly empty wave and
+// a CTA per row is sooner done. Timed with a flushed cache, CTA per row -> warp per row, us: d 1024: 2000 rows 8.2 -> 10.2, 2368 8.2 -> 8.2,
+// 8000 14.5 -> 12.3; d 2048: 3000 12.3 -> 14.3, 8000 20.5 -> 20.5, 20480 43 -> 35; d 4096: 4000 22.5 -> 26.6, 8000 38.9 -> 38.9,
+// 20480 84 -> 72; d 5120: 8000 49 -> 51, 20480 109 -> 98.
 template <int NV>
 __global__ void __launch_bounds__(256, 2) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                                            float* __restrict__ rstd_out, long long rows, int d, long long x_stride, long long y_stride, float eps) {
@@ -925,7 +927,7 @@ RLB_API int rlb_rmsnorm_fwd(const void* x, const void* res, const void* w, void*
                             void* stream) {
   if (rows <= 0) return 0;
   if (d % 8 || x_stride % 8 || y_stride % 8) return -2;
-  if (!res && rows >= 148 * 8 && d <= 5120) {
+  if (!res && d <= 5120 && rows >= 148ll * (d <= 1024 ? 16 : d <= 4096 ? 48 : 96)) {
     auto kern = d <= 1024 ? rmsnorm_rows_kernel<4> : d <= 2048 ? rmsnorm_rows_kernel<8> : d <= 4096 ? rmsnorm_rows_kernel<16> : rmsnorm_rows_kernel<20>;
     rlb_launch_pdl(kern, dim3(static_cast<unsigned>((rows + 7) / 8)), dim3(256), 0, S(stream), CBF(x), CBF(w), BF(y), rstd, rows, d, x_stride, y_stride, eps);
     return static_cast<int>(cudaGetLastError());
