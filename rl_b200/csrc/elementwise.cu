@@ -298,7 +298,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict
 
 // The same for head dimensions that are multiples of 16 and 16-byte aligned rows: a block takes `block_rows` rows, computes their angles once
 // and moves 16 bytes at a time (one warp per head recomputed 64 sines and cosines for each: 20480 rows of 40 heads of 128 took 169 us,
-// now 85 us, 4.4 TB/s).
+// now 85 us, 4.4 TB/s). From so many heads on that the SMs have several warps anyway: with fewer, a warp per head does not wait for a block's
+// angles (us in a captured chain, warp per head / block: 40 heads of 128, 64 rows 1.9 / 2.4, 128 rows 2.5 / 2.2; heads of 64, 8 rows 1.6 / 1.7, 64 rows 1.9 / 1.8).
 __global__ void __launch_bounds__(256) rope_rows_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict__ pos, const float* __restrict__ inv_freq, long long rows, int heads, int D,
                                                         long long row_stride, float sign, int block_rows) {
   extern __shared__ __align__(16) float2 rope_cs[];
@@ -963,8 +964,8 @@ RLB_API int rlb_rope(void* x, const int* pos, const float* inv_freq, long long r
                      long long row_stride, int backward, void* stream) {
   if (rows <= 0) return 0;
   if (D % 4) return -2;
-  if (!(D % 16) && D <= 512 && !(row_stride % 8) && !(reinterpret_cast<uintptr_t>(x) & 15)) {
-    const int block_rows = rows >= 148 * 16 ? 4 : 1;      // enough blocks for every SM before a block takes several rows
+  if (!(D % 16) && D <= 512 && !(row_stride % 8) && !(reinterpret_cast<uintptr_t>(x) & 15) && rows * heads > (D < 128 ? 512 : 4096)) {
+    const int block_rows = rows >= 148 * 16 ? 4 : 1;      // enough blocks for every SM before a block takes several rows (2368: 16.4 us either way, 20480: 74 and 78)
     rlb_launch_pdl(rope_rows_kernel, dim3(static_cast<unsigned>((rows + block_rows - 1) / block_rows)), dim3(256), block_rows * D / 2 * sizeof(float2), S(stream), BF(x), pos, inv_freq,
                    rows, heads, D, row_stride, backward ? -1.f : 1.f, block_rows);
     return static_cast<int>(cudaGetLastError());

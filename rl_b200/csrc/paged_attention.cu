@@ -97,7 +97,8 @@ __global__ void rope_kv_write_kernel(__nv_bfloat16* __restrict__ qkv, const int*
 
 // The same for head dimensions that are multiples of 16 and 16-byte aligned rows (the caches' heads are aligned then): a block takes `block_rows`
 // tokens, computes their angles once and moves 16 bytes at a time. One warp per head, as above, recomputed the sines and cosines for each:
-// 15000 tokens of 32 + 2 * 8 heads of 128, 208 -> 81 us.
+// 15000 tokens of 32 + 2 * 8 heads of 128, 208 -> 81 us. With fewer heads in all, as in most decode steps, a warp per head is sooner done (us in a
+// captured chain, warp per head / block: 48 heads of 128, 8 tokens 1.9 / 2.8, 64 2.1 / 3.0, 128 3.2 / 2.8; heads of 64, 8 2.0 / 2.0, 128 3.2 / 2.0).
 __global__ void __launch_bounds__(256) rope_kv_rows_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos, const float* __restrict__ inv_freq, const long long* __restrict__ slots,
                                                            __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, long long T, int Hq, int Hkv, int D, int block_size,
                                                            long long row_stride, long long num_slots, int* status, int block_rows) {
@@ -410,8 +411,8 @@ RLB_API int rlb_rope_kv_cache_write(void* qkv, const int* pos, const float* inv_
   if (T <= 0) return 0;
   if (D % 4 || row_stride % 2) return -2;
   if (!(D % 16) && D <= 512 && !(row_stride % 8) &&
-      !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15)) {
-    const int block_rows = T >= 148 * 16 ? 4 : 1;      // enough blocks for every SM before a block takes several tokens
+      !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) && T * (Hq + 2 * Hkv) > (D < 128 ? 512 : 4096)) {
+    const int block_rows = T >= 148 * 16 ? 4 : 1;      // enough blocks for every SM before a block takes several tokens (2368: 18.4 us either way, 20480: 94 and 99)
     rlb_launch_pdl(rope_kv_rows_kernel, dim3(static_cast<unsigned>((T + block_rows - 1) / block_rows)), dim3(256), block_rows * D / 2 * sizeof(float2), static_cast<cudaStream_t>(stream),
                    reinterpret_cast<__nv_bfloat16*>(qkv), pos, inv_freq, slots, reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache), T, Hq, Hkv, D, block_size,
                    row_stride, num_blocks * block_size, status, block_rows);
