@@ -1087,7 +1087,7 @@ RLB_API int rlb_adamw(void* p, void* p_lo, float* p32, const void* g, int grad_i
 // out += sum(x^2). `out` is a device float the caller zeroes.
 RLB_API int rlb_sumsq(const void* x, int is_bf16, long long n, float* out, void* stream) {
   if (n <= 0) return 0;
-  const int grid = grid_for(n, 1024, 148 * 8);
+  const int grid = grid_for(n, 1024, n < (1 << 24) ? 148 * 4 : 148 * 8);      // (few elements: half as many sums to add up)
   if (is_bf16) sumsq_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(CBF(x), n, out);
   else sumsq_kernel<float><<<grid, 256, 0, S(stream)>>>(reinterpret_cast<const float*>(x), n, out);
   return static_cast<int>(cudaGetLastError());
