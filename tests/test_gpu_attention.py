@@ -96,3 +96,24 @@ def test_flash_fwd_scales(native_lib, D, scale):
     assert check_status() == 0 and bool(lse.isfinite().all())
     ref = F._attention_ref(qkv.float(), cu, 4, 2, D, scale)
     assert (out.float() - ref).abs().max() < 3e-2
+
+
+@pytest.mark.parametrize("D", [128, 64])
+def test_flash_many_sequences(native_lib, D):
+    """More sequences than a warp has lanes, empty ones among them and at both ends."""
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import check_status
+
+    lens = [0] + [(7 * i) % 5 * 37 + i % 3 for i in range(71)] + [0, 0]
+    Hq, Hkv = 4, 2
+    qkv, cu, D = _case(lens, Hq, Hkv, seed=5, D=D)
+    x = qkv.clone().requires_grad_()
+    y = F.attention_varlen(x, cu, max(lens), Hq, Hkv, D)
+    g = torch.randn_like(y)
+    y.backward(g)
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    xr = qkv.float().requires_grad_()
+    yr = F._attention_ref(xr, cu, Hq, Hkv, D, 1.0 / math.sqrt(D))
+    yr.backward(g.float())
+    assert (y.float() - yr).abs().max() <= 3e-2 and (x.grad.float() - xr.grad).abs().max() <= 3e-2 * xr.grad.abs().max()

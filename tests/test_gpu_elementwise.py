@@ -469,7 +469,7 @@ def test_adamw_groups_of_eight(native_lib, n, shift, gdtype):
 @pytest.mark.parametrize("n", [1, 3, 8, 1000003])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_sumsq_sizes(native_lib, n, dtype):
-    """Against float64; fp32 partial sums of at most some hundred terms each: 1e-5 relative."""
+    """Against float64: sums of four or eight squares and of the blocks are fp32, some 1e-6 relative at these sizes."""
     from rl_b200.ops import functional as F
 
     x = torch.randn(n + 1, device="cuda").to(dtype)
@@ -479,8 +479,39 @@ def test_sumsq_sizes(native_lib, n, dtype):
         assert abs(out.item() - part.double().pow(2).sum().item()) <= 1e-5 * part.double().pow(2).sum().item()
 
 
+def test_sumsq_small_beside_large(native_lib):
+    """A large value in every 660, the others' squares nine tenths of half a unit in the last place of its square: fp32 sums over a thread's hundreds
+    of terms lose those that come after it, 1.7e-5 of the total. In fp64 the 1184 additions of block sums remain, whose roundings of at most 2^-24 of
+    the total each add up like sqrt(1184): 2e-6."""
+    from rl_b200.ops import functional as F
+
+    n = 100_000_000
+    x = torch.full((n,), (0.9 * 2.0 ** -12) ** 0.5, device="cuda")      # 64^2 = 2^12: half its last place is 2^-12
+    x[::660] = 64.0
+    out = torch.zeros(1, device="cuda")
+    F.sumsq_(x, out)
+    ref = sum(c.double().pow(2).sum().item() for c in x.split(10_000_000))
+    assert abs(out.item() - ref) <= 5e-6 * ref
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T,heads", [(5, 12), (300, 20), (2400, 4)])      # a warp per head, one row per block, four rows per block
+def test_rope_long_positions(native_lib, D, T, heads):
+    """Positions of thousands of tokens. The angle is rounded to fp32, and once more in the fast sines' reduction to a period: 2^-23 of it, which
+    turns a pair of values below 6 by as much; then one rounding of the result."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(D + T)
+    x = torch.randn(T, heads * D, generator=g, device="cuda").bfloat16().clamp(-6, 6)
+    pos = torch.randint(4000, 16000, (T,), generator=g, device="cuda", dtype=torch.int32)
+    inv = 1.0 / 10000.0 ** (torch.arange(0, D, 2, device="cuda").float() / D)
+    ref = F._rope_ref(x.double(), pos, inv.double(), heads, D)
+    F.call("rlb_rope", x.data_ptr(), pos.data_ptr(), inv.data_ptr(), T, heads, D, x.stride(0), 0, F.stream_ptr())
+    assert (x.double() - ref).abs().max() <= 2.0 ** -9 * 8.5 + 2.0 ** -23 * 16000 * 6 * 2 ** 0.5
+
+
 @pytest.mark.parametrize("D", [16, 64, 96, 128, 256])
-@pytest.mark.parametrize("T,heads", [(1, 3), (5, 12), (2371, 5)])      # one row per block, four rows per block and a cut last block
+@pytest.mark.parametrize("T,heads", [(1, 3), (5, 12), (2371, 5)])      # a warp per head, four rows per block and a cut last block
 @pytest.mark.parametrize("pad", [0, 8, 4])                             # a row stride without 16-byte alignment takes the plain kernel
 def test_rope_rows(native_lib, D, T, heads, pad):
     """Both directions against the fp32 statement: one rounding of the result (2^-8 of values up to 8) and the fast sines (2e-6 at these angles)."""
