@@ -394,7 +394,7 @@ class _QKNorm(torch.autograd.Function):
         buf, wq, wk, rstd = ctx.saved_tensors
         Hq, Hkv, D = ctx.meta
         T = buf.shape[0]
-        dout = dout if dout.stride(1) == 1 and dout.stride(0) % 2 == 0 else dout.contiguous()
+        dout = dout if dout.stride(1) == 1 and dout.stride(0) % 2 == 0 and dout.data_ptr() % 4 == 0 else dout.clone(memory_format=torch.contiguous_format)
         dbuf = torch.empty(buf.shape, dtype=buf.dtype, device=buf.device)
         part = torch.empty((max(1, _L.lib().rlb_qk_rmsnorm_bwd_parts(T)), 2, D), dtype=torch.float32, device=buf.device)
         dw = torch.zeros((2, D), dtype=torch.float32, device=buf.device)

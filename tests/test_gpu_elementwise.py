@@ -586,6 +586,21 @@ def test_qk_rmsnorm(native_lib, D, T, Hq, Hkv):
         assert F.qk_rmsnorm(z, wq, wk, Hq, Hkv, D, 1e-6) is z and torch.equal(z, y)
 
 
+def test_qk_rmsnorm_gradient_at_an_odd_place(native_lib):
+    """A gradient that is a slice of a wider one and starts at an odd element: its pairs are not aligned, and it is copied first."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(1)
+    x, up = (torch.randn(9, 4 * 64, generator=g, device="cuda").bfloat16() for _ in range(2))
+    w = torch.ones(64, device="cuda").bfloat16()
+    x.requires_grad_()
+    wide = torch.zeros(9, 4 * 64 + 2, device="cuda", dtype=torch.bfloat16)
+    wide[:, 1:-1] = up
+    grads = [torch.autograd.grad(F.qk_rmsnorm(x, w, w, 2, 1, 64, 1e-6), x, u)[0] for u in (up, wide[:, 1:-1])]
+    torch.cuda.synchronize()
+    assert torch.equal(*grads)
+
+
 @pytest.mark.parametrize("d", [8, 512, 1032, 2048, 4096, 5120, 5128])      # one register count each, cut rows of pieces, beyond the last
 @pytest.mark.parametrize("rows", [3, 1184, 1187])                           # a CTA per row; a warp per row, a cut last CTA
 def test_rmsnorm_many_rows(native_lib, d, rows):
