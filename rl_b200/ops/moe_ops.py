@@ -191,6 +191,7 @@ class _ExpertLayer(torch.autograd.Function):
         w, gate_up, down, xp, h, a, y = ctx.saved_tensors
         plan, (d, f), dev = ctx.plan, (xp.shape[1], a.shape[1]), xp.device
         g = dout.contiguous()
+        g = g if g.data_ptr() % 16 == 0 else g.clone()
         dy, dw = torch.empty_like(y), torch.zeros_like(w)
         call("rlb_moe_combine_rows_bwd", ptr(g), ptr(y), ptr(plan.row_copy), ptr(plan.tile_expert), ptr(w), plan.k, ptr(dy), ptr(dw), plan.mpad, d, stream_ptr())
         d_down = _grouped_wgrad(dy, a, down, plan) if ctx.needs_input_grad[4] else None
@@ -215,8 +216,9 @@ def expert_layer_takes(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
 def expert_layer(x: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, residual, gate_up: torch.Tensor, down: torch.Tensor) -> torch.Tensor:
     """(residual +) sum_j w[t, j] MLP_{idx[t, j]}(x[t]) for tokens ``x`` [T, d]; ``idx``, ``w`` [T, k]. The sum over a token's experts is fp32
     and in their order."""
-    def rows(t):
-        return t if t is None or (t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 and t.dtype == BF16) else t.to(BF16).contiguous()
+    def rows(t):      # (contiguous() would leave rows that start at an odd place where they are)
+        fits = t is None or (t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 and t.dtype == BF16)
+        return t if fits else t.to(BF16).clone(memory_format=torch.contiguous_format)
 
     return _ExpertLayer.apply(rows(x), w.float().contiguous(), rows(residual), gate_up, down, TokenPlan(idx, gate_up.shape[0]))
 

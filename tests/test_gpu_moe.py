@@ -212,6 +212,30 @@ def test_expert_layer(native_lib, T, E, k, skew, residual):
     assert gu.grad[counts == 0].abs().sum() == 0 and dn.grad is None
 
 
+@pytest.mark.parametrize("what", ["tokens", "residual", "gradient"])
+def test_expert_layer_rows_at_an_odd_place(native_lib, what):
+    """Contiguous rows that do not start on 16 bytes are copied first: the same values as from aligned ones."""
+    from rl_b200.ops import moe_ops as M
+    from rl_b200.ops.lib import check_status
+
+    g = torch.Generator("cuda").manual_seed(7)
+    T, d, f, E, k = 40, 128, 64, 4, 2
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    x, res, up, w = r(T, d).bfloat16(), r(T, d).bfloat16(), r(T, d).bfloat16(), torch.softmax(r(T, k), -1)
+    gu, dn, idx = (0.2 * r(E, 2 * f, d)).bfloat16(), (0.2 * r(E, d, f)).bfloat16(), r(T, E).topk(k, -1)[1]
+    odd = lambda t: torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(t.shape)      # noqa: E731
+
+    def run(x, res, up):
+        x, res = x.detach().requires_grad_(), res.detach().requires_grad_()
+        y = M.expert_layer(x, idx, w, res, gu, dn)
+        return [y, *torch.autograd.grad(y, (x, res), up)]
+
+    plain = run(x, res, up)
+    moved = run(odd(x) if what == "tokens" else x, odd(res) if what == "residual" else res, odd(up) if what == "gradient" else up)
+    torch.cuda.synchronize()
+    assert check_status() == 0 and all(torch.equal(a, b) for a, b in zip(plain, moved))
+
+
 @pytest.mark.parametrize("T,E,k,load", [(1, 8, 2, 32), (33, 16, 4, 32), (126, 64, 8, 32), (60, 16, 6, 64), (64, 8, 4, 64), (128, 8, 4, 128)])
 @pytest.mark.parametrize("one", [False, True])
 def test_few_token_layer(native_lib, T, E, k, load, one):
