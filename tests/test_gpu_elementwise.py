@@ -602,7 +602,7 @@ def test_qk_rmsnorm_gradient_at_an_odd_place(native_lib):
 
 
 @pytest.mark.parametrize("d", [8, 512, 1032, 2048, 4096, 5120, 5128])      # one register count each, cut rows of pieces, beyond the last
-@pytest.mark.parametrize("rows", [3, 1184, 1187])                           # a CTA per row; a warp per row, a cut last CTA
+@pytest.mark.parametrize("rows", [3, 1184, 1187])                           # a CTA per row
 def test_rmsnorm_many_rows(native_lib, d, rows):
     """Values, statistics and both gradients against float64: one bf16 rounding of a result (2^-8), a few in the gradient's two terms."""
     from rl_b200.ops import functional as F
@@ -618,6 +618,22 @@ def test_rmsnorm_many_rows(native_lib, d, rows):
     ref.backward(up.double())
     near = lambda a, b, t: (a.double() - b).norm() <= t * b.norm()      # noqa: E731
     assert near(y, ref, 2.0 ** -8) and near(x.grad, X.grad, 2.0 ** -7) and near(w.grad, W.grad, 2.0 ** -7)
+
+
+@pytest.mark.parametrize("d,rows", [(8, 2368), (512, 2371), (1024, 2368), (1032, 7109), (2048, 7104), (4096, 7109), (4104, 14213), (5120, 14208)])
+def test_rmsnorm_warp_rows(native_lib, d, rows):
+    """A warp per row: the first size that takes it, a cut last CTA, every register count. Against the fp32 statement: one bf16 rounding (2^-8)."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(d)
+    wide = torch.randn(rows, d + 8, generator=g, device="cuda").bfloat16()
+    x, w, y = wide[:, :d], (1 + 0.3 * torch.randn(d, generator=g, device="cuda")).bfloat16(), torch.zeros(rows + 1, d, dtype=torch.bfloat16, device="cuda")
+    rstd = torch.empty(rows, device="cuda")
+    F.call("rlb_rmsnorm_fwd", x.data_ptr(), None, w.data_ptr(), y.data_ptr(), None, rstd.data_ptr(), rows, d, x.stride(0), d, 1e-6, F.stream_ptr())
+    s = torch.rsqrt(x.float().pow(2).mean(-1) + 1e-6)
+    assert (rstd - s).abs().max() <= 1e-5 * s.max() and y[rows].abs().sum() == 0
+    ref = x.float() * s[:, None] * w.float()
+    assert ((y[:rows].float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6).all()
 
 
 @pytest.mark.parametrize("M", [1, 31, 33, 300])
