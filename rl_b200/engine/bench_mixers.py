@@ -177,7 +177,7 @@ def decode_ms(eng, n: int, ctx: int, steps: int, warmup: int) -> float:
         st["slots"][:n] = (st["block_table"][:n, per - 1].long() * 64 + 63)
 
     prev = E.skinny_static_weights(True)
-    splits = E.choose_splits(B, eng.hkv, max(eng.max_model_len // 2, 1), 64, eng._sm_count)
+    splits = E.choose_splits(B, eng.hkv, max(eng.max_model_len // 2, 1), 64, eng._sm_count, eng.hq)
     no, nml = E.decode_scratch_sizes(B, eng.hq, splits, eng.cfg.head_dim)
     scratch = (torch.empty(no, dtype=torch.float32, device="cuda"), torch.empty(nml, dtype=torch.float32, device="cuda")) if splits > 1 else None
     reset()
@@ -241,7 +241,7 @@ def kernel_table(name: str) -> list:
             nb = n * ctx * H * 128 * 2 * 2
             sets = copies(lambda: (torch.randn(n, 3 * H * 128, device=dev).to(bf), torch.randn(n * ctx // 64, H, 64, 128, device=dev).to(bf),
                                    torch.randn(n * ctx // 64, H, 64, 128, device=dev).to(bf)), nb)
-            sp = E.choose_splits(n, H, ctx // 2, 64)
+            sp = E.choose_splits(n, H, ctx // 2, 64, Hq=H)
             add(f"like: paged decode attention, {n} x {ctx}", timed_graph([lambda s=s: E.paged_decode(s[0], s[1], s[2], b.block_table, b.seq_lens, H, H, 128,
                                                                                                    num_splits=sp) for s in sets]), 4.0 * n * ctx * H * 128, nb)
             del sets
@@ -386,7 +386,7 @@ def redarax_table(name: str) -> list:
             nb = n * ctx * G * (m.dim + m.vdim) * 2
             sets = copies(lambda: (rows(n, m.in_width), *(torch.randn(n * ctx // 64, G, 64, w, device=dev).to(bf) for w in (m.dim, m.vdim))), nb)
             add(f"attention decode (all kernels), {n} x {ctx}", timed_graph([lambda s=s: S.attention(s[0], m, b, s[1], s[2]) for s in sets]), 4.0 * n * ctx * H * m.dim, nb)
-            sp = E.choose_splits(n, G, ctx // 2, 64)
+            sp = E.choose_splits(n, G, ctx // 2, 64, Hq=H)
             add("like: paged decode attention", timed_graph([lambda s=s: E.paged_decode(s[0][:, : H * m.dim], s[1], s[2], b.block_table, b.seq_lens, H, G, m.dim,
                                                                                       num_splits=sp) for s in sets]), 4.0 * n * ctx * H * m.dim, nb)
             del sets
@@ -504,7 +504,7 @@ def kikivik_table(name: str) -> list:
                 add(f"{label} decode (all kernels), {n} rows, {seen} keys seen", timed_graph([lambda s=s: S.attention(s[0], mx, b, s[1], s[2], s[3] if mx.v_mix else None) for s in sets]),
                     4.0 * n * seen * H * g.dim, nb)
                 if mx is twin:
-                    sp = E.choose_splits(n, G, seen // 2, 64)
+                    sp = E.choose_splits(n, G, seen // 2, 64, Hq=H)
                     add("like: paged decode attention", timed_graph([lambda s=s: E.paged_decode(s[0][:, : H * g.dim], s[1], s[2], b.block_table, b.seq_lens, H, G, g.dim, num_splits=sp)
                                                                      for s in sets]), 4.0 * n * seen * H * g.dim, nb)
                 del sets
