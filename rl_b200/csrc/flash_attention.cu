@@ -18,8 +18,8 @@
 // (before: one score buffer, P through shared memory): 16 x 4096 tokens 3.77 -> 2.24 ms (984 TFLOP/s); 64 x 1280 2.02 -> 1.18 ms.
 // Output: O[T, Hq*128] bf16 and the per-row log-sum-exp lse[Hq, T] (natural log) for the backward pass.
 //
-// Backward is two kernels without atomics: one per (64-key tile, kv head) accumulating dK / dV over all query tiles
-// and the G query heads of the group, one per (128-row query tile, query head) accumulating dQ over key tiles. Both
+// Backward (flash_attention_bwd.cu) is two kernels without atomics: one per (128-key tile, kv head) accumulating dK / dV over all query
+// tiles and the G query heads of the group, one per (128-row query tile, query head) accumulating dQ over key tiles. Both
 // recompute S and P from Q, K and lse.
 //
 // Replaces flash-attn 2 / cuDNN fused attention in the reference's policy workers

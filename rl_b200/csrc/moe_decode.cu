@@ -324,7 +324,7 @@ RLB_API int rlb_moe_route_topk(const void* logits, long long ld, int T, int E, i
   return static_cast<int>(cudaGetLastError());
 }
 
-// mpad: rows of the padded layout, a multiple of 128 and >= n_copies + El * 127 rounded up (worst case: all copies local).
+// mpad: rows of the padded layout, a multiple of `pad` (the rows of a tile) and >= n_copies + El * (pad - 1) (worst case: all copies local).
 RLB_API int rlb_moe_decode_plan(const int* idx, int n_copies, int k, int e_lo, int El, int mpad, int pad, int* src_tok, int* copy_row,
                                 int* tile_expert, int* row0, int* rows, int* status, void* stream) {
   if (n_copies <= 0 || n_copies > PLAN_MAX_COPIES || El < 1 || El > PLAN_MAX_EXPERTS || k < 1 || pad < 1 || (mpad % pad) ||

@@ -35,8 +35,8 @@ __device__ __forceinline__ void add_bf16x4(float4& v, uint32_t lo, uint32_t hi) 
 }
 
 // Writes the staged piece: rows row0.., columns col.. of C, with bias, residual and the old values where `ep` (an OutPiece or a struct with its
-// fields) has them. Old values (accumulation) and the residual are fetched by the caller's
-// warp in the same layout before the piece is complete.
+// fields) has them. Old values (accumulation), and the residual of a bf16 output, are requested in the same layout before the warp has met, so
+// that they arrive while it stages the piece; the residual of an fp32 output is read row by row.
 template <typename Out>
 __device__ __forceinline__ void store_piece(const Out& ep, uint32_t buf, int row0, int col, int M, int N, int lane) {
   if (ep.out_fp32) {

@@ -14,8 +14,8 @@
 // with a window of W and K kept first tokens the keys nearer than W and the first K. With sigmoid weights (SIG) there is no running maximum and no
 // sum: a key weighs sigmoid(score + a number per head), splits only add up. Where the output's place holds gates, out = y * sigmoid(gate).
 //
-// This first kernel serves the chunked, windowed and sigmoid forms; plain soft-max attention has its own below, in which neighbouring sequences
-// share a CTA. The CUDA-core kernel in paged_decode_tma.cu (same contract) is kept as the fallback for block sizes / head dims this
+// This first kernel serves the chunked, windowed and sigmoid forms, and plain soft-max attention of queries that do not start on 16 bytes; other
+// plain attention has its own kernel below, in which neighbouring sequences share a CTA. The CUDA-core kernel in paged_decode_tma.cu (same contract) is kept as the fallback for block sizes / head dims this
 // kernel does not cover. Reference counterpart: the FlashInfer / vLLM paged-attention decode kernels behind
 // nemo_rl/models/generation/vllm.
 #include "common.cuh"
