@@ -13,7 +13,8 @@
 // scores they have read, from where the second products take them as TMEM operands. The scores of tile j + 1 are computed while tile j is in
 // the warps' hands, so that the tensor core (768 cycles a tile in dQ, 1024 in dK / dV) and the exponentials (512) overlap.
 // Measured, 32 query and 8 KV heads of 128, causal (before: one score buffer, one group, P and dS through shared memory): 16 x 4096 tokens
-// 15.4 -> 10.9 ms (506 TFLOP/s of the five products that a gradient needs); 64 x 1280 7.7 -> 5.4 ms.
+// 15.4 -> 11.0 ms (499 TFLOP/s of the five products that a gradient needs); 64 x 1280 7.7 -> 5.5 ms; 8 x (513, 700, 333) 0.83 -> 0.65 ms; with
+// heads of 64 11.1 -> 8.8, 5.4 -> 4.4 and 0.59 -> 0.52 ms.
 // delta[h, t] = sum_d dO * O is computed beforehand by rlb_attn_delta.
 #include "common.cuh"
 
