@@ -395,9 +395,13 @@ __global__ void dm_combine_kernel(const float* __restrict__ part_o, const float*
 // A tile of one sequence is multiplied with the weights of all columns, zeros in the others', and zero times an infinite or undefined value is
 // undefined. So the accumulator starts anew with every run of tiles (the shared ones, then each sequence's own), and at the end of a run
 // only its own columns are taken from it: what one sequence holds does not reach its neighbours (1 to 3 % of a group's time).
+// Scores are scaled in fp32: queries that were scaled and rounded to bf16 again (head dimension 128; 1/8 is exact) made up half of the output's
+// squared error, and a reference maximum that may be stale leaves the largest weight of a tile rounded, which it is not where it is the reference.
+// So the error against 64 bits was 1 to 3 % above that of one CTA per sequence (64 sequences of 1000 tokens: 2.86e-3 of the norm, before 2.78e-3);
+// with the scale in fp32 it is below 2.6e-3, as with heads of 64 (2.32e-3).
 // Bound by the cache stream: K and V buffers of three CTAs per SM are in flight; one CTA-wide barrier per tile.
 // Measured, 8 KV heads of 128, 4 query heads each (one CTA per sequence, split and KV head, two per SM, before -> now): 48 sequences of 4000
-// tokens, 16 to a prompt, 169 -> 57 us, every prompt its own 206 -> 129 us (5.9 TB/s); 64 of 256 tokens, 8 to a prompt, 23 -> 18 us; 64 of 2000
+// tokens, 16 to a prompt, 166 -> 62 us, every prompt its own 206 -> 133 us (5.9 TB/s); 64 of 256 tokens, 8 to a prompt, 21 -> 16 us; 64 of 2000
 // tokens with heads of 64 (gathered and multiplied by library kernels before) 620 -> 47 us.
 constexpr int DG_ROWS = 4;       // most sequences of a group
 constexpr int DG_CLUSTER = 8;    // most splits that merge in a cluster
@@ -506,21 +510,13 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     same = __reduce_min_sync(0xffffffffu, same);
     if (lane == 0) s_same[warp] = same;
   }
-  // Q (pre-scaled) and a zeroed P^T, both in the swizzled K-major operand layout, 16 bytes at a time; row = sequence * G + head
+  // Q and a zeroed P^T, both in the swizzled K-major operand layout, 16 bytes at a time; row = sequence * G + head
   for (int i = threadIdx.x; i < 2 * Cfg::QP_BYTES / 16; i += DM_THREADS) {
     uint4 val = make_uint4(0, 0, 0, 0);
     const int which = i / (Cfg::QP_BYTES / 16), j = i % (Cfg::QP_BYTES / 16);
     const int c = j / 16, piece = j % 16;
     if (which == 0 && c < rows * G && piece < HD / 8) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(p.q + (seq0 + row_of(c)) * p.q_stride + static_cast<long long>(kvh * G + head_of(c)) * HD + piece * 8);
-      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-      uint32_t o[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float2 f = unpack_bf16x2(w[k]);
-        o[k] = pack_bf16x2(f.x * p.scale, f.y * p.scale);
-      }
-      val = make_uint4(o[0], o[1], o[2], o[3]);
+      val = *reinterpret_cast<const uint4*>(p.q + (seq0 + row_of(c)) * p.q_stride + static_cast<long long>(kvh * G + head_of(c)) * HD + piece * 8);
     }
     uint8_t* base = which == 0 ? q_sm : p_sm;
     *reinterpret_cast<uint4*>(base + sw128_off(c, piece * 8, DM_N * 128)) = val;
@@ -693,8 +689,8 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         if (RUNS && !(active >> c0 & 15u)) continue;
 #pragma unroll
         for (int c = c0; c < c0 + 4; ++c) {
-          if (!valid || !(active >> c & 1)) sr[c] = 0xff800000u;   // -inf
-          float mx = __uint_as_float(sr[c]);
+          float mx = valid && (active >> c & 1) ? __uint_as_float(sr[c]) * p.scale : -INFINITY;
+          sr[c] = __float_as_uint(mx);
 #pragma unroll
           for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
           if (lane == 0) red_max[quarter * DM_N + c] = mx;

@@ -408,6 +408,30 @@ def test_paged_decode_d64_forms(native_lib, form):
     assert check_status() == 0 and (got.cpu().float() - ref).norm() <= 2e-2 * ref.norm()
 
 
+@pytest.mark.parametrize("Hq,Hkv,D", [(32, 8, 128), (8, 1, 128), (32, 8, 64), (16, 1, 64), (16, 1, 128), (32, 2, 128)])
+@pytest.mark.parametrize("B,n", [(1, 1000), (16, 1000), (48, 513)])
+def test_paged_decode_error(native_lib, Hq, Hkv, D, B, n):
+    """Error against float64 over the norm. Weights and output are each rounded to bf16: values that are spread over a power of two lose 1.66e-3 of
+    their norm that way, together 2.35e-3; queries that are rounded a second time would make it 2.8e-3. A tenth on top
+    for the spread of a few thousand values."""
+    from rl_b200.ops import engine_ops as E
+    from rl_b200.ops.lib import check_status
+
+    bs, pages = 64, -(-n // 64)
+    g = torch.Generator("cuda").manual_seed(B + n + D)
+    q = torch.randn(B, Hq * D, generator=g, device="cuda").bfloat16()
+    kc, vc = (torch.randn(B * pages, Hkv, bs, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    bt = torch.randperm(B * pages, generator=g, device="cuda").int().view(B, pages)
+    lens = torch.full((B,), n, dtype=torch.int32, device="cuda")
+    out = E.paged_decode(q, kc, vc, bt, lens, Hq, Hkv, D, num_splits=E.choose_splits(B, Hkv, n, bs, 148, Hq))
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    k, v = (t[bt.long()].transpose(2, 3).reshape(B, pages * bs, Hkv, D)[:, :n].double() for t in (kc, vc))
+    s = torch.einsum("bhgd,bnhd->bhgn", q.double().view(B, Hkv, Hq // Hkv, D), k) / D ** 0.5
+    ref = torch.einsum("bhgn,bnhd->bhgd", s.softmax(-1), v).reshape(B, Hq * D)
+    assert (out.double() - ref).norm() <= 1.1 * 2.35e-3 * ref.norm()
+
+
 @pytest.mark.parametrize("Hq,Hkv,D", [(8, 2, 128), (8, 2, 64), (2, 2, 128)])
 @pytest.mark.parametrize("rows,splits", [(2, 1), (4, 1), (4, 3), (2, 11)])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
