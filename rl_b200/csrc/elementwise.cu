@@ -652,9 +652,11 @@ __global__ void adamw_kernel(__nv_bfloat16* __restrict__ p, int16_t* __restrict_
 }
 
 // Sums of four or eight squares are taken in fp32, everything above in fp64: thousands of fp32 additions in a row lost part of the
-// squares of small gradients beside large ones (2e-6 to 5e-6 of the norm at 1.2e9 to 1.9e9 parameters; now below 5e-7). Four 16-byte loads in flight: 2.28 -> 1.34 ms for 7.7 GB (5.7 TB/s).
+// squares of small gradients beside large ones (2e-6 to 5e-6 of the norm at 1.2e9 to 1.9e9 parameters; now below 5e-7). Four 16-byte loads in flight: 2.28 -> 1.34 ms for 7.7 GB (5.7 TB/s). The blocks' sums are added up in fp64 as well, by a
+// second kernel: as fp32 additions to `out`, a thousand sums that are nearly alike were all rounded the same way (5e-6 of the total).
+constexpr int SUMSQ_BLOCKS = 148 * 8;
 template <typename T>
-__global__ void sumsq_kernel(const T* __restrict__ x, long long n, float* __restrict__ out) {
+__global__ void sumsq_kernel(const T* __restrict__ x, long long n, double* __restrict__ part) {
   __shared__ double red[32];
   double s = 0.0;
   const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x, step = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -687,6 +689,20 @@ __global__ void sumsq_kernel(const T* __restrict__ x, long long n, float* __rest
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < (blockDim.x >> 5); ++w) s += red[w];
+    part[blockIdx.x] = s;
+  }
+}
+
+__global__ void sumsq_total_kernel(const double* __restrict__ part, int n, float* __restrict__ out) {
+  __shared__ double red[8];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += 256) s += part[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) s += red[w];
     atomicAdd(out, static_cast<float>(s));
   }
 }
@@ -1084,12 +1100,13 @@ RLB_API int rlb_adamw(void* p, void* p_lo, float* p32, const void* g, int grad_i
   return static_cast<int>(cudaGetLastError());
 }
 
-// out += sum(x^2). `out` is a device float the caller zeroes.
-RLB_API int rlb_sumsq(const void* x, int is_bf16, long long n, float* out, void* stream) {
+// out += sum(x^2). `out` is a device float the caller zeroes; `part` is scratch of SUMSQ_BLOCKS (1184) doubles.
+RLB_API int rlb_sumsq(const void* x, int is_bf16, long long n, float* out, double* part, void* stream) {
   if (n <= 0) return 0;
-  const int grid = grid_for(n, 1024, n < (1 << 24) ? 148 * 4 : 148 * 8);      // (few elements: half as many sums to add up)
-  if (is_bf16) sumsq_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(CBF(x), n, out);
-  else sumsq_kernel<float><<<grid, 256, 0, S(stream)>>>(reinterpret_cast<const float*>(x), n, out);
+  const int grid = grid_for(n, 1024, n < (1 << 24) ? SUMSQ_BLOCKS / 2 : SUMSQ_BLOCKS);      // (few elements: half as many sums to add up)
+  if (is_bf16) sumsq_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(CBF(x), n, part);
+  else sumsq_kernel<float><<<grid, 256, 0, S(stream)>>>(reinterpret_cast<const float*>(x), n, part);
+  sumsq_total_kernel<<<1, 256, 0, S(stream)>>>(part, grid, out);
   return static_cast<int>(cudaGetLastError());
 }
 RLB_API int rlb_clip_scale(const float* sumsq, float max_norm, float extra, float* scale_out, float* norm_out,
