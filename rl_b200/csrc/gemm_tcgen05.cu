@@ -26,6 +26,7 @@
 //   EPI_LOGPROB  for a vocab projection: per (row, n-tile) online-softmax partials (max, sum-exp,
 //                sum of z*exp) and the target logit; logits are never written. A small second
 //                kernel folds the partials into logprob / entropy / logsumexp per row.
+//   EPI_LOGPROB_KEEP  the same, and the scaled logits are written in fp32 for the backward pass (dlogits_kept_kernel)
 //   EPI_LAYER    products of a parallel mixer layer (LayerEpilogue in common.cuh): squared ReLU on a column range, or
 //                residual update + dynamic-tanh norm
 //   EPI_LINEAR   products of post-norm layers (LinearEpi in common.cuh): bias, then clamped gated unit or gated token input
@@ -67,10 +68,10 @@ struct Tile {
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 };
 
-enum { EPI_STORE = 0, EPI_LOGPROB = 1, EPI_DLOGITS = 2, EPI_LAYER = 3, EPI_LINEAR = 4 };
+enum { EPI_STORE = 0, EPI_LOGPROB = 1, EPI_DLOGITS = 2, EPI_LAYER = 3, EPI_LINEAR = 4, EPI_LOGPROB_KEEP = 5 };
 
 struct EpiParams {
-  void* C;              // output (EPI_STORE, EPI_DLOGITS)
+  void* C;              // output (EPI_STORE, EPI_DLOGITS), scaled logits (EPI_LOGPROB_KEEP)
   long long ldc;        // leading dimension of C in elements
   const float* bias;    // [N] or null
   const void* residual; // bf16 [M, ldr] added to the result (the residual stream), or null
@@ -110,6 +111,15 @@ __device__ __forceinline__ void unpack8(const uint4 r, float (&v)[8]) {
 __device__ __forceinline__ float4 square_relu4(float4 v) {
   v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f);
   return make_float4(v.x * v.x, v.y * v.y, v.z * v.z, v.w * v.w);
+}
+
+// Gradient of a logit whose scaled value is z: d logprob_t / dz_j = 1[j=t] - p_j ;  dH/dz_j = -p_j (logp_j + H)
+__device__ __forceinline__ float dlogit(float z, bool is_target, float lse, float g, float ge, float ent, float inv_temp) {
+  const float logp = z - lse;
+  const float p = __expf(logp);
+  float d = g * ((is_target ? 1.f : 0.f) - p);
+  d -= ge * p * (logp + ent);
+  return d * inv_temp;
 }
 
 // A load of this CTA's operands, signalling `bar`: with PAIR the first CTA's barrier.
@@ -449,7 +459,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
               *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(pack_bf16x2(v[q * 8], v[q * 8 + 1]), pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]),
                                                                   pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]), pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]));
         }
-      } else if (EPI == EPI_LOGPROB) {
+      } else if (EPI == EPI_LOGPROB || EPI == EPI_LOGPROB_KEEP) {
         // Online softmax statistics of this row over the tile's columns.
         float mx = -INFINITY, sum = 0.f, zsum = 0.f;
         const int tgt = row_ok ? ep.targets[row] : -1;
@@ -459,26 +469,56 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           tmem_ld_wait();
           const int col = col0 + c * 32;
           if (col >= N) continue;
-          float cmax = -INFINITY;
+          // Whole pieces go without a test of each column, whose branches cost more than the exponentials: the epilogue of a 256 x 256 tile was as
+          // long as a product of 2048, and longer with the logits' stores behind it (4096 x 128256 x 2048 with stores 2.39 ms, now 1.55).
+          float cmax[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          if (col + 32 <= N) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float z = __uint_as_float(r[i]) * ep.inv_temp;
-            r[i] = __float_as_uint(z);
-            if (col + i < N) cmax = fmaxf(cmax, z);
-          }
-          const float nmx = fmaxf(mx, cmax);
-          const float scale = __expf(mx - nmx);  // exp(-inf) = 0 on the first chunk
-          sum *= scale;
-          zsum *= scale;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (col + i < N) {
-              const float z = __uint_as_float(r[i]);
-              const float e = __expf(z - nmx);
-              sum += e;
-              zsum += z * e;
-              if (col + i == tgt) ep.target_logit[row] = z;
+            for (int i = 0; i < 32; ++i) {
+              const float z = __uint_as_float(r[i]) * ep.inv_temp;
+              r[i] = __float_as_uint(z);
+              cmax[i & 3] = fmaxf(cmax[i & 3], z);
             }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              r[i] = col + i < N ? __float_as_uint(__uint_as_float(r[i]) * ep.inv_temp) : __float_as_uint(-INFINITY);
+              cmax[i & 3] = fmaxf(cmax[i & 3], __uint_as_float(r[i]));
+            }
+          }
+          if (EPI == EPI_LOGPROB_KEEP) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              st_shared_f4(out_chunk(buf, lane, (c & 1) * 8 + q), __uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]),
+                           __uint_as_float(r[4 * q + 3]));
+            if ((c & 1) || col + 32 >= N) stream_piece(static_cast<float*>(ep.C), ep.ldc, buf, row0, col - (c & 1) * 32, M, N, lane);
+          }
+          const float nmx = fmaxf(mx, fmaxf(fmaxf(cmax[0], cmax[1]), fmaxf(cmax[2], cmax[3])));
+          const float scale = __expf(mx - nmx);  // exp(-inf) = 0 on the first chunk
+          float s4[4] = {sum * scale, 0.f, 0.f, 0.f}, z4[4] = {zsum * scale, 0.f, 0.f, 0.f};
+          if (col + 32 <= N) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const float z = __uint_as_float(r[i]), e = __expf(z - nmx);
+              s4[i & 3] += e;
+              z4[i & 3] += z * e;
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              if (col + i < N) {
+                const float z = __uint_as_float(r[i]), e = __expf(z - nmx);
+                s4[i & 3] += e;
+                z4[i & 3] += z * e;
+              }
+            }
+          }
+          sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+          zsum = (z4[0] + z4[1]) + (z4[2] + z4[3]);
+          if (static_cast<unsigned>(tgt - col) < 32u && tgt < N) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (col + i == tgt) ep.target_logit[row] = __uint_as_float(r[i]);
           }
           mx = nmx;
         }
@@ -503,13 +543,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           float v[64];
 #pragma unroll
           for (int i = 0; i < OUT_COLS; ++i) {
-            const float z = __uint_as_float(r[i]) * ep.inv_temp;
-            const float logp = z - lse;
-            const float p = __expf(logp);
-            // d logprob_t / dz_j = 1[j=t] - p_j ;  dH/dz_j = -p_j (logp_j + H)
-            float d = g * ((col + i == tgt ? 1.f : 0.f) - p);
-            d -= ge * p * (logp + ent);
-            v[i] = d * ep.inv_temp;
+            v[i] = dlogit(__uint_as_float(r[i]) * ep.inv_temp, col + i == tgt, lse, g, ge, ent, ep.inv_temp);
           }
 #pragma unroll
           for (int q = 0; q < OUT_COLS / 4; ++q) st_shared_f4(out_chunk(buf, lane, q), v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
@@ -532,6 +566,36 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     tc_fence_after();
     if constexpr (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
     else tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
+// EPI_DLOGITS without the product, from the logits that EPI_LOGPROB_KEEP wrote: 6 bytes a logit, bound by memory. A thread requests its 64 bytes
+// before it computes.
+constexpr int KEPT_COLS = 256 * 16;
+__global__ void __launch_bounds__(256) dlogits_kept_kernel(const float* __restrict__ z, __nv_bfloat16* __restrict__ dz, int N, long long ldz, long long lddz,
+                                                           const int* __restrict__ targets, float inv_temp, const float* __restrict__ lse_,
+                                                           const float* __restrict__ coef, const float* __restrict__ ent_coef,
+                                                           const float* __restrict__ entropy) {
+  const long long row = blockIdx.y;
+  const int col = blockIdx.x * KEPT_COLS + threadIdx.x * 8;      // and 2048 further on
+  const float* src = z + row * ldz + col;
+  float4 v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (col + (j >> 1) * 2048 < N) v[j] = __ldcs(reinterpret_cast<const float4*>(src + (j >> 1) * 2048) + (j & 1));
+  const int tgt = targets[row];
+  const float lse = lse_[row], g = coef[row];
+  const float ge = ent_coef ? ent_coef[row] : 0.f, ent = ent_coef ? entropy[row] : 0.f;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int c = col + j * 2048;
+    if (c >= N) continue;      // N is a multiple of 8
+    const float e[8] = {v[2 * j].x, v[2 * j].y, v[2 * j].z, v[2 * j].w, v[2 * j + 1].x, v[2 * j + 1].y, v[2 * j + 1].z, v[2 * j + 1].w};
+    float d[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d[i] = dlogit(e[i], c + i == tgt, lse, g, ge, ent, inv_temp);
+    *reinterpret_cast<uint4*>(dz + row * lddz + c) =
+        make_uint4(pack_bf16x2(d[0], d[1]), pack_bf16x2(d[2], d[3]), pack_bf16x2(d[4], d[5]), pack_bf16x2(d[6], d[7]));
   }
 }
 
@@ -775,9 +839,10 @@ RLB_API int rlb_gemm_num_n_tiles(int N) { return (N + BN - 1) / BN; }
 RLB_API int rlb_lm_head_logprob(const void* H, const void* W, int M, int N, int K, long long ldh, long long ldw,
                                 const int* targets, float inv_temp, float* part_max, float* part_sum,
                                 float* part_zsum, float* target_logit, float* logprob, float* entropy,
-                                float* lse, int* status, void* stream) {
+                                float* lse, float* logits, long long ldz, int* status, void* stream) {
   if (M <= 0) return 0;
   if ((ldh % 8) || (ldw % 8)) return -2;
+  if (logits && ((N % 8) || (ldz % 4) || (reinterpret_cast<uintptr_t>(logits) & 15))) return -2;
   CUtensorMap ta, tb;
   int rc = make_operand_maps(H, W, M, N, K, ldh, ldw, false, false, &ta, &tb);
   if (rc) return -100 - rc;
@@ -788,8 +853,11 @@ RLB_API int rlb_lm_head_logprob(const void* H, const void* W, int M, int N, int 
   ep.part_sum = part_sum;
   ep.part_zsum = part_zsum;
   ep.target_logit = target_logit;
+  ep.C = logits;
+  ep.ldc = ldz;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  rc = launch_gemm<false, false, EPI_LOGPROB>(ta, tb, M, N, K, ep, status, 0, s);
+  rc = logits ? launch_gemm<false, false, EPI_LOGPROB_KEEP>(ta, tb, M, N, K, ep, status, 0, s)
+              : launch_gemm<false, false, EPI_LOGPROB>(ta, tb, M, N, K, ep, status, 0, s);
   if (rc) return rc;
   const int parts = (N + BN - 1) / BN;
   logprob_combine_kernel<<<(M + 31) / 32, 256, 0, s>>>(part_max, part_sum, part_zsum, target_logit, M, parts,
@@ -849,4 +917,15 @@ RLB_API int rlb_lm_head_dlogits(const void* H, const void* W, void* dZ, int M, i
   ep.ent_coef = ent_coef;
   ep.entropy = entropy;
   return launch_gemm<false, false, EPI_DLOGITS>(ta, tb, M, N, K, ep, status, 0, static_cast<cudaStream_t>(stream));
+}
+
+// The same gradient from kept logits (rlb_lm_head_logprob). N and lddz multiples of 8, ldz of 4, both starting on 16 bytes.
+RLB_API int rlb_lm_head_dlogits_kept(const float* z, void* dZ, int M, int N, long long ldz, long long lddz, const int* targets, float inv_temp,
+                                     const float* lse, const float* coef, const float* ent_coef, const float* entropy, void* stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if ((ldz % 4) || (lddz % 8) || (N % 8) || M > 65535) return -2;
+  if ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(dZ)) & 15) return -3;
+  dlogits_kept_kernel<<<dim3((N + KEPT_COLS - 1) / KEPT_COLS, M), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      z, static_cast<__nv_bfloat16*>(dZ), N, ldz, lddz, targets, inv_temp, lse, coef, ent_coef, entropy);
+  return static_cast<int>(cudaGetLastError());
 }

@@ -33,7 +33,7 @@ def _local_stats(h, w, tg_local, inv_temp):
         tl = torch.zeros(M, dtype=torch.float32, device=dev)
         out = torch.empty((3, M), dtype=torch.float32, device=dev)
         call("rlb_lm_head_logprob", ptr(h), ptr(w), M, N, K, h.stride(0), w.stride(0), ptr(tg_local), inv_temp,
-             ptr(pm[0]), ptr(pm[1]), ptr(pm[2]), ptr(tl), ptr(out[2]), ptr(out[1]), ptr(out[0]), ptr(_L.status_word(dev)), stream_ptr())
+             ptr(pm[0]), ptr(pm[1]), ptr(pm[2]), ptr(tl), ptr(out[2]), ptr(out[1]), ptr(out[0]), None, 0, ptr(_L.status_word(dev)), stream_ptr())
         out[2].copy_(tl)
         return out
     z = (h.float() @ w.float().t()) * inv_temp

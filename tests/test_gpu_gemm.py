@@ -153,6 +153,37 @@ def test_lm_head_logprob(native_lib, M, V, K):
     assert _rel_err(w.grad, wr.grad) < 3e-2
 
 
+@pytest.mark.parametrize("M,V", [(1, 8), (33, 264), (129, 4096), (300, 4104), (257, 6152)])
+def test_lm_head_kept_logits(native_lib, monkeypatch, M, V):
+    """Gradients from the logits that forward kept (whole and partial runs of 4096 columns, last pieces of 8 and 32, rows in chunks) against
+    float64, and those of the recomputed product. dZ is rounded to bf16 (2^-9 a value), dH once more: below 2^-8 of the norm."""
+    from rl_b200.ops import functional as F
+
+    K = 192
+    g = torch.Generator("cuda").manual_seed(M)
+    h = (torch.randn(M, K, generator=g, device="cuda") * 0.5).bfloat16()
+    w = (torch.randn(V, K, generator=g, device="cuda") * 0.2).bfloat16()
+    tg = torch.randint(0, V, (M,), generator=g, device="cuda")
+    cl, ce = torch.randn(M, generator=g, device="cuda"), torch.randn(M, generator=g, device="cuda") * 0.1
+    monkeypatch.setattr(F._LMHeadLogprob, "CHUNK", 128)
+    kept = F._kept_logits
+    calls = []
+    grads = []
+    for keep in (True, False):
+        monkeypatch.setattr(F, "_kept_logits", lambda *a: (calls.append(a), kept(*a))[1] if keep else None)
+        hg, wg = h.clone().requires_grad_(), w.clone().requires_grad_()
+        lp, ent = F.lm_head_logprobs(hg, wg, tg, temperature=0.8, want_entropy=True)
+        (lp * cl + ent * ce).sum().backward()
+        grads.append((hg.grad, wg.grad))
+    assert len(calls) == 1
+    hd, wd = h.double().requires_grad_(), w.double().requires_grad_()
+    logp = torch.log_softmax(hd @ wd.t() / 0.8, -1)
+    (logp.gather(1, tg[:, None])[:, 0] * cl - (logp.exp() * logp).sum(-1) * ce).sum().backward()
+    for got in grads:
+        for x, ref in zip(got, (hd.grad, wd.grad)):
+            assert (x.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+
+
 @pytest.mark.parametrize("parts", [1, 3, 8, 21])
 def test_logprob_combine_empty_parts(native_lib, parts):
     """Parts without columns (maximum -inf, sums 0), as many as all of a warp's, count for nothing. Against float64: fp32 sums of at most 21 terms
