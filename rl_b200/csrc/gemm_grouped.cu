@@ -218,6 +218,14 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint32_t local_tile = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       const Work w = get_work<B_MN>(g, tile, num_m, num_n);
+      if (REDUCE && !w.valid && !g.accumulate) {      // an expert without rows: its product is zero
+        const int cols = min(BN, g.N - w.n_blk * BN), bytes = g.out_fp32 ? 4 : 2, per = cols * bytes / 16;      // N is a multiple of 8
+        const int first = w.m_blk * BM + quarter * 32, rows = min(32, g.M - first);
+        for (int i = lane; i < rows * per; i += 32) {
+          const long long at = w.c_off + static_cast<long long>(first + i / per) * g.ldc + w.n_blk * BN;
+          reinterpret_cast<uint4*>(static_cast<char*>(g.C) + at * bytes)[i % per] = make_uint4(0, 0, 0, 0);
+        }
+      }
       if (!w.valid) continue;
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;

@@ -80,6 +80,28 @@ def gemm(
     return out
 
 
+def grad_buffer(w) -> Optional[torch.Tensor]:
+    """``w.main_grad`` to add to, or None. A buffer whose old values count for nothing (``w.grad_stale``, set where gradients begin anew) is
+    zeroed first."""
+    g = getattr(w, "main_grad", None)
+    if g is not None and getattr(w, "grad_stale", False):
+        g.zero_()
+        w.grad_stale = False
+    return g
+
+
+def grad_output(w, rows: int) -> tuple[Optional[torch.Tensor], bool]:
+    """(``w.main_grad``, whether to add to it): a product over ``rows`` rows that covers all of it writes over a stale buffer, instead of a fill
+    and a read of zeros before it."""
+    g = getattr(w, "main_grad", None)
+    if g is None or not getattr(w, "grad_stale", False):
+        return g, True
+    if rows == 0:      # (a product over nothing is not launched)
+        return grad_buffer(w), True
+    w.grad_stale = False
+    return g, False
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, bias, residual):
@@ -107,10 +129,10 @@ class _Linear(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             dx = gemm(dy2, w, b_mn=True, out_dtype=x.dtype).view_as(x)
         if ctx.needs_input_grad[1]:
-            main_grad = getattr(w, "main_grad", None)
+            main_grad, add = grad_output(w, dy2.shape[0])
             if main_grad is not None:
-                # weight gradient accumulates straight into the (bf16 or fp32) gradient buffer
-                gemm(dy2, x2, a_mn=True, b_mn=True, out=main_grad, accumulate=True)
+                # weight gradient goes straight into the (bf16 or fp32) gradient buffer
+                gemm(dy2, x2, a_mn=True, b_mn=True, out=main_grad, accumulate=add)
                 dw = None
             else:
                 dw = gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=w.dtype)
@@ -229,7 +251,7 @@ class _MXLinear(torch.autograd.Function):
             # dW [N, K] = dY^T [N, M] X [M, K]: contraction over the tokens
             g = _mx_gemm(dy2.t().contiguous(), x2.t().contiguous())
             Fp8Training.stats["wgrad"] += 1
-            main_grad = getattr(w, "main_grad", None)
+            main_grad = grad_buffer(w)
             if main_grad is not None:
                 main_grad.add_(g.to(main_grad.dtype))
             else:
@@ -299,7 +321,7 @@ class _RMSNorm(torch.autograd.Function):
         dx = torch.empty((rows, d), dtype=x2.dtype, device=x2.device)
         parts = _L.lib().rlb_rmsnorm_bwd_parts(rows)
         partial = torch.empty((parts, d), dtype=torch.float32, device=x2.device)
-        main_grad = getattr(w, "main_grad", None)
+        main_grad = grad_buffer(w)
         if main_grad is not None:
             f32 = main_grad if main_grad.dtype == torch.float32 else None
             b16 = main_grad if main_grad.dtype == BF16 else None
@@ -360,7 +382,7 @@ class _HeadRMSNorm(torch.autograd.Function):
         dw = torch.zeros(D, dtype=torch.float32, device=buf.device)
         call("rlb_head_rmsnorm_bwd", ptr(dout[:, col0:]), ptr(buf[:, col0:]), ptr(w), ptr(rstd), ptr(dbuf[:, col0:]), ptr(dw),
              T, heads, D, buf.stride(0), dout.stride(0), dbuf.stride(0), stream_ptr())
-        main_grad = getattr(w, "main_grad", None)
+        main_grad = grad_buffer(w)
         if main_grad is not None:
             main_grad.add_(dw.to(main_grad.dtype))
             return dbuf, None, None, None, None, None
@@ -402,7 +424,7 @@ class _QKNorm(torch.autograd.Function):
              dout.stride(0), dbuf.stride(0), stream_ptr())
         grads = []
         for w, g, need in ((wq, dw[0], ctx.needs_input_grad[1]), (wk, dw[1], ctx.needs_input_grad[2])):
-            main_grad = getattr(w, "main_grad", None)
+            main_grad = grad_buffer(w)
             if main_grad is not None:
                 main_grad.add_(g.to(main_grad.dtype))
             grads.append(g.to(w.dtype) if need and main_grad is None else None)
@@ -538,7 +560,7 @@ class _Embedding(torch.autograd.Function):
         (flat,) = ctx.saved_tensors
         table = ctx.table
         dy2 = dy.reshape(-1, table.shape[1]).contiguous()
-        main_grad = getattr(table, "main_grad", None)
+        main_grad = grad_buffer(table)
         if main_grad is not None and main_grad.dtype == torch.float32:
             call("rlb_embedding_bwd", ptr(flat), ptr(dy2), ptr(main_grad), flat.numel(), table.shape[1], table.shape[0], stream_ptr())
             return None, None
@@ -651,7 +673,7 @@ class _LMHeadLogprob(torch.autograd.Function):
         coef = dlogp.float().contiguous()
         ecoef = dent.float().contiguous() if (dent is not None and ctx.want_entropy) else None
         dh = torch.empty_like(h) if ctx.needs_input_grad[0] else None
-        main_grad = getattr(w, "main_grad", None)
+        main_grad, add = grad_output(w, M)
         dw = None
         if ctx.needs_input_grad[1] and main_grad is None:
             dw = torch.zeros((N, K), dtype=torch.float32, device=dev)
@@ -671,7 +693,7 @@ class _LMHeadLogprob(torch.autograd.Function):
             if dh is not None:
                 gemm(dzc, w, b_mn=True, out=dh[s:e])
             if wgrad_target is not None:
-                gemm(dzc, h[s:e], a_mn=True, b_mn=True, out=wgrad_target, accumulate=True)
+                gemm(dzc, h[s:e], a_mn=True, b_mn=True, out=wgrad_target, accumulate=add or s > 0)
         if dw is not None:
             dw = dw.to(w.dtype)
         return dh, dw, None, None, None, None
@@ -686,9 +708,8 @@ def _kept_logits(M: int, N: int, dev) -> Optional[torch.Tensor]:
         return None
     step = max(64, (1 << M.bit_length()) // 8)
     rows = -(-M // step) * step
-    need = 4 * rows * N
-    if 4 * need > torch.cuda.mem_get_info(dev)[0] and 4 * need > (
-            torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)):
+    # (this process's own count: asking the driver took from 0.2 to 90 ms)
+    if torch.cuda.memory_allocated(dev) + 16 * rows * N > 0.95 * torch.cuda.get_device_properties(dev).total_memory:
         return None
     try:
         return torch.empty((rows, N), dtype=torch.float32, device=dev)

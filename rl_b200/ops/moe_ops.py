@@ -69,10 +69,10 @@ class _GroupedLinear(torch.autograd.Function):
             call("rlb_gemm_grouped_rows", ptr(dy), dy.stride(0), ptr(w), 1, ptr(dx), dx.stride(0), lay.mpad, K, N, E, ptr(lay.tile_expert),
                  0, ptr(_L.status_word(dy.device)), stream_ptr())
         if ctx.needs_input_grad[1]:
-            main_grad = getattr(w, "main_grad", None)
+            main_grad, add = F.grad_output(w, dy.shape[0])
             target = main_grad if main_grad is not None else torch.zeros((E, N, K), dtype=torch.float32, device=dy.device)
             call("rlb_gemm_grouped_reduce", ptr(dy), dy.stride(0), ptr(x), x.stride(0), ptr(target), lay.mpad, N, K, E, ptr(lay.row0),
-                 ptr(lay.rows), int(target.dtype == torch.float32), 1, ptr(_L.status_word(dy.device)), stream_ptr())
+                 ptr(lay.rows), int(target.dtype == torch.float32), int(add), ptr(_L.status_word(dy.device)), stream_ptr())
             dw = None if main_grad is not None else target.to(w.dtype)
         return dx, dw, None
 
@@ -160,10 +160,10 @@ def _grouped_rows(x, w, transposed: bool, plan) -> torch.Tensor:
 def _grouped_wgrad(dy, x, w, plan):
     """Adds the stacked weight gradient into ``w.main_grad``, or returns it."""
     E, N, K = w.shape
-    main_grad = getattr(w, "main_grad", None)
+    main_grad, add = F.grad_output(w, dy.shape[0])
     target = main_grad if main_grad is not None else torch.zeros((E, N, K), dtype=torch.float32, device=dy.device)
     call("rlb_gemm_grouped_reduce", ptr(dy), dy.stride(0), ptr(x), x.stride(0), ptr(target), plan.mpad, N, K, E, ptr(plan.row0), ptr(plan.rows),
-         int(target.dtype == torch.float32), 1, ptr(_L.status_word(dy.device)), stream_ptr())
+         int(target.dtype == torch.float32), int(add), ptr(_L.status_word(dy.device)), stream_ptr())
     return None if main_grad is not None else target.to(w.dtype)
 
 

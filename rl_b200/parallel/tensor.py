@@ -260,9 +260,9 @@ class TP:
 
 def _accum_dw(w, dy2, x2):
     """dW[N, K] += dy^T x, straight into the gradient buffer when the parameter has one."""
-    main_grad = getattr(w, "main_grad", None)
+    main_grad, add = F.grad_output(w, dy2.shape[0])
     if main_grad is not None:
-        F.gemm(dy2, x2, a_mn=True, b_mn=True, out=main_grad, accumulate=True)
+        F.gemm(dy2, x2, a_mn=True, b_mn=True, out=main_grad, accumulate=add)
         return None
     return F.gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=w.dtype)
 

@@ -76,7 +76,7 @@ class _VocabParallelLogprob(torch.autograd.Function):
         dev = h.device
         coef = dlogp.float().contiguous()
         ecoef = dent.float().contiguous() if (dent is not None and ctx.want_entropy) else None
-        main_grad = getattr(w, "main_grad", None)
+        main_grad = F.grad_buffer(w)
         need_w = ctx.needs_input_grad[1]
         dh = torch.empty((M, K), dtype=h.dtype, device=dev)
         dw = None

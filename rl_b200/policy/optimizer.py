@@ -91,11 +91,16 @@ class ShardedAdamW:
                           if min(b, self.hi) > max(a, self.lo)]
 
     # ------------------------------------------------------------------ step
-    def zero_grad(self) -> None:
+    def zero_grad(self, lazy: bool = False) -> None:
+        """``lazy``: the buffer itself is not read before the next step but through its parameters' backward passes (``FlatParams.begin_grads``)."""
+        if lazy and self.flat.grad is not None:
+            self.flat.begin_grads()
+            return
         if self.flat.grad is not None:
             self.flat.grad.zero_()
         for p in self.flat.params:
             p.grad = None
+            p.grad_stale = False
 
     def _reduce_scatter(self) -> torch.Tensor:
         g = self.flat.grad

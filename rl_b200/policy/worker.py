@@ -956,9 +956,11 @@ class PolicyWorker:
                 counts = counts / cpw
             global_valid_seqs, global_valid_toks = counts[0], counts[1]
             if not eval_mode:
-                self.optimizer.zero_grad()
-                if self.optimizer_e is not None:
-                    self.optimizer_e.zero_grad()
+                for opt in (self.optimizer, self.optimizer_e):
+                    if isinstance(opt, ShardedAdamW):
+                        opt.zero_grad(lazy=True)
+                    elif opt is not None:
+                        opt.zero_grad()
             gb_loss = torch.zeros((), device=self.device)
             budget = None if getattr(loss_fn, "requires_pairs", False) else self._token_budget("train")
             if self.pipeline is not None:
@@ -989,6 +991,9 @@ class PolicyWorker:
                 metrics["global_valid_toks"] = float(global_valid_toks)
                 all_mb_metrics.append(metrics)
             if not eval_mode:
+                for opt in (self.optimizer, self.optimizer_e):
+                    if isinstance(opt, ShardedAdamW) and opt.flat.grad is not None:
+                        opt.flat.settle_grads()
                 self._sync_replicated_grads()
                 if self.optimizer_e is None:
                     gn = self.optimizer.step()

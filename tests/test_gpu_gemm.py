@@ -184,6 +184,36 @@ def test_lm_head_kept_logits(native_lib, monkeypatch, M, V):
             assert (x.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
 
 
+@pytest.mark.parametrize("T", [0, 1, 130, 700])
+def test_stale_gradients_are_written_over(native_lib, monkeypatch, T):
+    """Gradients of a linear layer (used once and twice), of the vocabulary product in chunks and of an embedding into buffers whose old values are
+    undefined, equal to those added to zeros: x + 0 is x."""
+    from rl_b200.ops import functional as F
+
+    monkeypatch.setattr(F._LMHeadLogprob, "CHUNK", 64)
+    g = torch.Generator("cuda").manual_seed(T)
+    rnd = lambda *s: (torch.randn(*s, generator=g, device="cuda") * 0.1).bfloat16()      # noqa: E731
+    ids = torch.randint(0, 136, (T,), generator=g, device="cuda")
+    shapes = dict(once=(264, 128), twice=(128, 128), head=(136, 128), table=(136, 128))
+    weights = {n: rnd(*s) for n, s in shapes.items()}
+    x, up = rnd(T, 128), rnd(T, 264)
+    grads = []
+    for stale in (False, True):
+        ps = {n: torch.nn.Parameter(w.clone()) for n, w in weights.items()}
+        for p in ps.values():
+            p.main_grad = torch.full(p.shape, float("nan") if stale else 0.0, device="cuda")
+            p.grad_stale = stale
+        h = F.embedding(ids, ps["table"]) + x
+        h = F.linear(F.linear(h, ps["twice"]), ps["twice"])
+        loss = (F.linear(h, ps["once"]) * up).sum()
+        if T:
+            loss = loss + F.lm_head_logprobs(h, ps["head"], ids)[0].sum()
+        loss.backward()
+        grads.append({n: F.grad_buffer(p) for n, p in ps.items()})
+    for n in shapes:
+        assert torch.equal(grads[0][n], grads[1][n]) if n != "table" else torch.allclose(grads[0][n], grads[1][n], rtol=1e-4, atol=1e-6)
+
+
 @pytest.mark.parametrize("parts", [1, 3, 8, 21])
 def test_logprob_combine_empty_parts(native_lib, parts):
     """Parts without columns (maximum -inf, sums 0), as many as all of a warp's, count for nothing. Against float64: fp32 sums of at most 21 terms

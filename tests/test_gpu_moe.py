@@ -189,6 +189,10 @@ def test_expert_layer(native_lib, T, E, k, skew, residual):
     w = torch.softmax(r(T, k), -1).requires_grad_()
     gu, dn = (0.2 * r(E, 2 * f, d)).bfloat16().requires_grad_(), (0.2 * r(E, d, f)).bfloat16().requires_grad_()
     dn.main_grad = torch.ones(E, d, f, device="cuda")
+    dn2 = dn.detach().clone().requires_grad_()      # the same into a buffer whose old values are undefined; experts without tokens get zeros
+    dn2.main_grad, dn2.grad_stale = torch.full((E, d, f), float("nan"), device="cuda"), True
+    M.expert_layer(x.detach(), idx, w.detach(), None, gu.detach(), dn2).backward(torch.ones(T, d, device="cuda").bfloat16())
+    assert not dn2.grad_stale and bool(torch.isfinite(dn2.main_grad).all()) and not bool(dn2.main_grad[counts == 0].any())
     out = M.expert_layer(x, idx, w, res if residual else None, gu, dn)
     up = r(T, d).bfloat16()
     out.backward(up)

@@ -135,3 +135,27 @@ def test_native_build_sees_included_sources(tmp_path):
     before = _digest(tmp_path / "a_d64.cu", [])
     (tmp_path / "a.cu").write_text("int b;\n")
     assert _digest(tmp_path / "a_d64.cu", []) != before
+
+
+def test_gradients_that_begin_anew():
+    """After ``begin_grads`` every use sees zeros: a parameter that a backward pass reached, one that none did, and a small one."""
+    import torch
+
+    from rl_b200.models.transformer import FlatParams
+    from rl_b200.ops import functional as F
+
+    m = torch.nn.Module()
+    m.used, m.idle, m.norm = (torch.nn.Parameter(torch.randn(*s)) for s in ((300, 300), (300, 300), (300,)))
+    flat = FlatParams(m)
+    flat.attach_grad_buffer().fill_(float("nan"))
+    flat.begin_grads()
+    assert m.used.grad_stale and m.idle.grad_stale and not m.norm.grad_stale and not m.norm.main_grad.any()
+    out, add = F.grad_output(m.used, 0)
+    assert add and not out.any()
+    m.used.grad_stale = True
+    out, add = F.grad_output(m.used, 5)
+    assert not add and F.grad_output(m.used, 5)[1]
+    out.fill_(2.0)
+    m.norm.grad = torch.ones(300)
+    flat.fold_autograd_grads()
+    assert bool((m.used.main_grad == 2).all()) and not m.idle.main_grad.any() and bool((m.norm.main_grad == 1).all())
