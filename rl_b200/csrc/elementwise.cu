@@ -8,6 +8,8 @@
 // (nemo_rl/algorithms/loss/loss_functions.py:374-788).
 #include "common.cuh"
 
+#include <climits>
+
 #include <math.h>
 
 namespace {
@@ -77,11 +79,79 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
   }
 }
 
-// The same without a residual for many rows: one warp per row, which stays in registers between the two passes, all its loads in flight and no
-// barrier. NV: pieces of 8 elements per lane. Wide rows leave two CTAs to an SM, so that a few thousand of them end in a nearly empty wave and
-// a CTA per row is sooner done. Timed with a flushed cache, CTA per row -> warp per row, us: d 1024: 2000 rows 8.2 -> 10.2, 2368 8.2 -> 8.2,
-// 8000 14.5 -> 12.3; d 2048: 3000 12.3 -> 14.3, 8000 20.5 -> 20.5, 20480 43 -> 35; d 4096: 4000 22.5 -> 26.6, 8000 38.9 -> 38.9,
-// 20480 84 -> 72; d 5120: 8000 49 -> 51, 20480 109 -> 98.
+// The same for rows that fit the registers of one CTA, NV pieces of 8 elements a thread: all loads in flight at once, the row stays between the two
+// passes, and small CTAs, many to an SM, hide one another's barrier. Timed with a flushed cache against the kernel above / a warp per row, us:
+// d 2048: 600 rows 8.1 -> 8.0, 4000 14.6 -> 12.1, 20000 35.7 -> 30.7; d 4096: 600 10.1 -> 8.3, 4000 22.9 -> 16.6, 20000 70.4 -> 54.3 (6.0 TB/s);
+// d 5120: 4000 28.6 -> 20.2, 20000 98.2 -> 68.1. Two and eight pieces were slower above d 1024.
+template <int NV, bool RES>
+__global__ void __launch_bounds__(256) rmsnorm_regs_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
+                                                           __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out,
+                                                           int d, long long x_stride, long long y_stride, float eps) {
+  pdl_sync();
+  __shared__ float red[8];
+  const long long row = blockIdx.x;
+  const int threads = blockDim.x;
+  const __nv_bfloat16* xr = x + row * x_stride;
+  BF8 v[NV], r[NV], g[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = (threadIdx.x + j * threads) * 8;
+    v[j].w[0] = v[j].w[1] = v[j].w[2] = v[j].w[3] = 0u;
+    if (i < d) {
+      v[j] = *reinterpret_cast<const BF8*>(xr + i);
+      if (RES) r[j] = *reinterpret_cast<const BF8*>(res + row * d + i);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = (threadIdx.x + j * threads) * 8;
+    if (i < d) g[j] = *reinterpret_cast<const BF8*>(w + i);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = (threadIdx.x + j * threads) * 8;
+    if (RES && i < d) {      // the normalised value is the bf16-rounded residual stream, as a separate add would give
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = unpack_bf16x2(v[j].w[k]), e = unpack_bf16x2(r[j].w[k]);
+        v[j].w[k] = pack_bf16x2(f.x + e.x, f.y + e.y);
+      }
+      *reinterpret_cast<BF8*>(res_out + row * d + i) = v[j];
+    }
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 f = unpack_bf16x2(v[j].w[k]);
+      t += f.x * f.x + f.y * f.y;
+    }
+    ss += t;
+  }
+  ss = warp_sum(ss);
+  if (threads > 32) {
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = 0.f;
+    for (int i = 0; i < (threads >> 5); ++i) ss += red[i];
+  }
+  const float rstd = rsqrtf(ss / d + eps);
+  if (rstd_out && threadIdx.x == 0) rstd_out[row] = rstd;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = (threadIdx.x + j * threads) * 8;
+    if (i < d) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = unpack_bf16x2(v[j].w[k]), u = unpack_bf16x2(g[j].w[k]);
+        v[j].w[k] = pack_bf16x2(f.x * rstd * u.x, f.y * rstd * u.y);
+      }
+      *reinterpret_cast<BF8*>(y + row * y_stride + i) = v[j];
+    }
+  }
+}
+
+// The same without a residual for many short rows: one warp per row, which stays in registers between the two passes, all its loads in flight and no
+// barrier. NV: pieces of 8 elements per lane. d 1024, 20000 rows: 20.9 us (a CTA per row 26.4), 2400 rows 8.8 either way.
 template <int NV>
 __global__ void __launch_bounds__(256, 2) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                                            float* __restrict__ rstd_out, long long rows, int d, long long x_stride, long long y_stride, float eps) {
@@ -482,16 +552,23 @@ __global__ void head_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, co
 }
 
 // ------------------------------------------------------------------ SwiGLU
+// Row and vector of this thread where every vector has one of its own. Blocks start in order, so that those at work stay within some MB of one another:
+// with a loop over a capped grid the streams drifted apart (20000 rows of 14336: SwiGLU 294 us, without 244; squares of 1.2e9 values 0.75 ms and 0.65).
+__device__ __forceinline__ bool flat_vector(long long rows, int per_row, long long& row, int& v) {
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= rows * per_row) return false;
+  row = i <= 0xffffffffll ? static_cast<uint32_t>(i) / static_cast<uint32_t>(per_row) : i / per_row;
+  v = static_cast<int>(i - row * per_row);
+  return true;
+}
 // gu: [rows, 2F] (gate | up). y[rows, F] = silu(gate) * up.
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y,
                                   long long rows, int F) {
   pdl_sync();
-  const long long vecs_per_row = F / 8;
-  const long long total = rows * vecs_per_row;
-  for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < total;
-       v += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long row = v / vecs_per_row;
-    const int c = static_cast<int>(v - row * vecs_per_row) * 8;
+  long long row;
+  int c;
+  if (flat_vector(rows, F / 8, row, c)) {
+    c *= 8;
     float g[8], u[8], o[8];
     load8(gu + row * 2 * F + c, g);
     load8(gu + row * 2 * F + F + c, u);
@@ -502,12 +579,10 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 }
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gu,
                                   __nv_bfloat16* __restrict__ dgu, long long rows, int F) {
-  const long long vecs_per_row = F / 8;
-  const long long total = rows * vecs_per_row;
-  for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < total;
-       v += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long row = v / vecs_per_row;
-    const int c = static_cast<int>(v - row * vecs_per_row) * 8;
+  long long row;
+  int c;
+  if (flat_vector(rows, F / 8, row, c)) {
+    c *= 8;
     float g[8], u[8], d[8], dg[8], du[8];
     load8(gu + row * 2 * F + c, g);
     load8(gu + row * 2 * F + F + c, u);
@@ -590,39 +665,48 @@ __device__ __forceinline__ float adamw_element(float w, float grad, float& m, fl
   return w - a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
 }
 
-// Split master weights, eight elements (16 bytes read and 12 written an element with an fp32 gradient) per thread and step, all loads in flight before
-// the first use. Bound by memory: 1.9e9 parameters
-// 11.2 -> 10.4 ms (5.2 TB/s, reads and writes mixed).
+// Split master weights, bound by memory (16 bytes read and 12 written an element with an fp32 gradient). A thread takes four neighbouring elements
+// twice, a block's 2048 in whole 16-byte columns, all loads in flight before the first use. One block per 2048 elements and no loop: blocks start
+// in order, so that those at work are within some MB of one another in each of the nine streams. With a loop over the grid, a warp's rows hundreds of
+// MB apart, 1.2e9 parameters took 6.0 ms (eight elements a thread; 5.4 with four), through bulk copies and a ring in shared memory 5.0, now 4.86
+// (6.9 TB/s).
 template <typename GradT>
-__global__ void __launch_bounds__(256) adamw_split8_kernel(uint4* __restrict__ p, uint4* __restrict__ p_lo, const GradT* __restrict__ g, float4* __restrict__ m,
-                                                           float4* __restrict__ v, long long n8, AdamArgs a, const float* __restrict__ grad_scale) {
+__global__ void __launch_bounds__(256) adamw_split_kernel(uint2* __restrict__ p, uint2* __restrict__ p_lo, const GradT* __restrict__ g, float4* __restrict__ m,
+                                                          float4* __restrict__ v, long long n4, AdamArgs a, const float* __restrict__ grad_scale) {
   const float gs = grad_scale ? *grad_scale : 1.f;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8; i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    uint4 hi = p[i], lo = p_lo[i];
-    float gr[8], mm[8], vv[8];
+  const long long first = static_cast<long long>(blockIdx.x) * 512 + threadIdx.x;
+  uint2 hi[2], lo[2];
+  float4 gr[2], mm[2], vv[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const long long i = first + j * 256;
+    if (i >= n4) continue;
+    hi[j] = p[i];
+    lo[j] = p_lo[i];
     if constexpr (sizeof(GradT) == 4) {
-      const float4 g0 = __ldcs(reinterpret_cast<const float4*>(g) + 2 * i), g1 = __ldcs(reinterpret_cast<const float4*>(g) + 2 * i + 1);
-      gr[0] = g0.x; gr[1] = g0.y; gr[2] = g0.z; gr[3] = g0.w; gr[4] = g1.x; gr[5] = g1.y; gr[6] = g1.z; gr[7] = g1.w;
+      gr[j] = __ldcs(reinterpret_cast<const float4*>(g) + i);
     } else {
-      load8(reinterpret_cast<const __nv_bfloat16*>(g) + 8 * i, gr);
+      const uint2 b = __ldcs(reinterpret_cast<const uint2*>(g) + i);
+      const float2 x = unpack_bf16x2(b.x), y = unpack_bf16x2(b.y);
+      gr[j] = make_float4(x.x, x.y, y.x, y.y);
     }
+    mm[j] = m[i];
+    vv[j] = v[i];
+  }
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const float4 a4 = m[2 * i + q], b4 = v[2 * i + q];
-      mm[4 * q] = a4.x; mm[4 * q + 1] = a4.y; mm[4 * q + 2] = a4.z; mm[4 * q + 3] = a4.w;
-      vv[4 * q] = b4.x; vv[4 * q + 1] = b4.y; vv[4 * q + 2] = b4.z; vv[4 * q + 3] = b4.w;
-    }
-    __nv_bfloat16* h8 = reinterpret_cast<__nv_bfloat16*>(&hi);
-    int16_t* l8 = reinterpret_cast<int16_t*>(&lo);
+  for (int j = 0; j < 2; ++j) {
+    const long long i = first + j * 256;
+    if (i >= n4) continue;
+    __nv_bfloat16* h4 = reinterpret_cast<__nv_bfloat16*>(&hi[j]);
+    int16_t* l4 = reinterpret_cast<int16_t*>(&lo[j]);
+    const float ge[4] = {gr[j].x, gr[j].y, gr[j].z, gr[j].w};
+    float me[4] = {mm[j].x, mm[j].y, mm[j].z, mm[j].w}, ve[4] = {vv[j].x, vv[j].y, vv[j].z, vv[j].w};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) master_split(adamw_element(master_join(h8[j], l8[j]), gr[j] * gs, mm[j], vv[j], a), h8[j], l8[j]);
-    p[i] = hi;
-    p_lo[i] = lo;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      m[2 * i + q] = make_float4(mm[4 * q], mm[4 * q + 1], mm[4 * q + 2], mm[4 * q + 3]);
-      v[2 * i + q] = make_float4(vv[4 * q], vv[4 * q + 1], vv[4 * q + 2], vv[4 * q + 3]);
-    }
+    for (int k = 0; k < 4; ++k) master_split(adamw_element(master_join(h4[k], l4[k]), ge[k] * gs, me[k], ve[k], a), h4[k], l4[k]);
+    p[i] = hi[j];
+    p_lo[i] = lo[j];
+    m[i] = make_float4(me[0], me[1], me[2], me[3]);
+    v[i] = make_float4(ve[0], ve[1], ve[2], ve[3]);
   }
 }
 
@@ -654,19 +738,21 @@ __global__ void adamw_kernel(__nv_bfloat16* __restrict__ p, int16_t* __restrict_
 // Sums of four or eight squares are taken in fp32, everything above in fp64: thousands of fp32 additions in a row lost part of the
 // squares of small gradients beside large ones (2e-6 to 5e-6 of the norm at 1.2e9 to 1.9e9 parameters; now below 5e-7). Four 16-byte loads in flight: 2.28 -> 1.34 ms for 7.7 GB (5.7 TB/s). The blocks' sums are added up in fp64 as well, by a
 // second kernel: as fp32 additions to `out`, a thousand sums that are nearly alike were all rounded the same way (5e-6 of the total).
-constexpr int SUMSQ_BLOCKS = 148 * 8;
+// Runs of 64 KB a block, in order (flat_vector): 5.8 -> 6.9 TB/s.
+constexpr int SUMSQ_BYTES = 65536;
 template <typename T>
-__global__ void sumsq_kernel(const T* __restrict__ x, long long n, double* __restrict__ part) {
-  __shared__ double red[32];
+__global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, long long n, double* __restrict__ part) {
+  __shared__ double red[8];
   double s = 0.0;
-  const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x, step = static_cast<long long>(gridDim.x) * blockDim.x;
-  constexpr int PER = 16 / sizeof(T);
+  constexpr int PER = 16 / sizeof(T), VECS = SUMSQ_BYTES / 16;
   const long long nv = (reinterpret_cast<uintptr_t>(x) & 15) ? 0 : n / PER;
   const uint4* xv = reinterpret_cast<const uint4*>(x);
-  for (long long i = tid; i < nv; i += 4 * step) {
+  const long long first = static_cast<long long>(blockIdx.x) * VECS + threadIdx.x;
+#pragma unroll 1
+  for (long long i = first; i < nv && i < first + VECS; i += 4 * 256) {
     uint4 q[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = i + j * step < nv ? __ldcs(xv + i + j * step) : make_uint4(0, 0, 0, 0);
+    for (int j = 0; j < 4; ++j) q[j] = i + j * 256 < nv ? __ldcs(xv + i + j * 256) : make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const T* e = reinterpret_cast<const T*>(&q[j]);
@@ -679,7 +765,8 @@ __global__ void sumsq_kernel(const T* __restrict__ x, long long n, double* __res
       s += t;
     }
   }
-  for (long long i = nv * PER + tid; i < n; i += step) {
+  const long long step = static_cast<long long>(gridDim.x) * 256;
+  for (long long i = nv * PER + static_cast<long long>(blockIdx.x) * 256 + threadIdx.x; i < n; i += step) {
     const float f = static_cast<float>(x[i]);
     s += f * f;
   }
@@ -688,21 +775,22 @@ __global__ void sumsq_kernel(const T* __restrict__ x, long long n, double* __res
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (blockDim.x >> 5); ++w) s += red[w];
+    for (int w = 1; w < 8; ++w) s += red[w];
     part[blockIdx.x] = s;
   }
 }
 
-__global__ void sumsq_total_kernel(const double* __restrict__ part, int n, float* __restrict__ out) {
-  __shared__ double red[8];
+__global__ void __launch_bounds__(1024) sumsq_total_kernel(const double* __restrict__ part, int n, float* __restrict__ out) {
+  __shared__ double red[32];
   double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += 256) s += part[i];
+#pragma unroll 8
+  for (int i = threadIdx.x; i < n; i += 1024) s += part[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) s += red[w];
+    for (int w = 1; w < 32; ++w) s += red[w];
     atomicAdd(out, static_cast<float>(s));
   }
 }
@@ -944,9 +1032,14 @@ RLB_API int rlb_rmsnorm_fwd(const void* x, const void* res, const void* w, void*
                             void* stream) {
   if (rows <= 0) return 0;
   if (d % 8 || x_stride % 8 || y_stride % 8) return -2;
-  if (!res && d <= 5120 && rows >= 148ll * (d <= 1024 ? 16 : d <= 4096 ? 48 : 96)) {
-    auto kern = d <= 1024 ? rmsnorm_rows_kernel<4> : d <= 2048 ? rmsnorm_rows_kernel<8> : d <= 4096 ? rmsnorm_rows_kernel<16> : rmsnorm_rows_kernel<20>;
-    rlb_launch_pdl(kern, dim3(static_cast<unsigned>((rows + 7) / 8)), dim3(256), 0, S(stream), CBF(x), CBF(w), BF(y), rstd, rows, d, x_stride, y_stride, eps);
+  if (!res && d <= 1024 && rows >= 148 * 16) {
+    rlb_launch_pdl(rmsnorm_rows_kernel<4>, dim3(static_cast<unsigned>((rows + 7) / 8)), dim3(256), 0, S(stream), CBF(x), CBF(w), BF(y), rstd, rows, d, x_stride, y_stride, eps);
+    return static_cast<int>(cudaGetLastError());
+  }
+  if (d <= 8192) {
+    const int pieces = d <= 1024 ? 2 : 4, threads = (d / 8 + pieces * 32 - 1) / (pieces * 32) * 32;
+    auto kern = res ? (pieces == 2 ? rmsnorm_regs_kernel<2, true> : rmsnorm_regs_kernel<4, true>) : (pieces == 2 ? rmsnorm_regs_kernel<2, false> : rmsnorm_regs_kernel<4, false>);
+    rlb_launch_pdl(kern, dim3(static_cast<unsigned>(rows)), dim3(threads), 0, S(stream), CBF(x), CBF(res), CBF(w), BF(y), BF(res_out), rstd, d, x_stride, y_stride, eps);
     return static_cast<int>(cudaGetLastError());
   }
   rlb_launch_pdl(rmsnorm_fwd_kernel, dim3(static_cast<unsigned>(rows)), dim3(rms_threads(d)), 0, S(stream), 
@@ -1037,13 +1130,13 @@ RLB_API int rlb_qk_rmsnorm_bwd(const void* dy, const void* x, const void* wq, co
 RLB_API int rlb_swiglu_fwd(const void* gu, void* y, long long rows, int F, void* stream) {
   if (rows <= 0) return 0;
   if (F % 8) return -2;
-  rlb_launch_pdl(swiglu_fwd_kernel, dim3(grid_for(rows * (F / 8), 256)), dim3(256), 0, S(stream), CBF(gu), BF(y), rows, F);
+  rlb_launch_pdl(swiglu_fwd_kernel, dim3(grid_for(rows * (F / 8), 256, INT_MAX)), dim3(256), 0, S(stream), CBF(gu), BF(y), rows, F);
   return static_cast<int>(cudaGetLastError());
 }
 RLB_API int rlb_swiglu_bwd(const void* dy, const void* gu, void* dgu, long long rows, int F, void* stream) {
   if (rows <= 0) return 0;
   if (F % 8) return -2;
-  swiglu_bwd_kernel<<<grid_for(rows * (F / 8), 256), 256, 0, S(stream)>>>(CBF(dy), CBF(gu), BF(dgu), rows, F);
+  swiglu_bwd_kernel<<<grid_for(rows * (F / 8), 256, INT_MAX), 256, 0, S(stream)>>>(CBF(dy), CBF(gu), BF(dgu), rows, F);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1073,22 +1166,22 @@ RLB_API int rlb_adamw(void* p, void* p_lo, float* p32, const void* g, int grad_i
   AdamArgs a{lr, beta1, beta2, eps, weight_decay, 1.f - powf(beta1, static_cast<float>(step)),
              1.f - powf(beta2, static_cast<float>(step))};
   const uintptr_t all = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(p_lo) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v);
-  const long long n8 = p && p_lo && !p32 && !(all & 15) ? n / 8 : 0;      // the rest, if any, goes element by element
-  if (n8) {
-    const int blocks = grid_for(n8, 256, 148 * 16);
+  const long long n4 = p && p_lo && !p32 && !(all & 15) ? n / 4 : 0;      // the rest, if any, goes element by element
+  if (n4) {
+    const unsigned blocks = static_cast<unsigned>((n4 + 511) / 512);
     if (grad_is_bf16)
-      adamw_split8_kernel<__nv_bfloat16><<<blocks, 256, 0, S(stream)>>>(reinterpret_cast<uint4*>(p), reinterpret_cast<uint4*>(p_lo), CBF(g), reinterpret_cast<float4*>(m),
-                                                                        reinterpret_cast<float4*>(v), n8, a, grad_scale);
+      adamw_split_kernel<__nv_bfloat16><<<blocks, 256, 0, S(stream)>>>(reinterpret_cast<uint2*>(p), reinterpret_cast<uint2*>(p_lo), CBF(g), reinterpret_cast<float4*>(m),
+                                                                       reinterpret_cast<float4*>(v), n4, a, grad_scale);
     else
-      adamw_split8_kernel<float><<<blocks, 256, 0, S(stream)>>>(reinterpret_cast<uint4*>(p), reinterpret_cast<uint4*>(p_lo), reinterpret_cast<const float*>(g), reinterpret_cast<float4*>(m),
-                                                                reinterpret_cast<float4*>(v), n8, a, grad_scale);
-    if (n8 * 8 == n) return static_cast<int>(cudaGetLastError());
-    p = BF(p) + n8 * 8;
-    p_lo = static_cast<int16_t*>(p_lo) + n8 * 8;
-    g = static_cast<const char*>(g) + n8 * 8 * (grad_is_bf16 ? 2 : 4);
-    m += n8 * 8;
-    v += n8 * 8;
-    n -= n8 * 8;
+      adamw_split_kernel<float><<<blocks, 256, 0, S(stream)>>>(reinterpret_cast<uint2*>(p), reinterpret_cast<uint2*>(p_lo), reinterpret_cast<const float*>(g),
+                                                               reinterpret_cast<float4*>(m), reinterpret_cast<float4*>(v), n4, a, grad_scale);
+    if (n4 * 4 == n) return static_cast<int>(cudaGetLastError());
+    p = BF(p) + n4 * 4;
+    p_lo = static_cast<int16_t*>(p_lo) + n4 * 4;
+    g = static_cast<const char*>(g) + n4 * 4 * (grad_is_bf16 ? 2 : 4);
+    m += n4 * 4;
+    v += n4 * 4;
+    n -= n4 * 4;
   }
   const int grid = grid_for(n, 256, 148 * 8);
   if (grad_is_bf16)
@@ -1100,13 +1193,15 @@ RLB_API int rlb_adamw(void* p, void* p_lo, float* p32, const void* g, int grad_i
   return static_cast<int>(cudaGetLastError());
 }
 
-// out += sum(x^2). `out` is a device float the caller zeroes; `part` is scratch of SUMSQ_BLOCKS (1184) doubles.
+// Doubles of scratch that rlb_sumsq needs: one a block.
+RLB_API int rlb_sumsq_parts(long long n, int is_bf16) { return static_cast<int>((n * (is_bf16 ? 2 : 4) + SUMSQ_BYTES - 1) / SUMSQ_BYTES); }
+// out += sum(x^2). `out` is a device float the caller zeroes.
 RLB_API int rlb_sumsq(const void* x, int is_bf16, long long n, float* out, double* part, void* stream) {
   if (n <= 0) return 0;
-  const int grid = grid_for(n, 1024, n < (1 << 24) ? SUMSQ_BLOCKS / 2 : SUMSQ_BLOCKS);      // (few elements: half as many sums to add up)
+  const int grid = rlb_sumsq_parts(n, is_bf16);
   if (is_bf16) sumsq_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(CBF(x), n, part);
   else sumsq_kernel<float><<<grid, 256, 0, S(stream)>>>(reinterpret_cast<const float*>(x), n, part);
-  sumsq_total_kernel<<<1, 256, 0, S(stream)>>>(part, grid, out);
+  sumsq_total_kernel<<<1, 1024, 0, S(stream)>>>(part, grid, out);
   return static_cast<int>(cudaGetLastError());
 }
 RLB_API int rlb_clip_scale(const float* sumsq, float max_norm, float extra, float* scale_out, float* norm_out,

@@ -778,8 +778,9 @@ def sumsq_(x: torch.Tensor, out: torch.Tensor) -> None:
     if not use_native(x):
         out.add_(x.float().pow(2).sum())
         return
-    part = torch.empty(1184, dtype=torch.float64, device=x.device)      # a sum per block
-    call("rlb_sumsq", ptr(x), int(x.dtype == BF16), x.numel(), ptr(out), ptr(part), stream_ptr())
+    bf16 = int(x.dtype == BF16)
+    part = torch.empty(_L.lib().rlb_sumsq_parts(x.numel(), bf16), dtype=torch.float64, device=x.device)      # a sum per block
+    call("rlb_sumsq", ptr(x), bf16, x.numel(), ptr(out), ptr(part), stream_ptr())
 
 
 def clip_scale(sumsq: torch.Tensor, max_norm: float, extra: float, scale_out: torch.Tensor, norm_out: torch.Tensor) -> None:

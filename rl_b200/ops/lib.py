@@ -51,6 +51,7 @@ _SIGS: dict[str, list[Any]] = {
     "rlb_embedding_fwd": [P, P, P, L, I, I, P],
     "rlb_embedding_bwd": [P, P, P, L, I, I, P],
     "rlb_adamw": [P, P, P, P, I, P, P, L, F, F, F, F, F, I, P, P],
+    "rlb_sumsq_parts": [L, I],
     "rlb_sumsq": [P, I, L, P, P, P],
     "rlb_clip_scale": [P, F, F, P, P, P],
     "rlb_clipped_pg": [P, P, P, P, P, P, L, F, F, F, F, I, F, F, I, I, F, F, I, I, I, F, P, P, P],
