@@ -29,6 +29,7 @@ from rl_b200.ops import layer_ops as Y
 from rl_b200.ops import lib as _L
 from rl_b200.ops import mixer_ops as X
 from rl_b200.ops import sequence_ops as S
+from rl_b200.ops.dense_forward import dense_forward
 from rl_b200.parallel.tensor import gather_cols, row_linear
 
 _P, _I, _LL = C.c_void_p, C.c_int, C.c_longlong
@@ -757,13 +758,23 @@ class GenerationEngine:
             dist.broadcast(lp, src=src, group=self.tp.group)
         return tok, lp
 
+    def _dense_prefill(self, h, positions, slots, cu_seqlens, max_seqlen) -> Optional[torch.Tensor]:
+        """The residual stream after all layers on whole sequences, keys and values written to the caches, by one native call; None where the
+        layers are not plain dense ones (quantised copies of the weights, adapters, other families)."""
+        m = self.model
+        if not self.native or self.hybrid or getattr(m, "sharder", None) is not None:
+            return None
+        return dense_forward(m.layers, h, positions, [self._freq(layer) for layer in m.layers], cu_seqlens, max_seqlen, slots=slots,
+                             k_caches=self.k_cache, v_caches=self.v_cache)
+
     @torch.no_grad()
     def _prefill_forward(self, batch: PackedBatch, slots: torch.Tensor, last_idx: torch.Tensor, state_rows=None) -> torch.Tensor:
         m, c = self.model, self.cfg
         h = self._embed(batch.input_ids)
         if hasattr(m, "merge_vision"):
             h = m.merge_vision(h, batch.input_ids, getattr(batch, "mm", None))
-        for li, layer in enumerate(m.layers):
+        whole = self._dense_prefill(h, batch.positions, slots, batch.cu_seqlens, batch.max_seqlen)
+        for li, layer in enumerate(m.layers if whole is None else ()):
             if self.hybrid and layer.kind != "attention":
                 h = self._hybrid_block(li, layer, h, (batch.cu_seqlens, batch.max_seqlen, state_rows))
                 continue
@@ -772,7 +783,7 @@ class GenerationEngine:
             qkv = E.rope_kv_cache_write(qkv, batch.positions, self._freq(layer), slots, self.k_cache[li], self.v_cache[li], self.hq, self.hkv, c.head_dim)
             a = F.attention_varlen(qkv, batch.cu_seqlens, batch.max_seqlen, self.hq, self.hkv, c.head_dim, scale=c.attn_scale, window=layer.window)
             h = self._layer_tail(layer, h, a)
-        hl = E.gather_rows(h, last_idx.to(torch.int32))
+        hl = E.gather_rows(h if whole is None else whole, last_idx.to(torch.int32))
         hl = F.rmsnorm(hl, m.norm, c.rms_norm_eps)
         return self._output_logits(hl)
 
@@ -1352,7 +1363,8 @@ class GenerationEngine:
             fresh = [self._state_row[sid] for sid, _, p, _ in round_items if p == 0]
             if fresh:
                 self._zero_state_rows(torch.tensor(fresh, dtype=torch.int64, device=dev))
-        for li, layer in enumerate(m.layers):
+        whole = self._dense_prefill(h, positions, slots, cu, max(full_lens)) if not pre_slots else None
+        for li, layer in enumerate(m.layers if whole is None else ()):
             if self.hybrid and layer.kind != "attention":
                 h = self._hybrid_block(li, layer, h, (cu_new, max(news), st_rows))
                 continue
@@ -1369,7 +1381,7 @@ class GenerationEngine:
             else:
                 a = F.attention_varlen(qkv, cu, max(full_lens), hq, hkv, D, scale=c.attn_scale, window=layer.window)
             h = self._layer_tail(layer, h, a)
-        hl = E.gather_rows(h, torch.tensor(last, dtype=torch.int32, device=dev))
+        hl = E.gather_rows(h if whole is None else whole, torch.tensor(last, dtype=torch.int32, device=dev))
         return self._output_logits(F.rmsnorm(hl, m.norm, c.rms_norm_eps))
 
     def _window_steps(self, decode, reqs) -> int:

@@ -803,6 +803,13 @@ class CausalLM(nn.Module):
         if cap is not None:
             self.captured = {"embeds": h}
         lo, hi = (0, len(self.layers)) if self.active_chunk is None else self.chunk_bounds[self.active_chunk]
+        if cap is None and not torch.is_grad_enabled() and hi > lo:
+            from rl_b200.ops.dense_forward import dense_forward
+
+            freqs = [inv_freq[bool(layer.window)] if isinstance(inv_freq, tuple) else inv_freq for layer in self.layers[lo:hi]]
+            out = dense_forward(self.layers[lo:hi], h, batch.positions, freqs, batch.cu_seqlens, batch.max_seqlen)
+            if out is not None:
+                return out
         for i in range(lo, hi):
             layer = self.layers[i]
             if self.activation_checkpointing and torch.is_grad_enabled():
