@@ -13,6 +13,7 @@
 #define RLB_EXTERN extern "C"
 RLB_EXTERN int rlb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* res_out, float* rstd, long long rows, int d, long long x_stride,
                                long long y_stride, float eps, void* stream);
+RLB_EXTERN int rlb_gemm_takes_skinny(int M, int N, int K);
 RLB_EXTERN int rlb_gemm_skinny(const void* X, const void* W, void* Y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int out_fp32,
                                const float* bias, const void* residual, long long ldr, int split, int* status, void* stream);
 RLB_EXTERN int rlb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int a_mn_major,
@@ -45,14 +46,14 @@ struct RlbDenseForward {
   const int *positions, *cu_seqlens;
   const long long* slots;         // where keys and values go in the caches, or null
   int* status;
-  int L, T, B, d, Hq, Hkv, D, F, block_size, skinny_max;
+  int L, T, B, d, Hq, Hkv, D, F, block_size;
   long long num_blocks;
   float eps, scale;
 };
 
 namespace {
 int linear(const RlbDenseForward& p, const void* x, const void* w, void* y, int N, int K, const float* bias, const void* residual, void* stream) {
-  if (p.T <= p.skinny_max && K >= 256) return rlb_gemm_skinny(x, w, y, p.T, N, K, K, K, N, 0, bias, residual, residual ? N : 0, 0, p.status, stream);
+  if (rlb_gemm_takes_skinny(p.T, N, K)) return rlb_gemm_skinny(x, w, y, p.T, N, K, K, K, N, 0, bias, residual, residual ? N : 0, 0, p.status, stream);
   return rlb_gemm_bf16(x, w, y, p.T, N, K, K, K, N, 0, 0, 0, 0, bias, residual, residual ? N : 0, p.status, 0, stream);
 }
 }  // namespace

@@ -1,9 +1,11 @@
-// Small-batch ("skinny") bf16 GEMM for decode: Y[M, N] = X[M, K] W[N, K]^T with M <= 256 tokens.
+// Small-batch ("skinny") bf16 GEMM for decode and short passes: Y[M, N] = X[M, K] W[N, K]^T with up to some hundred tokens.
 //
 // At decode time a projection is a weight stream: every byte of W is read once and the arithmetic is nearly free, so
 // the kernel is organised around memory parallelism rather than tile reuse.
 //   * Operands are swapped: 128 rows of W form the M side of the tcgen05 MMA, the tokens form the N side
-//     (UMMA 128 x NT x 16 with NT = 32 / 64 / 128 / 256), so no tensor-core lanes idle on padding rows of X.
+//     (UMMA 128 x NT x 16 with NT = 32 / 64 / 128), so no tensor-core lanes idle on padding rows of X. More than 128 tokens are cut into tiles of 128
+//     (gridDim.y), which read the weights through L2: with all 256 in one tile a CTA had two stages of its ring and a partial sum of 128 KB
+//     (us, all in one tile -> tiles of 128, 240 tokens: 3072 x 2048 23 -> 12, 2048 x 8192 40 -> 17, 4096 x 14336 86 -> 36).
 //   * The reduction dimension is split over the CTAs of a thread-block cluster (1..8). Each CTA streams its K range
 //     through a deep TMA ring, parks its fp32 partial tile in its own shared memory, and after a cluster barrier every
 //     CTA of the cluster sums one slice of the tokens over all partials through distributed shared memory and writes
@@ -44,7 +46,7 @@ struct SkinnyCfg {
   static constexpr int B_BYTES = NT * SK_BK * 2;
   static constexpr int STAGE = A_BYTES + B_BYTES;
   // ring depth so that one CTA uses <= ~110 KB (two CTAs per SM)
-  static constexpr int STAGES = (NT <= 64) ? 4 : (NT == 128 ? 3 : 2);
+  static constexpr int STAGES = NT <= 64 ? 4 : 3;
   static constexpr int RING = STAGES * STAGE;
   static constexpr int PARTIAL = NT * SK_BM * 4;  // fp32 [NT][128]
   static constexpr int MAIN = RING > PARTIAL ? RING : PARTIAL;
@@ -114,6 +116,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       tma_load_2d(dst, &tmap_w, bar, kb * SK_BK, w_row0);
     }
   };
+  const int m0 = blockIdx.y * NT, rows = min(NT, p.M - m0);      // tokens of this tile
   const int num_k = (p.K + SK_BK - 1) / SK_BK;
   const int k_per = (num_k + split - 1) / split;
   const int kb_begin = krank * k_per;
@@ -159,7 +162,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   if (warp == 0) {
     if (lane == 0 && have_work) {
       for (int e = 0; e < early; ++e)
-        tma_load_2d(smem_u32(smem + e * Cfg::STAGE) + Cfg::A_BYTES, &tmap_x, smem_u32(&full_bar[e]), (kb_begin + e) * SK_BK, 0);
+        tma_load_2d(smem_u32(smem + e * Cfg::STAGE) + Cfg::A_BYTES, &tmap_x, smem_u32(&full_bar[e]), (kb_begin + e) * SK_BK, m0);
       uint32_t stage = early == Cfg::STAGES ? 0 : early, phase = early == Cfg::STAGES ? 1 : 0;
       for (int kb = kb_begin + early; kb < kb_end; ++kb) {
         if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.status, RLB_ERR_WAIT_EMPTY)) break;
@@ -167,7 +170,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         const uint32_t a_dst = smem_u32(smem + stage * Cfg::STAGE);
         mbar_arrive_expect_tx(bar, Cfg::STAGE);
         load_w(a_dst, bar, kb);
-        tma_load_2d(a_dst + Cfg::A_BYTES, &tmap_x, bar, kb * SK_BK, 0);
+        tma_load_2d(a_dst + Cfg::A_BYTES, &tmap_x, bar, kb * SK_BK, m0);
         if (++stage == Cfg::STAGES) {
           stage = 0;
           phase ^= 1;
@@ -209,9 +212,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       // per-token reciprocal RMS of the input from the producer's per-tile partial sums (this runs under the mainloop)
       for (int m = threadIdx.x - 64; m < NT; m += 128) {
         float ss = 0.f;
-        if (m < p.M)
-          for (int t = 0; t < p.ssq_in_tiles; ++t) ss += p.ssq_in[t * p.ssq_in_stride + m];
-        s_rstd[m] = m < p.M ? rsqrtf(ss / static_cast<float>(p.K) + p.eps) : 0.f;
+        if (m < rows)
+          for (int t = 0; t < p.ssq_in_tiles; ++t) ss += p.ssq_in[t * p.ssq_in_stride + m0 + m];
+        s_rstd[m] = m < rows ? rsqrtf(ss / static_cast<float>(p.K) + p.eps) : 0.f;
       }
     }
     bool ok = have_work && mbar_wait(smem_u32(acc_bar), 0, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
@@ -242,7 +245,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   {
     const int tok_per = (NT + split - 1) / split;
     const int m_begin = krank * tok_per;
-    const int m_end = min(min(NT, p.M), m_begin + tok_per);
+    const int m_end = min(rows, m_begin + tok_per);
     const uint32_t part_addr = smem_u32(smem);
     const int out_cols = p.swiglu ? 64 : SK_BM;      // output columns of this tile
     const int groups = out_cols / 4;                 // work item: (token m, 4 consecutive output columns)
@@ -255,7 +258,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     auto finish = [&](auto alone) {      // alone: a CTA on its own, without the loops over the cluster, whose instructions cost more than they hide
       for (int it = threadIdx.x; it < items_pad; it += SK_THREADS) {
         const bool live = it < items;
-        const int m = m_begin + (live ? it / groups : 0);
+        const int ml = m_begin + (live ? it / groups : 0), m = m0 + ml;      // in this tile, of all
         const int n4 = (live ? it % groups : 0) * 4;
         const int n = n0 + n4;
         const bool valid = live && n < p.N;  // N is a multiple of 8, so a group of 4 is all in or all out
@@ -265,7 +268,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
           // All that the item needs from memory and from the other CTAs is requested before any of it is waited for: one latency instead of one
           // per CTA of the cluster (projections of an 8B layer in a captured chain, 64 sequences 98.7 -> 97.0 us, one 85.5 -> 83.6; of a 1B
           // layer 46.5 -> 45.1 and 37.9 -> 36.9).
-          const uint32_t off = static_cast<uint32_t>((m * SK_BM + n4) * 4);
+          const uint32_t off = static_cast<uint32_t>((ml * SK_BM + n4) * 4);
           if (p.residual) rv = *reinterpret_cast<const uint2*>(p.residual + static_cast<long long>(m) * p.ldr + n);
           if (p.ssq_out) wv = *reinterpret_cast<const uint2*>(p.norm_w + n);
           if (p.use_layer && p.layer.x) {
@@ -293,7 +296,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
           }
           if (p.ssq_in) {
-            const float rs = s_rstd[m];
+            const float rs = s_rstd[ml];
             acc.x *= rs; acc.y *= rs; acc.z *= rs; acc.w *= rs;
             acc_u.x *= rs; acc_u.y *= rs; acc_u.z *= rs; acc_u.w *= rs;
           }
@@ -360,7 +363,7 @@ int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyPara
   }
   const int tiles = p.swiglu ? (p.N + 63) / 64 : (p.N + SK_BM - 1) / SK_BM;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles * split, 1, 1);
+  cfg.gridDim = dim3(tiles * split, (p.M + NT - 1) / NT, 1);
   cfg.blockDim = dim3(SK_THREADS, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM;
   cfg.stream = stream;
@@ -381,23 +384,22 @@ int launch_skinny_nt(int NT, const CUtensorMap& tw, const CUtensorMap& tx, const
   switch (NT) {
     case 32: return launch_skinny<32>(tw, tx, p, split, s);
     case 64: return launch_skinny<64>(tw, tx, p, split, s);
-    case 128: return launch_skinny<128>(tw, tx, p, split, s);
-    default: return launch_skinny<256>(tw, tx, p, split, s);
+    default: return launch_skinny<128>(tw, tx, p, split, s);
   }
 }
 
 }  // namespace
 
-// Picks the cluster size (K split) for a projection: enough CTAs to cover the SMs twice over at most, never more than
-// 8 (the portable cluster limit), never more than one CTA per 4 k-blocks.
-RLB_API int rlb_gemm_skinny_split(int N, int K) {
+// Cluster size (K split) for a projection of M tokens: the largest power of two up to 8 (the portable cluster limit) with which all CTAs are
+// resident, two to an SM, and each has at least four k-blocks.
+static int skinny_split(int M, int N, int K) {
   if (g_sk_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_sk_sms, cudaDevAttrMultiProcessorCount, dev);
     if (g_sk_sms <= 0) g_sk_sms = 148;
   }
-  const int tiles = (N + SK_BM - 1) / SK_BM;
+  const int tiles = (N + SK_BM - 1) / SK_BM * ((M + 127) / 128);
   const int num_k = (K + SK_BK - 1) / SK_BK;
   int best = 1;
   for (int s = 1; s <= 8; s *= 2) {
@@ -406,6 +408,18 @@ RLB_API int rlb_gemm_skinny_split(int N, int K) {
     best = s;
   }
   return best;
+}
+RLB_API int rlb_gemm_skinny_split(int N, int K) { return skinny_split(1, N, K); }
+
+// Whether a product of M tokens is sooner done here than on the tiled kernel (gemm_tcgen05.cu): up to 128 tokens, and up to 1024 where the
+// contraction can be split at least in two. Timed both ways, weights from memory, us (here / tiled): 3072 x 2048: 129 tokens 12 / 18, 256 12 / 19,
+// 512 17 / 19, 768 17 / 19, 1024 (one part) 24 / 19; 2048 x 8192: 256 17 / 46, 512 23 / 46, 1024 38 / 46; 6144 x 4096: 256 25 / 29, 384 25 / 29, 512
+// (one part) 37 / 29; 4096 x 14336: 256 36 / 74, 512 62 / 74, 640 (one part) 96 / 78; 16384 x 2048 (one part): 256 27 / 22; 28672 x 4096 (one part):
+// 256 91 / 61, but 128 tokens 52 / 49 and 65 49 / 49.
+constexpr int SK_MAX_TOKENS = 1024;
+RLB_API int rlb_gemm_takes_skinny(int M, int N, int K) {
+  if (K < 256 || M > SK_MAX_TOKENS) return 0;
+  return M <= 128 || skinny_split(M, N, K) > 1;
 }
 
 // While set, callers promise that the W operand of every skinny GEMM was not written by the kernel launched just before
@@ -417,7 +431,7 @@ RLB_API int rlb_gemm_skinny_static_weights(int on) {
   return prev;
 }
 
-// Y[M, N] = X[M, K] W[N, K]^T (+ bias) (+ residual); M <= 256. ldx / ldw / ldy / ldr in elements (multiples of 8;
+// Y[M, N] = X[M, K] W[N, K]^T (+ bias) (+ residual); M <= 1024. ldx / ldw / ldy / ldr in elements (multiples of 8;
 // fp32 output: ldy multiple of 4). `split` = 0 lets the library choose. Returns 0, a CUDA error or a negative code.
 //
 // Optional fusions (see the head of this file), each switched on by a non-null pointer / non-zero flag:
@@ -432,12 +446,15 @@ RLB_API int rlb_gemm_skinny_fused(const void* X, const void* W, void* Y, int M, 
                                   float* ssq_out, long long ssq_out_stride, const void* norm_w, void* Y2, long long ldy2,
                                   int swiglu, int* status, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (M > 256) return -7;
+  if (M > SK_MAX_TOKENS) return -7;
   if ((ldx % 8) || (ldw % 8) || (N % 8) || (ldy % (out_fp32 ? 4 : 8)) || (residual && (ldr % 4))) return -2;
+  // (beyond 256 tokens with the tiled kernel's alignments)
+  if (M > 256 && residual && ((ldr % 8) || (reinterpret_cast<uintptr_t>(residual) & 15))) return -2;
+  if (M > 256 && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(Y)) & 15)) return -3;
   if (swiglu && ((N % 64) || bias || residual || ssq_out)) return -2;
   if (ssq_out && (out_fp32 || !norm_w || !Y2 || (ldy2 % 4) || ssq_out_stride < M)) return -2;
   if (ssq_in && (ssq_in_tiles <= 0 || ssq_in_stride < M)) return -2;
-  const int NT = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256));
+  const int NT = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
   CUtensorMap tw, tx;
   const int w_rows = swiglu ? 2 * N : N;
   int rc = rlb_make_tmap_2d(&tw, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, w_rows, ldw * 2, SK_BK, swiglu ? 64 : SK_BM,
@@ -446,7 +463,7 @@ RLB_API int rlb_gemm_skinny_fused(const void* X, const void* W, void* Y, int M, 
   rc = rlb_make_tmap_2d(&tx, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, ldx * 2, SK_BK, NT,
                         CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return -100 - rc;
-  if (split <= 0) split = rlb_gemm_skinny_split(w_rows, K);
+  if (split <= 0) split = skinny_split(M, w_rows, K);
   if (split > 8) split = 8;
   SkinnyParams p;
   p.Y = Y;
@@ -475,18 +492,18 @@ RLB_API int rlb_gemm_skinny_fused(const void* X, const void* W, void* Y, int M, 
   return launch_skinny_nt(NT, tw, tx, p, split, static_cast<cudaStream_t>(stream));
 }
 
-// rlb_gemm_layer for M <= 256 rows on the weight-streaming kernel.
+// rlb_gemm_layer for M <= 1024 rows on the weight-streaming kernel.
 RLB_API int rlb_gemm_skinny_layer(const void* X, const void* W, void* out, int M, int N, int K, long long ldx_in, long long ldw, long long ldo,
                                   int act_from, float* x, long long ldx, const float* e, const void* step, const void* alpha,
                                   const void* nw, const void* nb, int* status, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (M > 256) return -7;
+  if (M > SK_MAX_TOKENS) return -7;
   if ((ldx_in % 8) || (ldw % 8) || (ldo % 8) || (N % 8) || (K % 8) || (act_from % 8) || (ldx % 4)) return -2;
   if (x && (!alpha || !nw || !nb)) return -2;
   if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(x) |
        reinterpret_cast<uintptr_t>(e) | reinterpret_cast<uintptr_t>(step) | reinterpret_cast<uintptr_t>(nw) | reinterpret_cast<uintptr_t>(nb)) & 15)
     return -3;
-  const int NT = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256));
+  const int NT = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
   CUtensorMap tw, tx;
   int rc = rlb_make_tmap_2d(&tw, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, ldw * 2, SK_BK, SK_BM, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return -100 - rc;
@@ -503,17 +520,17 @@ RLB_API int rlb_gemm_skinny_layer(const void* X, const void* W, void* out, int M
   p.use_layer = 1;
   p.layer = LayerEpilogue{x, ldx, e, static_cast<const __nv_bfloat16*>(step), static_cast<const __nv_bfloat16*>(alpha),
                           static_cast<const __nv_bfloat16*>(nw), static_cast<const __nv_bfloat16*>(nb), act_from, LinearEpi{}};
-  return launch_skinny_nt(NT, tw, tx, p, rlb_gemm_skinny_split(N, K), static_cast<cudaStream_t>(stream));
+  return launch_skinny_nt(NT, tw, tx, p, skinny_split(M, N, K), static_cast<cudaStream_t>(stream));
 }
 
-// rlb_linear_tiled for M <= 256 rows on the weight-streaming kernel; out bf16 or fp32 (fp32: no gated unit).
+// rlb_linear_tiled for M <= 1024 rows on the weight-streaming kernel; out bf16 or fp32 (fp32: no gated unit).
 RLB_API int rlb_linear_skinny(const RlbLinear* l, void* stream) {
   if (l->M <= 0 || l->N <= 0 || l->K <= 0) return 0;
-  if (l->M > 256) return -7;
+  if (l->M > SK_MAX_TOKENS) return -7;
   if ((l->lda % 8) || (l->ldw % 8) || (l->ldo % (l->out_f32 ? 4 : 8)) || (l->N % 8) || (l->K % 8) || l->in_f32 || l->tile_expert || l->row_scale) return -2;
   if (l->out_f32 && lin_gated(l->act)) return -2;
   if ((reinterpret_cast<uintptr_t>(l->a) | reinterpret_cast<uintptr_t>(l->w) | reinterpret_cast<uintptr_t>(l->out) | reinterpret_cast<uintptr_t>(l->bias)) & 15) return -3;
-  const int NT = l->M <= 32 ? 32 : (l->M <= 64 ? 64 : (l->M <= 128 ? 128 : 256));
+  const int NT = l->M <= 32 ? 32 : (l->M <= 64 ? 64 : 128);
   CUtensorMap tw, tx;
   int rc = rlb_make_tmap_2d(&tw, l->w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, l->K, l->N, l->ldw * 2, SK_BK, SK_BM, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return -100 - rc;
@@ -531,7 +548,7 @@ RLB_API int rlb_linear_skinny(const RlbLinear* l, void* stream) {
   p.use_layer = 1;
   p.layer.act_from = 1 << 30;
   p.layer.lin = rlb_linear_epi(*l);
-  return launch_skinny_nt(NT, tw, tx, p, rlb_gemm_skinny_split(l->N, l->K), static_cast<cudaStream_t>(stream));
+  return launch_skinny_nt(NT, tw, tx, p, skinny_split(l->M, l->N, l->K), static_cast<cudaStream_t>(stream));
 }
 
 RLB_API int rlb_gemm_skinny(const void* X, const void* W, void* Y, int M, int N, int K, long long ldx, long long ldw,

@@ -25,7 +25,7 @@ class _Layer(C.Structure):
 
 class _Forward(C.Structure):
     _fields_ = [(n, _P) for n in ("layers", "h", "out", "mid", "x", "qkv", "att", "gate_up", "act", "positions", "cu_seqlens", "slots", "status")]
-    _fields_ += [(n, _I) for n in ("L", "T", "B", "d", "Hq", "Hkv", "D", "F", "block_size", "skinny_max")]
+    _fields_ += [(n, _I) for n in ("L", "T", "B", "d", "Hq", "Hkv", "D", "F", "block_size")]
     _fields_ += [("num_blocks", _LL), ("eps", _F), ("scale", _F)]
 
 
@@ -39,7 +39,8 @@ def _weights(layer) -> Optional[tuple]:
 
     if type(layer) is not DecoderLayer or layer.cfg.sandwich_norm:
         return None
-    at, mlp = layer.self_attn, layer.mlp
+    mods = layer._modules      # (attribute access of modules and parameters by name goes through a Python function each time)
+    at, mlp = mods["self_attn"], mods["mlp"]
     if type(at) is not Attention or type(mlp) is not DenseMLP or not mlp.gated or mlp.act != "silu" or at.cp is not None or at.tp.world > 1 or mlp.tp.world > 1:
         return None
     if at.qkv_lora is not None or at.o_lora is not None or mlp.gate_up_lora is not None or mlp.down_lora is not None:
@@ -47,12 +48,13 @@ def _weights(layer) -> Optional[tuple]:
     for m in (layer, at, mlp):
         if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
             return None
-    norms = (at.q_norm, at.k_norm) if layer.cfg.qk_norm else (None, None)
-    ws = (layer.input_layernorm, at.qkv_proj, at.o_proj, layer.post_attention_layernorm, mlp.gate_up_proj, mlp.down_proj, *norms, at.qkv_bias)
+    own, a, f = layer._parameters, at._parameters, mlp._parameters
+    ws = (own["input_layernorm"], a["qkv_proj"], a["o_proj"], own["post_attention_layernorm"], f["gate_up_proj"], f["down_proj"], a.get("q_norm"), a.get("k_norm"),
+          a.get("qkv_bias"))
     if any(w.dim() != 2 or not w.numel() for w in (ws[1], ws[2], ws[4], ws[5])):      # (sharded elsewhere)
         return None
     for w in ws:
-        if w is not None and (w.dtype != torch.bfloat16 or not w.is_contiguous() or w.data_ptr() % 16 or hasattr(w, "_rlb_qat") or hasattr(w, "_rlb_q")):
+        if w is not None and (w.dtype != torch.bfloat16 or not w.is_contiguous() or w.data_ptr() % 16 or "_rlb_qat" in w.__dict__ or "_rlb_q" in w.__dict__):
             return None
     return ws
 
@@ -98,7 +100,7 @@ def dense_forward(layers: Sequence, h: torch.Tensor, positions: torch.Tensor, in
         layers=C.cast(array, _P), h=ptr(h), out=ptr(out), mid=ptr(mid), x=ptr(x), qkv=ptr(qkv), att=ptr(att), gate_up=ptr(gu), act=ptr(act),
         positions=ptr(positions), cu_seqlens=ptr(cu), slots=ptr(slots),
         status=ptr(_L.status_word(h.device)), L=len(layers), T=T, B=cu.numel() - 1, d=d, Hq=Hq, Hkv=Hkv, D=D, F=ff,
-        block_size=k_caches[0].shape[2] if slots is not None else 0, skinny_max=F.SKINNY_MAX_M,
+        block_size=k_caches[0].shape[2] if slots is not None else 0,
         num_blocks=k_caches[0].shape[0] if slots is not None else 0, eps=c.rms_norm_eps,
         scale=c.attn_scale if c.attn_scale is not None else 1.0 / math.sqrt(D))), stream_ptr())
     Counters.launches += len(layers) * (9 + bool(c.qk_norm)) - 1

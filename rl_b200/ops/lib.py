@@ -31,6 +31,7 @@ _SIGS: dict[str, list[Any]] = {
     "rlb_gemm_skinny": [P, P, P, I, I, I, L, L, L, I, P, P, L, I, P, P],
     "rlb_gemm_skinny_fused": [P, P, P, I, I, I, L, L, L, I, P, P, L, I, P, I, L, F, P, L, P, P, L, I, P, P],
     "rlb_gemm_skinny_split": [I, I],
+    "rlb_gemm_takes_skinny": [I, I, I],
     "rlb_gemm_skinny_static_weights": [I],
     "rlb_lm_head_logprob": [P, P, I, I, I, L, L, P, F, P, P, P, P, P, P, P, P, L, P, P],
     "rlb_lm_head_dlogits_kept": [P, P, I, I, L, L, P, F, P, P, P, P, P],

@@ -256,6 +256,35 @@ def test_skinny_gemm(native_lib, M, N, K):
     assert _rel_err(y2, ref + bias + res.float()) < 2e-3
 
 
+@pytest.mark.parametrize("M", [129, 130, 255, 257, 384, 385, 512, 640, 1000, 1024])      # token tiles of 128, whole and cut
+@pytest.mark.parametrize("N,K", [(1000, 512), (2048, 264), (264, 8192), (4096, 1024)])
+def test_skinny_token_tiles(native_lib, M, N, K):
+    """More tokens than one tile holds, with norm statistics from and for the neighbours, against fp32. Inputs of one: a bf16 result is off by 2^-9
+    of itself, the sums of its squares by fp32 rounding and that."""
+    from rl_b200.ops import engine_ops as E
+    from rl_b200.ops.lib import call, check_status, lib, ptr, status_word, stream_ptr
+
+    g = torch.Generator("cuda").manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=g, device="cuda").bfloat16(), (torch.randn(N, K, generator=g, device="cuda") / K ** 0.5).bfloat16()
+    res, bias = torch.randn(M, N, generator=g, device="cuda").bfloat16(), torch.randn(N, generator=g, device="cuda")
+    ref = x.float() @ w.float().t() + bias + res.float()
+    for split in (0, 1, 3, 8):
+        y = torch.full((M + 1, N), 7.0, device="cuda").bfloat16()
+        call("rlb_gemm_skinny", ptr(x), ptr(w), ptr(y), M, N, K, K, K, N, 0, ptr(bias), ptr(res), N, split, ptr(status_word(x.device)), stream_ptr())
+        assert (y[:M].float() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max() and bool((y[M] == 7).all())
+    assert check_status() == 0
+    if N % 128 == 0 and M <= 256:      # the decode step's hand-off of norm statistics
+        ssq, hw, nw = torch.zeros(N // 128, 256, device="cuda"), torch.empty(M, N, device="cuda").bfloat16(), torch.rand(N, generator=g, device="cuda").bfloat16()
+        h = E.skinny_linear(x, w, residual=res, ssq_out=ssq, norm_w=nw, out2=hw)
+        assert torch.allclose(ssq[:, :M].sum(0), h.float().pow(2).sum(1), rtol=1e-4)
+        assert (hw.float() - h.float() * nw.float()).abs().max() <= 2.0 ** -8 * h.float().abs().max()
+        w2 = (torch.randn(256, N, generator=g, device="cuda") / N ** 0.5).bfloat16()
+        act = E.skinny_linear(hw, w2, ssq_in=ssq, eps=1e-5, swiglu=True)
+        z = (hw.float() @ w2.float().t()) * torch.rsqrt(h.float().pow(2).mean(1, keepdim=True) + 1e-5)
+        want = torch.nn.functional.silu(z[:, :128]) * z[:, 128:]
+        assert (act.float() - want).abs().max() <= 2.0 ** -7 * want.abs().max()
+
+
 def test_skinny_split_values(native_lib):
     from rl_b200.ops.lib import call, lib, ptr, status_word, stream_ptr
 
