@@ -16,7 +16,7 @@ from typing import Any, Optional
 
 import torch
 
-from rl_b200.algorithms.utils import calculate_kl, masked_mean
+from rl_b200.algorithms.utils import DeferredMetrics, calculate_kl, masked_mean
 from rl_b200.ops import lib as _L
 
 from .interfaces import LossInputType, LossType
@@ -44,6 +44,12 @@ CLIPPED_PG_DEFAULTS = dict(
 )
 
 
+def host_value(count) -> float:
+    """A global count as a number: the one that came along with the tensor (``host``), else read from it."""
+    known = getattr(count, "host", None)
+    return float(count if known is None else known)
+
+
 def _nan_to_zero(x: torch.Tensor) -> torch.Tensor:
     return torch.nan_to_num(x, nan=0.0, posinf=0.0, neginf=0.0)
 
@@ -55,7 +61,7 @@ class _FusedPG(torch.autograd.Function):
     def forward(ctx, curr, prev, gen, ref, adv, mask, cfg, inv_norm):
         T = curr.numel()
         dev = curr.device
-        sums = torch.empty(16, dtype=torch.float32, device=dev)
+        sums = torch.empty(16, dtype=torch.float64, device=dev)
         dcurr = torch.empty(T, dtype=torch.float32, device=dev)
         kl_type = {"k1": 1, "k2": 2, "k3": 3}[cfg["reference_policy_kl_type"]]
         tis_ratio = cfg["truncated_importance_sampling_ratio"]
@@ -78,7 +84,7 @@ class _FusedPG(torch.autograd.Function):
         ctx.save_for_backward(dcurr)
         ctx.shape = curr.shape
         beta = float(cfg["reference_policy_kl_penalty"]) if ref is not None else 0.0
-        loss = (sums[0] + beta * sums[1]) * inv_norm
+        loss = ((sums[0] + beta * sums[1]) * inv_norm).float()
         ctx.mark_non_differentiable(sums)
         return loss, sums
 
@@ -144,35 +150,36 @@ class ClippedPGLossFn:
     def _fused(self, curr, prev, gen, ref, adv, mask, sample_mask, global_valid_toks):
         c = self.cfg
         beta = c["reference_policy_kl_penalty"]
-        inv_norm = 1.0 / (float(global_valid_toks) + 1e-8)
+        inv_norm = 1.0 / (host_value(global_valid_toks) + 1e-8)
         f = lambda t: None if t is None else t.float().contiguous()
         loss, sums = _FusedPG.apply(f(curr), f(prev), f(gen), f(ref), f(adv), f(mask), c, inv_norm)
-        s = (sums.detach() * inv_norm).tolist()
-        raw = sums.detach()
-        rmin, rmax, cmin, cmax = raw[10].item(), raw[11].item(), raw[12].item(), raw[13].item()
-        if raw[5].item() == 0:
-            rmin, rmax, cmin, cmax = float("inf"), float("-inf"), float("inf"), float("-inf")
-        metrics = {
-            "loss": loss.item(),
-            "probs_ratio": s[2],
-            "probs_ratio_clamped": s[3],
-            "probs_ratio_min": rmin,
-            "probs_ratio_max": rmax,
-            "probs_ratio_clamped_min": cmin,
-            "probs_ratio_clamped_max": cmax,
-            "kl_penalty": s[1] if beta != 0 else 0,
-            "token_mult_prob_error": s[4],
-            "gen_kl_error": s[6],
-            "policy_kl_error": s[7],
-            "js_divergence_error": s[14],
-            "sampling_importance_ratio": s[8],
-            "num_valid_samples": sample_mask.sum().item(),
-            "approx_entropy": s[9],
-            "positive_nll_loss": 0.0,
-        }
-        if c["truncated_importance_sampling_ratio"] is not None:
-            metrics["is_oob_ratio"] = s[15]
-        return loss, metrics
+
+        def make(raw):
+            s = [v * inv_norm for v in raw[:16]]
+            rmin, rmax, cmin, cmax = raw[10:14] if raw[5] != 0 else (float("inf"), float("-inf"), float("inf"), float("-inf"))
+            metrics = {
+                "loss": raw[16],
+                "probs_ratio": s[2],
+                "probs_ratio_clamped": s[3],
+                "probs_ratio_min": rmin,
+                "probs_ratio_max": rmax,
+                "probs_ratio_clamped_min": cmin,
+                "probs_ratio_clamped_max": cmax,
+                "kl_penalty": s[1] if beta != 0 else 0,
+                "token_mult_prob_error": s[4],
+                "gen_kl_error": s[6],
+                "policy_kl_error": s[7],
+                "js_divergence_error": s[14],
+                "sampling_importance_ratio": s[8],
+                "num_valid_samples": raw[17],
+                "approx_entropy": s[9],
+                "positive_nll_loss": 0.0,
+            }
+            if c["truncated_importance_sampling_ratio"] is not None:
+                metrics["is_oob_ratio"] = s[15]
+            return metrics
+
+        return loss, DeferredMetrics(torch.cat([sums.detach(), torch.stack([loss.detach(), sample_mask.sum()]).double()]), make)
 
     # ---- PyTorch statement of the same math (CPU path, oracle, and every non-fused configuration)
     def _reference(self, curr, prev, gen, ref, adv, token_mask, sample_mask, mask, data, gvs, gvt):
@@ -324,8 +331,10 @@ class NLLLossFn:
         else:
             num_unmasked = mask.sum()
             loss = -masked_mean(next_token_logprobs, mask, global_normalization_factor=global_valid_toks)
-        return loss, {"loss": loss.item() if loss.dim() == 0 else loss,
-                      "num_unmasked_tokens": num_unmasked.item(), "num_valid_samples": sample_mask.sum().item()}
+        if loss.dim() != 0:
+            return loss, {"loss": loss, "num_unmasked_tokens": num_unmasked.item(), "num_valid_samples": sample_mask.sum().item()}
+        names = ("loss", "num_unmasked_tokens", "num_valid_samples")
+        return loss, DeferredMetrics(torch.stack([loss.detach(), num_unmasked, sample_mask.sum()]), lambda v: dict(zip(names, v)))
 
 
 class PreferenceLossFn:

@@ -44,6 +44,77 @@ def calculate_kl(logprobs: torch.Tensor, logprobs_reference: torch.Tensor, kl_ty
     return kl
 
 
+class DeferredMetrics(dict):
+    """Metrics whose numbers are still on the device: ``make(numbers)`` turns the values of ``device_values`` (a 1-D tensor) into the dict, which
+    happens at the first look at it. A training step that looks only when its kernels are all enqueued does not wait for them in between."""
+
+    def __init__(self, device_values: torch.Tensor, make):
+        super().__init__()
+        self._pending = (device_values, make)
+
+    def _resolve(self):
+        if self._pending is not None:
+            values, make = self._pending
+            self._pending = None
+            added = dict(dict.items(self))
+            dict.update(self, make(values.tolist()))
+            dict.update(self, added)
+        return self
+
+    def __reduce__(self):
+        return dict, (dict(self._resolve()),)
+
+    def __iter__(self):
+        return dict.__iter__(self._resolve())
+
+    def __len__(self):
+        return dict.__len__(self._resolve())
+
+    def __contains__(self, k):
+        return dict.__contains__(self._resolve(), k)
+
+    def __getitem__(self, k):
+        return dict.__getitem__(self._resolve(), k)
+
+    def __eq__(self, other):
+        return dict.__eq__(self._resolve(), other)
+
+    __hash__ = None
+
+    def __repr__(self):
+        return dict.__repr__(self._resolve())
+
+    def keys(self):
+        return dict.keys(self._resolve())
+
+    def values(self):
+        return dict.values(self._resolve())
+
+    def items(self):
+        return dict.items(self._resolve())
+
+    def get(self, k, default=None):
+        return dict.get(self._resolve(), k, default)
+
+    def pop(self, *a):
+        return dict.pop(self._resolve(), *a)
+
+    def setdefault(self, *a):
+        return dict.setdefault(self._resolve(), *a)
+
+    def __delitem__(self, k):
+        dict.__delitem__(self._resolve(), k)
+
+    def copy(self):
+        return dict(self._resolve())
+
+    def __or__(self, other):
+        return dict(self._resolve()) | other
+
+    def __ror__(self, other):
+        return other | dict(self._resolve())
+
+
 def masked_mean(values: torch.Tensor, mask: torch.Tensor, dim: Optional[int] = None,
                 global_normalization_factor=None) -> torch.Tensor:
     """sum(values * mask) / (N + 1e-8), with N the mask sum or a caller-supplied global count."""

@@ -827,11 +827,26 @@ struct PGArgs {
   float inv_norm;    // 1 / (global valid tokens + 1e-8)
 };
 
+// Sum over the block, in fp64: terms of either sign nearly cancel in the loss, and blocks add their sums in any order.
+__device__ __forceinline__ double block_sum64(double v, double* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if (lane == 0) red[w] = v;
+  __syncthreads();
+  double s = 0.0;
+  if (threadIdx.x == 0)
+    for (int i = 0; i < nw; ++i) s += red[i];
+  return s;      // (thread 0)
+}
+
 __global__ void clipped_pg_kernel(const float* __restrict__ curr, const float* __restrict__ prev,
                                   const float* __restrict__ gen, const float* __restrict__ ref,
                                   const float* __restrict__ adv, const float* __restrict__ mask, long long T,
-                                  PGArgs a, float* __restrict__ sums, float* __restrict__ dcurr) {
+                                  PGArgs a, double* __restrict__ sums, float* __restrict__ dcurr) {
   __shared__ float red[32];
+  __shared__ double red64[32];
   float acc[10];
 #pragma unroll
   for (int i = 0; i < 10; ++i) acc[i] = 0.f;
@@ -955,34 +970,35 @@ __global__ void clipped_pg_kernel(const float* __restrict__ curr, const float* _
   }
 #pragma unroll
   for (int i = 0; i < 10; ++i) {
-    const float s = block_sum(acc[i], red);
+    const double s = block_sum64(acc[i], red64);
     if (threadIdx.x == 0) atomicAdd(sums + i, s);
   }
   {
-    const float s = block_sum(js, red);
+    const double s = block_sum64(js, red64);
     if (threadIdx.x == 0) atomicAdd(sums + 14, s);
     (void)nclip;
-    const float s2 = block_sum(oob, red);
+    const double s2 = block_sum64(oob, red64);
     if (threadIdx.x == 0) atomicAdd(sums + 15, s2);
   }
-  // min/max via integer atomics on non-negative floats (ratios are > 0)
+  // min/max via integer atomics on non-negative values (ratios are > 0)
   rmin = -block_max(-rmin, red);
   rmax = block_max(rmax, red);
   cmin = -block_max(-cmin, red);
   cmax = block_max(cmax, red);
   if (threadIdx.x == 0) {
-    if (isfinite(rmin)) atomicMin(reinterpret_cast<int*>(sums + 10), __float_as_int(rmin));
-    if (isfinite(rmax)) atomicMax(reinterpret_cast<int*>(sums + 11), __float_as_int(rmax));
-    if (isfinite(cmin)) atomicMin(reinterpret_cast<int*>(sums + 12), __float_as_int(cmin));
-    if (isfinite(cmax)) atomicMax(reinterpret_cast<int*>(sums + 13), __float_as_int(cmax));
+    long long* bits = reinterpret_cast<long long*>(sums);
+    if (isfinite(rmin)) atomicMin(bits + 10, __double_as_longlong(rmin));
+    if (isfinite(rmax)) atomicMax(bits + 11, __double_as_longlong(rmax));
+    if (isfinite(cmin)) atomicMin(bits + 12, __double_as_longlong(cmin));
+    if (isfinite(cmax)) atomicMax(bits + 13, __double_as_longlong(cmax));
   }
 }
 
-__global__ void pg_init_sums_kernel(float* sums) {
+__global__ void pg_init_sums_kernel(double* sums) {
   const int i = threadIdx.x;
   if (i < 16) {
-    float v = 0.f;
-    if (i == 10 || i == 12) v = 3.0e38f;  // running minima start high
+    double v = 0.0;
+    if (i == 10 || i == 12) v = 3.0e38;  // running minima start high
     sums[i] = v;
   }
 }
@@ -1214,7 +1230,7 @@ RLB_API int rlb_clipped_pg(const float* curr, const float* prev, const float* ge
                            const float* adv, const float* mask, long long T, float eps_lo, float eps_hi,
                            float dual_c, float kl_beta, int kl_type, float kl_in_clamp, float kl_out_clamp,
                            int use_is, int tis_type, float tis_max, float tis_min, int force_on_policy,
-                           int use_cispo, int on_policy_kl_approx, float inv_norm, float* sums, float* dcurr,
+                           int use_cispo, int on_policy_kl_approx, float inv_norm, double* sums, float* dcurr,
                            void* stream) {
   PGArgs a{eps_lo, eps_hi, dual_c, kl_beta, kl_type, kl_in_clamp, kl_out_clamp, use_is, tis_type, tis_max,
            tis_min, force_on_policy, use_cispo, on_policy_kl_approx, inv_norm};

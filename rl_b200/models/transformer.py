@@ -14,7 +14,7 @@ from __future__ import annotations
 
 import math
 from dataclasses import dataclass
-from typing import Optional
+from typing import Optional, Sequence
 
 import torch
 import torch.nn as nn
@@ -453,6 +453,7 @@ class PackedBatch:
     cu_seqlens: torch.Tensor
     max_seqlen: int
     num_real_tokens: Optional[int] = None  # set when a dummy tail sequence pads the stream (see pad_to_multiple)
+    rows: Optional[torch.Tensor] = None    # sequence of every real token, where the lengths were known on the host
 
     def pad_to_multiple(self, m: int, pad_id: int = 0) -> "PackedBatch":
         """Appends one dummy sequence of pad tokens so that the token count divides by ``m`` (sequence-parallel rows
@@ -465,12 +466,22 @@ class PackedBatch:
         ids = torch.cat([self.input_ids, torch.full((r,), pad_id, dtype=self.input_ids.dtype, device=dev)])
         pos = torch.cat([self.positions, torch.arange(r, dtype=self.positions.dtype, device=dev)])
         cu = torch.cat([self.cu_seqlens, torch.tensor([T + r], dtype=self.cu_seqlens.dtype, device=dev)])
-        return PackedBatch(ids, pos, cu, max(self.max_seqlen, r), num_real_tokens=T)
+        return PackedBatch(ids, pos, cu, max(self.max_seqlen, r), num_real_tokens=T, rows=self.rows)
 
     @staticmethod
-    def from_padded(input_ids: torch.Tensor, lengths: torch.Tensor) -> "PackedBatch":
-        """[B, S] right-padded ids + lengths [B] -> packed stream (pads dropped)."""
+    def from_padded(input_ids: torch.Tensor, lengths: torch.Tensor, host_lengths: Optional[Sequence[int]] = None) -> "PackedBatch":
+        """[B, S] right-padded ids + lengths [B] -> packed stream (pads dropped). With the lengths also on the host nothing waits for the device."""
         B, S = input_ids.shape
+        if host_lengths is not None and B:
+            n = [min(max(int(x), 0), S) for x in host_lengths]
+            dev, T = input_ids.device, sum(n)
+            lengths = lengths.to(dev).long().clamp(min=0, max=S)
+            rows = torch.repeat_interleave(torch.arange(B, device=dev), lengths, output_size=T)
+            ends = lengths.cumsum(0)
+            pos = torch.arange(T, device=dev) - (ends - lengths)[rows]
+            cu = torch.zeros(B + 1, dtype=torch.int32, device=dev)
+            cu[1:] = ends
+            return PackedBatch(input_ids[rows, pos], pos.to(torch.int32), cu, max(n), rows=rows)
         lengths = lengths.to(input_ids.device).long().clamp(max=S)
         ar = torch.arange(S, device=input_ids.device)
         keep = ar[None, :] < lengths[:, None]
@@ -486,8 +497,11 @@ class PackedBatch:
         if self.num_real_tokens is not None:  # drop the dummy tail sequence
             cu, flat = cu[:-1], flat[: self.num_real_tokens]
         B = cu.numel() - 1
-        lengths = (cu[1:] - cu[:-1]).long()
         out = flat.new_full((B, S) + tuple(flat.shape[1:]), fill)
+        if self.rows is not None and self.max_seqlen <= S and flat.shape[0] == self.rows.shape[0]:
+            out[self.rows, self.positions[: self.rows.shape[0]].long()] = flat
+            return out
+        lengths = (cu[1:] - cu[:-1]).long()
         ar = torch.arange(S, device=flat.device)
         keep = ar[None, :] < lengths[:, None]
         out[keep] = flat
@@ -868,9 +882,8 @@ class CausalLM(nn.Module):
         """``h``: normed final hidden states (this rank's rows). out[t] = log p(ids[t] | ids[<t]), 0 at sequence starts."""
         ids = batch.input_ids.long()
         T = ids.shape[0]
-        starts = batch.cu_seqlens[:-1].long()
-        is_start = torch.zeros(T, dtype=torch.bool, device=h.device)
-        is_start[starts[starts < T]] = True
+        is_start = torch.zeros(T + 1, dtype=torch.bool, device=h.device)
+        is_start = is_start.index_fill_(0, batch.cu_seqlens[:-1].long(), True)[:T]      # (empty sequences at the end begin behind the last token)
         # hidden state t predicts token t+1: every row is scored against the next token, then shifted by one
         targets = torch.roll(ids, -1)
         if self.cfg.caps_logits:

@@ -708,7 +708,9 @@ def _kept_logits(M: int, N: int, dev) -> Optional[torch.Tensor]:
     step = max(64, (1 << M.bit_length()) // 8)
     rows = -(-M // step) * step
     # (this process's own count: asking the driver took from 0.2 to 90 ms)
-    if torch.cuda.memory_allocated(dev) + 16 * rows * N > 0.95 * torch.cuda.get_device_properties(dev).total_memory:
+    stats = torch.cuda.memory.memory_stats_as_nested_dict(dev)      # (as a flat dict 0.2 ms)
+    used = stats["allocated_bytes"]["all"]["current"] if "allocated_bytes" in stats else math.inf
+    if used + 16 * rows * N > 0.95 * torch.cuda.get_device_properties(dev).total_memory:
         return None
     try:
         return torch.empty((rows, N), dtype=torch.float32, device=dev)

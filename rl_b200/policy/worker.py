@@ -23,6 +23,7 @@ import torch
 import torch.distributed as dist
 
 from rl_b200.algorithms.loss.interfaces import LossInputType, LossType
+from rl_b200.algorithms.utils import DeferredMetrics
 from rl_b200.distributed.batched_data_dict import BatchedDataDict
 from rl_b200.models.config import ModelConfig, preset
 from rl_b200.models.transformer import CausalLM, PackedBatch, build_model
@@ -797,7 +798,8 @@ class PolicyWorker:
     def _pack(self, mb: BatchedDataDict) -> tuple[PackedBatch, int]:
         ids = to_device(mb["input_ids"], self.device)
         lens = to_device(mb["input_lengths"], self.device)
-        batch = PackedBatch.from_padded(ids, lens)
+        known = mb["input_lengths"] if mb["input_lengths"].device.type == "cpu" else None
+        batch = PackedBatch.from_padded(ids, lens, known.tolist() if known is not None else None)
         if self.device.type == "cuda":
             batch.input_ids = batch.input_ids.to(torch.int32)
         if self.tp.world > 1 and self.tp.sequence_parallel:
@@ -805,14 +807,14 @@ class PolicyWorker:
         elif self.cp.world > 1:
             batch = batch.pad_to_multiple(16 * self.cp.world)   # 2 cp chunks of whole 8-row groups
         if self.router_replay:
-            self._set_router_replay(mb, lens, ids.shape[1], int(batch.input_ids.numel()))
+            self._set_router_replay(mb, lens, ids.shape[1], batch)
         if "pixel_patches" in mb:   # vision-language batch: image patch rows in sample order (models/vision.py)
             parts = [t for t in mb["pixel_patches"] if t is not None]
             batch.mm = dict(patches=to_device(torch.cat(parts), self.device) if parts else None,
                             sizes=[int(x) for row in mb["image_sizes"] for x in (row or [])])
         return batch, ids.shape[1]
 
-    def _set_router_replay(self, mb: BatchedDataDict, lens: torch.Tensor, S: int, packed_rows: int) -> None:
+    def _set_router_replay(self, mb: BatchedDataDict, lens: torch.Tensor, S: int, batch: PackedBatch) -> None:
         """Hands every MoE layer the engine's expert choices for the rows of the next forward pass (packed order); without a
         record in the batch the routers decide themselves."""
         from rl_b200.utils import routing_trace as RT
@@ -823,9 +825,12 @@ class PolicyWorker:
         if re is None:
             RT.replay(self.model, None)
             return
-        re = to_device(re[:, :S], self.device)
-        keep = torch.arange(S, device=self.device)[None, :] < lens[:, None].clamp(max=S)
-        rows = re[keep]                                   # [T, MoE layers, k], the order PackedBatch.from_padded uses
+        re, packed_rows = to_device(re[:, :S], self.device), int(batch.input_ids.numel())
+        if batch.rows is not None:
+            rows = re[batch.rows, batch.positions[: batch.rows.shape[0]].long()]
+        else:
+            rows = re[torch.arange(S, device=self.device)[None, :] < lens[:, None].clamp(max=S)]
+        # [T, MoE layers, k], the order PackedBatch.from_padded uses
         if rows.shape[0] < packed_rows:                   # rows appended for tensor / context parallel alignment
             rows = torch.cat([rows, rows.new_full((packed_rows - rows.shape[0],) + tuple(rows.shape[1:]), -1)])
         RT.replay_rows(self.model, rows)
@@ -950,11 +955,14 @@ class PolicyWorker:
             gb = data.slice(g * local_gbs, min(n_local, (g + 1) * local_gbs))
             tm = gb["token_mask"][:, 1:].float() if "token_mask" in gb else None
             sm = gb["sample_mask"].float() if "sample_mask" in gb else torch.ones(gb.size)
-            counts = torch.stack([sm.sum(), (tm * sm[:, None]).sum() if tm is not None else sm.sum()]).to(self.device)
+            counts = torch.stack([sm.sum(), (tm * sm[:, None]).sum() if tm is not None else sm.sum()])
+            known = counts.tolist() if counts.device.type == "cpu" and self.world == 1 else None
+            counts = counts.to(self.device)
             if self.world > 1:
                 dist.all_reduce(counts, group=self.dp_group)
                 counts = counts / cpw
             global_valid_seqs, global_valid_toks = counts[0], counts[1]
+            global_valid_seqs.host, global_valid_toks.host = known or counts.tolist()      # (losses that need them on the host do not wait for the pass)
             if not eval_mode:
                 for opt in (self.optimizer, self.optimizer_e):
                     if isinstance(opt, ShardedAdamW):
@@ -985,10 +993,11 @@ class PolicyWorker:
                     if not eval_mode:
                         loss.backward()
                 gb_loss += loss.detach()
-                metrics = dict(metrics)
+                if not isinstance(metrics, DeferredMetrics):
+                    metrics = dict(metrics)
                 metrics["lr"] = self.optimizer.lr if self.optimizer else 0.0
-                metrics["global_valid_seqs"] = float(global_valid_seqs)
-                metrics["global_valid_toks"] = float(global_valid_toks)
+                metrics["global_valid_seqs"] = global_valid_seqs.host
+                metrics["global_valid_toks"] = global_valid_toks.host
                 all_mb_metrics.append(metrics)
             if not eval_mode:
                 for opt in (self.optimizer, self.optimizer_e):

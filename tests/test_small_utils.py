@@ -159,3 +159,37 @@ def test_gradients_that_begin_anew():
     m.norm.grad = torch.ones(300)
     flat.fold_autograd_grads()
     assert bool((m.used.main_grad == 2).all()) and not m.idle.main_grad.any() and bool((m.norm.main_grad == 1).all())
+
+
+def test_deferred_metrics_and_packing_without_a_wait():
+    """Metrics are made at the first look, additions made before it stay; lengths on the host give the same pack as lengths on the device."""
+    import pickle
+
+    import torch
+
+    from rl_b200.algorithms.utils import DeferredMetrics
+    from rl_b200.models.transformer import PackedBatch
+
+    made = []
+    fresh = lambda: DeferredMetrics(torch.tensor([1.0, 2.0]), lambda v: (made.append(1), dict(a=v[0], b=v[1]))[1])      # noqa: E731
+    m = fresh()
+    m["lr"] = 3.0
+    assert not made
+    want = dict(a=1.0, b=2.0, lr=3.0)
+    assert m["a"] == 1.0 and dict(m) == want and {**m} == want and sorted(m) == ["a", "b", "lr"] and len(made) == 1
+    for look in (lambda x: dict(x), lambda x: {**x}, lambda x: pickle.loads(pickle.dumps(x)), lambda x: dict(x.items()), lambda x: x.copy(), lambda x: {} | x):
+        assert look(fresh()) == dict(a=1.0, b=2.0)
+    d = dict(z=0)
+    d.update(fresh())
+    assert d == dict(z=0, a=1.0, b=2.0) and "a" in fresh() and len(fresh()) == 2 and fresh().get("b") == 2.0 and isinstance(fresh(), dict)
+    ids = torch.arange(40).view(4, 10)
+    for lens in ([3, 10, 1, 7], [0, 5, 12, 2], [4, 0, 0, 0]):
+        t = torch.tensor(lens)
+        a, b = PackedBatch.from_padded(ids, t), PackedBatch.from_padded(ids, t, lens)
+        assert torch.equal(a.input_ids, b.input_ids) and torch.equal(a.positions, b.positions) and torch.equal(a.cu_seqlens, b.cu_seqlens)
+        assert a.max_seqlen == b.max_seqlen and b.rows is not None and a.positions.dtype == b.positions.dtype and a.cu_seqlens.dtype == b.cu_seqlens.dtype
+        x = torch.randn(a.input_ids.numel(), 2)
+        assert torch.equal(a.unpack(x, 10), b.unpack(x, 10))
+        pa, pb = a.pad_to_multiple(8), b.pad_to_multiple(8)
+        y = torch.randn(pa.input_ids.numel())
+        assert torch.equal(pa.unpack(y, 10), pb.unpack(y, 10))
