@@ -327,13 +327,21 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const _
   }
 }
 
-// Column sums of a [parts, d] fp32 matrix, added into (or written to) a gradient buffer.
-__global__ void colsum_kernel(const float* __restrict__ partial, int parts, int d, float* __restrict__ out_f32,
-                              __nv_bfloat16* __restrict__ out_bf16, int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d) return;
+// Column sums of a [parts, d] fp32 matrix, added into (or written to) a gradient buffer: 32 columns a block, the parts dealt out to its eight warps
+// (a thread walked all of them, 17 us for 296 parts of 4096; now 8).
+__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ partial, int parts, int d, float* __restrict__ out_f32,
+                                                     __nv_bfloat16* __restrict__ out_bf16, int accumulate) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int p = 0; p < parts; ++p) s += partial[static_cast<long long>(p) * d + c];
+  if (c < d) {
+#pragma unroll 8
+    for (int p = warp; p < parts; p += 8) s += partial[static_cast<long long>(p) * d + c];
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || c >= d) return;
+  for (int w = 1; w < 8; ++w) s += red[w][lane];
   if (out_f32) out_f32[c] = accumulate ? out_f32[c] + s : s;
   if (out_bf16) out_bf16[c] = __float2bfloat16(accumulate ? __bfloat162float(out_bf16[c]) + s : s);
 }
@@ -1081,7 +1089,7 @@ RLB_API int rlb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   else
     rmsnorm_bwd_kernel<<<parts, threads, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial,
                                                          static_cast<int>(rows), d, x_stride, dy_stride, add_to_dx);
-  colsum_kernel<<<(d + 255) / 256, 256, 0, S(stream)>>>(dw_partial, parts, d, dw_f32, BF(dw_bf16), dw_accumulate);
+  colsum_kernel<<<(d + 31) / 32, 256, 0, S(stream)>>>(dw_partial, parts, d, dw_f32, BF(dw_bf16), dw_accumulate);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1139,7 +1147,7 @@ RLB_API int rlb_qk_rmsnorm_bwd(const void* dy, const void* x, const void* wq, co
   if ((D % 64) || D > 256 || (x_stride % 2) || (dy_stride % 2) || (dx_stride % 2)) return -2;
   const int parts = rlb_qk_rmsnorm_bwd_parts(rows);
   qk_rmsnorm_bwd_kernel<<<parts, 256, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(wq), CBF(wk), rstd, BF(dx), dw_part, rows, Hq, Hkv, D, x_stride, dy_stride, dx_stride);
-  colsum_kernel<<<(2 * D + 255) / 256, 256, 0, S(stream)>>>(dw_part, parts, 2 * D, dw, nullptr, 0);
+  colsum_kernel<<<(2 * D + 31) / 32, 256, 0, S(stream)>>>(dw_part, parts, 2 * D, dw, nullptr, 0);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1305,7 +1313,7 @@ RLB_API int rlb_rmsnorm_bwd_static(const void* dy, const void* x, const void* w,
   // call left in the array is never read.
   rmsnorm_bwd_kernel<<<parts, threads, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), scratch,
                                                        static_cast<int>(rows), d, x_stride, dy_stride, 0);
-  colsum_kernel<<<(d + 255) / 256, 256, 0, S(stream)>>>(scratch, parts, d, dw_f32, nullptr, dw_accumulate);
+  colsum_kernel<<<(d + 31) / 32, 256, 0, S(stream)>>>(scratch, parts, d, dw_f32, nullptr, dw_accumulate);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -194,7 +194,7 @@ class MoEMLP(nn.Module):
             ws = self._small_workspace(T)
             if ws is not None:
                 out, idx = ws.forward(x, residual, self.router, self.gate_up_proj, self.down_proj, bool(c.norm_topk_prob))
-                self.last_routing = idx.clone()   # the workspace's copy is overwritten by the next layer
+                self.last_routing = idx
                 if self.routing_sink is not None:
                     self.routing_sink(self, self.last_routing)
                 return out

@@ -275,7 +275,6 @@ class SmallTokenMoE:
         self.max_mpad = max(self.mpad_for(self.maxT), -(-(n_all * top_k + self.El * 127) // 128) * 128)
         i32 = dict(dtype=torch.int32, device=device)
         self.w = torch.empty((n_all, top_k), dtype=torch.float32, device=device)
-        self.idx = torch.empty((n_all, top_k), **i32)
         self.src_tok = torch.empty(self.max_mpad, **i32)
         self.copy_row = torch.empty(n_all * top_k, **i32)
         self.tile_expert = torch.empty(self.max_mpad // 32, **i32)
@@ -344,7 +343,7 @@ class SmallTokenMoE:
         else:
             xa = x
         logits = F.linear(xa, router)
-        wts, idx = self.w[:n_all], self.idx[:n_all]
+        wts, idx = self.w[:n_all], torch.empty((n_all, k), dtype=torch.int32, device=x.device)      # (the experts outlive the call)
         call("rlb_moe_route_topk", ptr(logits), logits.stride(0), n_all, self.E, k, int(renorm), ptr(wts), ptr(idx), st)
         mpad, pad = self.mpad_for(T), self.tile_rows(T)
         call("rlb_moe_decode_plan", ptr(idx), n_all * k, k, self.e_lo, self.El, mpad, pad, ptr(self.src_tok), ptr(self.copy_row),
