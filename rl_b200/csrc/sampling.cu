@@ -1,5 +1,9 @@
 // Token sampling for the generation engine: temperature, top-k, top-p, multinomial draw and the
-// log-probability of the drawn token under the *processed* distribution, one CTA per sequence.
+// log-probability of the drawn token under the *processed* distribution.
+//
+// Without filters a row goes to a cluster of four or eight CTAs, where all rows' CTAs are resident, which draw over parts of it and merge maximum,
+// sum and best key through distributed shared memory. One CTA per row: 31 us greedy and 44 sampled for 128256 logits, whatever the number of rows up to
+// 128; eight 14 and 16 (32 rows), four 17 and 25 (64 rows).
 //
 // The draw uses the Gumbel-max construction: argmax_i (z_i / T + g_i) with g_i ~ Gumbel(0,1) is a
 // sample of softmax(z / T). That needs no normalisation and no prefix sums, so the unfiltered case
@@ -85,21 +89,38 @@ __device__ __forceinline__ ArgBest block_argmax(ArgBest v, ArgBest* red) {
   return r;
 }
 
+struct RowPart {      // of a CTA's share of a row
+  float mx, sum;
+  ArgBest best;
+};
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+
 // Per-row parameters may be null (then the scalar defaults apply).
-template <typename T>
+template <typename T, bool SHARED>
 __global__ void __launch_bounds__(1024)
 sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const float* __restrict__ temps,
               const int* __restrict__ top_ks, const float* __restrict__ top_ps, float def_temp, int def_top_k,
               float def_top_p, int greedy, unsigned long long seed, unsigned long long step,
               const unsigned long long* __restrict__ step_ptr, const long long* __restrict__ row_keys,
               int* __restrict__ out_tok, float* __restrict__ out_logprob) {
+  pdl_sync();
+  uint32_t parts = 1, part = 0;
+  if (SHARED) {
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(parts));
+    part = cluster_ctarank();
+  }
+  const int row = SHARED ? blockIdx.x / parts : blockIdx.x;
   if (step_ptr) step = *step_ptr;  // a counter in device memory lets a captured graph draw fresh numbers
   // With row_keys the random stream of a row depends only on (seed, key), e.g. key = request id and token position:
   // the draw is then independent of which other rows share the batch or which rank serves the request.
-  const unsigned long long rk = row_keys ? static_cast<unsigned long long>(row_keys[blockIdx.x]) : 0ull;
+  const unsigned long long rk = row_keys ? static_cast<unsigned long long>(row_keys[row]) : 0ull;
   __shared__ float red[32];
   __shared__ ArgBest redb[32];
-  const int row = blockIdx.x;
+  __shared__ RowPart mine;
   const T* z = logits + static_cast<long long>(row) * row_stride;
   float temp = temps ? temps[row] : def_temp;
   const int top_k = top_ks ? top_ks[row] : def_top_k;
@@ -108,7 +129,7 @@ sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const f
   if (temp <= 0.f) temp = 1.f;
   const float inv_t = 1.f / temp;
 
-  const bool filtered = (top_k > 0 && top_k < V) || top_p < 1.f;
+  const bool filtered = !SHARED && ((top_k > 0 && top_k < V) || top_p < 1.f);
   // pass 1: maximum (only the filters need it up front; the unfiltered draw below finds it on the way)
   float mx = -INFINITY;
   if (filtered) {
@@ -120,8 +141,8 @@ sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const f
   // train-side filter and vLLM apply them: top-k first, then the nucleus inside the renormalised top-k set. Both are a
   // bisection on the ordered-uint image of fp32; invariant: `lo` satisfies the predicate.
   float thr = -INFINITY;
-  const bool need_k = top_k > 0 && top_k < V;
-  const bool need_p = top_p < 1.f;
+  const bool need_k = !SHARED && top_k > 0 && top_k < V;
+  const bool need_p = !SHARED && top_p < 1.f;
   if (need_k) {
     // x_k = largest x with count(z >= x) >= k, i.e. the k-th largest logit (ties at x_k are all kept)
     uint32_t lo = 0u, hi = f2ord(mx);
@@ -168,7 +189,7 @@ sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const f
   const uint32_t k0 = static_cast<uint32_t>(seed), k1 = static_cast<uint32_t>(seed >> 32);
   // fp32 rows that start on a 16-byte boundary are read four logits at a time
   const bool vec4 = sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(z) & 15u) == 0;
-  for (int i4 = threadIdx.x * 4; i4 < V; i4 += blockDim.x * 4) {
+  for (int i4 = (part * blockDim.x + threadIdx.x) * 4; i4 < V; i4 += parts * blockDim.x * 4) {
     uint32_t rnd[4] = {0, 0, 0, 0};
     if (!is_greedy)
       philox4x32(static_cast<uint32_t>(i4 >> 2), row_keys ? static_cast<uint32_t>(rk) : static_cast<uint32_t>(row),
@@ -213,13 +234,58 @@ sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const f
   }
   sum = block_sum(sum, red);
   best = block_argmax(best, redb);
-  if (threadIdx.x == 0) {
+  if (SHARED) {
+    if (threadIdx.x == 0) mine = RowPart{mx, sum, best};
+    cluster_sync();
+  }
+  if (part == 0 && threadIdx.x == 0) {
+    if (SHARED) {
+      for (uint32_t r = 1; r < parts; ++r) {
+        const uint32_t at = mapa_shared(smem_u32(&mine), r);
+        const float m2 = __uint_as_float(ld_cluster_u32(at)), s2 = __uint_as_float(ld_cluster_u32(at + 4));
+        best = better(best, ArgBest{__uint_as_float(ld_cluster_u32(at + 8)), static_cast<int>(ld_cluster_u32(at + 12))});
+        const float top = fmaxf(mx, m2);
+        sum = (mx > -INFINITY ? sum * __expf((mx - top) * inv_t) : 0.f) + (m2 > -INFINITY ? s2 * __expf((m2 - top) * inv_t) : 0.f);
+        mx = top;
+      }
+    }
     out_tok[row] = best.idx;
     if (out_logprob) {
       const float zt = ldz(z, best.idx);
       out_logprob[row] = (zt - mx) * inv_t - __logf(sum);
     }
   }
+  if (SHARED) cluster_sync();      // the first CTA may still read this one's part
+}
+
+template <typename T>
+int launch_sample(const T* logits, long long row_stride, int B, int V, const float* temps, const int* top_ks, const float* top_ps, float def_temp, int def_top_k,
+                  float def_top_p, int greedy, unsigned long long seed, unsigned long long step, const unsigned long long* step_ptr,
+                  const long long* row_keys, int* out_tok, float* out_logprob, cudaStream_t s) {
+  // Clusters where no row can have a filter and at least four CTAs a row fit, two to an SM, with 4096 logits each.
+  const bool plain = !top_ks && !top_ps && !(def_top_k > 0 && def_top_k < V) && !(def_top_p < 1.f);
+  int parts = plain ? 8 : 1;
+  while (parts > 1 && (static_cast<long long>(parts) * B > 2 * 148 || parts * 4096 > V)) parts /= 2;
+  if (parts < 4) {
+    rlb_launch_pdl(sample_kernel<T, false>, dim3(B), dim3(1024), 0, s, logits, row_stride, V, temps, top_ks, top_ps, def_temp, def_top_k, def_top_p, greedy, seed,
+                   step, step_ptr, row_keys, out_tok, out_logprob);
+    return static_cast<int>(cudaGetLastError());
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(parts) * B);
+  cfg.blockDim = dim3(1024);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = rlb_pdl_enabled() ? 2 : 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, sample_kernel<T, true>, logits, row_stride, V, temps, top_ks, top_ps, def_temp, def_top_k, def_top_p, greedy,
+                                             seed, step, step_ptr, row_keys, out_tok, out_logprob));
 }
 
 }  // namespace
@@ -234,14 +300,10 @@ RLB_API int rlb_sample(const void* logits, int dtype, long long row_stride, int 
   if (B <= 0) return 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == 0)
-    sample_kernel<float><<<B, 1024, 0, s>>>(reinterpret_cast<const float*>(logits), row_stride, V, temps, top_ks,
-                                           top_ps, def_temp, def_top_k, def_top_p, greedy, seed, step, step_ptr,
-                                           row_keys, out_tok, out_logprob);
-  else
-    sample_kernel<__nv_bfloat16><<<B, 1024, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(logits), row_stride, V,
-                                                    temps, top_ks, top_ps, def_temp, def_top_k, def_top_p, greedy,
-                                                    seed, step, step_ptr, row_keys, out_tok, out_logprob);
-  return static_cast<int>(cudaGetLastError());
+    return launch_sample(reinterpret_cast<const float*>(logits), row_stride, B, V, temps, top_ks, top_ps, def_temp, def_top_k, def_top_p, greedy, seed, step,
+                         step_ptr, row_keys, out_tok, out_logprob, s);
+  return launch_sample(reinterpret_cast<const __nv_bfloat16*>(logits), row_stride, B, V, temps, top_ks, top_ps, def_temp, def_top_k, def_top_p, greedy, seed,
+                       step, step_ptr, row_keys, out_tok, out_logprob, s);
 }
 
 // ---------------------------------------------------------------- device-resident decode state

@@ -672,3 +672,26 @@ def test_logprob_combine(native_lib, M, V):
     lp, ent = F.lm_head_logprobs(h, w, t, 1.0, True)
     z = torch.log_softmax(h.double() @ w.double().T, -1)
     assert (lp.double() - z.gather(1, t[:, None])[:, 0]).abs().max() < 1e-4 and (ent.double() + (z.exp() * z).sum(-1)).abs().max() < 1e-3
+
+
+@pytest.mark.parametrize("B,V", [(1, 128256), (3, 16384), (37, 32771), (38, 32771), (74, 20000), (75, 20000), (2, 16383)])      # eight, four and one CTA a row
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("greedy", [False, True])
+def test_sampling_over_parts_of_rows(native_lib, B, V, dtype, greedy):
+    """The token equals that of one CTA per row (asked for by a filter that keeps every logit in reach), ties go to the first, rows may hold -inf;
+    log-probabilities against float64: fp32 sums in parts, 2e-5."""
+    from rl_b200.ops import engine_ops as E
+
+    g = torch.Generator("cuda").manual_seed(B + V)
+    z = (torch.randn(B, V + 8, generator=g, device="cuda") * 3).to(dtype)[:, :V]
+    z[0, 5 : V // 2] = -float("inf")
+    if greedy:
+        z[:, 100], z[:, V - 7] = 30.0, 30.0
+        z[0, 100] = 30.0
+    keys, temps = torch.arange(B, device="cuda") * 77, torch.full((B,), 0.7, device="cuda")
+    kw = dict(greedy=greedy, seed=11, row_keys=keys, temps=temps)
+    tok, lp = E.sample(z, **kw)
+    one, _ = E.sample(z, top_ks=torch.full((B,), 0, dtype=torch.int32, device="cuda"), **kw)
+    assert torch.equal(tok, one) and (not greedy or bool((tok == 100).all()))
+    want = torch.log_softmax(z.double() / 0.7, -1).gather(1, tok.long()[:, None])[:, 0]
+    assert (lp - want).abs().max() <= 2e-5 * (1 + want.abs().max())
