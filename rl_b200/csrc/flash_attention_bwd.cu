@@ -16,7 +16,7 @@
 // 15.4 -> 11.0 ms (499 TFLOP/s of the five products that a gradient needs); 64 x 1280 7.7 -> 5.5 ms; 8 x (513, 700, 333) 0.83 -> 0.65 ms; with
 // heads of 64 11.1 -> 8.8, 5.4 -> 4.4 and 0.59 -> 0.52 ms.
 // delta[h, t] = sum_d dO * O is computed beforehand by rlb_attn_delta.
-#include "common.cuh"
+#include "attention_tiles.cuh"
 
 #include <math.h>
 
@@ -35,32 +35,6 @@ constexpr int ATOMS = HD / 64;   // [rows x 64] swizzle atoms per operand tile a
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr int BWD_THREADS = 320;      // TMA, MMA, two groups of four warps
 
-// Sequence and tile of a flat tile index, found by a whole warp, 32 sequences at a time.
-__device__ __forceinline__ bool locate_tile_b(const int* __restrict__ cu, int num_seqs, int rows, int tile, int& start, int& len, int& tile_in_seq) {
-  const int lane = threadIdx.x & 31;
-  int acc = 0;
-  for (int s0 = 0; s0 < num_seqs; s0 += 32) {
-    const int s = min(s0 + lane, num_seqs - 1);
-    const int b = cu[s], e = cu[s + 1];
-    const int n = s0 + lane < num_seqs ? (e - b + rows - 1) / rows : 0;
-    int end = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, end, o);
-      if (lane >= o) end += v;
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, tile < acc + end);
-    if (hit) {
-      const int src = __ffs(hit) - 1;
-      start = __shfl_sync(0xffffffffu, b, src);
-      len = __shfl_sync(0xffffffffu, e - b, src);
-      tile_in_seq = tile - acc - __shfl_sync(0xffffffffu, end - n, src);
-      return true;
-    }
-    acc += __shfl_sync(0xffffffffu, end, 31);
-  }
-  return false;
-}
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
@@ -127,12 +101,11 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   int* info = reinterpret_cast<int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.y;
+  const int head = blockIdx.x % p.Hq;
   const int kv_head = head / (p.Hq / p.Hkv);
   if (warp == 0) {
     int start = 0, len = 0, tis = 0;
-    // late tiles of a sequence see the most keys: they go first
-    const bool ok = locate_tile_b(p.cu_seqlens, p.num_seqs, DQ_BQ, gridDim.x - 1 - blockIdx.x, start, len, tis) && (smem_u32(smem) & 1023u) == 0;
+    const bool ok = locate_longest_first(p.cu_seqlens, p.num_seqs, DQ_BQ, blockIdx.x / p.Hq, gridDim.x / p.Hq, true, start, len, tis) && (smem_u32(smem) & 1023u) == 0;
     if (lane == 0) {
       info[0] = start; info[1] = len; info[2] = tis; info[3] = ok ? 1 : 0;
       mbar_init(smem_u32(q_full), 1);
@@ -332,11 +305,11 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_kv128, const __gri
   int* info = reinterpret_cast<int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kv_head = blockIdx.y;
+  const int kv_head = blockIdx.x % p.Hkv;
   const int G = p.Hq / p.Hkv;
   if (warp == 0) {
     int start = 0, len = 0, tis = 0;
-    const bool ok = locate_tile_b(p.cu_seqlens, p.num_seqs, KV_BKV, blockIdx.x, start, len, tis) && (smem_u32(smem) & 1023u) == 0;
+    const bool ok = locate_longest_first(p.cu_seqlens, p.num_seqs, KV_BKV, blockIdx.x / p.Hkv, gridDim.x / p.Hkv, false, start, len, tis) && (smem_u32(smem) & 1023u) == 0;
     if (lane == 0) {
       info[0] = start; info[1] = len; info[2] = tis; info[3] = ok ? 1 : 0;
       for (int i = 0; i < 11; ++i) mbar_init(smem_u32(&bars[i]), 1);
@@ -564,7 +537,9 @@ RLB_API int RLB_NAME(rlb_flash_attn_bwd)(const void* qkv, long long qkv_stride, 
   p.dqkv_stride = dqkv_stride;
   p.status = status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  flash_bwd_dq_kernel<<<dim3(max_q_tiles, Hq), BWD_THREADS, DQ_SMEM, s>>>(tq128, tkv64, tdo128, p);
-  flash_bwd_dkv_kernel<<<dim3(max_kv_tiles, Hkv), BWD_THREADS, KV_SMEM, s>>>(tkv128, tq64, tdo64, p);
+  const int most = (T + KV_BKV - 1) / KV_BKV + num_seqs;
+  if (max_kv_tiles > most) max_kv_tiles = most;      // (blocks without a tile end at once, but take their turn)
+  flash_bwd_dq_kernel<<<max_q_tiles * Hq, BWD_THREADS, DQ_SMEM, s>>>(tq128, tkv64, tdo128, p);
+  flash_bwd_dkv_kernel<<<max_kv_tiles * Hkv, BWD_THREADS, KV_SMEM, s>>>(tkv128, tq64, tdo64, p);
   return static_cast<int>(cudaGetLastError());
 }

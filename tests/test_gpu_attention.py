@@ -99,6 +99,28 @@ def test_flash_fwd_scales(native_lib, D, scale):
 
 
 @pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("lens", [[300] * 3, [1, 640, 129, 128, 640, 0, 257], [33] * 128, [150, 20] * 64 + [40], [2000] + [10] * 20, [200] * 140])
+def test_flash_tiles_of_every_sequence(native_lib, lens, D):
+    """Equal lengths, all levels of work with several sequences in each, as many sequences as are sorted and one more, and enough tiles for the
+    forward pass to go head by head: outputs and gradients of the longest and the shortest row of each, within the bf16 bounds above."""
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import check_status
+
+    Hq, Hkv = (32, 4) if len(lens) == 140 else (4, 2)
+    qkv, cu, D = _case(lens, Hq, Hkv, seed=len(lens), D=D)
+    x = qkv.clone().requires_grad_()
+    y = F.attention_varlen(x, cu, max(lens), Hq, Hkv, D)
+    g = torch.randn_like(y)
+    y.backward(g)
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    xr = qkv.float().requires_grad_()
+    yr = F._attention_ref(xr, cu, Hq, Hkv, D, 1.0 / math.sqrt(D))
+    yr.backward(g.float())
+    assert (y.float() - yr).abs().max() <= 3e-2 and (x.grad.float() - xr.grad).abs().max() <= 3e-2 * xr.grad.abs().max()
+
+
+@pytest.mark.parametrize("D", [64, 128])
 def test_flash_many_sequences(native_lib, D):
     """More sequences than a warp has lanes, empty ones among them and at both ends."""
     from rl_b200.ops import functional as F
