@@ -354,24 +354,26 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   }
 }
 
-// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]  (one warp per (t, h))
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                                  float* __restrict__ delta, int T, int Hq, long long do_stride, long long o_stride) {
-  const long long wid = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (wid >= static_cast<long long>(T) * Hq) return;
-  const int t = static_cast<int>(wid / Hq), h = static_cast<int>(wid % Hq);
-  constexpr int PER = HD / 32;   // elements per lane: 4 or 2
-  const __nv_bfloat16* a = dout + t * do_stride + h * HD + lane * PER;
-  const __nv_bfloat16* b = out + t * o_stride + h * HD + lane * PER;
+// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]: eight elements a thread, so many lanes a head (a warp per head moved 8 bytes a lane: 4000 tokens of 32
+// heads of 128 26 us, now 20; of 64 23 and 14).
+__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
+                                                         float* __restrict__ delta, int T, int Hq, long long do_stride, long long o_stride) {
+  constexpr int LANES = HD / 8;
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x, head = i / LANES;
+  const int piece = static_cast<int>(i % LANES);
+  const bool in = head < static_cast<long long>(T) * Hq;
+  const int t = in ? static_cast<int>(head / Hq) : 0, h = in ? static_cast<int>(head % Hq) : 0;
+  const uint4 a = *reinterpret_cast<const uint4*>(dout + t * do_stride + h * HD + piece * 8), b = *reinterpret_cast<const uint4*>(out + t * o_stride + h * HD + piece * 8);
+  const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
   float s = 0.f;
 #pragma unroll
-  for (int q = 0; q < PER / 2; ++q) {
-    const float2 x = unpack_bf16x2(reinterpret_cast<const uint32_t*>(a)[q]), y = unpack_bf16x2(reinterpret_cast<const uint32_t*>(b)[q]);
-    s += x.x * y.x + x.y * y.y;
+  for (int q = 0; q < 4; ++q) {
+    const float2 u = unpack_bf16x2(x[q]), v = unpack_bf16x2(y[q]);
+    s += u.x * v.x + u.y * v.y;
   }
-  s = warp_sum(s);
-  if (lane == 0) delta[static_cast<long long>(h) * T + t] = s;
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (in && piece == 0) delta[static_cast<long long>(h) * T + t] = s;
 }
 
 int g_fwd_configured = 0;
@@ -422,8 +424,8 @@ RLB_API int RLB_NAME(rlb_flash_attn_fwd)(const void* qkv, long long qkv_stride, 
 RLB_API int RLB_NAME(rlb_attn_delta)(const void* dout, const void* out, float* delta, int T, int Hq, long long do_stride,
                            long long o_stride, void* stream) {
   if (T <= 0) return 0;
-  const long long warps = static_cast<long long>(T) * Hq;
-  const long long blocks = (warps * 32 + 255) / 256;
+  if ((do_stride % 8) || (o_stride % 8) || ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(out)) & 15)) return -3;      // (as the gradient's loads want it)
+  const long long blocks = (static_cast<long long>(T) * Hq * (HD / 8) + 255) / 256;
   attn_delta_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const __nv_bfloat16*>(dout), reinterpret_cast<const __nv_bfloat16*>(out), delta, T, Hq,
       do_stride, o_stride);

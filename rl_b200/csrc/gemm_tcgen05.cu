@@ -599,20 +599,22 @@ __global__ void __launch_bounds__(256) dlogits_kept_kernel(const float* __restri
   }
 }
 
-// Folds the per-n-tile partials of EPI_LOGPROB into per-row results: 32 rows per CTA, the parts dealt out to its eight warps (one thread per row
-// walked 501 parts twice, 126 us at 240 rows, now 20 us).
-__global__ void __launch_bounds__(256) logprob_combine_kernel(const float* __restrict__ part_max, const float* __restrict__ part_sum,
+// Folds the per-n-tile partials of EPI_LOGPROB into per-row results: 32 rows per CTA, the parts dealt out to its warps (one thread per row
+// walked 501 parts twice, 126 us at 240 rows; eight warps
+// take 37 us for 32 to 4000 rows, 32 warps 15 to 17; from 20000 rows on, where the CTAs fill the SMs several times, eight: 52 and 61).
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) logprob_combine_kernel(const float* __restrict__ part_max, const float* __restrict__ part_sum,
                                                               const float* __restrict__ part_zsum, const float* __restrict__ target_logit, int M, int num_parts,
                                                               float* __restrict__ logprob, float* __restrict__ entropy, float* __restrict__ lse_out) {
-  __shared__ float s_max[8][32], s_sum[8][32], s_zsum[8][32];
+  __shared__ float s_max[WARPS][32], s_sum[WARPS][32], s_zsum[WARPS][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * 32 + lane;
   float mx = -INFINITY, sum = 0.f, zsum = 0.f;
   if (row < M) {
 #pragma unroll 4
-    for (int p = warp; p < num_parts; p += 8) mx = fmaxf(mx, part_max[static_cast<long long>(p) * M + row]);
+    for (int p = warp; p < num_parts; p += WARPS) mx = fmaxf(mx, part_max[static_cast<long long>(p) * M + row]);
 #pragma unroll 4
-    for (int p = warp; p < num_parts; p += 8) {
+    for (int p = warp; p < num_parts; p += WARPS) {
       const long long i = static_cast<long long>(p) * M + row;
       const float s = part_max[i] == -INFINITY ? 0.f : __expf(part_max[i] - mx);      // (a part without columns, or all of this warp's)
       sum += part_sum[i] * s;
@@ -624,9 +626,9 @@ __global__ void __launch_bounds__(256) logprob_combine_kernel(const float* __res
   s_zsum[warp][lane] = zsum;
   __syncthreads();
   if (warp != 0 || row >= M) return;
-  for (int w = 1; w < 8; ++w) mx = fmaxf(mx, s_max[w][lane]);
+  for (int w = 1; w < WARPS; ++w) mx = fmaxf(mx, s_max[w][lane]);
   sum = zsum = 0.f;
-  for (int w = 0; w < 8; ++w) {
+  for (int w = 0; w < WARPS; ++w) {
     const float s = s_max[w][lane] == -INFINITY ? 0.f : __expf(s_max[w][lane] - mx);
     sum += s_sum[w][lane] * s;
     zsum += s_zsum[w][lane] * s;
@@ -645,6 +647,13 @@ int sm_count() {
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
   }
   return n;
+}
+
+template <typename... Args>
+void launch_combine(cudaStream_t s, const float* part_max, const float* part_sum, const float* part_zsum, const float* target_logit, int M, Args... args) {
+  const int blocks = (M + 31) / 32;
+  if (blocks <= 2 * sm_count()) logprob_combine_kernel<32><<<blocks, 1024, 0, s>>>(part_max, part_sum, part_zsum, target_logit, M, args...);
+  else logprob_combine_kernel<8><<<blocks, 256, 0, s>>>(part_max, part_sum, part_zsum, target_logit, M, args...);
 }
 
 // Tiles of this size, and the waves of them on at most `max_ctas` CTAs (0: as many as there are SMs).
@@ -860,8 +869,7 @@ RLB_API int rlb_lm_head_logprob(const void* H, const void* W, int M, int N, int 
               : launch_gemm<false, false, EPI_LOGPROB>(ta, tb, M, N, K, ep, status, 0, s);
   if (rc) return rc;
   const int parts = (N + BN - 1) / BN;
-  logprob_combine_kernel<<<(M + 31) / 32, 256, 0, s>>>(part_max, part_sum, part_zsum, target_logit, M, parts,
-                                                          logprob, entropy, lse);
+  launch_combine(s, part_max, part_sum, part_zsum, target_logit, M, parts, logprob, entropy, lse);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -870,8 +878,7 @@ RLB_API int rlb_logprob_combine(const float* part_max, const float* part_sum, co
                                 const float* target_logit, int M, int parts, float* logprob, float* entropy,
                                 float* lse, void* stream) {
   if (M <= 0) return 0;
-  logprob_combine_kernel<<<(M + 31) / 32, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      part_max, part_sum, part_zsum, target_logit, M, parts, logprob, entropy, lse);
+  launch_combine(static_cast<cudaStream_t>(stream), part_max, part_sum, part_zsum, target_logit, M, parts, logprob, entropy, lse);
   return static_cast<int>(cudaGetLastError());
 }
 
