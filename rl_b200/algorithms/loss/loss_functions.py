@@ -50,6 +50,12 @@ def host_value(count) -> float:
     return float(count if known is None else known)
 
 
+def device_metrics(values: torch.Tensor, make, count) -> dict:
+    """``make(numbers of values)``: a plain dict, or, where the caller gave a count whose number it knew (a training step, which looks at its
+    metrics at its end), one that is made at the first look."""
+    return make(values.tolist()) if getattr(count, "host", None) is None else DeferredMetrics(values, make)
+
+
 def _nan_to_zero(x: torch.Tensor) -> torch.Tensor:
     return torch.nan_to_num(x, nan=0.0, posinf=0.0, neginf=0.0)
 
@@ -179,7 +185,7 @@ class ClippedPGLossFn:
                 metrics["is_oob_ratio"] = s[15]
             return metrics
 
-        return loss, DeferredMetrics(torch.cat([sums.detach(), torch.stack([loss.detach(), sample_mask.sum()]).double()]), make)
+        return loss, device_metrics(torch.cat([sums.detach(), torch.stack([loss.detach(), sample_mask.sum()]).double()]), make, global_valid_toks)
 
     # ---- PyTorch statement of the same math (CPU path, oracle, and every non-fused configuration)
     def _reference(self, curr, prev, gen, ref, adv, token_mask, sample_mask, mask, data, gvs, gvt):
@@ -334,7 +340,7 @@ class NLLLossFn:
         if loss.dim() != 0:
             return loss, {"loss": loss, "num_unmasked_tokens": num_unmasked.item(), "num_valid_samples": sample_mask.sum().item()}
         names = ("loss", "num_unmasked_tokens", "num_valid_samples")
-        return loss, DeferredMetrics(torch.stack([loss.detach(), num_unmasked, sample_mask.sum()]), lambda v: dict(zip(names, v)))
+        return loss, device_metrics(torch.stack([loss.detach(), num_unmasked, sample_mask.sum()]), lambda v: dict(zip(names, v)), global_valid_toks)
 
 
 class PreferenceLossFn:

@@ -46,7 +46,7 @@ def calculate_kl(logprobs: torch.Tensor, logprobs_reference: torch.Tensor, kl_ty
 
 class DeferredMetrics(dict):
     """Metrics whose numbers are still on the device: ``make(numbers)`` turns the values of ``device_values`` (a 1-D tensor) into the dict, which
-    happens at the first look at it. A training step that looks only when its kernels are all enqueued does not wait for them in between."""
+    happens at the first look at it (C code that reads the storage itself, such as ``json.dumps``, is no look: hand it a plain copy). A training step that looks only when its kernels are all enqueued does not wait for them in between."""
 
     def __init__(self, device_values: torch.Tensor, make):
         super().__init__()
@@ -57,6 +57,7 @@ class DeferredMetrics(dict):
             values, make = self._pending
             self._pending = None
             added = dict(dict.items(self))
+            dict.clear(self)
             dict.update(self, make(values.tolist()))
             dict.update(self, added)
         return self
@@ -79,6 +80,9 @@ class DeferredMetrics(dict):
     def __eq__(self, other):
         return dict.__eq__(self._resolve(), other)
 
+    def __ne__(self, other):
+        return dict.__ne__(self._resolve(), other)
+
     __hash__ = None
 
     def __repr__(self):
@@ -98,6 +102,15 @@ class DeferredMetrics(dict):
 
     def pop(self, *a):
         return dict.pop(self._resolve(), *a)
+
+    def popitem(self):
+        return dict.popitem(self._resolve())
+
+    def clear(self):
+        dict.clear(self._resolve())
+
+    def __reversed__(self):
+        return dict.__reversed__(self._resolve())
 
     def setdefault(self, *a):
         return dict.setdefault(self._resolve(), *a)

@@ -182,6 +182,16 @@ def test_deferred_metrics_and_packing_without_a_wait():
     d = dict(z=0)
     d.update(fresh())
     assert d == dict(z=0, a=1.0, b=2.0) and "a" in fresh() and len(fresh()) == 2 and fresh().get("b") == 2.0 and isinstance(fresh(), dict)
+    assert not (fresh() != dict(a=1.0, b=2.0)) and fresh().popitem() == ("b", 2.0)
+    # only a caller that knows its counts on the host gets them: every other one has a plain dict
+    from rl_b200.algorithms.loss.loss_functions import NLLLossFn
+
+    counts = torch.tensor([2.0, 5.0])
+    call = lambda toks: NLLLossFn()(-torch.rand(2, 4), dict(token_mask=torch.ones(2, 5), sample_mask=torch.ones(2)), counts[0], toks)[1]      # noqa: E731
+    assert type(call(counts[1])) is dict
+    known = counts[1]
+    known.host = 5.0
+    assert type(call(known)) is DeferredMetrics and call(known)["num_unmasked_tokens"] == 8
     ids = torch.arange(40).view(4, 10)
     for lens in ([3, 10, 1, 7], [0, 5, 12, 2], [4, 0, 0, 0]):
         t = torch.tensor(lens)
