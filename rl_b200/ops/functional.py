@@ -707,10 +707,13 @@ def _kept_logits(M: int, N: int, dev) -> Optional[torch.Tensor]:
         return None
     step = max(64, (1 << M.bit_length()) // 8)
     rows = -(-M // step) * step
-    # (this process's own count: asking the driver took from 0.2 to 90 ms)
+    size, props = 4 * rows * N, torch.cuda.get_device_properties(dev)
     stats = torch.cuda.memory.memory_stats_as_nested_dict(dev)      # (as a flat dict 0.2 ms)
-    used = stats["allocated_bytes"]["all"]["current"] if "allocated_bytes" in stats else math.inf
-    if used + 16 * rows * N > 0.95 * torch.cuda.get_device_properties(dev).total_memory:
+    used, held = ((stats[k]["all"]["current"] if k in stats else math.inf) for k in ("allocated_bytes", "reserved_bytes"))
+    if used + 4 * size > 0.95 * torch.cuda.get_per_process_memory_fraction(dev) * props.total_memory:
+        return None
+    # What the allocator holds is this process's. Where it has to grow the driver is asked what other processes leave (0.2 ms, up to 90 on a busy host).
+    if held - used < size and torch.cuda.mem_get_info(dev)[0] + held - used < 4 * size + 0.05 * props.total_memory:
         return None
     try:
         return torch.empty((rows, N), dtype=torch.float32, device=dev)

@@ -203,3 +203,36 @@ def test_deferred_metrics_and_packing_without_a_wait():
         pa, pb = a.pad_to_multiple(8), b.pad_to_multiple(8)
         y = torch.randn(pa.input_ids.numel())
         assert torch.equal(pa.unpack(y, 10), pb.unpack(y, 10))
+
+
+def test_kept_logits_leave_room(monkeypatch):
+    """Logits are kept for a backward pass only where four times their size is free: of this process's share, and, where its allocator would have to
+    grow, of what other processes leave."""
+    import types
+
+    import torch
+
+    from rl_b200.ops import functional as F
+
+    M, N = 64, 1024
+    size, total = 4 * M * N, 100 << 20
+    asked = []
+
+    def kept(used, held, free, fraction=1.0, capturing=False, words=N):
+        asked.clear()
+        now = dict(allocated_bytes=dict(all=dict(current=used)), reserved_bytes=dict(all=dict(current=held)))
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+        monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: types.SimpleNamespace(total_memory=total))
+        monkeypatch.setattr(torch.cuda.memory, "memory_stats_as_nested_dict", lambda d: now)
+        monkeypatch.setattr(torch.cuda, "get_per_process_memory_fraction", lambda d: fraction)
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (asked.append(1), (free, total))[1])
+        z = F._kept_logits(M, words, torch.device("cpu"))
+        assert z is None or (z.shape[0] >= M and z.shape[1] == words and z.dtype == torch.float32)
+        return z is not None
+
+    assert kept(0, size, 0) and not asked                                    # the allocator has it: nobody is asked
+    assert kept(0, 0, 90 << 20) and asked
+    assert not kept(0, 0, 4 * size) and kept(0, 0, 4 * size + total // 20 + 1)      # another process holds the rest
+    assert not kept(int(0.95 * total) - 4 * size + 1, total, 0) and kept(int(0.95 * total) - 4 * size - 1, total, 0)
+    assert not kept(total // 2, total, 0, fraction=0.5)
+    assert not kept(0, size, 0, capturing=True) and not kept(0, size, 0, words=N + 4)
