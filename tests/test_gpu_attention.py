@@ -83,6 +83,13 @@ def test_flash_bwd_few_tiles(native_lib, n, Hq, Hkv, D):
 
 
 @pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("n", [384, 385, 512, 513, 770])
+def test_flash_bwd_more_tiles(native_lib, n, D):
+    """The same with three to seven tiles of 128 opposite a tile: every slot of the rings and both places of the scores come round again."""
+    test_flash_bwd_few_tiles(native_lib, n, 3, 1, D)
+
+
+@pytest.mark.parametrize("D", [128, 64])
 @pytest.mark.parametrize("scale", [0.0, -0.0, 1e-39, -1e-39, -0.09, 1e-3])
 def test_flash_fwd_scales(native_lib, D, scale):
     """Scales of zero, too small for a normal number, and negative ones, where the least score has the largest weight. Bounds of test_flash_fwd."""
