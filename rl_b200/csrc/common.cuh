@@ -41,6 +41,9 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
+// One thread of a converged warp, for the roles that issue loads and products. The compiler knows that a block under it runs one thread and keeps descriptors and
+// addresses in uniform registers, where the instructions want them; under `lane == 0` it moves them there for each instruction, and issuing a product took 105
+// cycles (128 x 128 x 16 executes in 64): flash attention forward, 4 x 4096 tokens, 32 and 8 heads of 128: 670 -> 546 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
@@ -88,14 +91,15 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // wait ran out, so that the others stop early instead of each waiting out the full limit.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code, unsigned long long limit_ns = kWaitLimitNs) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
+  unsigned long long t0 = 0;      // (from the 256th poll on)
   uint32_t polls = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if (((++polls) & 255u) == 0u) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > limit_ns) {
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > limit_ns) {
         *abort_flag = 1;
         if (status) atomicCAS(status, 0, code);
         return false;

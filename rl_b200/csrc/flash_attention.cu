@@ -15,7 +15,7 @@
 //               uses the same reference).
 // Bound by the exponentials and the tensor cores alike (512 cycles each per tile and CTA), so both have to run all the time: the next
 // tile's scores are computed under this one's softmax, and two CTAs cover each other's hand-offs. Measured, 32 query and 8 KV heads of 128
-// (before: one score buffer, P through shared memory): 16 x 4096 tokens 3.77 -> 2.24 ms (984 TFLOP/s); 64 x 1280 2.02 -> 1.18 ms.
+// (before: one score buffer, P through shared memory): 16 x 4096 tokens 3.77 -> 2.24 ms (984 TFLOP/s); 64 x 1280 2.02 -> 1.18 ms. Since then, by the order of the tiles and an elected issuer: 4 x 4096 670 -> 546 us, 1 x 7600 541 -> 422.
 // Output: O[T, Hq*128] bf16 and the per-row log-sum-exp lse[Hq, T] (natural log) for the backward pass.
 //
 // Backward (flash_attention_bwd.cu) is two kernels without atomics: one per (128-key tile, kv head) accumulating dK / dV over all query
@@ -155,7 +155,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int v_col = (p.Hq + p.Hkv + kv_head) * HD;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tmap(&tmap_q);
       prefetch_tmap(&tmap_kv);
       mbar_arrive_expect_tx(smem_u32(q_full), Q_BYTES);
@@ -184,7 +184,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(BQ, BKV, false, false);
       constexpr uint32_t idesc_o = make_idesc_bf16(BQ, HD, false, true);
       // S = Q K^T of tile j over the head dimension: steps of 16, swizzle atoms of 64. Its buffer held P of tile j - 2, whose product has

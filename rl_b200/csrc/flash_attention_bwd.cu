@@ -193,7 +193,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
   const int q_col = head * HD, k_col = (p.Hq + kv_head) * HD, v_col = (p.Hq + p.Hkv + kv_head) * HD;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       load_rows(q_s, &tmap_qkv, &q_full[0], q_col, seq_start + q0);
       bool ok = true;
       for (int j = 0; j < n_kv && ok; ++j) {
@@ -377,7 +377,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
   const int k_col = (p.Hq + kv_head) * HD, v_col = (p.Hq + p.Hkv + kv_head) * HD;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       load_rows(k_s, &tmap_qkv, &kv_full[0], k_col, seq_start + kv0);
       bool ok = true;
       for (int it = 0; it < n_iter && ok; ++it) {

@@ -160,7 +160,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   pdl_sync();  // everything above overlaps the tail of the previous kernel on the stream
 
   if (warp == 0) {
-    if (lane == 0 && have_work) {
+    if (have_work && elect_one()) {
       for (int e = 0; e < early; ++e)
         tma_load_2d(smem_u32(smem + e * Cfg::STAGE) + Cfg::A_BYTES, &tmap_x, smem_u32(&full_bar[e]), (kb_begin + e) * SK_BK, m0);
       uint32_t stage = early == Cfg::STAGES ? 0 : early, phase = early == Cfg::STAGES ? 1 : 0;
@@ -178,7 +178,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && have_work) {
+    if (have_work && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(SK_BM, NT, false, false);
       uint32_t stage = 0, phase = 0;
       bool ok = true;

@@ -146,7 +146,7 @@ flash_latent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   auto tile_of = [&](int j) { return j < sinks ? j : first_tile + j - sinks; };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tmap(&tmap_q);
       prefetch_tmap(&tmap_kv);
       prefetch_tmap(&tmap_lat);
@@ -169,7 +169,7 @@ flash_latent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(LA_BQ, LA_BKV, false, false);
       const uint32_t idesc_o = make_idesc_bf16(LA_BQ, p.vcols, false, true);
       const int steps_n = p.dim / 16, steps_r = (p.rot_dim + 15) / 16;

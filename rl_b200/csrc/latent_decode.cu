@@ -77,7 +77,7 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int num_k = (g.K + HG_K - 1) / HG_K;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int kb = 0; kb < num_k; ++kb) {
         const int s = kb % HG_STAGES;
         if (!mbar_wait(smem_u32(empty + s), ((kb / HG_STAGES) & 1) ^ 1, abort_flag, g.status, RLB_ERR_WAIT_EMPTY)) break;
@@ -94,7 +94,7 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(HG_T, BN, false, B_MN);
       bool ok = true;
       for (int kb = 0; kb < num_k; ++kb) {

@@ -73,7 +73,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int num_k = g.K / MS_BK, work = g.max_tiles * g.w_tiles;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < work && ok; w += gridDim.x) {
@@ -102,7 +102,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(128, NT, false, false);
       uint32_t stage = 0, phase = 0, local = 0;
       bool ok = true;

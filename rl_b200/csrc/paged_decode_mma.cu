@@ -163,7 +163,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const int* bt = p.block_table + static_cast<long long>(seq) * p.max_blocks_per_seq;
       const int box_rows = bs < DM_TOK ? bs : DM_TOK;
       const int nbox = DM_TOK / box_rows;
@@ -195,7 +195,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(DM_TOK, DM_N, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(DM_D, DM_N, true, false);
       auto issue_qk = [&](int i) -> bool {
@@ -567,7 +567,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const int box_rows = bs < DM_TOK ? bs : DM_TOK;
       const int nbox = DM_TOK / box_rows;
       bool ok = true;
@@ -602,7 +602,7 @@ paged_decode_group_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(DM_TOK, DM_N, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(128, DM_N, true, false);
       auto issue_qk = [&](int i) -> bool {

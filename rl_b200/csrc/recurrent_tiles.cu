@@ -625,7 +625,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmap_whi, const __grid_con
   const int c0 = piece_chunk[piece], c1 = piece_chunk[piece + 1];
   const int atoms_d = (p.dim + 63) / 64;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int c = c0; c < c1; ++c) {
         const uint32_t ph = (c - c0) & 1;
         const int row = (c * p.heads + head) * RT_C;
@@ -644,7 +644,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmap_whi, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_w2 = make_idesc_bf16(RT_C, 2 * VB, false, true), idesc_w1 = make_idesc_bf16(RT_C, VB, false, true);
       constexpr uint32_t idesc_k2 = make_idesc_bf16(RT_C, 2 * VB, true, true), idesc_k1 = make_idesc_bf16(RT_C, VB, true, true);
       const int steps = (p.dim + 15) / 16;
