@@ -29,12 +29,10 @@
 // (nemo_rl/models/generation/vllm/vllm_worker.py:570-597).
 #include "common.cuh"
 
-#include <cooperative_groups.h>
 #include <type_traits>
 
 namespace {
 using namespace rlb;
-namespace cg = cooperative_groups;
 
 constexpr int SK_BM = 128;     // rows of W per tile
 constexpr int SK_BK = 64;
@@ -86,14 +84,21 @@ __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
   return v;
 }
 
-template <int NT>
+// What a kernel's epilogue can do. Every CTA runs through it once, so that instructions come from memory: code for what a launch does not do costs time. A kernel per kind, two
+// items a thread in flight, no cluster barrier for a CTA on its own and the last one split around the stores, projections of a layer in a captured chain, us:
+// 8B one sequence 84.1 -> 81.5, 64 sequences 93.3 -> 90.0; 1B 35.7 -> 34.3 and 44.0 -> 43.1. What is left at 64 sequences is the traffic between the CTAs of
+// a cluster: 28 KB of partial sums to each, some 10 bytes a cycle.
+enum { SK_PLAIN = 0, SK_SWIGLU = 1, SK_LAYER = 2 };
+
+template <int NT, int MODE>
 __global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    SkinnyParams p) {
   using Cfg = SkinnyCfg<NT>;
   extern __shared__ __align__(1024) uint8_t smem[];
-  cg::cluster_group cluster = cg::this_cluster();
-  const uint32_t split = cluster.num_blocks();
+  constexpr bool GLU = MODE == SK_SWIGLU, LAYER = MODE == SK_LAYER;
+  uint32_t split;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(split));
   const uint32_t krank = cluster_ctarank();
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::MAIN);
   uint64_t* full_bar = bars;
@@ -106,10 +111,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_blk = blockIdx.x / split;  // tile of 128 W rows (SwiGLU: 64 gate rows + the 64 matching up rows)
   // W rows of the tile: one 128-row box, or two 64-row boxes (gate rows, then up rows F further down)
-  const int w_row0 = p.swiglu ? n_blk * 64 : n_blk * SK_BM;
+  const int w_row0 = GLU ? n_blk * 64 : n_blk * SK_BM;
   const int w_row1 = p.N + n_blk * 64;
   auto load_w = [&](uint32_t dst, uint32_t bar, int kb) {
-    if (p.swiglu) {
+    if (GLU) {
       tma_load_2d(dst, &tmap_w, bar, kb * SK_BK, w_row0);
       tma_load_2d(dst + Cfg::A_BYTES / 2, &tmap_w, bar, kb * SK_BK, w_row1);
     } else {
@@ -213,6 +218,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       for (int m = threadIdx.x - 64; m < NT; m += 128) {
         float ss = 0.f;
         if (m < rows)
+#pragma unroll 8
           for (int t = 0; t < p.ssq_in_tiles; ++t) ss += p.ssq_in[t * p.ssq_in_stride + m0 + m];
         s_rstd[m] = m < rows ? rsqrtf(ss / static_cast<float>(p.K) + p.eps) : 0.f;
       }
@@ -241,127 +247,147 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     tmem_dealloc(tmem_acc, Cfg::TMEM);
   }
   // Epilogue part 2: every CTA of the cluster reduces a slice of the tokens over all partial tiles.
-  cluster.sync();
-  {
-    const int tok_per = (NT + split - 1) / split;
-    const int m_begin = krank * tok_per;
-    const int m_end = min(rows, m_begin + tok_per);
-    const uint32_t part_addr = smem_u32(smem);
-    const int out_cols = p.swiglu ? 64 : SK_BM;      // output columns of this tile
-    const int groups = out_cols / 4;                 // work item: (token m, 4 consecutive output columns)
-    const int n0 = n_blk * out_cols;
-    const float layer_alpha = p.use_layer && p.layer.x ? __bfloat162float(*p.layer.alpha) : 0.f;
-    // a warp always works on one token (groups is 16 or 32, the stride a multiple of 32), so the per-token sum of
-    // squares for the next norm is one warp reduction
-    const int items = max(m_end - m_begin, 0) * groups;
-    const int items_pad = (items + 31) & ~31;
-    auto finish = [&](auto alone) {      // alone: a CTA on its own, without the loops over the cluster, whose instructions cost more than they hide
-      for (int it = threadIdx.x; it < items_pad; it += SK_THREADS) {
-        const bool live = it < items;
-        const int ml = m_begin + (live ? it / groups : 0), m = m0 + ml;      // in this tile, of all
-        const int n4 = (live ? it % groups : 0) * 4;
-        const int n = n0 + n4;
-        const bool valid = live && n < p.N;  // N is a multiple of 8, so a group of 4 is all in or all out
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc_u = acc, x_old = acc, x_e = acc;
-        uint2 rv = make_uint2(0u, 0u), wv = rv;
-        if (valid) {
-          // All that the item needs from memory and from the other CTAs is requested before any of it is waited for: one latency instead of one
-          // per CTA of the cluster (projections of an 8B layer in a captured chain, 64 sequences 98.7 -> 97.0 us, one 85.5 -> 83.6; of a 1B
-          // layer 46.5 -> 45.1 and 37.9 -> 36.9).
+  if (split > 1) cluster_sync();
+  const int tok_per = (NT + split - 1) / split;
+  const int m_begin = krank * tok_per;
+  const int m_end = min(rows, m_begin + tok_per);
+  const uint32_t part_addr = smem_u32(smem);
+  constexpr int OUT_COLS = GLU ? 64 : SK_BM;       // output columns of this tile
+  constexpr int GROUPS = OUT_COLS / 4;             // work item: (token m, 4 consecutive output columns)
+  const int n0 = n_blk * OUT_COLS;
+  const float layer_alpha = LAYER && p.layer.x ? __bfloat162float(*p.layer.alpha) : 0.f;
+  // a warp always works on one token or two (the stride is a multiple of 32), one where the sum of squares for the next norm is wanted, which is one
+  // warp reduction
+  const int items = max(m_end - m_begin, 0) * GROUPS;
+  const int items_pad = (items + 31) & ~31;
+  bool arrived = false;
+  auto finish = [&](auto alone) {      // alone: a CTA on its own, without the loops over the cluster, whose instructions cost more than they hide
+    constexpr int U = 2;               // items in flight per thread
+    for (int it0 = threadIdx.x; it0 < items_pad; it0 += U * SK_THREADS) {
+      // All that the items need from memory and from the other CTAs is requested before any of it is waited for: one latency instead of one
+      // per CTA of the cluster and item.
+      float4 acc[U], acc_u[U], x_old[U], x_e[U];
+      uint2 rv[U], wv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int it = it0 + u * SK_THREADS;
+        const int ml = m_begin + it / GROUPS, n4 = it % GROUPS * 4, m = m0 + ml, n = n0 + n4;      // ml: in this tile, m: of all
+        acc[u] = acc_u[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (it < items && n < p.N) {      // (N is a multiple of 8, so a group of 4 is all in or all out)
           const uint32_t off = static_cast<uint32_t>((ml * SK_BM + n4) * 4);
-          if (p.residual) rv = *reinterpret_cast<const uint2*>(p.residual + static_cast<long long>(m) * p.ldr + n);
-          if (p.ssq_out) wv = *reinterpret_cast<const uint2*>(p.norm_w + n);
-          if (p.use_layer && p.layer.x) {
-            x_old = *reinterpret_cast<const float4*>(p.layer.x + m * p.layer.ldx + n);
-            if (p.layer.e) x_e = *reinterpret_cast<const float4*>(p.layer.e + m * p.layer.ldx + n);
+          if (!GLU && p.residual) rv[u] = *reinterpret_cast<const uint2*>(p.residual + static_cast<long long>(m) * p.ldr + n);
+          if (!GLU && !LAYER && p.ssq_out) wv[u] = *reinterpret_cast<const uint2*>(p.norm_w + n);
+          if (LAYER && p.layer.x) {
+            x_old[u] = *reinterpret_cast<const float4*>(p.layer.x + m * p.layer.ldx + n);
+            if (p.layer.e) x_e[u] = *reinterpret_cast<const float4*>(p.layer.e + m * p.layer.ldx + n);
           }
           if constexpr (decltype(alone)::value) {
-            acc = *reinterpret_cast<const float4*>(smem + off);
-            if (p.swiglu) acc_u = *reinterpret_cast<const float4*>(smem + off + 64 * 4);
+            acc[u] = *reinterpret_cast<const float4*>(smem + off);
+            if (GLU) acc_u[u] = *reinterpret_cast<const float4*>(smem + off + 64 * 4);
           } else {
             float4 part[8], part_u[8];      // 8: the largest cluster
 #pragma unroll
-            for (uint32_t r = 0; r < 8; ++r) {
-              if (r < split) {
-                part[r] = ld_dsmem_f4(mapa_shared(part_addr + off, r));
-                if (p.swiglu) part_u[r] = ld_dsmem_f4(mapa_shared(part_addr + off + 64 * 4, r));
+            for (uint32_t q = 0; q < 8; ++q) {
+              if (q < split) {
+                part[q] = ld_dsmem_f4(mapa_shared(part_addr + off, q));
+                if (GLU) part_u[q] = ld_dsmem_f4(mapa_shared(part_addr + off + 64 * 4, q));
               }
             }
 #pragma unroll
-            for (uint32_t r = 0; r < 8; ++r) {
-              if (r < split) {
-                acc.x += part[r].x; acc.y += part[r].y; acc.z += part[r].z; acc.w += part[r].w;
-                if (p.swiglu) { acc_u.x += part_u[r].x; acc_u.y += part_u[r].y; acc_u.z += part_u[r].z; acc_u.w += part_u[r].w; }
+            for (uint32_t q = 0; q < 8; ++q) {
+              if (q < split) {
+                acc[u].x += part[q].x; acc[u].y += part[q].y; acc[u].z += part[q].z; acc[u].w += part[q].w;
+                if (GLU) { acc_u[u].x += part_u[q].x; acc_u[u].y += part_u[q].y; acc_u[u].z += part_u[q].z; acc_u[u].w += part_u[q].w; }
               }
             }
           }
+        }
+      }
+      if (!decltype(alone)::value && it0 + U * SK_THREADS >= items_pad) {      // (the same for a whole warp) nothing is read from the others any more
+        __syncwarp();
+        cluster_arrive();
+        arrived = true;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int it = it0 + u * SK_THREADS;
+        const int ml = m_begin + it / GROUPS, n4 = it % GROUPS * 4, m = m0 + ml, n = n0 + n4;
+        const bool live = it < items, valid = live && n < p.N;
+        float4 v = acc[u];
+        if (valid) {
           if (p.ssq_in) {
             const float rs = s_rstd[ml];
-            acc.x *= rs; acc.y *= rs; acc.z *= rs; acc.w *= rs;
-            acc_u.x *= rs; acc_u.y *= rs; acc_u.z *= rs; acc_u.w *= rs;
+            v.x *= rs; v.y *= rs; v.z *= rs; v.w *= rs;
+            if (GLU) { acc_u[u].x *= rs; acc_u[u].y *= rs; acc_u[u].z *= rs; acc_u[u].w *= rs; }
           }
-          if (p.swiglu) {
-            acc.x = acc.x / (1.f + __expf(-acc.x)) * acc_u.x;
-            acc.y = acc.y / (1.f + __expf(-acc.y)) * acc_u.y;
-            acc.z = acc.z / (1.f + __expf(-acc.z)) * acc_u.z;
-            acc.w = acc.w / (1.f + __expf(-acc.w)) * acc_u.w;
+          if (GLU) {
+            v.x = v.x / (1.f + __expf(-v.x)) * acc_u[u].x;
+            v.y = v.y / (1.f + __expf(-v.y)) * acc_u[u].y;
+            v.z = v.z / (1.f + __expf(-v.z)) * acc_u[u].z;
+            v.w = v.w / (1.f + __expf(-v.w)) * acc_u[u].w;
+          } else {
+            if (p.bias) {
+              v.x += p.bias[n]; v.y += p.bias[n + 1]; v.z += p.bias[n + 2]; v.w += p.bias[n + 3];
+            }
+            if (p.residual) {
+              const float2 r0 = unpack_bf16x2(rv[u].x), r1 = unpack_bf16x2(rv[u].y);
+              v.x += r0.x; v.y += r0.y; v.z += r1.x; v.w += r1.y;
+            }
           }
-          if (p.bias) {
-            acc.x += p.bias[n]; acc.y += p.bias[n + 1]; acc.z += p.bias[n + 2]; acc.w += p.bias[n + 3];
-          }
-          if (p.residual) {
-            const float2 r0 = unpack_bf16x2(rv.x), r1 = unpack_bf16x2(rv.y);
-            acc.x += r0.x; acc.y += r0.y; acc.z += r1.x; acc.w += r1.y;
-          }
-          if (p.use_layer) acc = layer_epilogue4(p.layer, acc, m, n, layer_alpha, x_old, x_e);
+          if (LAYER) v = layer_epilogue4(p.layer, v, m, n, layer_alpha, x_old[u], x_e[u]);
           if (p.out_fp32) {
-            *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.Y) + static_cast<long long>(m) * p.ldy + n) = acc;
-          } else if (p.use_layer && lin_gated(p.layer.lin.act)) {
-            *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.Y) + static_cast<long long>(m) * p.ldy + n / 2) = pack_bf16x2(acc.x, acc.y);
+            *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.Y) + static_cast<long long>(m) * p.ldy + n) = v;
+          } else if (LAYER && lin_gated(p.layer.lin.act)) {
+            *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.Y) + static_cast<long long>(m) * p.ldy + n / 2) = pack_bf16x2(v.x, v.y);
           } else {
             uint2 o;
-            o.x = pack_bf16x2(acc.x, acc.y);
-            o.y = pack_bf16x2(acc.z, acc.w);
+            o.x = pack_bf16x2(v.x, v.y);
+            o.y = pack_bf16x2(v.z, v.w);
             *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.Y) + static_cast<long long>(m) * p.ldy + n) = o;
-            if (p.ssq_out) {
+            if (MODE == SK_PLAIN && p.ssq_out) {
               // what the next norm sees is the bf16 value that was just stored
               const float2 h0 = unpack_bf16x2(o.x), h1 = unpack_bf16x2(o.y);
-              acc = make_float4(h0.x, h0.y, h1.x, h1.y);
-              const float2 w0 = unpack_bf16x2(wv.x), w1 = unpack_bf16x2(wv.y);
+              v = make_float4(h0.x, h0.y, h1.x, h1.y);
+              const float2 w0 = unpack_bf16x2(wv[u].x), w1 = unpack_bf16x2(wv[u].y);
               uint2 o2;
-              o2.x = pack_bf16x2(acc.x * w0.x, acc.y * w0.y);
-              o2.y = pack_bf16x2(acc.z * w1.x, acc.w * w1.y);
+              o2.x = pack_bf16x2(v.x * w0.x, v.y * w0.y);
+              o2.y = pack_bf16x2(v.z * w1.x, v.w * w1.y);
               *reinterpret_cast<uint2*>(p.Y2 + static_cast<long long>(m) * p.ldy2 + n) = o2;
             }
           }
         }
-        if (p.ssq_out) {
-          float sq = valid ? acc.x * acc.x + acc.y * acc.y + acc.z * acc.z + acc.w * acc.w : 0.f;
+        if (MODE == SK_PLAIN && p.ssq_out && it < items_pad) {      // (items_pad: the same for a whole warp)
+          float sq = valid ? v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w : 0.f;
           sq = warp_sum(sq);
           if (live && (threadIdx.x & 31) == 0) p.ssq_out[n_blk * p.ssq_out_stride + m] = sq;
         }
       }
-    };
-    if (split == 1) finish(std::true_type{});
-    else finish(std::false_type{});
+    }
+  };
+  if (split == 1) {
+    finish(std::true_type{});
+  } else {
+    finish(std::false_type{});
+    __syncwarp();
+    if (!arrived) cluster_arrive();
+    cluster_wait();      // peers may still be reading this CTA's partial tile
   }
-  cluster.sync();  // peers may still be reading this CTA's partial tile
 }
 
 int g_sk_sms = 0;
 int g_sk_static_w = 0;
 
-template <int NT>
+template <int NT, int MODE>
 int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int split, cudaStream_t stream) {
   using Cfg = SkinnyCfg<NT>;
-  auto kern = gemm_skinny_kernel<NT>;
+  auto kern = gemm_skinny_kernel<NT, MODE>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
-  const int tiles = p.swiglu ? (p.N + 63) / 64 : (p.N + SK_BM - 1) / SK_BM;
+  const int tiles = MODE == SK_SWIGLU ? (p.N + 63) / 64 : (p.N + SK_BM - 1) / SK_BM;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles * split, (p.M + NT - 1) / NT, 1);
   cfg.blockDim = dim3(SK_THREADS, 1, 1);
@@ -381,11 +407,9 @@ int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyPara
 }
 
 int launch_skinny_nt(int NT, const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int split, cudaStream_t s) {
-  switch (NT) {
-    case 32: return launch_skinny<32>(tw, tx, p, split, s);
-    case 64: return launch_skinny<64>(tw, tx, p, split, s);
-    default: return launch_skinny<128>(tw, tx, p, split, s);
-  }
+#define RLB_SK(mode) (NT == 32 ? launch_skinny<32, mode>(tw, tx, p, split, s) : NT == 64 ? launch_skinny<64, mode>(tw, tx, p, split, s) : launch_skinny<128, mode>(tw, tx, p, split, s))
+  return p.swiglu ? RLB_SK(SK_SWIGLU) : p.use_layer ? RLB_SK(SK_LAYER) : RLB_SK(SK_PLAIN);
+#undef RLB_SK
 }
 
 }  // namespace
