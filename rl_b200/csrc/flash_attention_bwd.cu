@@ -153,8 +153,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
   uint64_t* dq_done = bars + 15;   // the second product of a tile is complete
   uint64_t* all_done = bars + 16;  // every product is
   uint64_t* s_read = bars + 17;
-  uint64_t* ds_full = bars + 18;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  uint64_t* ds_full = bars + 18;   // [2]: a group may be done with the next tile before the other is with this one
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* info = reinterpret_cast<int*>(tmem_slot + 2);
 
@@ -168,7 +168,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
       info[0] = start; info[1] = len; info[2] = tis; info[3] = ok ? 1 : 0;
       for (int i = 0; i < 17; ++i) mbar_init(smem_u32(&bars[i]), 1);
       mbar_init(smem_u32(s_read), 8);
-      mbar_init(smem_u32(ds_full), 8);
+      for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ds_full[i]), 8);
       *abort_flag = 0;
       mbar_fence_init();
       fence_proxy_async();
@@ -235,7 +235,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
           if (j > 0 && !mbar_wait(smem_u32(dq_done), (j - 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) break;
           if (!dprobs(j + 1)) break;
         }
-        if (!mbar_wait(smem_u32(ds_full), j & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) break;
+        if (!mbar_wait(smem_u32(&ds_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) break;
         tc_fence_after();
         gradient_mma(tmem_dq, tmem_dp + (j & 1) * TILE, smem_u32(k_s + (j % DQ_K_STAGES) * TILE_BYTES), j != 0);
         umma_commit(smem_u32(&k_empty[j % DQ_K_STAGES]));
@@ -286,7 +286,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
         for (int i = 0; i < 32; ++i) w[c * 32 + i] *= (__uint_as_float(dpv[i]) - dlt) * p.scale;
         store_bf16(dp_at + c * 16, w + c * 32);
       }
-      hand_over(ds_full, lane);
+      hand_over(&ds_full[j & 1], lane);
     }
     if (ok && mbar_wait(smem_u32(all_done), 0, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
       tc_fence_after();
