@@ -85,7 +85,7 @@ __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
 }
 
 // What a kernel's epilogue can do. Every CTA runs through it once, so that instructions come from memory: code for what a launch does not do costs time. A kernel per kind, two
-// items a thread in flight, no cluster barrier for a CTA on its own and the last one split around the stores, projections of a layer in a captured chain, us:
+// items a thread in flight, no cluster barrier for a CTA on its own and no fence at the last one, projections of a layer in a captured chain, us:
 // 8B one sequence 84.1 -> 81.5, 64 sequences 93.3 -> 90.0; 1B 35.7 -> 34.3 and 44.0 -> 43.1. What is left at 64 sequences is the traffic between the CTAs of
 // a cluster: 28 KB of partial sums to each, some 10 bytes a cycle.
 enum { SK_PLAIN = 0, SK_SWIGLU = 1, SK_LAYER = 2 };
@@ -241,13 +241,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
   }
   tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem_acc, Cfg::TMEM);
-  }
+  __syncwarp();
   // Epilogue part 2: every CTA of the cluster reduces a slice of the tokens over all partial tiles.
   if (split > 1) cluster_sync();
+  else __syncthreads();
   const int tok_per = (NT + split - 1) / split;
   const int m_begin = krank * tok_per;
   const int m_end = min(rows, m_begin + tok_per);
@@ -260,7 +257,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   // warp reduction
   const int items = max(m_end - m_begin, 0) * GROUPS;
   const int items_pad = (items + 31) & ~31;
-  bool arrived = false;
   auto finish = [&](auto alone) {      // alone: a CTA on its own, without the loops over the cluster, whose instructions cost more than they hide
     constexpr int U = 2;               // items in flight per thread
     for (int it0 = threadIdx.x; it0 < items_pad; it0 += U * SK_THREADS) {
@@ -302,11 +298,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
           }
         }
-      }
-      if (!decltype(alone)::value && it0 + U * SK_THREADS >= items_pad) {      // (the same for a whole warp) nothing is read from the others any more
-        __syncwarp();
-        cluster_arrive();
-        arrived = true;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -368,9 +359,15 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     finish(std::true_type{});
   } else {
     finish(std::false_type{});
+    // Peers may still be reading this CTA's partial tile. What this one read has come, since its stores took it, and nothing is handed over: no fence, which
+    // would wait for those stores.
     __syncwarp();
-    if (!arrived) cluster_arrive();
-    cluster_wait();      // peers may still be reading this CTA's partial tile
+    cluster_arrive_relaxed();
+    cluster_wait();
+  }
+  if (warp == 1) {      // (every warp has read its part of the accumulators before the barrier of the partial tiles)
+    tc_fence_after();
+    tmem_dealloc(tmem_acc, Cfg::TMEM);
   }
 }
 
