@@ -86,8 +86,8 @@ __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
 
 // What a kernel's epilogue can do. Every CTA runs through it once, so that instructions come from memory: code for what a launch does not do costs time. A kernel per kind, two
 // items a thread in flight, no cluster barrier for a CTA on its own and no fence at the last one, projections of a layer in a captured chain, us:
-// 8B one sequence 84.1 -> 81.5, 64 sequences 93.3 -> 90.0; 1B 35.7 -> 34.3 and 44.0 -> 43.1. What is left at 64 sequences is the traffic between the CTAs of
-// a cluster: 28 KB of partial sums to each, some 10 bytes a cycle.
+// 8B one sequence 84.1 -> 80.2, 64 sequences 93.3 -> 88.9; 1B 35.7 -> 31.5 and 44.0 -> 40.0. What is left at 64 sequences is the reading of the other CTAs'
+// partial sums, 28 KB to each CTA: 1300 to 4500 cycles (sent by bulk copies instead: 92.1 us a layer).
 enum { SK_PLAIN = 0, SK_SWIGLU = 1, SK_LAYER = 2 };
 
 template <int NT, int MODE>
