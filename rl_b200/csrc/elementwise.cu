@@ -1128,8 +1128,8 @@ RLB_API int rlb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   if (d <= 2048)
     rmsnorm_bwd_rows_kernel<1, 4><<<parts, (d / 8 + 31) / 32 * 32, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial, static_cast<int>(rows), d, x_stride,
                                                                                   dy_stride, add_to_dx);
-  else if (d <= 4096)
-    rmsnorm_bwd_rows_kernel<2, 2><<<parts, (d / 16 + 31) / 32 * 32, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial, static_cast<int>(rows), d, x_stride,
+  else if (d <= 4096)      // whole warps of two pieces a thread, the last of them cut
+    rmsnorm_bwd_rows_kernel<2, 2><<<parts, (d / 8 + 63) / 64 * 32, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial, static_cast<int>(rows), d, x_stride,
                                                                                    dy_stride, add_to_dx);
   else
     rmsnorm_bwd_kernel<<<parts, threads, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial,

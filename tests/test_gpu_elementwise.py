@@ -644,6 +644,27 @@ def test_rmsnorm_many_rows(native_lib, d, rows):
     assert near(y, ref, 2.0 ** -8) and near(x.grad, X.grad, 2.0 ** -7) and near(w.grad, W.grad, 2.0 ** -7)
 
 
+@pytest.mark.parametrize("d", [2040, 2048, 2056, 2064, 2568, 2688, 3080, 3584, 3592, 4088, 4096, 4104])      # a piece a thread, two, two of which the last warp has one, the looping kernel
+@pytest.mark.parametrize("rows", [1, 5, 700])
+def test_rmsnorm_gradient_covers_every_column(native_lib, d, rows):
+    """Gradients of widths whose last warp has part of its pieces, into buffers that hold NaN before, against float64: one bf16 rounding of dx (2^-9 a
+    value) and fp32 sums of the weight gradient (rows' terms of size 1 to 10: 1e-5)."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(d + rows)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    x, dy, w = r(rows, d).bfloat16(), r(rows, d).bfloat16(), (1 + 0.3 * r(d)).bfloat16()
+    rstd = torch.rsqrt(x.float().pow(2).mean(-1) + 1e-6)
+    parts = F._L.lib().rlb_rmsnorm_bwd_parts(rows)
+    dx, partial, dw = torch.full_like(x, float("nan")), torch.full((parts, d), float("nan"), device="cuda"), torch.full((d,), float("nan"), device="cuda")
+    F.call("rlb_rmsnorm_bwd", dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dx.data_ptr(), partial.data_ptr(), dw.data_ptr(), None, 0,
+           rows, d, d, d, 0, F.stream_ptr())
+    X, D, W, s = x.double(), dy.double(), w.double(), rstd.double()[:, None]
+    ref = s * (D * W - X * s * s * (D * W * X).mean(-1, keepdim=True))
+    want = (D * X * s).sum(0)
+    assert (dx.double() - ref).norm() <= 2.0 ** -8 * ref.norm() and (dw.double() - want).norm() <= 1e-5 * want.norm()
+
+
 @pytest.mark.parametrize("d,rows", [(8, 2368), (512, 2371), (1024, 2368), (1032, 7109), (2048, 7104), (4096, 7109), (4104, 14213), (5120, 14208)])
 def test_rmsnorm_warp_rows(native_lib, d, rows):
     """A warp per row: the first size that takes it, a cut last CTA, every register count. Against the fp32 statement: one bf16 rounding (2^-8)."""
