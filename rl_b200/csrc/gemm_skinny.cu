@@ -472,6 +472,10 @@ RLB_API int rlb_gemm_skinny_fused(const void* X, const void* W, void* Y, int M, 
   // (beyond 256 tokens with the tiled kernel's alignments)
   if (M > 256 && residual && ((ldr % 8) || (reinterpret_cast<uintptr_t>(residual) & 15))) return -2;
   if (M > 256 && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(Y)) & 15)) return -3;
+  // four values of output, residual and norm weight at a time
+  if ((reinterpret_cast<uintptr_t>(Y) & (out_fp32 ? 15 : 7)) ||
+      ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(Y2)) & 7))
+    return -3;
   if (swiglu && ((N % 64) || bias || residual || ssq_out)) return -2;
   if (ssq_out && (out_fp32 || !norm_w || !Y2 || (ldy2 % 4) || ssq_out_stride < M)) return -2;
   if (ssq_in && (ssq_in_tiles <= 0 || ssq_in_stride < M)) return -2;

@@ -20,6 +20,16 @@ BF16 = torch.bfloat16
 
 
 # --------------------------------------------------------------------------------------- GEMM
+def _streams_weights(M: int, N: int, K: int, out: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
+    """Whether a product goes to the weight-streaming kernel: where it is sooner done there (``rlb_gemm_takes_skinny``), and up to 256 rows also
+    where output or residual do not start their rows on 16 bytes, which the tiled kernel wants and this one does not."""
+    if M > 1024 or K < 256:
+        return False
+    if _L.lib().rlb_gemm_takes_skinny(M, N, K):
+        return True
+    return M <= 256 and (out.data_ptr() % 16 != 0 or (residual is not None and (residual.data_ptr() % 16 != 0 or residual.stride(0) % 8 != 0)))
+
+
 def gemm(
     a: torch.Tensor,
     b: torch.Tensor,
@@ -64,7 +74,7 @@ def gemm(
     assert out.stride(1) == 1 and out.dtype in (BF16, torch.float32)
     if bias is not None:
         bias = bias.float().contiguous()
-    if not a_mn and not b_mn and not accumulate and max_ctas == 0 and M <= 1024 and _L.lib().rlb_gemm_takes_skinny(M, N, K):
+    if not a_mn and not b_mn and not accumulate and max_ctas == 0 and _streams_weights(M, N, K, out, residual):
         # decode-sized batches and short passes: weight-streaming kernel with cluster split-K
         call("rlb_gemm_skinny", ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
              int(out.dtype == torch.float32), ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,

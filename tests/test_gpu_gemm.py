@@ -256,6 +256,34 @@ def test_skinny_gemm(native_lib, M, N, K):
     assert _rel_err(y2, ref + bias + res.float()) < 2e-3
 
 
+@pytest.mark.parametrize("M", [5, 128, 129, 256])
+@pytest.mark.parametrize("N,K", [(19072, 512), (18952, 264), (9480, 448), (264, 256), (1000, 2048)])      # too wide to be split, contractions too short, split
+@pytest.mark.parametrize("place", ["residual stride", "residual", "output", "both"])
+def test_gemm_of_places_on_8_bytes(native_lib, M, N, K, place):
+    """Up to 256 rows a residual's rows may be a multiple of four elements apart, and it and a bf16 output may start on 8 bytes. Against float64: fp32
+    sums and one bf16 rounding of at most 2^-8, and not a value beside the output is written. 257 rows of such a residual are refused, and so is an
+    fp32 output on 8 bytes, whatever the number of rows."""
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import NativeLibraryError, check_status
+
+    g = torch.Generator("cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    a, b = r(M, K).bfloat16(), (0.1 * r(N, K)).bfloat16()
+    res = r(M, N + 4).bfloat16()[:, :N] if place == "residual stride" else r(M, N + 8).bfloat16()[:, 0 if place == "output" else 4 :][:, :N]
+    wide = r(M, N + 8).bfloat16()
+    old, at = wide.clone(), 4 if place in ("output", "both") else 0
+    F.gemm(a, b, out=wide[:, at : at + N], residual=res)
+    ref = a.double() @ b.double().t() + res
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    assert (wide[:, at : at + N].double() - ref).abs().max() <= (2.0 ** -8 + 1e-5) * ref.abs().max()
+    assert torch.equal(wide[:, :at], old[:, :at]) and torch.equal(wide[:, at + N :], old[:, at + N :])
+    with pytest.raises(NativeLibraryError):
+        F.gemm(a, b, out=r(M, N + 4)[:, 2 : 2 + N])
+    with pytest.raises(NativeLibraryError):
+        F.gemm(r(257, K).bfloat16(), b, residual=r(257, N + 4).bfloat16()[:, :N])
+
+
 @pytest.mark.parametrize("M", [129, 130, 255, 257, 384, 385, 512, 640, 1000, 1024])      # token tiles of 128, whole and cut
 @pytest.mark.parametrize("N,K", [(1000, 512), (2048, 264), (264, 8192), (4096, 1024)])
 def test_skinny_token_tiles(native_lib, M, N, K):
