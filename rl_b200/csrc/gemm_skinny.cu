@@ -49,7 +49,6 @@ struct SkinnyCfg {
   static constexpr int PARTIAL = NT * SK_BM * 4;  // fp32 [NT][128]
   static constexpr int MAIN = RING > PARTIAL ? RING : PARTIAL;
   static constexpr int SMEM = MAIN + 256 + 1024;  // ring / partial tile, barriers, per-token rstd (256 floats)
-  static constexpr int TMEM = NT < 32 ? 32 : NT;
 };
 
 struct SkinnyParams {
@@ -60,6 +59,7 @@ struct SkinnyParams {
   long long ldr;
   int M, N, K;
   int out_fp32;
+  int chains;    // 2: a CTA sums the two halves of its K range apart (skinny_chains)
   int w_static;  // W is not written by the kernel that precedes this one on the stream: its stream may start early
   int* status;
   // fused RMSNorm of the input: partial sums of squares [ssq_in_tiles][ssq_in_stride] written by the producer of X
@@ -126,6 +126,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const int k_per = (num_k + split - 1) / split;
   const int kb_begin = krank * k_per;
   const int kb_end = min(num_k, kb_begin + k_per);
+  const int kb_mid = NT == 128 && p.chains > 1 ? (kb_begin + kb_end + 1) / 2 : kb_end;      // from here on into the second accumulator
+  const uint32_t tmem_cols = NT == 128 && p.chains > 1 ? 2 * NT : NT;
   const bool aligned = (smem_u32(smem) & 1023u) == 0;
 
   if (threadIdx.x == 0) {
@@ -155,7 +157,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), Cfg::TMEM);
+    tmem_alloc(smem_u32(tmem_slot), tmem_cols);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -198,7 +200,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         const uint64_t b_desc = make_smem_desc_sw128(a_addr + Cfg::A_BYTES, 16, 1024);
 #pragma unroll
         for (int kk = 0; kk < SK_BK / 16; ++kk)
-          umma_f16(tmem_acc, a_desc + kk * 2, b_desc + kk * 2, idesc, (kb > kb_begin || kk > 0) ? 1u : 0u);
+          umma_f16(tmem_acc + (kb < kb_mid ? 0 : NT), a_desc + kk * 2, b_desc + kk * 2, idesc, (kb > kb_begin && kb != kb_mid) || kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&empty_bar[stage]));
         if (++stage == Cfg::STAGES) {
           stage = 0;
@@ -232,6 +234,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       if (ok) {
         tmem_ld_32x32b_x32(taddr + c * 32, r);
         tmem_ld_wait();
+        if (NT == 128 && kb_mid < kb_end) {
+          uint32_t r2[32];
+          tmem_ld_32x32b_x32(taddr + NT + c * 32, r2);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
+        }
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) r[i] = 0u;  // a CTA without a K range contributes zeros
@@ -367,7 +376,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   }
   if (warp == 1) {      // (every warp has read its part of the accumulators before the barrier of the partial tiles)
     tc_fence_after();
-    tmem_dealloc(tmem_acc, Cfg::TMEM);
+    tmem_dealloc(tmem_acc, tmem_cols);
   }
 }
 
@@ -432,15 +441,21 @@ static int skinny_split(int M, int N, int K) {
 }
 RLB_API int rlb_gemm_skinny_split(int N, int K) { return skinny_split(1, N, K); }
 
+// Two tiles of tokens leave CTAs for half the split, and the tensor core's sums lose with their length (they are cut, not rounded: 6144 x 4096 off by
+// 1.0e-6 of the norm in eighths, 2.1e-6 in quarters). A CTA of such a product sums the halves of its range in two accumulators, so that products
+// of up to 256 tokens are as exact as those of 128.
+static int skinny_chains(int M, int N, int K, int split) { return M > 128 && M <= 256 && skinny_split(1, N, K) > split ? 2 : 1; }
+
 // Whether a product of M tokens is sooner done here than on the tiled kernel (gemm_tcgen05.cu): up to 128 tokens, and up to 1024 where the
 // contraction can be split at least in two. Timed both ways, weights from memory, us (here / tiled): 3072 x 2048: 129 tokens 12 / 18, 256 12 / 19,
 // 512 17 / 19, 768 17 / 19, 1024 (one part) 24 / 19; 2048 x 8192: 256 17 / 46, 512 23 / 46, 1024 38 / 46; 6144 x 4096: 256 25 / 29, 384 25 / 29, 512
 // (one part) 37 / 29; 4096 x 14336: 256 36 / 74, 512 62 / 74, 640 (one part) 96 / 78; 16384 x 2048 (one part): 256 27 / 22; 28672 x 4096 (one part):
-// 256 91 / 61, but 128 tokens 52 / 49 and 65 49 / 49.
+// 256 91 / 61, but 128 tokens 52 / 49 and 65 49 / 49. Up to 256 tokens whatever is split at 128 comes
+// here, for the sake of its sums (skinny_chains): 16384 x 2048 2 us longer than on the tiled kernel, half its error.
 constexpr int SK_MAX_TOKENS = 1024;
 RLB_API int rlb_gemm_takes_skinny(int M, int N, int K) {
   if (K < 256 || M > SK_MAX_TOKENS) return 0;
-  return M <= 128 || skinny_split(M, N, K) > 1;
+  return M <= 128 || skinny_split(M <= 256 ? 1 : M, N, K) > 1;
 }
 
 // While set, callers promise that the W operand of every skinny GEMM was not written by the kernel launched just before
@@ -488,9 +503,13 @@ RLB_API int rlb_gemm_skinny_fused(const void* X, const void* W, void* Y, int M, 
   rc = rlb_make_tmap_2d(&tx, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, ldx * 2, SK_BK, NT,
                         CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return -100 - rc;
-  if (split <= 0) split = skinny_split(M, w_rows, K);
-  if (split > 8) split = 8;
   SkinnyParams p;
+  p.chains = 1;
+  if (split <= 0) {
+    split = skinny_split(M, w_rows, K);
+    p.chains = skinny_chains(M, w_rows, K, split);
+  }
+  if (split > 8) split = 8;
   p.Y = Y;
   p.ldy = ldy;
   p.bias = bias;
@@ -545,7 +564,9 @@ RLB_API int rlb_gemm_skinny_layer(const void* X, const void* W, void* out, int M
   p.use_layer = 1;
   p.layer = LayerEpilogue{x, ldx, e, static_cast<const __nv_bfloat16*>(step), static_cast<const __nv_bfloat16*>(alpha),
                           static_cast<const __nv_bfloat16*>(nw), static_cast<const __nv_bfloat16*>(nb), act_from, LinearEpi{}};
-  return launch_skinny_nt(NT, tw, tx, p, skinny_split(M, N, K), static_cast<cudaStream_t>(stream));
+  const int split = skinny_split(M, N, K);
+  p.chains = skinny_chains(M, N, K, split);
+  return launch_skinny_nt(NT, tw, tx, p, split, static_cast<cudaStream_t>(stream));
 }
 
 // rlb_linear_tiled for M <= 1024 rows on the weight-streaming kernel; out bf16 or fp32 (fp32: no gated unit).
@@ -573,7 +594,9 @@ RLB_API int rlb_linear_skinny(const RlbLinear* l, void* stream) {
   p.use_layer = 1;
   p.layer.act_from = 1 << 30;
   p.layer.lin = rlb_linear_epi(*l);
-  return launch_skinny_nt(NT, tw, tx, p, skinny_split(l->M, l->N, l->K), static_cast<cudaStream_t>(stream));
+  const int split = skinny_split(l->M, l->N, l->K);
+  p.chains = skinny_chains(l->M, l->N, l->K, split);
+  return launch_skinny_nt(NT, tw, tx, p, split, static_cast<cudaStream_t>(stream));
 }
 
 RLB_API int rlb_gemm_skinny(const void* X, const void* W, void* Y, int M, int N, int K, long long ldx, long long ldw,

@@ -284,6 +284,34 @@ def test_gemm_of_places_on_8_bytes(native_lib, M, N, K, place):
         F.gemm(r(257, K).bfloat16(), b, residual=r(257, N + 4).bfloat16()[:, :N])
 
 
+@pytest.mark.parametrize("M", [129, 200, 256])
+@pytest.mark.parametrize("N,K", [(3072, 2048), (6144, 4096), (4096, 14336), (16384, 2048), (16384, 576), (2048, 4992), (264, 520)])      # split by 8, 4, 2; halves of odd lengths
+@pytest.mark.parametrize("kind", ["plain", "unit", "layer"])
+def test_products_of_two_token_tiles_are_as_exact(native_lib, M, N, K, kind):
+    """Sums over the contraction lose with their length. A product of 129 to 256 rows is cut into the same lengths as one of 128: its error against
+    float64 is that of its first 128 rows (which differ by the chance of their values, some per cent; sums twice as long are off by twice as much)."""
+    from rl_b200.ops import engine_ops as E
+    from rl_b200.ops import functional as F
+    from rl_b200.ops import layer_ops as Y
+    from rl_b200.ops.lib import check_status
+
+    g = torch.Generator("cuda").manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=g, device="cuda").bfloat16(), (0.05 * torch.randn(N, K, generator=g, device="cuda")).bfloat16()
+    z = x.double() @ w.double().t()
+    if kind == "unit":
+        if N % 128:
+            pytest.skip("the unit's halves are whole tiles")
+        run = lambda t: E.skinny_linear(t, w, out_dtype=torch.float32, swiglu=True)      # noqa: E731
+        z = torch.nn.functional.silu(z[:, : N // 2]) * z[:, N // 2 :]
+    elif kind == "layer":
+        run = lambda t: Y.capped_logits(t, w, 1.0, 0.0)      # noqa: E731
+    else:
+        run = lambda t: F.gemm(t, w, out_dtype=torch.float32)      # noqa: E731
+    err = [((run(x[:m]) - z[:m]).norm() / z[:m].norm()).item() for m in (128, M)]
+    assert check_status() == 0
+    assert err[1] <= 1.2 * err[0] and err[0] < 1e-5
+
+
 @pytest.mark.parametrize("M", [129, 130, 255, 257, 384, 385, 512, 640, 1000, 1024])      # token tiles of 128, whole and cut
 @pytest.mark.parametrize("N,K", [(1000, 512), (2048, 264), (264, 8192), (4096, 1024)])
 def test_skinny_token_tiles(native_lib, M, N, K):
