@@ -236,6 +236,7 @@ sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const f
   best = block_argmax(best, redb);
   if (SHARED) {
     if (threadIdx.x == 0) mine = RowPart{mx, sum, best};
+    __syncwarp();      // (the cluster's barrier wants whole warps)
     cluster_sync();
   }
   if (part == 0 && threadIdx.x == 0) {
@@ -255,7 +256,10 @@ sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const f
       out_logprob[row] = (zt - mx) * inv_t - __logf(sum);
     }
   }
-  if (SHARED) cluster_sync();      // the first CTA may still read this one's part
+  if (SHARED) {      // the first CTA may still read this one's part
+    __syncwarp();
+    cluster_sync();
+  }
 }
 
 template <typename T>
