@@ -250,9 +250,10 @@ sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const f
         mx = top;
       }
     }
-    out_tok[row] = best.idx;
+    const int tok = best.idx < V ? best.idx : 0;      // (a row without a number above -inf draws nothing: its first token, whose log-probability is NaN)
+    out_tok[row] = tok;
     if (out_logprob) {
-      const float zt = ldz(z, best.idx);
+      const float zt = ldz(z, tok);
       out_logprob[row] = (zt - mx) * inv_t - __logf(sum);
     }
   }

@@ -716,3 +716,20 @@ def test_sampling_over_parts_of_rows(native_lib, B, V, dtype, greedy):
     assert torch.equal(tok, one) and (not greedy or bool((tok == 100).all()))
     want = torch.log_softmax(z.double() / 0.7, -1).gather(1, tok.long()[:, None])[:, 0]
     assert (lp - want).abs().max() <= 2e-5 * (1 + want.abs().max())
+
+
+@pytest.mark.parametrize("B,V", [(4, 128256), (40, 32771), (80, 4099)])      # eight, four and one CTA a row
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kw", [dict(greedy=True), dict(temperature=0.7, seed=3), dict(temperature=0.7, seed=3, top_k=5), dict(seed=3, top_p=0.9)])
+def test_sampling_rows_without_a_number(native_lib, B, V, dtype, kw):
+    """Rows of -inf or NaN alone give their first token and NaN; the others give what they give without such rows beside them."""
+    from rl_b200.ops import engine_ops as E
+
+    z = torch.randn(B, V, generator=torch.Generator("cuda").manual_seed(V), device="cuda").to(dtype)
+    want = E.sample(z, **kw)
+    z[1], z[-1] = -float("inf"), float("nan")
+    tok, lp = E.sample(z, **kw)
+    rest = torch.ones(B, dtype=torch.bool, device="cuda")
+    rest[1] = rest[-1] = False
+    assert tok[1] == tok[-1] == 0 and bool(lp[~rest].isnan().all())
+    assert torch.equal(tok[rest], want[0][rest]) and torch.equal(lp[rest], want[1][rest])
