@@ -263,14 +263,54 @@ sample_kernel(const T* __restrict__ logits, long long row_stride, int V, const f
   }
 }
 
+int sm_count() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    n = sms;
+  }
+  return n;
+}
+
+// Clusters of 8 or 4 CTAs that the device holds at once.
+template <typename T>
+int resident_clusters(int parts) {
+  static int known[2] = {-1, -1};
+  int& n = known[parts == 8];
+  if (n < 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(parts));
+    cfg.blockDim = dim3(1024);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = parts;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, sample_kernel<T, true>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      fit = 0;
+    }
+    n = fit;
+  }
+  return n;
+}
+
 template <typename T>
 int launch_sample(const T* logits, long long row_stride, int B, int V, const float* temps, const int* top_ks, const float* top_ps, float def_temp, int def_top_k,
                   float def_top_p, int greedy, unsigned long long seed, unsigned long long step, const unsigned long long* step_ptr,
                   const long long* row_keys, int* out_tok, float* out_logprob, cudaStream_t s) {
-  // Clusters where no row can have a filter and at least four CTAs a row fit, two to an SM, with 4096 logits each.
+  // Clusters where no row can have a filter, at most two CTAs come to an SM and each has 4096 logits; 12288 where not all clusters are resident
+  // at once (SMs of a group that do not fill a cluster are left over): greedy, 74 rows in fours 16384 logits 9.3 us, a CTA a row 5.9; 32000 11.2
+  // and 9.1; 50000 13.9 and 12.9, but drawn 17.7 and 18.8; 128256 22.8 and 27.7. 37 rows in eights and fours: 65536 12.3 and 10.6, 128256 16.0 and 16.2,
+  // drawn 21.2 and 23.3.
   const bool plain = !top_ks && !top_ps && !(def_top_k > 0 && def_top_k < V) && !(def_top_p < 1.f);
   int parts = plain ? 8 : 1;
-  while (parts > 1 && (static_cast<long long>(parts) * B > 2 * 148 || parts * 4096 > V)) parts /= 2;
+  while (parts >= 4 && (static_cast<long long>(parts) * B > 2 * sm_count() || parts * (B > resident_clusters<T>(parts) ? 12288 : 4096) > V)) parts /= 2;
   if (parts < 4) {
     rlb_launch_pdl(sample_kernel<T, false>, dim3(B), dim3(1024), 0, s, logits, row_stride, V, temps, top_ks, top_ps, def_temp, def_top_k, def_top_p, greedy, seed,
                    step, step_ptr, row_keys, out_tok, out_logprob);

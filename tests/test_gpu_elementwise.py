@@ -695,7 +695,7 @@ def test_logprob_combine(native_lib, M, V):
     assert (lp.double() - z.gather(1, t[:, None])[:, 0]).abs().max() < 1e-4 and (ent.double() + (z.exp() * z).sum(-1)).abs().max() < 1e-3
 
 
-@pytest.mark.parametrize("B,V", [(1, 128256), (3, 16384), (37, 32771), (38, 32771), (74, 20000), (75, 20000), (2, 16383)])      # eight, four and one CTA a row
+@pytest.mark.parametrize("B,V", [(1, 128256), (3, 16384), (37, 32771), (38, 32771), (74, 20000), (75, 20000), (2, 16383), (74, 50000)])      # eight, four and one CTA a row, clusters in two waves
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("greedy", [False, True])
 def test_sampling_over_parts_of_rows(native_lib, B, V, dtype, greedy):
