@@ -143,17 +143,16 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   }
   const bool have_work = kb_end > kb_begin && aligned;
   // Weights that the preceding kernel cannot have written are requested before the dependency wait: the first ring
-  // stages fill while that kernel drains. The activations of the same stages follow after the wait.
-  int early = 0;
+  // stages fill while that kernel drains. The activations of the same stages follow after the wait. (Every thread knows how many: the one that is
+  // elected below need not be the one here.)
+  const int early = p.w_static && have_work ? min(Cfg::STAGES, kb_end - kb_begin) : 0;
   if (threadIdx.x == 0 && have_work) {
     prefetch_tmap(&tmap_w);
     prefetch_tmap(&tmap_x);
-    if (p.w_static) {
-      for (; early < Cfg::STAGES && kb_begin + early < kb_end; ++early) {
-        const uint32_t bar = smem_u32(&full_bar[early]);
-        mbar_arrive_expect_tx(bar, Cfg::STAGE);
-        load_w(smem_u32(smem + early * Cfg::STAGE), bar, kb_begin + early);
-      }
+    for (int e = 0; e < early; ++e) {
+      const uint32_t bar = smem_u32(&full_bar[e]);
+      mbar_arrive_expect_tx(bar, Cfg::STAGE);
+      load_w(smem_u32(smem + e * Cfg::STAGE), bar, kb_begin + e);
     }
   }
   if (warp == 1) {

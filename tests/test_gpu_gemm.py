@@ -357,6 +357,31 @@ def test_skinny_split_values(native_lib):
     assert lib().rlb_gemm_skinny_split(4096, 4096) in (1, 2, 4, 8)
 
 
+@pytest.mark.parametrize("M", [1, 33, 65, 130])      # rings of four, four and three stages, two token tiles
+@pytest.mark.parametrize("K", [64, 192, 256, 264, 320, 576, 1088])
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+def test_skinny_early_weights(native_lib, M, K, split):
+    """Weights requested ahead of the dependency: ranges shorter than the ring, as long, longer and empty (more CTAs than blocks of 64). The same
+    products in the same order as without, so equal bit for bit; against float64 one bf16 rounding and fp32 sums."""
+    from rl_b200.ops.engine_ops import skinny_static_weights
+    from rl_b200.ops.lib import call, check_status, ptr, status_word, stream_ptr
+
+    g = torch.Generator("cuda").manual_seed(K + M)
+    x, w = torch.randn(M, K, generator=g, device="cuda").bfloat16(), torch.randn(384, K, generator=g, device="cuda").bfloat16()
+    outs = []
+    for on in (False, True):
+        y = torch.empty(M, 384, device="cuda", dtype=torch.bfloat16)
+        torch.cuda.synchronize()      # (the promise holds: nothing writes the weights behind this)
+        before = skinny_static_weights(on)
+        for _ in range(3):
+            call("rlb_gemm_skinny", ptr(x), ptr(w), ptr(y), M, 384, K, K, K, 384, 0, None, None, 0, split, ptr(status_word()), stream_ptr())
+        skinny_static_weights(bool(before))
+        outs.append(y)
+    ref = x.double() @ w.double().t()
+    assert check_status() == 0 and torch.equal(*outs)
+    assert (outs[0].double() - ref).abs().max() <= (2.0 ** -8 + 1e-5) * ref.abs().max()
+
+
 @pytest.mark.parametrize("M", [5, 64, 130])
 def test_skinny_gemm_epilogue_fusions_match_fp32_reference(native_lib, M):
     """RMSNorm folded into two projections (producer writes h * w and per-tile sums of squares, consumer scales its rows)
