@@ -38,16 +38,20 @@ __device__ __forceinline__ bool locate_tile(const int* __restrict__ cu, int num_
 // (key tiles), so all tiles that see d of them come before those that see d - 1. Block `index` of `most` (some past the last tile: false). More
 // than 128 sequences go one after the other. With the CTAs of all heads side by side (the heads as the fast part of the block index) the last ones are the
 // shortest of all; one head after the other, each with its own short and long tiles, left SMs without work for up to a quarter of the time (backward of
-// 32 query and 8 KV heads of 128, us: 4 x 1000 383 -> 321, 8 x 500 277 -> 251, 7600 2755 -> 2371, 4 x 4096 3042 -> 2808).
+// 32 query and 8 KV heads of 128, us: 4 x 1000 383 -> 321, 8 x 500 277 -> 251, 7600 2755 -> 2371, 4 x 4096 3042 -> 2808). The place in the order comes from the grid's
+// dimensions and the bounds stay in registers: with a division for head and tile each and the bounds read again, some 800 cycles, tiles of short sequences
+// took a tenth longer (forward, 256 x 64 tokens 278 us, now 262; 1 x 64 8.3 and 7.2).
 __device__ __forceinline__ bool locate_longest_first(const int* __restrict__ cu, int num_seqs, int rows, int index, int most, bool late, int& start, int& len,
                                                      int& tile_in_seq) {
   if (num_seqs > SORTED_SEQS) return locate_tile(cu, num_seqs, rows, late ? most - 1 - index : index, start, len, tile_in_seq);
   const int lane = threadIdx.x & 31;
-  int tiles[SORTED_SEQS / 32], top = 0;
+  int tiles[SORTED_SEQS / 32], begin[SORTED_SEQS / 32], length[SORTED_SEQS / 32], top = 0;
 #pragma unroll
   for (int k = 0; k < SORTED_SEQS / 32; ++k) {
     const int s = lane + 32 * k;
-    tiles[k] = s < num_seqs ? (cu[s + 1] - cu[s] + rows - 1) / rows : 0;
+    begin[k] = s < num_seqs ? cu[s] : 0;
+    length[k] = s < num_seqs ? cu[s + 1] - begin[k] : 0;
+    tiles[k] = (length[k] + rows - 1) / rows;
     top = max(top, tiles[k]);
   }
   auto at_least = [&](int d) {      // tiles that see d others or more
@@ -73,9 +77,9 @@ __device__ __forceinline__ bool locate_longest_first(const int* __restrict__ cu,
       continue;
     }
     for (; j > 0; --j) has &= has - 1;
-    const int src = __ffs(has) - 1, s = 32 * k + src;
-    start = cu[s];
-    len = cu[s + 1] - start;
+    const int src = __ffs(has) - 1;
+    start = __shfl_sync(0xffffffffu, begin[k], src);
+    len = __shfl_sync(0xffffffffu, length[k], src);
     tile_in_seq = late ? lo - 1 : __shfl_sync(0xffffffffu, tiles[k], src) - lo;
     return true;
   }

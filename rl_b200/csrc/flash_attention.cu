@@ -106,33 +106,36 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   int* tile_info = reinterpret_cast<int*>(tmem_slot + 2);  // seq_start, seq_len, tile_in_seq, valid
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles = gridDim.x / p.Hq, head = p.longest_first ? blockIdx.x % p.Hq : blockIdx.x / tiles;
+  const int head = p.longest_first ? blockIdx.x : blockIdx.y;
   const int kv_head = head / (p.Hq / p.Hkv);
 
   if (warp == 0) {
     int start = 0, len = 0, tis = 0;
-    const bool ok = p.longest_first ? locate_longest_first(p.cu_seqlens, p.num_seqs, BQ, blockIdx.x / p.Hq, tiles, true, start, len, tis)
-                                    : locate_tile(p.cu_seqlens, p.num_seqs, BQ, tiles - 1 - blockIdx.x % tiles, start, len, tis);      // late tiles of a sequence see the most keys
+    const bool ok = p.longest_first ? locate_longest_first(p.cu_seqlens, p.num_seqs, BQ, blockIdx.y, gridDim.y, true, start, len, tis)
+                                    : locate_tile(p.cu_seqlens, p.num_seqs, BQ, gridDim.x - 1 - blockIdx.x, start, len, tis);      // late tiles of a sequence see the most keys
     if (lane == 0) {
       tile_info[0] = start;
       tile_info[1] = len;
       tile_info[2] = tis;
       tile_info[3] = ok ? 1 : 0;
-      mbar_init(smem_u32(q_full), 1);
-      for (int s = 0; s < K_STAGES; ++s) {
-        mbar_init(smem_u32(&k_full[s]), 1);
-        mbar_init(smem_u32(&k_empty[s]), 1);
-      }
-      for (int s = 0; s < 2; ++s) {
-        mbar_init(smem_u32(&v_full[s]), 1);
-        mbar_init(smem_u32(&v_empty[s]), 1);
-        mbar_init(smem_u32(&s_full[s]), 1);
-        mbar_init(smem_u32(&p_full[s]), 4);
-      }
-      *abort_flag = 0;
-      mbar_fence_init();
-      fence_proxy_async();
     }
+  } else if (threadIdx.x == 64) {      // (while the first warp waits for the sequences' bounds)
+    prefetch_tmap(&tmap_q);
+    prefetch_tmap(&tmap_kv);
+    mbar_init(smem_u32(q_full), 1);
+    for (int s = 0; s < K_STAGES; ++s) {
+      mbar_init(smem_u32(&k_full[s]), 1);
+      mbar_init(smem_u32(&k_empty[s]), 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&v_full[s]), 1);
+      mbar_init(smem_u32(&v_empty[s]), 1);
+      mbar_init(smem_u32(&s_full[s]), 1);
+      mbar_init(smem_u32(&p_full[s]), 4);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+    fence_proxy_async();
   }
   __syncthreads();
   if (!tile_info[3]) return;  // uniform: past the last tile (before any TMEM allocation)
@@ -156,8 +159,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
   if (warp == 0) {
     if (elect_one()) {
-      prefetch_tmap(&tmap_q);
-      prefetch_tmap(&tmap_kv);
       mbar_arrive_expect_tx(smem_u32(q_full), Q_BYTES);
 #pragma unroll
       for (int a = 0; a < ATOMS; ++a)
@@ -417,7 +418,8 @@ RLB_API int RLB_NAME(rlb_flash_attn_fwd)(const void* qkv, long long qkv_stride, 
   // 32 heads of 128: 543 -> 488 us; 8 x 500 71 -> 69); with more there is little to save, and neighbouring tiles of a head find their keys in the
   // nearer cache (16 x 1200: 323 us, longest first 336).
   p.longest_first = static_cast<long long>(max_tiles) * Hq <= 10 * 2 * 148;
-  flash_fwd_kernel<<<max_tiles * Hq, FWD_THREADS, FWD_SMEM, static_cast<cudaStream_t>(stream)>>>(tq, tkv, p);
+  const dim3 grid = p.longest_first ? dim3(Hq, max_tiles) : dim3(max_tiles, Hq);
+  flash_fwd_kernel<<<grid, FWD_THREADS, FWD_SMEM, static_cast<cudaStream_t>(stream)>>>(tq, tkv, p);
   return static_cast<int>(cudaGetLastError());
 }
 

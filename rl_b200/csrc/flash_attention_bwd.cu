@@ -159,20 +159,23 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
   int* info = reinterpret_cast<int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.x % p.Hq;
+  const int head = blockIdx.x;
   const int kv_head = head / (p.Hq / p.Hkv);
   if (warp == 0) {
     int start = 0, len = 0, tis = 0;
-    const bool ok = locate_longest_first(p.cu_seqlens, p.num_seqs, TILE, blockIdx.x / p.Hq, gridDim.x / p.Hq, true, start, len, tis) && (smem_u32(smem) & 1023u) == 0;
+    const bool ok = locate_longest_first(p.cu_seqlens, p.num_seqs, TILE, blockIdx.z * gridDim.y + blockIdx.y, gridDim.y * gridDim.z, true, start, len, tis) && (smem_u32(smem) & 1023u) == 0;
     if (lane == 0) {
       info[0] = start; info[1] = len; info[2] = tis; info[3] = ok ? 1 : 0;
-      for (int i = 0; i < 17; ++i) mbar_init(smem_u32(&bars[i]), 1);
-      mbar_init(smem_u32(s_read), 8);
-      for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ds_full[i]), 8);
-      *abort_flag = 0;
-      mbar_fence_init();
-      fence_proxy_async();
     }
+  } else if (threadIdx.x == 64) {      // (while the first warp waits for the sequences' bounds)
+    prefetch_tmap(&tmap_qkv);
+    prefetch_tmap(&tmap_do);
+    for (int i = 0; i < 17; ++i) mbar_init(smem_u32(&bars[i]), 1);
+    mbar_init(smem_u32(s_read), 8);
+    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ds_full[i]), 8);
+    *abort_flag = 0;
+    mbar_fence_init();
+    fence_proxy_async();
   }
   __syncthreads();
   if (!info[3]) return;
@@ -340,21 +343,24 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
   int* info = reinterpret_cast<int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kv_head = blockIdx.x % p.Hkv;
+  const int kv_head = blockIdx.x;
   const int G = p.Hq / p.Hkv;
   if (warp == 0) {
     int start = 0, len = 0, tis = 0;
-    const bool ok = locate_longest_first(p.cu_seqlens, p.num_seqs, TILE, blockIdx.x / p.Hkv, gridDim.x / p.Hkv, false, start, len, tis) && (smem_u32(smem) & 1023u) == 0;
+    const bool ok = locate_longest_first(p.cu_seqlens, p.num_seqs, TILE, blockIdx.z * gridDim.y + blockIdx.y, gridDim.y * gridDim.z, false, start, len, tis) && (smem_u32(smem) & 1023u) == 0;
     if (lane == 0) {
       info[0] = start; info[1] = len; info[2] = tis; info[3] = ok ? 1 : 0;
-      for (int i = 0; i < 16; ++i) mbar_init(smem_u32(&bars[i]), 1);
-      mbar_init(smem_u32(p_full), 8);
-      mbar_init(smem_u32(dp_read), 8);
-      mbar_init(smem_u32(ds_full), 8);
-      *abort_flag = 0;
-      mbar_fence_init();
-      fence_proxy_async();
     }
+  } else if (threadIdx.x == 64) {      // (while the first warp waits for the sequences' bounds)
+    prefetch_tmap(&tmap_qkv);
+    prefetch_tmap(&tmap_do);
+    for (int i = 0; i < 16; ++i) mbar_init(smem_u32(&bars[i]), 1);
+    mbar_init(smem_u32(p_full), 8);
+    mbar_init(smem_u32(dp_read), 8);
+    mbar_init(smem_u32(ds_full), 8);
+    *abort_flag = 0;
+    mbar_fence_init();
+    fence_proxy_async();
   }
   __syncthreads();
   if (!info[3]) return;
@@ -560,7 +566,9 @@ RLB_API int RLB_NAME(rlb_flash_attn_bwd)(const void* qkv, long long qkv_stride, 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int most = (T + TILE - 1) / TILE + num_seqs;
   if (max_kv_tiles > most) max_kv_tiles = most;      // (blocks without a tile end at once, but take their turn)
-  flash_bwd_dq_kernel<<<max_q_tiles * Hq, BWD_THREADS, DQ_SMEM, s>>>(tqkv, tdo, p);
-  flash_bwd_dkv_kernel<<<max_kv_tiles * Hkv, BWD_THREADS, KV_SMEM, s>>>(tqkv, tdo, p);
+  // Heads are the fast dimension; tiles take two where they are more than one can count.
+  auto grid = [](int heads, int tiles) { return tiles <= 65535 ? dim3(heads, tiles) : dim3(heads, 65535, (tiles + 65534) / 65535); };
+  flash_bwd_dq_kernel<<<grid(Hq, max_q_tiles), BWD_THREADS, DQ_SMEM, s>>>(tqkv, tdo, p);
+  flash_bwd_dkv_kernel<<<grid(Hkv, max_kv_tiles), BWD_THREADS, KV_SMEM, s>>>(tqkv, tdo, p);
   return static_cast<int>(cudaGetLastError());
 }

@@ -146,3 +146,28 @@ def test_flash_many_sequences(native_lib, D):
     yr = F._attention_ref(xr, cu, Hq, Hkv, D, 1.0 / math.sqrt(D))
     yr.backward(g.float())
     assert (y.float() - yr).abs().max() <= 3e-2 and (x.grad.float() - xr.grad).abs().max() <= 3e-2 * xr.grad.abs().max()
+
+
+@pytest.mark.parametrize("D", [128, 64])
+def test_flash_more_tiles_than_a_grid_dimension(native_lib, D):
+    """65600 sequences of one token and two of 200, one of them last: more tiles than the second dimension of a grid can count. A token on its own
+    gets its value, hands its gradient on to it (one bf16 rounding of a product with 1) and nothing to its query and key; the others as in
+    test_flash_bwd_few_tiles."""
+    from rl_b200.ops import functional as F
+    from rl_b200.ops.lib import check_status
+
+    n = 65600
+    qkv, cu, D = _case([200] + [1] * n + [200], 1, 1, seed=D, D=D)
+    x = qkv.clone().requires_grad_()
+    y = F.attention_varlen(x, cu, 200, 1, 1, D)
+    g = torch.randn_like(y)
+    y.backward(g)
+    torch.cuda.synchronize()
+    assert check_status() == 0
+    one = slice(200, 200 + n)
+    assert torch.equal(y[one], qkv[one, 2 * D :]) and torch.equal(x.grad[one, 2 * D :], g[one]) and float(x.grad[one, : 2 * D].abs().max()) <= 1e-2
+    for part in (slice(0, 200), slice(200 + n, 400 + n)):
+        xr = qkv[part].float().requires_grad_()
+        yr = F._attention_ref(xr, torch.tensor([0, 200], dtype=torch.int32, device="cuda"), 1, 1, D, 1.0 / math.sqrt(D))
+        yr.backward(g[part].float())
+        assert (y[part].float() - yr).abs().max() <= 3e-2 and (x.grad[part].float() - xr.grad).abs().max() <= 3e-2 * xr.grad.abs().max()
