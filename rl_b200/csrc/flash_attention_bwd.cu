@@ -18,10 +18,13 @@
 // Measured, 32 query and 8 KV heads of 128, causal, dQ + dK / dV (before: tiles of 64, each group its own, lane 0 issuing), us: 4 x 4096 tokens
 // 1433 + 1501 -> 774 + 951 (796 TFLOP/s of the five products that a gradient needs); 1 x 7600 1176 + 1327 -> 590 + 801; 16 x 1280 738 + 670 ->
 // 475 + 471; 4 x 1000 129 + 116 -> 89 + 79; 16 x 300 114 + 74 -> 94 + 68.
+// What lies behind a sequence's end is left out, by warps of 32 rows and by halves of the other side: sequences of up to 64 tokens, half of a tile, took up to a
+// fifth longer than with tiles of 64 without that. 64 x 64 tokens 155 -> 139 us, 256 x 16 507 -> 440 (tiles of 64: 144 and 476).
 // delta[h, t] = sum_d dO * O is computed beforehand by rlb_attn_delta.
 #include "attention_tiles.cuh"
 
 #include <math.h>
+#include <type_traits>
 
 namespace {
 using namespace rlb;
@@ -91,12 +94,13 @@ __device__ __forceinline__ void scores_mma(uint32_t d, uint32_t a_s, uint32_t b_
   }
 }
 // D[TILE x HD] (+)= A B with A [TILE x TILE] in TMEM, the two groups' halves 64 columns apart, and B a tile of rows read as an MN-major operand: 16 rows per
-// step, 64-column groups an atom apart.
+// step, 64-column groups an atom apart. BOTH: the second half holds something, too (else nothing was written there).
+template <bool BOTH>
 __device__ __forceinline__ void gradient_mma(uint32_t d, uint32_t a, uint32_t b_s, bool add) {
   constexpr uint32_t idesc = make_idesc_bf16(TILE, HD, false, true);
   const uint64_t b = make_smem_desc_sw128(b_s, ATOM, 1024);
 #pragma unroll
-  for (int kk = 0; kk < TILE / 16; ++kk) umma_f16_ts(d, a + (kk / 4) * HALF + (kk % 4) * 8, desc_at(b, kk * 2048), idesc, add || kk != 0);
+  for (int kk = 0; kk < (BOTH ? TILE : HALF) / 16; ++kk) umma_f16_ts(d, a + (kk / 4) * HALF + (kk % 4) * 8, desc_at(b, kk * 2048), idesc, add || kk != 0);
 }
 __device__ __forceinline__ void load_rows(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col, int row) {
   mbar_arrive_expect_tx(smem_u32(bar), TILE_BYTES);
@@ -122,6 +126,11 @@ __device__ __forceinline__ void load_scores(uint32_t at, float* v, uint64_t* rea
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(read));
   }
+}
+// The same from a warp that has nothing to read or store.
+__device__ __forceinline__ void pass_on(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(smem_u32(bar));
 }
 // After a warp's stores to TMEM: its arrival at a barrier that the MMA warp waits for.
 __device__ __forceinline__ void hand_over(uint64_t* bar, int lane) {
@@ -212,6 +221,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
       if (!ok) let_loads_land();
     }
   } else if (warp == 1) {
+    const int cut = __shfl_sync(0xffffffffu, (q0 + q_rows - 1) % TILE < HALF ? 1 : 0, 0);      // 1: the last tile has keys in its first half only
     if (elect_one()) {
       auto scores = [&](int j) -> bool {      // S of tile j
         const int ks = j % DQ_K_STAGES;
@@ -232,22 +242,26 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
       };
       bool ok = mbar_wait(smem_u32(&q_full[0]), 0, abort_flag, p.status, RLB_ERR_WAIT_FULL) && scores(0) &&
                 mbar_wait(smem_u32(&q_full[1]), 0, abort_flag, p.status, RLB_ERR_WAIT_FULL) && dprobs(0);
-      for (int j = 0; j < n_kv && ok; ++j) {
+      auto product = [&](int j, auto both) -> bool {      // of tile j; the next tile's before it
         if (j + 1 < n_kv) {      // scores as soon as the warps have read the last ones, dP in the place of the last dS but one
-          if (!mbar_wait(smem_u32(s_read), j & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG) || !scores(j + 1)) break;
-          if (j > 0 && !mbar_wait(smem_u32(dq_done), (j - 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) break;
-          if (!dprobs(j + 1)) break;
+          if (!mbar_wait(smem_u32(s_read), j & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG) || !scores(j + 1)) return false;
+          if (j > 0 && !mbar_wait(smem_u32(dq_done), (j - 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) return false;
+          if (!dprobs(j + 1)) return false;
         }
-        if (!mbar_wait(smem_u32(&ds_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) break;
+        if (!mbar_wait(smem_u32(&ds_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) return false;
         tc_fence_after();
-        gradient_mma(tmem_dq, tmem_dp + (j & 1) * TILE, smem_u32(k_s + (j % DQ_K_STAGES) * TILE_BYTES), j != 0);
+        gradient_mma<decltype(both)::value>(tmem_dq, tmem_dp + (j & 1) * TILE, smem_u32(k_s + (j % DQ_K_STAGES) * TILE_BYTES), j != 0);
         umma_commit(smem_u32(&k_empty[j % DQ_K_STAGES]));
         umma_commit(smem_u32(dq_done));
         if (j + 1 == n_kv) umma_commit(smem_u32(all_done));
-      }
+        return true;
+      };
+      for (int j = 0; j < n_kv - cut && ok; ++j) ok = product(j, std::true_type{});
+      if (cut && ok) product(n_kv - 1, std::false_type{});
     }
   } else {
-    const int group = (warp - 2) >> 2;      // takes this half of a tile's keys
+    const int warp_u = __shfl_sync(0xffffffffu, warp, 0);      // (the compiler sees that a branch on it is one of the whole warp)
+    const int group = (warp_u - 2) >> 2;      // takes this half of a tile's keys
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
@@ -257,8 +271,11 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
     const float lse2 = row_ok ? p.lse[stat_idx] * LOG2E : INFINITY;      // (rows behind the sequence: weights of zero)
     const float dlt = row_ok ? p.delta[stat_idx] : 0.f;
     const uint32_t s_at = tmem_base + group * HALF + lane_addr;
+    // Tiles that have something for this warp: none where all of its rows are behind the sequence (what the products make of them is not stored), not the last
+    // one where its half of the keys is.
+    const int n_live = (warp_u & 3) * 32 >= q_rows ? 0 : q0 + q_rows > (n_kv - 1) * TILE + group * HALF ? n_kv : n_kv - 1;
     bool ok = true;
-    for (int j = 0; j < n_kv; ++j) {
+    for (int j = 0; j < n_live; ++j) {
       const uint32_t dp_at = tmem_dp + (j & 1) * TILE + group * HALF + lane_addr;
       if (!mbar_wait(smem_u32(s_full), j & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL)) {
         ok = false;
@@ -290,6 +307,12 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_c
         store_bf16(dp_at + c * 16, w + c * 32);
       }
       hand_over(&ds_full[j & 1], lane);
+    }
+    for (int j = n_live; j < n_kv && ok; ++j) {
+      ok = mbar_wait(smem_u32(s_full), j & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
+      if (ok) pass_on(s_read, lane);
+      ok = ok && mbar_wait(smem_u32(&dp_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
+      if (ok) pass_on(&ds_full[j & 1], lane);
     }
     if (ok && mbar_wait(smem_u32(all_done), 0, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
       tc_fence_after();
@@ -401,6 +424,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       if (!ok) let_loads_land();
     }
   } else if (warp == 1) {
+    const int cut = __shfl_sync(0xffffffffu, (seq_len - 1) % TILE < HALF ? 1 : 0, 0);      // 1: the last query tile has rows in its first half only
     if (elect_one()) {
       auto scores = [&](int it) -> bool {      // S^T
         const int qs = it % KV_Q_STAGES;
@@ -420,25 +444,30 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       };
       bool ok = n_iter > 0 && mbar_wait(smem_u32(&kv_full[0]), 0, abort_flag, p.status, RLB_ERR_WAIT_FULL) && scores(0) &&
                 mbar_wait(smem_u32(&kv_full[1]), 0, abort_flag, p.status, RLB_ERR_WAIT_FULL) && dprobs(0);
-      for (int it = 0; it < n_iter && ok; ++it) {
+      auto products = [&](int it, auto both) -> bool {
         const int qs = it % KV_Q_STAGES, os = it % KV_DO_STAGES;
-        if (!mbar_wait(smem_u32(p_full), it & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) break;
+        if (!mbar_wait(smem_u32(p_full), it & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) return false;
         tc_fence_after();
-        gradient_mma(tmem_dv, tmem_base + (it & 1) * TILE, smem_u32(do_s + os * TILE_BYTES), it != 0);
+        gradient_mma<decltype(both)::value>(tmem_dv, tmem_base + (it & 1) * TILE, smem_u32(do_s + os * TILE_BYTES), it != 0);
         umma_commit(smem_u32(&do_empty[os]));      // (dP^T of this tile was issued before)
         // the next scores take the place of this tile's dP as soon as the warps have read it, the next dP that of its P and dS
-        if (it + 1 < n_iter && !(mbar_wait(smem_u32(dp_read), it & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG) && scores(it + 1))) break;
-        if (!mbar_wait(smem_u32(ds_full), it & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) break;
+        if (it + 1 < n_iter && !(mbar_wait(smem_u32(dp_read), it & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG) && scores(it + 1))) return false;
+        if (!mbar_wait(smem_u32(ds_full), it & 1, abort_flag, p.status, RLB_ERR_WAIT_FLAG)) return false;
         tc_fence_after();
-        gradient_mma(tmem_dk, tmem_base + (it & 1) * TILE + 32, smem_u32(q_s + qs * TILE_BYTES), it != 0);
+        gradient_mma<decltype(both)::value>(tmem_dk, tmem_base + (it & 1) * TILE + 32, smem_u32(q_s + qs * TILE_BYTES), it != 0);
         umma_commit(smem_u32(&q_empty[qs]));
         umma_commit(smem_u32(dk_done));
         if (it + 1 == n_iter) umma_commit(smem_u32(all_done));
-        if (it + 1 < n_iter && !(mbar_wait(smem_u32(dk_done), it & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY) && dprobs(it + 1))) break;
+        return it + 1 == n_iter || (mbar_wait(smem_u32(dk_done), it & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY) && dprobs(it + 1));
+      };
+      for (int it = 0; it < n_iter && ok;) {      // a head's query tiles
+        for (const int whole = it + qt_count - cut; it < whole && ok; ++it) ok = products(it, std::true_type{});
+        if (cut && ok) ok = products(it++, std::false_type{});
       }
     }
   } else {
-    const int group = (warp - 2) >> 2;      // takes this half of a tile's query rows
+    const int warp_u = __shfl_sync(0xffffffffu, warp, 0);      // (the compiler sees that a branch on it is one of the whole warp)
+    const int group = (warp_u - 2) >> 2;      // takes this half of a tile's query rows
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;   // key row of this thread
     const int ct = (threadIdx.x - 64) & 127;     // 0..127 among the group's threads
@@ -453,54 +482,70 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       return ct < 64 ? p.lse[idx] * LOG2E : p.delta[idx];
     };
     float next = statistic(0);
+    // Query tiles of a head that have something for this warp: none where all of its keys are behind the sequence, not the last one where its half of the rows is.
+    const int n_live = (warp_u & 3) * 32 >= kv_rows ? 0 : seq_len > (qt_first + qt_count - 1) * TILE + group * HALF ? qt_count : qt_count - 1;
     bool ok = true;
-    for (int it = 0; it < n_iter; ++it) {
-      const int qbase = (qt_first + it % qt_count) * TILE + group * HALF;
-      float* st_lse = stat_s + (group * 2 + (it & 1)) * 2 * HALF;
-      st_lse[ct] = next;
+    // The statistics of tile `it` in their place and its scores computed. Every warp of the group meets every barrier, also after a wait that ran out.
+    auto begin = [&](int it) {
+      stat_s[(group * 2 + (it & 1)) * 2 * HALF + ct] = next;
       next = statistic(it + 1);
       named_bar_sync(1 + group, 128);
       ok = ok && mbar_wait(smem_u32(s_full), it & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
-      if (!ok) continue;      // every warp of the group meets every barrier, also after a wait that ran out
-      tc_fence_after();
-      const uint32_t s_at = tmem_base + (it & 1) * TILE + group * HALF + lane_addr, dp_at = tmem_base + (~it & 1) * TILE + group * HALF + lane_addr;
-      float w[HALF];
-      load_scores(s_at, w, nullptr, lane);
+    };
+    for (int it = 0; it < n_iter;) {
+      const int live_end = it + n_live, head_end = it + qt_count;
+      int qbase = qt_first * TILE + group * HALF;
+      for (; it < live_end; ++it, qbase += TILE) {
+        begin(it);
+        if (!ok) continue;
+        const float* st_lse = stat_s + (group * 2 + (it & 1)) * 2 * HALF;
+        tc_fence_after();
+        const uint32_t s_at = tmem_base + (it & 1) * TILE + group * HALF + lane_addr, dp_at = tmem_base + (~it & 1) * TILE + group * HALF + lane_addr;
+        float w[HALF];
+        load_scores(s_at, w, nullptr, lane);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < 2; ++c) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(st_lse + c * 32 + i);
-          w[c * 32 + i] = exp2f(w[c * 32 + i] * p.scale_log2 - l4.x);
-          w[c * 32 + i + 1] = exp2f(w[c * 32 + i + 1] * p.scale_log2 - l4.y);
-          w[c * 32 + i + 2] = exp2f(w[c * 32 + i + 2] * p.scale_log2 - l4.z);
-          w[c * 32 + i + 3] = exp2f(w[c * 32 + i + 3] * p.scale_log2 - l4.w);
+          for (int i = 0; i < 32; i += 4) {
+            const float4 l4 = *reinterpret_cast<const float4*>(st_lse + c * 32 + i);
+            w[c * 32 + i] = exp2f(w[c * 32 + i] * p.scale_log2 - l4.x);
+            w[c * 32 + i + 1] = exp2f(w[c * 32 + i + 1] * p.scale_log2 - l4.y);
+            w[c * 32 + i + 2] = exp2f(w[c * 32 + i + 2] * p.scale_log2 - l4.z);
+            w[c * 32 + i + 3] = exp2f(w[c * 32 + i + 3] * p.scale_log2 - l4.w);
+          }
+          if (qbase < kv0 + TILE - 1) {      // on the diagonal
+#pragma unroll
+            for (int i = 0; i < 32; ++i) w[c * 32 + i] = qbase + c * 32 + i < kj ? 0.f : w[c * 32 + i];
+          }
+          store_bf16(s_at + c * 16, w + c * 32);
         }
-        if (qbase < kv0 + TILE - 1) {      // on the diagonal
+        hand_over(p_full, lane);
+        ok = mbar_wait(smem_u32(dp_full), it & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
+        if (!ok) continue;
+        tc_fence_after();
+        float dpv[HALF];
+        load_scores(dp_at, dpv, dp_read, lane);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) w[c * 32 + i] = qbase + c * 32 + i < kj ? 0.f : w[c * 32 + i];
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            const float4 d4 = *reinterpret_cast<const float4*>(st_lse + HALF + c * 32 + i);
+            w[c * 32 + i] *= (dpv[c * 32 + i] - d4.x) * p.scale;
+            w[c * 32 + i + 1] *= (dpv[c * 32 + i + 1] - d4.y) * p.scale;
+            w[c * 32 + i + 2] *= (dpv[c * 32 + i + 2] - d4.z) * p.scale;
+            w[c * 32 + i + 3] *= (dpv[c * 32 + i + 3] - d4.w) * p.scale;
+          }
+          store_bf16(s_at + 32 + c * 16, w + c * 32);
         }
-        store_bf16(s_at + c * 16, w + c * 32);
+        hand_over(ds_full, lane);
       }
-      hand_over(p_full, lane);
-      ok = mbar_wait(smem_u32(dp_full), it & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
-      if (!ok) continue;
-      tc_fence_after();
-      float dpv[HALF];
-      load_scores(dp_at, dpv, dp_read, lane);
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 d4 = *reinterpret_cast<const float4*>(st_lse + HALF + c * 32 + i);
-          w[c * 32 + i] *= (dpv[c * 32 + i] - d4.x) * p.scale;
-          w[c * 32 + i + 1] *= (dpv[c * 32 + i + 1] - d4.y) * p.scale;
-          w[c * 32 + i + 2] *= (dpv[c * 32 + i + 2] - d4.z) * p.scale;
-          w[c * 32 + i + 3] *= (dpv[c * 32 + i + 3] - d4.w) * p.scale;
-        }
-        store_bf16(s_at + 32 + c * 16, w + c * 32);
+      for (; it < head_end; ++it) {
+        begin(it);
+        if (ok) pass_on(p_full, lane);
+        ok = ok && mbar_wait(smem_u32(dp_full), it & 1, abort_flag, p.status, RLB_ERR_WAIT_TMEM_FULL);
+        if (ok) pass_on(dp_read, lane);
+        if (ok) pass_on(ds_full, lane);
       }
-      hand_over(ds_full, lane);
     }
     if (ok && n_iter > 0 && mbar_wait(smem_u32(all_done), 0, abort_flag, p.status, RLB_ERR_WAIT_TMEM_EMPTY)) {
       tc_fence_after();

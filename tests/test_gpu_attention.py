@@ -171,3 +171,12 @@ def test_flash_more_tiles_than_a_grid_dimension(native_lib, D):
         yr = F._attention_ref(xr, torch.tensor([0, 200], dtype=torch.int32, device="cuda"), 1, 1, D, 1.0 / math.sqrt(D))
         yr.backward(g[part].float())
         assert (y[part].float() - yr).abs().max() <= 3e-2 and (x.grad[part].float() - xr.grad).abs().max() <= 3e-2 * xr.grad.abs().max()
+
+
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("n", [1, 16, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128])
+@pytest.mark.parametrize("before", [0, 128, 256])
+def test_flash_bwd_cut_tiles(native_lib, n, before, D):
+    """Tiles of which only the first warps' rows, or the first half of the other side, belong to the sequence, alone and as the last of several. Bounds
+    and repeats as in test_flash_bwd_few_tiles."""
+    test_flash_bwd_few_tiles(native_lib, before + n, 4, 2, D)
