@@ -199,10 +199,13 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_rows_kernel(const __nv_bfloat1
 }
 
 // Gradient for d up to 4096: a CTA takes ROWS rows at a time, so that a barrier serves all of them, keeps them in registers, NV pieces of 8 columns a
-// thread, and has requested the next ones before it works on these. 4000 rows with
-// a flushed cache, the sums of the weight gradient included, before these and the requests ahead -> now: of 2048 38 -> 32 us, of 4096 59 -> 40.
-template <int NV, int ROWS>
-__global__ void __launch_bounds__(256, 2) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+// thread, and has requested the next ones before it works on these. As many rows as the registers hold: a requested value that is spilled is waited for
+// at once. With a row more (256 threads of 128 registers, 56 to 100 bytes of them spilled) rows of 2048 were no sooner done than without requests ahead.
+// 20000 rows, one launch after the other, the sums of the weight gradient included, one row at a time or four without requests / with spills / now, us: of 512
+// 41 / 47 / 29, of 1024 64 / 64 / 37, of 2048 82 / 82 / 60, of 4096 170 / 128 / 113; 4000 of 2048 29 / 25 / 21, of 4096 51 / 35 / 31; 16 of 1024
+// 8.3 / 10.3 / 8.3.
+template <int NV, int ROWS, int THREADS>
+__global__ void __launch_bounds__(THREADS, 2) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
                                                                   float* __restrict__ dw_partial, int rows, int d, long long x_stride, long long dy_stride, int add_to_dx) {
   __shared__ float red[2][ROWS][8];
@@ -1125,15 +1128,17 @@ RLB_API int rlb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   const int threads = rms_threads(d);
   if (d > threads * 8 * 8) return -4;
   const int parts = rlb_rmsnorm_bwd_parts(rows);
-  if (d <= 2048)
-    rmsnorm_bwd_rows_kernel<1, 4><<<parts, (d / 8 + 31) / 32 * 32, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial, static_cast<int>(rows), d, x_stride,
-                                                                                  dy_stride, add_to_dx);
-  else if (d <= 4096)      // whole warps of two pieces a thread, the last of them cut
-    rmsnorm_bwd_rows_kernel<2, 2><<<parts, (d / 8 + 63) / 64 * 32, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial, static_cast<int>(rows), d, x_stride,
-                                                                                   dy_stride, add_to_dx);
-  else
+  if (d <= 4096) {
+    const int pieces = d <= 2048 ? 1 : 2, width = (d / 8 + pieces * 32 - 1) / (pieces * 32) * 32;      // whole warps, the last of them cut
+    auto kern = pieces == 2     ? rmsnorm_bwd_rows_kernel<2, 1, 256>
+                : rows <= parts ? rmsnorm_bwd_rows_kernel<1, 1, 256>      // (a row a CTA)
+                : width > 128   ? rmsnorm_bwd_rows_kernel<1, 3, 256>
+                                : rmsnorm_bwd_rows_kernel<1, 4, 128>;
+    kern<<<parts, width, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial, static_cast<int>(rows), d, x_stride, dy_stride, add_to_dx);
+  } else {
     rmsnorm_bwd_kernel<<<parts, threads, 0, S(stream)>>>(CBF(dy), CBF(x), CBF(w), rstd, BF(dx), dw_partial,
                                                          static_cast<int>(rows), d, x_stride, dy_stride, add_to_dx);
+  }
   colsum_kernel<<<(d + 31) / 32, 256, 0, S(stream)>>>(dw_partial, parts, d, dw_f32, BF(dw_bf16), dw_accumulate);
   return static_cast<int>(cudaGetLastError());
 }

@@ -665,6 +665,13 @@ def test_rmsnorm_gradient_covers_every_column(native_lib, d, rows):
     assert (dx.double() - ref).norm() <= 2.0 ** -8 * ref.norm() and (dw.double() - want).norm() <= 1e-5 * want.norm()
 
 
+@pytest.mark.parametrize("d,rows", [(8, 296), (8, 297), (264, 2400), (1024, 296), (1024, 297), (1024, 1184), (1024, 1185), (1032, 296), (1032, 297), (1032, 888), (1032, 889), (2048, 1777),
+                                    (2056, 296), (2056, 297), (4096, 593), (4104, 297)])
+def test_rmsnorm_gradient_rows_of_a_cta(native_lib, d, rows):
+    """One row to a CTA and one more, rounds of four, three and one row, whole and begun. Bounds as above."""
+    test_rmsnorm_gradient_covers_every_column(native_lib, d, rows)
+
+
 @pytest.mark.parametrize("d,rows", [(8, 2368), (512, 2371), (1024, 2368), (1032, 7109), (2048, 7104), (4096, 7109), (4104, 14213), (5120, 14208)])
 def test_rmsnorm_warp_rows(native_lib, d, rows):
     """A warp per row: the first size that takes it, a cut last CTA, every register count. Against the fp32 statement: one bf16 rounding (2^-8)."""
