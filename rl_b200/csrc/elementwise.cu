@@ -790,18 +790,20 @@ __global__ void adamw_kernel(__nv_bfloat16* __restrict__ p, int16_t* __restrict_
 // Sums of four or eight squares are taken in fp32, everything above in fp64: thousands of fp32 additions in a row lost part of the
 // squares of small gradients beside large ones (2e-6 to 5e-6 of the norm at 1.2e9 to 1.9e9 parameters; now below 5e-7). Four 16-byte loads in flight: 2.28 -> 1.34 ms for 7.7 GB (5.7 TB/s). The blocks' sums are added up in fp64 as well, by a
 // second kernel: as fp32 additions to `out`, a thousand sums that are nearly alike were all rounded the same way (5e-6 of the total).
-// Runs of 64 KB a block, in order (flat_vector): 5.8 -> 6.9 TB/s.
-constexpr int SUMSQ_BYTES = 65536;
+// Runs of 64 KB a block, in order (flat_vector): 5.8 -> 6.9 TB/s; of 16 KB, one round of loads, where 64 would leave SMs without a block. A block on its own
+// needs no second kernel, and that one is launched ahead of the first one's end (in a row, us, one kernel of fp32 additions / 64 KB and plain launches / now:
+// 1000 values 4.2 / 6.3 / 4.1, 100000 4.2 / 6.5 / 4.7, 1048576 4.2 / 8.3 / 6.2, 1e7 10.4 / 14.5 / 12.1).
+inline int sumsq_run(long long bytes) { return bytes < 4 * 148 * 65536ll ? 16384 : 65536; }
 template <typename T>
-__global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, long long n, double* __restrict__ part) {
+__global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, long long n, int vecs, double* __restrict__ part, float* __restrict__ out) {
   __shared__ double red[8];
   double s = 0.0;
-  constexpr int PER = 16 / sizeof(T), VECS = SUMSQ_BYTES / 16;
+  constexpr int PER = 16 / sizeof(T);
   const long long nv = (reinterpret_cast<uintptr_t>(x) & 15) ? 0 : n / PER;
   const uint4* xv = reinterpret_cast<const uint4*>(x);
-  const long long first = static_cast<long long>(blockIdx.x) * VECS + threadIdx.x;
+  const long long first = static_cast<long long>(blockIdx.x) * vecs + threadIdx.x;
 #pragma unroll 1
-  for (long long i = first; i < nv && i < first + VECS; i += 4 * 256) {
+  for (long long i = first; i < nv && i < first + vecs; i += 4 * 256) {
     uint4 q[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) q[j] = i + j * 256 < nv ? __ldcs(xv + i + j * 256) : make_uint4(0, 0, 0, 0);
@@ -828,11 +830,13 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, lon
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < 8; ++w) s += red[w];
-    part[blockIdx.x] = s;
+    if (gridDim.x == 1) atomicAdd(out, static_cast<float>(s));
+    else part[blockIdx.x] = s;
   }
 }
 
 __global__ void __launch_bounds__(1024) sumsq_total_kernel(const double* __restrict__ part, int n, float* __restrict__ out) {
+  pdl_sync();
   __shared__ double red[32];
   double s = 0.0;
 #pragma unroll 8
@@ -1268,14 +1272,18 @@ RLB_API int rlb_adamw(void* p, void* p_lo, float* p32, const void* g, int grad_i
 }
 
 // Doubles of scratch that rlb_sumsq needs: one a block.
-RLB_API int rlb_sumsq_parts(long long n, int is_bf16) { return static_cast<int>((n * (is_bf16 ? 2 : 4) + SUMSQ_BYTES - 1) / SUMSQ_BYTES); }
+RLB_API int rlb_sumsq_parts(long long n, int is_bf16) {
+  const long long bytes = n * (is_bf16 ? 2 : 4);
+  const int run = sumsq_run(bytes);
+  return static_cast<int>((bytes + run - 1) / run);
+}
 // out += sum(x^2). `out` is a device float the caller zeroes.
 RLB_API int rlb_sumsq(const void* x, int is_bf16, long long n, float* out, double* part, void* stream) {
   if (n <= 0) return 0;
-  const int grid = rlb_sumsq_parts(n, is_bf16);
-  if (is_bf16) sumsq_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(CBF(x), n, part);
-  else sumsq_kernel<float><<<grid, 256, 0, S(stream)>>>(reinterpret_cast<const float*>(x), n, part);
-  sumsq_total_kernel<<<1, 1024, 0, S(stream)>>>(part, grid, out);
+  const int grid = rlb_sumsq_parts(n, is_bf16), vecs = sumsq_run(n * (is_bf16 ? 2 : 4)) / 16;
+  if (is_bf16) sumsq_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(CBF(x), n, vecs, part, out);
+  else sumsq_kernel<float><<<grid, 256, 0, S(stream)>>>(reinterpret_cast<const float*>(x), n, vecs, part, out);
+  if (grid > 1) rlb_launch_pdl(sumsq_total_kernel, dim3(1), dim3(1024), 0, S(stream), part, grid, out);
   return static_cast<int>(cudaGetLastError());
 }
 RLB_API int rlb_clip_scale(const float* sumsq, float max_norm, float extra, float* scale_out, float* norm_out,

@@ -503,6 +503,21 @@ def test_sumsq_sizes(native_lib, n, dtype):
         assert abs(out.item() - part.double().pow(2).sum().item()) <= 1e-5 * part.double().pow(2).sum().item()
 
 
+@pytest.mark.parametrize("nbytes", [16384, 16400, 4 * 148 * 65536 - 16, 4 * 148 * 65536, 4 * 148 * 65536 + 65552])      # one block, two, the shorter runs' last, the longer ones
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sumsq_runs(native_lib, nbytes, dtype):
+    """Both lengths of a block's run, one block on its own, cut last ones, added to what `out` holds; and the same values where they do not start on
+    16 bytes. Bounds as above."""
+    from rl_b200.ops import functional as F
+
+    n = nbytes // (2 if dtype == torch.bfloat16 else 4)
+    x = torch.randn(n + 1, device="cuda").to(dtype)
+    for part in (x[:n], x[1:]):
+        out, ref = torch.full((1,), 7.0, device="cuda"), 7 + part.double().pow(2).sum().item()
+        F.sumsq_(part, out)
+        assert abs(out.item() - ref) <= 1e-5 * ref
+
+
 def test_sumsq_small_beside_large(native_lib):
     """A large value in every 660, the others' squares nine tenths of half a unit in the last place of its square: fp32 sums over a thread's hundreds
     of terms lose those that come after it, 1.7e-5 of the total. In fp64 the 1184 additions of block sums remain, whose roundings of at most 2^-24 of
