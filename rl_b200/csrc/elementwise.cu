@@ -82,7 +82,9 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
 // The same for rows that fit the registers of one CTA, NV pieces of 8 elements a thread: all loads in flight at once, the row stays between the two
 // passes, and small CTAs, many to an SM, hide one another's barrier. Timed with a flushed cache against the kernel above / a warp per row, us:
 // d 2048: 600 rows 8.1 -> 8.0, 4000 14.6 -> 12.1, 20000 35.7 -> 30.7; d 4096: 600 10.1 -> 8.3, 4000 22.9 -> 16.6, 20000 70.4 -> 54.3 (6.0 TB/s);
-// d 5120: 4000 28.6 -> 20.2, 20000 98.2 -> 68.1. Two and eight pieces were slower above d 1024.
+// d 5120: 4000 28.6 -> 20.2, 20000 98.2 -> 68.1. Two and eight pieces were slower above d 1024; with a
+// residual, which waits for two rows and stores one more, two are sooner done up to 4096 (one row of 2048, four / two / the kernel above: 2.2, 1.8, 2.0; 4000
+// of 4096 21.6, 19.3, 22.8).
 template <int NV, bool RES>
 __global__ void __launch_bounds__(256) rmsnorm_regs_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
                                                            __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out,
@@ -1109,7 +1111,7 @@ RLB_API int rlb_rmsnorm_fwd(const void* x, const void* res, const void* w, void*
     return static_cast<int>(cudaGetLastError());
   }
   if (d <= 8192) {
-    const int pieces = d <= 1024 ? 2 : 4, threads = (d / 8 + pieces * 32 - 1) / (pieces * 32) * 32;
+    const int pieces = d <= (res ? 4096 : 1024) ? 2 : 4, threads = (d / 8 + pieces * 32 - 1) / (pieces * 32) * 32;
     auto kern = res ? (pieces == 2 ? rmsnorm_regs_kernel<2, true> : rmsnorm_regs_kernel<4, true>) : (pieces == 2 ? rmsnorm_regs_kernel<2, false> : rmsnorm_regs_kernel<4, false>);
     rlb_launch_pdl(kern, dim3(static_cast<unsigned>(rows)), dim3(threads), 0, S(stream), CBF(x), CBF(res), CBF(w), BF(y), BF(res_out), rstd, d, x_stride, y_stride, eps);
     return static_cast<int>(cudaGetLastError());

@@ -53,6 +53,24 @@ def test_rmsnorm_residual(native_lib):
     _close(y, y_ref, 1e-2)
 
 
+@pytest.mark.parametrize("d", [8, 1024, 1032, 2048, 2056, 4088, 4096, 4104, 8184, 8192, 8200, 10248])      # two and four pieces a thread, cut ones, the looping kernel
+@pytest.mark.parametrize("rows", [1, 300])
+def test_rmsnorm_forward_widths(native_lib, d, rows):
+    """With and without a residual, whose sum is rounded to bf16 before the norm; one bf16 rounding of the result (2^-8)."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(d)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()      # noqa: E731
+    x, res, w = r(rows, d), r(rows, d), r(d)
+    both = (x.float() + res.float()).bfloat16()
+    with torch.no_grad():
+        plain, fused = F.rmsnorm(x, w, 1e-6), F.rmsnorm_residual_(x, res, w, 1e-6)
+    assert torch.equal(res, both)
+    for y, z in ((plain, x.double()), (fused, both.double())):
+        ref = z * torch.rsqrt(z.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+        assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-30).all()
+
+
 def test_rope_and_inverse(native_lib):
     from rl_b200.ops import functional as F
 
