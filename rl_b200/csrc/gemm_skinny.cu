@@ -130,7 +130,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const uint32_t tmem_cols = NT == 128 && p.chains > 1 ? 2 * NT : NT;
   const bool aligned = (smem_u32(smem) & 1023u) == 0;
 
-  if (threadIdx.x == 0) {
+  // The elected thread of the first warp also loads below: of the same warp elect.sync picks the same one each time.
+  const bool lead = warp == 0 && elect_one();
+  if (lead) {
     for (int s = 0; s < Cfg::STAGES; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 1);
       mbar_init(smem_u32(&empty_bar[s]), 1);
@@ -143,16 +145,17 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   }
   const bool have_work = kb_end > kb_begin && aligned;
   // Weights that the preceding kernel cannot have written are requested before the dependency wait: the first ring
-  // stages fill while that kernel drains. The activations of the same stages follow after the wait. (Every thread knows how many: the one that is
-  // elected below need not be the one here.)
-  const int early = p.w_static && have_work ? min(Cfg::STAGES, kb_end - kb_begin) : 0;
-  if (threadIdx.x == 0 && have_work) {
+  // stages fill while that kernel drains. The activations of the same stages follow after the wait.
+  int early = 0;
+  if (lead && have_work) {
     prefetch_tmap(&tmap_w);
     prefetch_tmap(&tmap_x);
-    for (int e = 0; e < early; ++e) {
-      const uint32_t bar = smem_u32(&full_bar[e]);
-      mbar_arrive_expect_tx(bar, Cfg::STAGE);
-      load_w(smem_u32(smem + e * Cfg::STAGE), bar, kb_begin + e);
+    if (p.w_static) {
+      for (; early < Cfg::STAGES && kb_begin + early < kb_end; ++early) {
+        const uint32_t bar = smem_u32(&full_bar[early]);
+        mbar_arrive_expect_tx(bar, Cfg::STAGE);
+        load_w(smem_u32(smem + early * Cfg::STAGE), bar, kb_begin + early);
+      }
     }
   }
   if (warp == 1) {
