@@ -444,20 +444,24 @@ static int skinny_split(int M, int N, int K) {
 RLB_API int rlb_gemm_skinny_split(int N, int K) { return skinny_split(1, N, K); }
 
 // Two tiles of tokens leave CTAs for half the split, and the tensor core's sums lose with their length (they are cut, not rounded: 6144 x 4096 off by
-// 1.0e-6 of the norm in eighths, 2.1e-6 in quarters). A CTA of such a product sums the halves of its range in two accumulators, so that products
-// of up to 256 tokens are as exact as those of 128.
-static int skinny_chains(int M, int N, int K, int split) { return M > 128 && M <= 256 && skinny_split(1, N, K) > split ? 2 : 1; }
+// 1.0e-6 of the norm in eighths, 2.1e-6 in quarters). Where the result is fp32 a CTA of such a product sums the halves of its range in two accumulators, so
+// that products of up to 256 tokens are as exact as those of 128. A bf16 result, whose own rounding is a thousand times that, is as far off either way
+// (6144 x 4096, 240 tokens: 1.6558e-3).
+static int skinny_chains(bool fp32, int M, int N, int K, int split) { return fp32 && M > 128 && M <= 256 && skinny_split(1, N, K) > split ? 2 : 1; }
 
 // Whether a product of M tokens is sooner done here than on the tiled kernel (gemm_tcgen05.cu): up to 128 tokens, and up to 1024 where the
 // contraction can be split at least in two. Timed both ways, weights from memory, us (here / tiled): 3072 x 2048: 129 tokens 12 / 18, 256 12 / 19,
 // 512 17 / 19, 768 17 / 19, 1024 (one part) 24 / 19; 2048 x 8192: 256 17 / 46, 512 23 / 46, 1024 38 / 46; 6144 x 4096: 256 25 / 29, 384 25 / 29, 512
 // (one part) 37 / 29; 4096 x 14336: 256 36 / 74, 512 62 / 74, 640 (one part) 96 / 78; 16384 x 2048 (one part): 256 27 / 22; 28672 x 4096 (one part):
-// 256 91 / 61, but 128 tokens 52 / 49 and 65 49 / 49. Up to 256 tokens whatever is split at 128 comes
-// here, for the sake of its sums (skinny_chains): 16384 x 2048 2 us longer than on the tiled kernel, half its error.
+// 256 91 / 61, but 128 tokens 52 / 49 and 65 49 / 49. An fp32 result of up to 256 tokens
+// comes here wherever 128 are split, for the sake of its sums (skinny_chains; 16384 x 2048 2 us longer than on the tiled kernel, half its error). What is fused into the epilogue
+// (the decode step's norms and units, the layers of layer lists) comes here up to 256 tokens whatever its width: 8B gate / up with its unit 82 us where
+// the tiled kernel and a unit of its own take 68, the vocabulary of 128256 x 4096 391 / 227, a layer's 32768 x 4096 103 / 64 (in one tile of 256 tokens: 123, 494
+// and 153).
 constexpr int SK_MAX_TOKENS = 1024;
 RLB_API int rlb_gemm_takes_skinny(int M, int N, int K) {
   if (K < 256 || M > SK_MAX_TOKENS) return 0;
-  return M <= 128 || skinny_split(M <= 256 ? 1 : M, N, K) > 1;
+  return M <= 128 || skinny_split(M, N, K) > 1;
 }
 
 // While set, callers promise that the W operand of every skinny GEMM was not written by the kernel launched just before
@@ -509,7 +513,7 @@ RLB_API int rlb_gemm_skinny_fused(const void* X, const void* W, void* Y, int M, 
   p.chains = 1;
   if (split <= 0) {
     split = skinny_split(M, w_rows, K);
-    p.chains = skinny_chains(M, w_rows, K, split);
+    p.chains = skinny_chains(out_fp32 != 0, M, w_rows, K, split);
   }
   if (split > 8) split = 8;
   p.Y = Y;
@@ -567,7 +571,7 @@ RLB_API int rlb_gemm_skinny_layer(const void* X, const void* W, void* out, int M
   p.layer = LayerEpilogue{x, ldx, e, static_cast<const __nv_bfloat16*>(step), static_cast<const __nv_bfloat16*>(alpha),
                           static_cast<const __nv_bfloat16*>(nw), static_cast<const __nv_bfloat16*>(nb), act_from, LinearEpi{}};
   const int split = skinny_split(M, N, K);
-  p.chains = skinny_chains(M, N, K, split);
+  p.chains = skinny_chains(x != nullptr, M, N, K, split);
   return launch_skinny_nt(NT, tw, tx, p, split, static_cast<cudaStream_t>(stream));
 }
 
@@ -597,7 +601,7 @@ RLB_API int rlb_linear_skinny(const RlbLinear* l, void* stream) {
   p.layer.act_from = 1 << 30;
   p.layer.lin = rlb_linear_epi(*l);
   const int split = skinny_split(l->M, l->N, l->K);
-  p.chains = skinny_chains(l->M, l->N, l->K, split);
+  p.chains = skinny_chains(l->out_f32 != 0, l->M, l->N, l->K, split);
   return launch_skinny_nt(NT, tw, tx, p, split, static_cast<cudaStream_t>(stream));
 }
 

@@ -22,10 +22,13 @@ BF16 = torch.bfloat16
 # --------------------------------------------------------------------------------------- GEMM
 def _streams_weights(M: int, N: int, K: int, out: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
     """Whether a product goes to the weight-streaming kernel: where it is sooner done there (``rlb_gemm_takes_skinny``), and up to 256 rows also
-    where output or residual do not start their rows on 16 bytes, which the tiled kernel wants and this one does not."""
+    where the result is fp32 and the contraction is split, with half the tiled kernel's error, and where output or residual do not start their rows on 16
+    bytes, which the tiled kernel wants and this one does not."""
     if M > 1024 or K < 256:
         return False
     if _L.lib().rlb_gemm_takes_skinny(M, N, K):
+        return True
+    if M <= 256 and out.dtype == torch.float32 and _L.lib().rlb_gemm_skinny_split(N, K) > 1:
         return True
     return M <= 256 and (out.data_ptr() % 16 != 0 or (residual is not None and (residual.data_ptr() % 16 != 0 or residual.stride(0) % 8 != 0)))
 
