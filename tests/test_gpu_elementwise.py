@@ -735,7 +735,7 @@ def test_logprob_combine(native_lib, M, V):
     assert (lp.double() - z.gather(1, t[:, None])[:, 0]).abs().max() < 1e-4 and (ent.double() + (z.exp() * z).sum(-1)).abs().max() < 1e-3
 
 
-@pytest.mark.parametrize("B,V", [(1, 128256), (3, 16384), (37, 32771), (38, 32771), (74, 20000), (75, 20000), (2, 16383), (74, 50000)])      # eight, four and one CTA a row, clusters in two waves
+@pytest.mark.parametrize("B,V", [(1, 128256), (3, 16384), (37, 32771), (38, 32771), (74, 20000), (75, 20000), (2, 16383)])      # eight, four and one CTA a row
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("greedy", [False, True])
 def test_sampling_over_parts_of_rows(native_lib, B, V, dtype, greedy):
@@ -756,6 +756,13 @@ def test_sampling_over_parts_of_rows(native_lib, B, V, dtype, greedy):
     assert torch.equal(tok, one) and (not greedy or bool((tok == 100).all()))
     want = torch.log_softmax(z.double() / 0.7, -1).gather(1, tok.long()[:, None])[:, 0]
     assert (lp - want).abs().max() <= 2e-5 * (1 + want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("greedy", [False, True])
+def test_sampling_clusters_in_two_waves(native_lib, dtype, greedy):
+    """More clusters than the device holds at once, of rows long enough to be shared all the same."""
+    test_sampling_over_parts_of_rows(native_lib, 74, 50000, dtype, greedy)
 
 
 @pytest.mark.parametrize("B,V", [(4, 128256), (40, 32771), (80, 4099)])      # eight, four and one CTA a row
