@@ -184,6 +184,33 @@ def test_lm_head_kept_logits(native_lib, monkeypatch, M, V):
             assert (x.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
 
 
+@pytest.mark.parametrize("M,V", [(1, 8), (33, 264), (129, 4096), (300, 4104), (257, 6152)])
+def test_lm_head_kept_logits_are_those_of_the_product(native_lib, monkeypatch, M, V):
+    """Storage is given whatever the device has free, so that the kept logits are written and read; the values behind the last row and the gradients are
+    looked at. Both ways start from the same scaled fp32 logits: dZ differs where one exponential lies on the other side of a rounding, 2^-8 of
+    a value, a few in a thousand."""
+    from rl_b200.ops import functional as F
+
+    g = torch.Generator("cuda").manual_seed(M)
+    h = (torch.randn(M, 192, generator=g, device="cuda") * 0.5).bfloat16()
+    w = (torch.randn(V, 192, generator=g, device="cuda") * 0.2).bfloat16()
+    tg = torch.randint(0, V, (M,), generator=g, device="cuda")
+    cl, ce = torch.randn(M, generator=g, device="cuda"), torch.randn(M, generator=g, device="cuda") * 0.1
+    monkeypatch.setattr(F._LMHeadLogprob, "CHUNK", 128)
+    room = torch.full((M + 3, V), float("nan"), device="cuda")
+    grads = []
+    for z in (room, None):
+        monkeypatch.setattr(F, "_kept_logits", lambda *a: z)
+        hg, wg = h.clone().requires_grad_(), w.clone().requires_grad_()
+        lp, ent = F.lm_head_logprobs(hg, wg, tg, temperature=0.8, want_entropy=True)
+        (lp * cl + ent * ce).sum().backward()
+        grads.append((hg.grad.double(), wg.grad.double()))
+    want = h.double() @ w.double().t() / 0.8
+    assert (room[:M].double() - want).abs().max() <= 1e-5 * want.abs().max() and bool(room[M:].isnan().all())
+    for kept, again in zip(*grads):
+        assert (kept - again).norm() <= 2.0 ** -9 * again.norm()
+
+
 @pytest.mark.parametrize("T", [0, 1, 130, 700])
 def test_stale_gradients_are_written_over(native_lib, monkeypatch, T):
     """Gradients of a linear layer (used once and twice), of the vocabulary product in chunks and of an embedding into buffers whose old values are
