@@ -13,8 +13,9 @@
 //               max / sum in the exp2 domain, writes P in bf16 over the scores it has read, and rescales the O accumulator in
 //               TMEM only when the row maximum moved by more than 2^8 (stale maxima are exact because the final normalisation
 //               uses the same reference).
-// Bound by the exponentials and the tensor cores alike (512 cycles each per tile and CTA), so both have to run all the time: the next
-// tile's scores are computed under this one's softmax, and two CTAs cover each other's hand-offs. Measured, 32 query and 8 KV heads of 128
+// Bound by the tensor core (768 cycles per tile and CTA with heads of 128: eight steps of the scores, which take 64 cycles although only 64 columns wide, and
+// four of the output; 512 with heads of 64) and the exponentials (512), so both have to run all the time: the next tile's scores are computed under this
+// one's softmax, and two CTAs cover each other's hand-offs. Measured, 32 query and 8 KV heads of 128
 // (before: one score buffer, P through shared memory): 16 x 4096 tokens 3.77 -> 2.24 ms (984 TFLOP/s); 64 x 1280 2.02 -> 1.18 ms. Since then, by the order of the tiles and an elected issuer: 4 x 4096 670 -> 546 us, 1 x 7600 541 -> 422.
 // Output: O[T, Hq*128] bf16 and the per-row log-sum-exp lse[Hq, T] (natural log) for the backward pass.
 //

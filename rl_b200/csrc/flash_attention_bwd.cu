@@ -575,7 +575,7 @@ int g_bwd_configured = 0;
 
 // dqkv[T, (Hq+2Hkv)*128] = gradient of the packed causal attention w.r.t. the fused [q | k | v] buffer.
 // lse and delta are [Hq, T] fp32 (lse from the forward pass, delta from rlb_attn_delta).
-// max_q_tiles / max_kv_tiles: upper bounds on the number of 128-row tiles (ceil(T/128) + num_seqs is enough for both).
+// max_q_tiles / max_kv_tiles: upper bounds on the number of 128-row tiles (ceil(T/128) + num_seqs is enough for both; blocks without a tile end at once, but take their turn).
 RLB_API int RLB_NAME(rlb_flash_attn_bwd)(const void* qkv, long long qkv_stride, const void* dout, long long do_stride,
                                const float* lse, const float* delta, const int* cu_seqlens, int num_seqs, int T, int Hq,
                                int Hkv, int D, float scale, void* dqkv, long long dqkv_stride, int max_q_tiles,
@@ -609,8 +609,6 @@ RLB_API int RLB_NAME(rlb_flash_attn_bwd)(const void* qkv, long long qkv_stride, 
   p.dqkv_stride = dqkv_stride;
   p.status = status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int most = (T + TILE - 1) / TILE + num_seqs;
-  if (max_kv_tiles > most) max_kv_tiles = most;      // (blocks without a tile end at once, but take their turn)
   // Heads are the fast dimension; tiles take two where they are more than one can count.
   auto grid = [](int heads, int tiles) { return tiles <= 65535 ? dim3(heads, tiles) : dim3(heads, 65535, (tiles + 65534) / 65535); };
   flash_bwd_dq_kernel<<<grid(Hq, max_q_tiles), BWD_THREADS, DQ_SMEM, s>>>(tqkv, tdo, p);

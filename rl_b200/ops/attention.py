@@ -61,7 +61,7 @@ class _FlashAttn(torch.autograd.Function):
             delta = torch.empty((Hq, T), dtype=torch.float32, device=qkv.device)
             call("rlb_attn_delta" + _sfx(D), ptr(dout), ptr(out), ptr(delta), T, Hq, dout.stride(0), out.stride(0), stream_ptr())
             call("rlb_flash_attn_bwd" + _sfx(D), ptr(qkv), qkv.stride(0), ptr(dout), dout.stride(0), ptr(lse), ptr(delta), ptr(cu), B, T,
-                 Hq, Hkv, D, scale, ptr(dqkv), dqkv.stride(0), (T + 127) // 128 + B, (T + 63) // 64 + B,
+                 Hq, Hkv, D, scale, ptr(dqkv), dqkv.stride(0), (T + 127) // 128 + B, (T + 127) // 128 + B,
                  ptr(_L.status_word(qkv.device)), stream_ptr())
             return dqkv, None, None, None, None, None, None
         # interim: differentiate the PyTorch restatement

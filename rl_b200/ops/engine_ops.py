@@ -265,7 +265,7 @@ def skinny_linear(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tenso
                   bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
                   ssq_in: Optional[torch.Tensor] = None, eps: float = 1e-6, ssq_out: Optional[torch.Tensor] = None,
                   norm_w: Optional[torch.Tensor] = None, out2: Optional[torch.Tensor] = None, swiglu: bool = False) -> torch.Tensor:
-    """Decode-sized projection (at most 256 rows) with the epilogue fusions of ``rlb_gemm_skinny_fused``.
+    """Decode-sized projection (at most 1024 rows, in tiles of 128) with the epilogue fusions of ``rlb_gemm_skinny_fused``.
 
     ``ssq_in`` [tiles, stride]: ``x`` is ``h * w_norm`` and the output rows are scaled by the reciprocal RMS of ``h`` built
     from these partial sums (RMSNorm folded into the projection). ``ssq_out`` + ``norm_w`` + ``out2``: also writes
